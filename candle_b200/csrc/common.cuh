@@ -29,6 +29,13 @@ inline bool dtype_supported(int dtype) {
 // k-quants, Q8_0 (32) for Q8_0.
 __host__ __device__ inline int act_block(int dtype) { return dtype == CANDLE_GGML_Q8_0 ? 32 : 256; }
 
+// Repacked weights (candle_moe_prepack): half-tile blocks of 8 rows x 256 elements (Q8_0: x 128), [n / 8][k / 256][bytes].
+// A block starts with 512-byte regions of 8 rows x four 16-byte chunks t; row g's chunk t is the chunk_pos(g, t)-th of its
+// region.  Both ways the kernels read a region are then free of shared-memory bank conflicts: eight rows at one t (a lane
+// per row, the GEMM) and two rows at all four t (a lane per (g, t), the decode kernels).
+constexpr int Q4K_HTB_BYTES = 1184, Q6K_HTB_BYTES = 1680, Q80_HTB_BYTES = 1088;
+__host__ __device__ constexpr int chunk_pos(int g, int t) { return 8 * t + ((g + 2 * t) & 7); }
+
 // Per-expert weight base pointers travel as a kernel parameter (no device-side table to allocate).
 struct ExpertPtrs {
     const uint8_t* p[CANDLE_MOE_MAX_EXPERTS];

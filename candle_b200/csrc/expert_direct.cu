@@ -37,8 +37,6 @@ __device__ __forceinline__ int imad(int a, int b, int c) {
     return d;
 }
 
-constexpr int Q4K_HTB = 1184;
-constexpr int Q6K_HTB = 1680;
 constexpr int DIRECT_WARPS = 16;
 constexpr int DIRECT_THREADS = 32 * DIRECT_WARPS;
 
@@ -54,7 +52,7 @@ struct ActArgs {
 
 // ------------------------------------------------------------------------------------------------
 struct DirQ4K {
-    static constexpr int HTB = Q4K_HTB;
+    static constexpr int HTB = Q4K_HTB_BYTES;
     static constexpr int BS_PER_BLOCK = 8;
     __device__ static __forceinline__ int bs_value(const int16_t* bs16, int i) { return (int)bs16[2 * i] + (int)bs16[2 * i + 1]; }
     __device__ static __forceinline__ void bs_split(int v, uint8_t& hi, uint8_t& lo) {
@@ -69,7 +67,7 @@ struct DirQ4K {
     // hta: shared-window address of the first half-tile block inside the warp's ring slot; the second follows it
     __device__ static __forceinline__ void load(Frag& F, uint32_t hta, int lane) {
         const int g = lane >> 2;
-        const uint32_t bq = hta + lane * 16, bd = hta + 4 * g, bs = hta + 8 * g;
+        const uint32_t bq = hta + 16 * chunk_pos(g, lane & 3), bd = hta + 4 * g, bs = hta + 8 * g;
         F.qa[0] = lds128_o<0>(bq);
         F.qa[1] = lds128_o<512>(bq);
         F.qb[0] = lds128_o<HTB>(bq);
@@ -144,7 +142,7 @@ struct DirQ4K {
 
 // ------------------------------------------------------------------------------------------------
 struct DirQ6K {
-    static constexpr int HTB = Q6K_HTB;
+    static constexpr int HTB = Q6K_HTB_BYTES;
     static constexpr int BS_PER_BLOCK = 16;
     __device__ static __forceinline__ int bs_value(const int16_t* bs16, int i) { return (int)bs16[i]; }
     __device__ static __forceinline__ void bs_split(int v, uint8_t& hi, uint8_t& lo) {
@@ -159,7 +157,7 @@ struct DirQ6K {
     };
     __device__ static __forceinline__ void load(Frag& F, uint32_t hta, int lane) {
         const int g = lane >> 2;
-        const uint32_t bq = hta + lane * 16, bs = hta + 16 * g, bd = hta + 2 * g;
+        const uint32_t bq = hta + 16 * chunk_pos(g, lane & 3), bs = hta + 16 * g, bd = hta + 2 * g;
         F.qlA[0] = lds128_o<0>(bq);
         F.qlA[1] = lds128_o<512>(bq);
         F.qhA = lds128_o<1024>(bq);
@@ -273,7 +271,7 @@ template <class F, bool GATE_UP, int NT, int DEPTH>
 // and Q6_K would spill): the
 // registers a CTA leaves free let the CTAs of the next kernel on the stream become resident and run their
 // prologue under programmatic dependent launch while this one drains.
-__global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB ? 608 : DIRECT_THREADS, 1) expert_direct_kernel(const __grid_constant__ DirectParams P) {
+__global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB_BYTES ? 608 : DIRECT_THREADS, 1) expert_direct_kernel(const __grid_constant__ DirectParams P) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint32_t s_offs[CANDLE_MOE_MAX_EXPERTS + 1];
     __shared__ int s_rows[16];
@@ -548,11 +546,11 @@ __global__ void __launch_bounds__(256) prepack_q4k_kernel(const uint8_t* __restr
     const int ht = blockIdx.x / kb, blk = blockIdx.x - ht * kb;
     const size_t row_bytes = (size_t)kb * Q4K_BYTES;
     const uint8_t* src = raw + (size_t)ht * 8 * row_bytes + (size_t)blk * Q4K_BYTES;  // row g at + g * row_bytes
-    uint8_t* out = dst + ((size_t)ht * kb + blk) * Q4K_HTB;
+    uint8_t* out = dst + ((size_t)ht * kb + blk) * Q4K_HTB_BYTES;
     const int w = threadIdx.x;  // output word 0..255 of the quant region
     {
-        const int u = w >> 7, lane = (w >> 2) & 31, cw = w & 3;
-        const int g = lane >> 2, t = lane & 3;
+        const int u = w >> 7, pos = (w >> 2) & 31, cw = w & 3;
+        const int t = pos >> 3, g = ((pos & 7) - 2 * t) & 7;  // inverse of chunk_pos
         const int grp = 2 * u + (cw >> 1), isb = cw & 1;
         const uint32_t v = *reinterpret_cast<const uint32_t*>(src + (size_t)g * row_bytes + 16 + 32 * grp + 16 * isb + 4 * t);
         reinterpret_cast<uint32_t*>(out)[w] = v;
@@ -571,11 +569,11 @@ __global__ void __launch_bounds__(384) prepack_q6k_kernel(const uint8_t* __restr
     const int ht = blockIdx.x / kb, blk = blockIdx.x - ht * kb;
     const size_t row_bytes = (size_t)kb * Q6K_BYTES;
     const uint8_t* src = raw + (size_t)ht * 8 * row_bytes + (size_t)blk * Q6K_BYTES;
-    uint8_t* out = dst + ((size_t)ht * kb + blk) * Q6K_HTB;
+    uint8_t* out = dst + ((size_t)ht * kb + blk) * Q6K_HTB_BYTES;
     const int w = threadIdx.x;  // output word 0..383
     {
-        const int u = w >> 7, lane = (w >> 2) & 31, cw = w & 3;
-        const int g = lane >> 2, t = lane & 3;
+        const int u = w >> 7, pos = (w >> 2) & 31, cw = w & 3;
+        const int t = pos >> 3, g = ((pos & 7) - 2 * t) & 7;  // inverse of chunk_pos
         int off;
         if (u < 2)
             off = 64 * u + 32 * (cw >> 1) + 16 * (cw & 1) + 4 * t;  // ql, half u, xo = cw >> 1, lr = cw & 1
@@ -602,7 +600,7 @@ cudaError_t launch_dir(cudaStream_t st, const DirectParams& P, size_t smem_bytes
 
 size_t prepacked_bytes(int dtype, int64_t n_rows, int k) {
     if (k % 256 || n_rows % 8) return 0;
-    const size_t htb = dtype == CANDLE_GGML_Q4K ? Q4K_HTB : (dtype == CANDLE_GGML_Q6K ? Q6K_HTB : 0);
+    const size_t htb = dtype == CANDLE_GGML_Q4K ? Q4K_HTB_BYTES : (dtype == CANDLE_GGML_Q6K ? Q6K_HTB_BYTES : 0);
     return (size_t)(n_rows / 8) * (size_t)(k / 256) * htb;
 }
 
@@ -676,7 +674,7 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
         P.off_bs = take((uint32_t)2 * MT * ks_blocks * bs_per_block);
         // per-warp rings of DEPTH K-blocks: 4 slots for Q4_K (2368 B each), 3 for Q6_K (3360 B each)
         const int depth = dtype == CANDLE_GGML_Q4K ? 4 : 3;
-        const uint32_t slot_bytes = 2u * (dtype == CANDLE_GGML_Q4K ? Q4K_HTB : Q6K_HTB);
+        const uint32_t slot_bytes = 2u * (dtype == CANDLE_GGML_Q4K ? Q4K_HTB_BYTES : Q6K_HTB_BYTES);
         P.off_ring = take((uint32_t)DIRECT_WARPS * depth * slot_bytes);
         P.off_part = NT == 1 ? take((uint32_t)DIRECT_WARPS * 512u) : 0u;
         if ((int)off > g_dir_max_smem - 1024) continue;

@@ -56,7 +56,6 @@ constexpr int G_REGS_EPI = 128, G_REGS_MISC = 32;  // budgets after the trade: 2
 constexpr int G_TMEM_COLS = 512;
 constexpr int G_TM_MAIN = 0;    // + 128 * buffer
 constexpr int G_TM_A = 256;     // weight operand ring: columns 256..511
-constexpr int Q6K_HTB_BYTES = 1680;  // repacked half-tile block: 8 rows x 256 elements (expert_direct.cu)
 
 // ---------------------------------------------------------------------------------------------
 // Operand preparation: the int8 activation rows in grouped order as fp16 (B operand), the block scales
@@ -157,28 +156,40 @@ prep_gemm_b_q80_kernel(const int8_t* __restrict__ aq, const float* __restrict__ 
     if (lane == 0) d8t[(int64_t)blk * P_pad + p] = exact ? 1.0f / 64.0f : 1.0f;
 }
 
-// Q8_0 GGUF rows [n][K / 32 blocks of 34 bytes] -> [n][K_pad / 256][272]: 256 int8 then 8 f16 scales, zeros past K.
-// One warp per (row, 256-block); a lane moves eight values with 2-byte loads (the 34-byte blocks are 2-byte aligned).
-__global__ void __launch_bounds__(256)
-prepack_q80_kernel(const uint8_t* __restrict__ raw, int64_t n_rows, int K, int K_pad, uint8_t* __restrict__ dst) {
-    const int kb = K_pad >> 8, lane = threadIdx.x & 31;
-    const int64_t unit = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (unit >= n_rows * kb) return;
-    const int64_t row = unit / kb;
-    const int blk = (int)(unit - row * kb);
-    uint8_t* out = dst + unit * 272;
-    const int k0 = blk * 256 + lane * 8;  // this lane's eight values
-    uint16_t v[4] = {0, 0, 0, 0};
-    if (k0 < K) {
-        const uint8_t* b = raw + (row * (K / 32) + (k0 >> 5)) * Q8_0_BYTES;
-        const uint16_t* q = reinterpret_cast<const uint16_t*>(b + 2 + (k0 & 31));
+// Q8_0 GGUF rows [n][K / 32 blocks of 34 bytes] -> [ceil(n / 8)][2 * ceil(K / 256)][1088]: 8 rows x 128 elements, two
+// 512-byte regions of 64 elements (chunk_pos order, a chunk of row g holds the words at 4 t, 16 + 4 t, 32 + 4 t, 48 + 4 t)
+// and [8 rows][4] f16 scales; zeros past K and past n.  The pieces the decode kernels' fragments and the GEMM's
+// row-per-lane reads both take with conflict-free 128-bit shared loads.  One CTA per half-tile block, one output word per
+// thread.
+__global__ void __launch_bounds__(288)
+prepack_q80_kernel(const uint8_t* __restrict__ raw, int64_t n_rows, int K, int kb, uint8_t* __restrict__ dst) {
+    const int64_t ht = blockIdx.x / kb;
+    const int blk = (int)(blockIdx.x - ht * kb);
+    uint32_t* out = reinterpret_cast<uint32_t*>(dst + (size_t)blockIdx.x * Q80_HTB_BYTES);
+    const int w = threadIdx.x;
+    if (w < 256) {
+        const int region = w >> 7, pos = (w >> 2) & 31, cw = w & 3;
+        const int t = pos >> 3, g = ((pos & 7) - 2 * t) & 7;  // inverse of chunk_pos
+        const int64_t row = ht * 8 + g;
+        const int k0 = blk * 128 + 64 * region + 16 * cw + 4 * t;
+        uint32_t v = 0;
+        if (row < n_rows && k0 < K) {
+            const uint16_t* q = reinterpret_cast<const uint16_t*>(raw + (row * (K / 32) + (k0 >> 5)) * Q8_0_BYTES + 2 + (k0 & 31));
+            v = (uint32_t)q[0] | ((uint32_t)q[1] << 16);
+        }
+        out[w] = v;
+    } else if (w < 272) {
+        uint32_t v = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = q[i];
-        if ((lane & 3) == 0) reinterpret_cast<uint16_t*>(out + 256)[lane >> 2] = *reinterpret_cast<const uint16_t*>(b);
-    } else if ((lane & 3) == 0) {
-        reinterpret_cast<uint16_t*>(out + 256)[lane >> 2] = 0;
+        for (int i = 0; i < 2; ++i) {
+            const int idx = 2 * (w - 256) + i;  // [g][j]
+            const int64_t row = ht * 8 + (idx >> 2);
+            const int b32 = blk * 4 + (idx & 3);
+            if (row < n_rows && b32 * 32 < K)
+                v |= (uint32_t)*reinterpret_cast<const uint16_t*>(raw + (row * (K / 32) + b32) * Q8_0_BYTES) << (16 * i);
+        }
+        out[w] = v;
     }
-    reinterpret_cast<uint2*>(out)[lane] = make_uint2((uint32_t)v[0] | ((uint32_t)v[1] << 16), (uint32_t)v[2] | ((uint32_t)v[3] << 16));
 }
 
 struct GemmParams {
@@ -207,40 +218,37 @@ __device__ __forceinline__ uint4 ldg128(const uint8_t* p) { return __ldg(reinter
 __device__ __forceinline__ uint32_t w4(const uint4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
 
 // ------------------------------------------------------------------------------------------------
-// Q4_K, GGUF layout (144-byte blocks: d, dmin, 12 scale bytes, 128 nibble bytes).  Thread (row, h) owns
-// bytes 16h..16h+15 of each 32-byte group: low nibbles are k = 16h.. of the 64-wide slab, high
-// nibbles k = 32 + 16h..; one TMEM column holds two k, so the 16 + 16 values are columns 8h.. and 16+8h..
+// The unpack formats.  An unpack thread owns (tile row, K half h): elements 128 h .. 128 h + 127 of every 256-block,
+// i.e. slabs 2h and 2h + 1 of 64 elements, handed over as one pair.  (Splitting a row's bytes between two threads inside
+// every slab instead made both decode the same scales.)  A slab is 32 TMEM columns of two elements each; element k of
+// the slab belongs to column k / 2, inside a group of four in the order (0, 2), (1, 3).
+//
+// Q4_K, GGUF layout (144-byte blocks: d, dmin, 12 scale bytes, 128 nibble bytes): bytes 32 s .. 32 s + 31 of the nibbles
+// are slab s, low nibbles k = 0..31, high nibbles k = 32..63.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ4K {
     static constexpr bool HAS_MIN = true;
     static constexpr int A_COLS = 32, A_PARTS = 1, A_PAIRS = 4;  // 8 slabs of 32 columns: two blocks in flight
     static constexpr int B_PARTS = 1;
-    static constexpr bool STAGE_W = true;                         // raw blocks of the tile pass through shared memory
+    static constexpr bool STAGE_W = true;      // raw blocks of the tile pass through shared memory
+    static constexpr bool HALF_TILES = false;  // ... as rows of GGUF blocks (tensor-map boxes)
     static constexpr int W_ROW_BYTES = Q4K_BYTES;
-    static constexpr int W_MAP_ELEM = 1;     // the tensor map of the raw blocks counts bytes
-    static constexpr int W_STAGES_WIDE = 1;  // staged blocks that fit beside 128-wide activation stages
-    struct Row {
-        const uint8_t* p;
-    };
-    __device__ static __forceinline__ Row row(const uint8_t* w, int n, int kb) { return Row{w + (size_t)n * kb * Q4K_BYTES}; }
+    static constexpr int W_STAGES_WIDE = 1;    // staged blocks that fit beside 128-wide activation stages
+    struct Row {};
     struct Pre {
         uint4 hdr, q[4];
     };
-    __device__ static __forceinline__ void load(Pre& pr, const Row& r, int blk, int h) {
-        const uint8_t* b = r.p + (size_t)blk * Q4K_BYTES;
-        pr.hdr = ldg128(b);
-#pragma unroll
-        for (int s = 0; s < 4; ++s) pr.q[s] = ldg128(b + 16 + 32 * s + 16 * h);
-    }
-    // the same pieces from the staged copy of the block (row_addr: shared-window address of the row's 144 bytes;
-    // rows are 36 words apart, so the eight lanes of a 16-byte load phase cover all 32 banks once)
+    __device__ static __forceinline__ void load(Pre&, const Row&, int, int) {}
+    __device__ static __forceinline__ Row row(const uint8_t*, int, int) { return Row{}; }
+    // this thread's pieces of the staged row (rows are 36 words apart: the eight lanes of a 16-byte load phase cover all
+    // 32 banks once)
     __device__ static __forceinline__ void load_staged(Pre& pr, uint32_t row_addr, int h) {
         pr.hdr = lds128_o<0>(row_addr);
-        const uint32_t rb = row_addr + 16 * h;
+        const uint32_t rb = row_addr + 64 * h;
         pr.q[0] = lds128_o<16>(rb);
-        pr.q[1] = lds128_o<48>(rb);
-        pr.q[2] = lds128_o<80>(rb);
-        pr.q[3] = lds128_o<112>(rb);
+        pr.q[1] = lds128_o<32>(rb);
+        pr.q[2] = lds128_o<48>(rb);
+        pr.q[3] = lds128_o<64>(rb);
     }
     // one word of every vector load_staged fetched: a value that exists only when all of them have arrived
     __device__ static __forceinline__ uint32_t staged_words(const Pre& pr) {
@@ -249,15 +257,18 @@ struct GemmQ4K {
     // d (low half) and dmin (high half) of the block, fp16 bits
     __device__ static __forceinline__ uint32_t hdr_of(const Pre& pr) { return pr.hdr.x; }
     struct Ctx {
-        uint32_t sc[2], mn[2];  // 6-bit scales / mins as bytes: [0] = sub-blocks 0..3, [1] = 4..7 (utils.rs:50-60)
+        uint32_t sc, mn;  // 6-bit scales / mins of this half's sub-blocks 4h .. 4h + 3 as bytes (utils.rs:50-60)
     };
-    __device__ static __forceinline__ void begin(const Pre& pr, Ctx& c) {
+    __device__ static __forceinline__ void begin(const Pre& pr, Ctx& c, int h) {
         const uint32_t s0 = pr.hdr.y, s1 = pr.hdr.z, s2 = pr.hdr.w;
-        c.sc[0] = s0 & 0x3f3f3f3fu;
-        c.mn[0] = s1 & 0x3f3f3f3fu;
-        c.sc[1] = (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
-        c.mn[1] = ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4);
-        if ((pr.hdr.x & 0x7fffu) == 0) c.sc[0] = c.sc[1] = 0;  // d = 0: the block is its min term alone (see scale_of)
+        if (h == 0) {
+            c.sc = s0 & 0x3f3f3f3fu;
+            c.mn = s1 & 0x3f3f3f3fu;
+        } else {
+            c.sc = (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
+            c.mn = ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4);
+        }
+        if ((pr.hdr.x & 0x7fffu) == 0) c.sc = 0;  // d = 0: the block is its min term alone (see scale_of)
     }
     // The epilogue multiplies the block's accumulator by d; a block with d = 0 (and no main sum, above) is
     // scaled by dmin instead so that its min term survives, or by 1 if both are zero.
@@ -265,58 +276,50 @@ struct GemmQ4K {
         const uint32_t hb = (hdr & 0x7fffu) ? (hdr & 0xffffu) : (((hdr >> 16) & 0x7fffu) ? (hdr >> 16) : 0x3c00u);
         return half_bits_to_float((uint16_t)hb);
     }
-    // slab s = sub-blocks 2s (low nibbles) and 2s+1 (high nibbles).  0x6400 | n is 1024 + n and
-    // fma(1024 + n, sc, -1024 sc) rounds the exact n * sc once; 0x6400 | (n << 4) is 1024 + 16 n and
+    // slab s of this half = sub-blocks 2s (low nibbles) and 2s + 1 (high nibbles) of the half.  0x6400 | n is 1024 + n
+    // and fma(1024 + n, sc, -1024 sc) rounds the exact n * sc once; 0x6400 | (n << 4) is 1024 + 16 n and
     // fma(1024 + 16 n, sc / 16, -64 sc) does the same for a nibble left in the high half of its byte.
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx& c, uint32_t ta, int h) {
-        const int jl = 2 * s, jh = 2 * s + 1;
+    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx& c, uint32_t ta) {
         const __half2 k1024 = __float2half2_rn(1024.f);
-        const __half2 scl = __hsub2(byte_magic2(c.sc[jl >> 2], jl & 3), k1024);
-        const __half2 sch = __hsub2(byte_magic2(c.sc[jh >> 2], jh & 3), k1024);
+        const __half2 scl = __hsub2(byte_magic2(c.sc, 2 * s), k1024);
+        const __half2 sch = __hsub2(byte_magic2(c.sc, 2 * s + 1), k1024);
         const __half2 offl = __hmul2(scl, __float2half2_rn(-1024.f));
         const __half2 sch16 = __hmul2(sch, __float2half2_rn(0.0625f)), offh = __hmul2(sch, __float2half2_rn(-64.f));
-        const uint32_t w[4] = {pr.q[s].x, pr.q[s].y, pr.q[s].z, pr.q[s].w};
-        uint32_t lo[8], hi[8];
+        uint32_t o[32];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t x = w[i], y = w[i] >> 8;  // bytes (0, 2) and (1, 3) of the four
-            lo[2 * i] = bits_h2(__hfma2(h2_bits((x & 0x000F000Fu) | 0x64006400u), scl, offl));
-            lo[2 * i + 1] = bits_h2(__hfma2(h2_bits((y & 0x000F000Fu) | 0x64006400u), scl, offl));
-            hi[2 * i] = bits_h2(__hfma2(h2_bits((x & 0x00F000F0u) | 0x64006400u), sch16, offh));
-            hi[2 * i + 1] = bits_h2(__hfma2(h2_bits((y & 0x00F000F0u) | 0x64006400u), sch16, offh));
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t x = w4(pr.q[2 * s + (i >> 2)], i & 3), y = x >> 8;  // bytes (0, 2) and (1, 3) of the four
+            o[2 * i] = bits_h2(__hfma2(h2_bits((x & 0x000F000Fu) | 0x64006400u), scl, offl));
+            o[2 * i + 1] = bits_h2(__hfma2(h2_bits((y & 0x000F000Fu) | 0x64006400u), scl, offl));
+            o[16 + 2 * i] = bits_h2(__hfma2(h2_bits((x & 0x00F000F0u) | 0x64006400u), sch16, offh));
+            o[16 + 2 * i + 1] = bits_h2(__hfma2(h2_bits((y & 0x00F000F0u) | 0x64006400u), sch16, offh));
         }
-        tmem_st8(ta + 8 * h, lo);
-        tmem_st8(ta + 16 + 8 * h, hi);
+        tmem_st32(ta, o);
     }
     // weight side of the min term (see prep_gemm_b_kernel): -rho_j = -dmin m_j / d split into tf32 terms.  One
-    // row is 32 floats [r1 (8) | r2 (8) | r1 (8) | unused]; thread h = 0 writes the four 16-byte chunks of r1,
-    // thread h = 1 the two of r2.  2^23 + m as float bits is 0x4B000000 | m.
+    // row is 32 floats [r1 (8) | r2 (8) | r1 (8) | unused]; half h writes its four values of each.  2^23 + m as float
+    // bits is 0x4B000000 | m.
     __device__ static __forceinline__ void emit_min(const Pre& pr, const Ctx& c, uint8_t* arow, int h, int sw) {
         const float ratio = -__fdividef(half_bits_to_float((uint16_t)(pr.hdr.x >> 16)), scale_of(pr.hdr.x));
-        uint32_t o[8];
+        uint32_t r1[4], r2[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float mf = __uint_as_float(0x4B000000u | byte_u(c.mn[j >> 2], j & 3)) - 8388608.f;
+        for (int j = 0; j < 4; ++j) {
+            const float mf = __uint_as_float(__byte_perm(c.mn, 0x4B000000u, 0x7650 | j)) - 8388608.f;
             const float a = __fmul_rn(ratio, mf), a1 = tf32_head(a);
-            o[j] = __float_as_uint(h == 0 ? a1 : tf32_head(__fsub_rn(a, a1)));
+            r1[j] = __float_as_uint(a1);
+            r2[j] = __float_as_uint(tf32_head(__fsub_rn(a, a1)));
         }
-        if (h == 0) {
-            *reinterpret_cast<uint4*>(arow + ((0 ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4*>(arow + ((1 ^ sw) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
-            *reinterpret_cast<uint4*>(arow + ((4 ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4*>(arow + ((5 ^ sw) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
-        } else {
-            *reinterpret_cast<uint4*>(arow + ((2 ^ sw) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4*>(arow + ((3 ^ sw) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
-        }
+        *reinterpret_cast<uint4*>(arow + ((h ^ sw) << 4)) = make_uint4(r1[0], r1[1], r1[2], r1[3]);
+        *reinterpret_cast<uint4*>(arow + (((2 + h) ^ sw) << 4)) = make_uint4(r2[0], r2[1], r2[2], r2[3]);
+        *reinterpret_cast<uint4*>(arow + (((4 + h) ^ sw) << 4)) = make_uint4(r1[0], r1[1], r1[2], r1[3]);
     }
 };
 
 // ------------------------------------------------------------------------------------------------
 // Q6_K, repacked layout (expert_direct.cu: per 8 rows x 256 elements, 1680 bytes: low nibbles 2 x 512,
-// high bit pairs 512, 128 scales, 8 d).  Row g's 64 nibble bytes of half n sit at 512 n + 64 g in four
-// 16-byte chunks t; word cw of chunk t holds elements k0 = 16 cw + 4 t .. + 3 of the half's two slabs
-// (low nibbles: even slab, high nibbles: odd slab).  Thread (row, h) takes chunks t = 2h, 2h + 1.
+// high bit pairs 512, 128 scales, 8 d; a row's four 16-byte chunks t of a 512-byte region lie in chunk_pos order).  Word
+// cw of chunk t of half h holds elements k0 = 16 cw + 4 t .. + 3 of the half's two slabs (low nibbles: first slab, high
+// nibbles: second), words 2h, 2h + 1 of chunk t of the third region their high bit pairs.
 // The quant is placed at mantissa bits 4..9 (0x6400 | q << 4 = 1024 + 16 q); minus 1536 leaves
 // 16 (q - 32), times ceil(sc/2)/16 and floor(sc/2)/16 gives the two exact operand parts.
 // ------------------------------------------------------------------------------------------------
@@ -325,8 +328,8 @@ struct GemmQ6K {
     static constexpr int A_COLS = 64, A_PARTS = 2, A_PAIRS = 2;  // 4 slabs of 64 columns (two operand parts each)
     static constexpr int B_PARTS = 1;
     static constexpr bool STAGE_W = false;
+    static constexpr bool HALF_TILES = false;
     static constexpr int W_ROW_BYTES = 0;
-    static constexpr int W_MAP_ELEM = 1;
     static constexpr int W_STAGES_WIDE = 1;
     struct Row {
         const uint8_t* p;  // half-tile block 0 of the row's group of 8
@@ -336,62 +339,61 @@ struct GemmQ6K {
         return Row{w + (size_t)(n >> 3) * kb * Q6K_HTB_BYTES, n & 7};
     }
     struct Pre {
-        uint4 ql[2][2], qh[2], sc;
+        uint4 ql[4];
+        uint2 qh[4], sc;
         uint32_t d;  // fp16 bits
     };
     __device__ static __forceinline__ uint32_t hdr_of(const Pre& pr) { return pr.d; }
     __device__ static __forceinline__ void load_staged(Pre&, uint32_t, int) {}
     __device__ static __forceinline__ uint32_t staged_words(const Pre&) { return 0u; }
     __device__ static __forceinline__ void load(Pre& pr, const Row& r, int blk, int h) {
-        const uint8_t* b = r.p + (size_t)blk * Q6K_HTB_BYTES + 64 * r.g + 32 * h;
+        const uint8_t* b = r.p + (size_t)blk * Q6K_HTB_BYTES;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            pr.ql[0][j] = ldg128(b + 16 * j);
-            pr.ql[1][j] = ldg128(b + 512 + 16 * j);
-            pr.qh[j] = ldg128(b + 1024 + 16 * j);
+        for (int t = 0; t < 4; ++t) {
+            const int c = 16 * chunk_pos(r.g, t);
+            pr.ql[t] = ldg128(b + 512 * h + c);
+            pr.qh[t] = __ldg(reinterpret_cast<const uint2*>(b + 1024 + c + 8 * h));
         }
-        pr.sc = ldg128(r.p + (size_t)blk * Q6K_HTB_BYTES + 1536 + 16 * r.g);
-        pr.d = (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(r.p + (size_t)blk * Q6K_HTB_BYTES + 1664 + 2 * r.g));
+        pr.sc = __ldg(reinterpret_cast<const uint2*>(b + 1536 + 16 * r.g + 8 * h));
+        pr.d = (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(b + 1664 + 2 * r.g));
     }
     struct Ctx {
-        uint32_t xc[4], xh[4];  // per scale byte: ceil(sc/2) + 64 and floor(sc/2) + 64
+        uint32_t xc[2], xh[2];  // per scale byte: ceil(sc/2) + 64 and floor(sc/2) + 64
     };
-    __device__ static __forceinline__ void begin(const Pre& pr, Ctx& c) {
-        const uint32_t w[4] = {pr.sc.x, pr.sc.y, pr.sc.z, pr.sc.w};
+    __device__ static __forceinline__ void begin(const Pre& pr, Ctx& c, int) {
+        const uint32_t w[2] = {pr.sc.x, pr.sc.y};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 2; ++i) {
             const uint32_t x = w[i] ^ 0x80808080u;  // sc + 128 per byte
             c.xh[i] = (x >> 1) & 0x7f7f7f7fu;
             c.xc[i] = c.xh[i] + (x & 0x01010101u);
         }
     }
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx& c, uint32_t ta, int h) {
-        const int n = s >> 1, odd = s & 1;
+    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx& c, uint32_t ta) {
         const __half2 k16th = __float2half2_rn(0.0625f), km68 = __float2half2_rn(-68.f), km1536 = __float2half2_rn(-1536.f);
 #pragma unroll
         for (int cw = 0; cw < 4; ++cw) {
-            const int idx = 4 * s + cw;
             // (1024 + x) / 16 - 68 = (x - 64) / 16: the half scale over 16; c = -1536 m, so that
             // fma(1024 + 16 q, m, c) = (q - 32) * (half scale), an integer of at most 2048: exact
-            const __half2 m1 = __hfma2(byte_magic2(c.xc[idx >> 2], idx & 3), k16th, km68);
-            const __half2 m2 = __hfma2(byte_magic2(c.xh[idx >> 2], idx & 3), k16th, km68);
+            const __half2 m1 = __hfma2(byte_magic2(c.xc[s], cw), k16th, km68);
+            const __half2 m2 = __hfma2(byte_magic2(c.xh[s], cw), k16th, km68);
             const __half2 c1 = __hmul2(m1, km1536), c2 = __hmul2(m2, km1536);
-            const int bq = 2 * ((cw >> 1) + 2 * odd);  // bit position of this quarter's pair in the qh byte
-            uint32_t o1[4], o2[4];
+            const int bq = 2 * ((cw >> 1) + 2 * s);  // bit position of this quarter's pair in the qh byte
+            uint32_t o1[8], o2[8];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const uint32_t qlw = w4(pr.ql[n][j], cw), qhw = w4(pr.qh[j], 2 * n + (cw & 1));
-                const uint32_t a02 = odd ? qlw : (qlw << 4), a13 = odd ? (qlw >> 8) : (qlw >> 4);
+            for (int t = 0; t < 4; ++t) {
+                const uint32_t qlw = w4(pr.ql[t], cw), qhw = (cw & 1) ? pr.qh[t].y : pr.qh[t].x;
+                const uint32_t a02 = s ? qlw : (qlw << 4), a13 = s ? (qlw >> 8) : (qlw >> 4);
                 const uint32_t b02 = qhw << (8 - bq), b13 = qhw >> bq;
                 const __half2 v02 = h2_bits(((a02 & 0x00F000F0u) | 0x64006400u) | (b02 & 0x03000300u));
                 const __half2 v13 = h2_bits(((a13 & 0x00F000F0u) | 0x64006400u) | (b13 & 0x03000300u));
-                o1[2 * j] = bits_h2(__hfma2(v02, m1, c1));
-                o1[2 * j + 1] = bits_h2(__hfma2(v13, m1, c1));
-                o2[2 * j] = bits_h2(__hfma2(v02, m2, c2));
-                o2[2 * j + 1] = bits_h2(__hfma2(v13, m2, c2));
+                o1[2 * t] = bits_h2(__hfma2(v02, m1, c1));
+                o1[2 * t + 1] = bits_h2(__hfma2(v13, m1, c1));
+                o2[2 * t] = bits_h2(__hfma2(v02, m2, c2));
+                o2[2 * t + 1] = bits_h2(__hfma2(v13, m2, c2));
             }
-            tmem_st4(ta + 8 * cw + 4 * h, o1[0], o1[1], o1[2], o1[3]);
-            tmem_st4(ta + 32 + 8 * cw + 4 * h, o2[0], o2[1], o2[2], o2[3]);
+            tmem_st8(ta + 8 * cw, o1);
+            tmem_st8(ta + 32 + 8 * cw, o2);
         }
     }
     __device__ static __forceinline__ void emit_min(const Pre&, const Ctx&, uint8_t*, int, int) {}
@@ -399,74 +401,76 @@ struct GemmQ6K {
 };
 
 // ------------------------------------------------------------------------------------------------
-// Q8_0, repacked layout (prepack_q80_kernel): per row and 256 elements a 272-byte record [256 int8 | 8 f16
-// scales], rows padded with zero records to a multiple of 256 elements.  The reference multiplies per 32-element
+// Q8_0, repacked layout (prepack_q80_kernel): half-tile blocks of 8 rows x 128 elements, two of them per 256-block, rows
+// padded with zeros to a multiple of 256 elements.  The reference multiplies per 32-element
 // block (sum of int8 products) * d_w * d_a in f32 (k_quants.rs:636-668); here both scales are folded into the fp16
 // operands -- weight d_w * q, activation d_a * q, each rounded once to fp16 (2^-12 relative) -- and the products
 // are accumulated in f32 by the tensor core over the whole row, so no per-block scaling is left for the epilogue.
 // The rounding of the operands is the one deviation from the reference's arithmetic on this path: it shows as a
 // relative L2 error of a few 1e-4 on a product, inside the block's bound (1e-3), and is measured by the tests.
 // Used for the down product only (see launch_expert_gemm for why gate_up cannot afford that rounding).
-// Thread (row, h) owns bytes 16h..16h+15 and 32+16h..32+16h+15 of each 64-element slab, like the Q4_K thread.
+// Half h of a 256-block is its half-tile block h; word cw of chunk t of region s holds elements 16 cw + 4 t .. + 3.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ80 {
     static constexpr bool HAS_MIN = false;
     static constexpr int A_COLS = 32, A_PARTS = 1, A_PAIRS = 4;
     static constexpr int B_PARTS = 1;
     static constexpr bool STAGE_W = true;
-    static constexpr int W_ROW_BYTES = 272;
-    static constexpr int W_MAP_ELEM = 4;     // the tensor map counts 4-byte elements (a box row of 272 bytes exceeds 256 bytes)
+    static constexpr bool HALF_TILES = true;  // staged as half-tile blocks, one bulk copy per 8 rows
+    static constexpr int W_ROW_BYTES = 2 * Q80_HTB_BYTES / 8;
     static constexpr int W_STAGES_WIDE = 2;  // staged blocks beside 128-wide activation stages
-    struct Row {
-        const uint8_t* p;
-    };
-    __device__ static __forceinline__ Row row(const uint8_t* w, int n, int kb) { return Row{w + (size_t)n * kb * W_ROW_BYTES}; }
+    struct Row {};
+    __device__ static __forceinline__ Row row(const uint8_t*, int, int) { return Row{}; }
     struct Pre {
-        uint4 sc;       // 8 f16 scales
-        uint4 q[4][2];  // per slab: bytes 16h.. and 32 + 16h..
+        uint2 sc;       // 4 f16 scales
+        uint4 q[2][4];  // per slab: chunks t = 0..3
     };
     __device__ static __forceinline__ void load(Pre&, const Row&, int, int) {}
-    __device__ static __forceinline__ void load_staged(Pre& pr, uint32_t row_addr, int h) {
-        pr.sc = lds128_o<256>(row_addr);
-        const uint32_t rb = row_addr + 16 * h;
-        pr.q[0][0] = lds128_o<0>(rb);
-        pr.q[0][1] = lds128_o<32>(rb);
-        pr.q[1][0] = lds128_o<64>(rb);
-        pr.q[1][1] = lds128_o<96>(rb);
-        pr.q[2][0] = lds128_o<128>(rb);
-        pr.q[2][1] = lds128_o<160>(rb);
-        pr.q[3][0] = lds128_o<192>(rb);
-        pr.q[3][1] = lds128_o<224>(rb);
-    }
-    __device__ static __forceinline__ uint32_t staged_words(const Pre& pr) {
-        return pr.sc.x | pr.q[0][0].x | pr.q[0][1].x | pr.q[1][0].x | pr.q[1][1].x | pr.q[2][0].x | pr.q[2][1].x | pr.q[3][0].x | pr.q[3][1].x;
-    }
-    __device__ static __forceinline__ uint32_t hdr_of(const Pre&) { return 0u; }
-    struct Ctx {};
-    __device__ static __forceinline__ void begin(const Pre&, Ctx&) {}
-    __device__ static __forceinline__ float scale_of(uint32_t) { return 1.0f; }  // the scales are inside the operands
-    // 16 int8 -> 8 columns of fp16 pairs (k0, k2), (k1, k3) per word, times d: the byte plus 128 is dropped into the
-    // mantissa of 1024 (0x6400 | b + 128 = 1152 + b), 1152 comes off exactly, one multiply rounds
-    __device__ static __forceinline__ void cvt16(const uint4& v, __half2 d, uint32_t (&o)[8]) {
-        const uint32_t w[4] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u, v.z ^ 0x80808080u, v.w ^ 0x80808080u};
-        const __half2 k1152 = __float2half2_rn(1152.f);
+    // ht_addr: the row's half-tile (both blocks) in the stage, g: its row inside
+    __device__ static __forceinline__ void load_half_tile(Pre& pr, uint32_t ht_addr, int g, int h) {
+        const uint32_t b = ht_addr + h * Q80_HTB_BYTES;
+        pr.sc = lds64_o<1024>(b + 8 * g);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint32_t e, f;
-            asm("prmt.b32 %0, %1, %2, 0x4240;" : "=r"(e) : "r"(w[i]), "r"(0x64646464u));  // bytes 0 and 2
-            asm("prmt.b32 %0, %1, %2, 0x4341;" : "=r"(f) : "r"(w[i]), "r"(0x64646464u));  // bytes 1 and 3
-            o[2 * i] = bits_h2(__hmul2(__hsub2(h2_bits(e), k1152), d));
-            o[2 * i + 1] = bits_h2(__hmul2(__hsub2(h2_bits(f), k1152), d));
+        for (int t = 0; t < 4; ++t) {
+            const uint32_t c = b + 16 * chunk_pos(g, t);
+            pr.q[0][t] = lds128_o<0>(c);
+            pr.q[1][t] = lds128_o<512>(c);
         }
     }
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx&, uint32_t ta, int h) {
-        const uint32_t dw = s == 0 ? pr.sc.x : (s == 1 ? pr.sc.y : (s == 2 ? pr.sc.z : pr.sc.w));  // scales of blocks 2s, 2s + 1
-        const __half2 d2 = h2_bits(dw);
-        uint32_t lo[8], hi[8];
-        cvt16(pr.q[s][0], __low2half2(d2), lo);
-        cvt16(pr.q[s][1], __high2half2(d2), hi);
-        tmem_st8(ta + 8 * h, lo);
-        tmem_st8(ta + 16 + 8 * h, hi);
+    __device__ static __forceinline__ void load_staged(Pre&, uint32_t, int) {}
+    __device__ static __forceinline__ uint32_t staged_words(const Pre&) { return 0u; }  // a ring of two or more stages always
+    __device__ static __forceinline__ uint32_t hdr_of(const Pre&) { return 0u; }
+    struct Ctx {};
+    __device__ static __forceinline__ void begin(const Pre&, Ctx&, int) {}
+    __device__ static __forceinline__ float scale_of(uint32_t) { return 1.0f; }  // the scales are inside the operands
+    // 4 int8 -> 2 columns of fp16 pairs (k0, k2), (k1, k3): the byte plus 128 is dropped into the mantissa of 1024
+    // (0x6400 | b + 128 = 1152 + b), 1152 comes off exactly, one multiply rounds
+    __device__ static __forceinline__ void split4(uint32_t v, __half2& e, __half2& f) {
+        const __half2 k1152 = __float2half2_rn(1152.f);
+        uint32_t a, b;
+        const uint32_t w = v ^ 0x80808080u;
+        asm("prmt.b32 %0, %1, %2, 0x4240;" : "=r"(a) : "r"(w), "r"(0x64646464u));  // bytes 0 and 2
+        asm("prmt.b32 %0, %1, %2, 0x4341;" : "=r"(b) : "r"(w), "r"(0x64646464u));  // bytes 1 and 3
+        e = __hsub2(h2_bits(a), k1152);
+        f = __hsub2(h2_bits(b), k1152);
+    }
+    // scales of the two 32-element blocks of slab s
+    __device__ static __forceinline__ __half2 scales(const Pre& pr, int s) { return h2_bits(s ? pr.sc.y : pr.sc.x); }
+    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx&, uint32_t ta) {
+        const __half2 d2 = scales(pr, s);
+        uint32_t o[32];
+#pragma unroll
+        for (int cw = 0; cw < 4; ++cw) {
+            const __half2 d = cw < 2 ? __low2half2(d2) : __high2half2(d2);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                __half2 e, f;
+                split4(w4(pr.q[s][t], cw), e, f);
+                o[8 * cw + 2 * t] = bits_h2(__hmul2(e, d));
+                o[8 * cw + 2 * t + 1] = bits_h2(__hmul2(f, d));
+            }
+        }
+        tmem_st32(ta, o);
     }
     __device__ static __forceinline__ void emit_min(const Pre&, const Ctx&, uint8_t*, int, int) {}
 };
@@ -486,32 +490,27 @@ struct GemmQ80X : GemmQ80 {
     static constexpr int B_PARTS = 2;
     static constexpr int W_STAGES_WIDE = 2;
     __device__ static __forceinline__ float scale_of(uint32_t) { return 1.0f / 4096.0f; }
-    __device__ static __forceinline__ void cvt16x(const uint4& v, __half2 d, uint32_t (&p0)[8], uint32_t (&p1)[8]) {
-        const uint32_t w[4] = {v.x ^ 0x80808080u, v.y ^ 0x80808080u, v.z ^ 0x80808080u, v.w ^ 0x80808080u};
-        const __half2 k1152 = __float2half2_rn(1152.f);
+    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx&, uint32_t ta) {
+        const __half2 d2 = __hmul2(scales(pr, s), __float2half2_rn(4096.f));  // exact (a power of two)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint32_t e, f;
-            asm("prmt.b32 %0, %1, %2, 0x4240;" : "=r"(e) : "r"(w[i]), "r"(0x64646464u));
-            asm("prmt.b32 %0, %1, %2, 0x4341;" : "=r"(f) : "r"(w[i]), "r"(0x64646464u));
-            const __half2 xe = __hsub2(h2_bits(e), k1152), xf = __hsub2(h2_bits(f), k1152);
-            const __half2 re = __hmul2(xe, d), rf = __hmul2(xf, d);
-            p0[2 * i] = bits_h2(re);
-            p0[2 * i + 1] = bits_h2(rf);
-            p1[2 * i] = bits_h2(__hfma2(xe, d, __hneg2(re)));  // exact: the residual of a 19-bit product has at most 8 bits
-            p1[2 * i + 1] = bits_h2(__hfma2(xf, d, __hneg2(rf)));
+        for (int c2 = 0; c2 < 2; ++c2) {  // one 32-element block of the slab
+            const __half2 d = c2 ? __high2half2(d2) : __low2half2(d2);
+            uint32_t p0[16], p1[16];
+#pragma unroll
+            for (int cw = 0; cw < 2; ++cw)
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    __half2 e, f;
+                    split4(w4(pr.q[s][t], 2 * c2 + cw), e, f);
+                    const __half2 re = __hmul2(e, d), rf = __hmul2(f, d);
+                    p0[8 * cw + 2 * t] = bits_h2(re);
+                    p0[8 * cw + 2 * t + 1] = bits_h2(rf);
+                    p1[8 * cw + 2 * t] = bits_h2(__hfma2(e, d, __hneg2(re)));  // exact: the residual of a 19-bit product has at most 8 bits
+                    p1[8 * cw + 2 * t + 1] = bits_h2(__hfma2(f, d, __hneg2(rf)));
+                }
+            tmem_st16(ta + 16 * c2, p0);
+            tmem_st16(ta + 32 + 16 * c2, p1);
         }
-    }
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx&, uint32_t ta, int h) {
-        const uint32_t dw = s == 0 ? pr.sc.x : (s == 1 ? pr.sc.y : (s == 2 ? pr.sc.z : pr.sc.w));
-        const __half2 d2 = __hmul2(h2_bits(dw), __float2half2_rn(4096.f));  // exact (a power of two)
-        uint32_t a0[8], a1[8];
-        cvt16x(pr.q[s][0], __low2half2(d2), a0, a1);
-        tmem_st8(ta + 8 * h, a0);
-        tmem_st8(ta + 32 + 8 * h, a1);
-        cvt16x(pr.q[s][1], __high2half2(d2), a0, a1);
-        tmem_st8(ta + 16 + 8 * h, a0);
-        tmem_st8(ta + 48 + 8 * h, a1);
     }
 };
 
@@ -519,6 +518,12 @@ struct GemmQ80X : GemmQ80 {
 template <class F, int TN>
 __host__ __device__ constexpr int w_stages() {
     return !F::STAGE_W ? 1 : (TN <= 32 ? 4 : (TN <= 64 ? (F::B_PARTS == 2 ? 4 : 3) : F::W_STAGES_WIDE));
+}
+
+// weight row of tile row r: gate_up tiles hold 8 rows of W1, then the same 8 rows of W3, and so on (64 rows of each)
+template <bool GATE_UP>
+__device__ __forceinline__ int weight_row(int mt, int r) {
+    return GATE_UP ? mt * 64 + (r >> 4) * 8 + (r & 7) : mt * 128 + r;
 }
 
 struct TileCoord {
@@ -594,7 +599,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
     if (threadIdx.x == 0) {
         s_abort = 0;
         for (int s = 0; s < 4; ++s) {
-            mbar_init(&full_a[s], G_DQ_WARPS);
+            mbar_init(&full_a[s], G_DQ_WARPS / 2);
             mbar_init(&empty_a[s], 1);
         }
         for (int s = 0; s < G_B_STAGES; ++s) {
@@ -701,17 +706,18 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
 #pragma unroll
             for (int i = 0; i < CH / 2; ++i) f32x2_unpack(acc2[i], acc[2 * i], acc[2 * i + 1]);
             // ---- store the tile ----
-            const int n = GATE_UP ? tc.mt * 64 + (r >> 1) : tc.mt * 128 + r;
+            const int n = weight_row<GATE_UP>(tc.mt, r);
             const uint32_t pc0 = tc.p0 + colhalf * CH;
             float* out_k = P.out + (size_t)tc.ks * P.split_stride;
             if (GATE_UP) {
-                // even lane holds w1 x, odd lane w3 x of the same output row: the even lane finishes the first
-                // half of this warp's columns, the odd lane the second half, one exchange per pair of columns
+                // the lane with bit 3 clear holds w1 x, its partner w3 x of the same output row: the first finishes the
+                // first half of this warp's columns, the other the second half, one exchange per pair of columns
+                const bool up = lane & 8;
 #pragma unroll
                 for (int c = 0; c < CH / 2; ++c) {
-                    const float recv = __shfl_xor_sync(0xffffffffu, (lane & 1) ? acc[c] : acc[c + CH / 2], 1);
-                    const float gv = (lane & 1) ? recv : acc[c], uv = (lane & 1) ? acc[c + CH / 2] : recv;
-                    const uint32_t p = pc0 + c + ((lane & 1) ? CH / 2 : 0);
+                    const float recv = __shfl_xor_sync(0xffffffffu, up ? acc[c] : acc[c + CH / 2], 8);
+                    const float gv = up ? recv : acc[c], uv = up ? acc[c + CH / 2] : recv;
+                    const uint32_t p = pc0 + c + (up ? CH / 2 : 0);
                     if (p < tc.p_end) out_k[(size_t)p * P.N + n] = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
                 }
             } else {
@@ -729,39 +735,42 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         const int r = 32 * quarter + lane;
         const uint32_t ta_lane = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)G_TM_A;
         const uint32_t min_row_off = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
-        uint32_t ita = 0, ab = 0;
+        uint32_t ab = 0;
         long long tile = blockIdx.x;
         TileCoord tc, tcn;
         bool have = decode_tile<TN>(tile, s_offs, P.E, P.m_tiles, P.ksplit, P.kb, tc);
         typename F::Row rowc{}, rown{};
         typename F::Pre cur, nxt;
-        // staged row of tile row r: gate_up keeps the W1 rows first, then the W3 rows
-        const uint32_t w_row = smem_u32(smem_w) + (GATE_UP ? (uint32_t)((r & 1) * (G_TILE_M / 2 * F::W_ROW_BYTES) + (r >> 1) * F::W_ROW_BYTES)
-                                                           : (uint32_t)(r * F::W_ROW_BYTES));
+        // where tile row r lies in a stage: rows (gate_up: the W1 rows first, then the W3 rows) or half-tiles in tile order
+        const uint32_t w_row = smem_u32(smem_w) +
+                               (F::HALF_TILES ? (uint32_t)((r >> 3) * 8 * F::W_ROW_BYTES)
+                                : GATE_UP ? (uint32_t)((((r >> 3) & 1) * (G_TILE_M / 2) + (r >> 4) * 8 + (r & 7)) * F::W_ROW_BYTES)
+                                          : (uint32_t)(r * F::W_ROW_BYTES));
+        const bool is_w3 = GATE_UP && ((r >> 3) & 1);
         if (have && !F::STAGE_W) {
-            const int n = GATE_UP ? tc.mt * 64 + (r >> 1) : tc.mt * 128 + r;
-            rowc = F::row((GATE_UP && (r & 1)) ? P.wb.p[tc.e] : P.wa.p[tc.e], n, P.kb);
+            rowc = F::row(is_w3 ? P.wb.p[tc.e] : P.wa.p[tc.e], weight_row<GATE_UP>(tc.mt, r), P.kb);
             F::load(cur, rowc, tc.kb0, h);
             nxt = cur;
         }
         while (have) {
             const bool have_n = decode_tile<TN>(tile + gridDim.x, s_offs, P.E, P.m_tiles, P.ksplit, P.kb, tcn);
-            if (have_n && !F::STAGE_W) {
-                const int nn = GATE_UP ? tcn.mt * 64 + (r >> 1) : tcn.mt * 128 + r;
-                rown = F::row((GATE_UP && (r & 1)) ? P.wb.p[tcn.e] : P.wa.p[tcn.e], nn, P.kb);
-            }
+            if (have_n && !F::STAGE_W)
+                rown = F::row(is_w3 ? P.wb.p[tcn.e] : P.wa.p[tcn.e], weight_row<GATE_UP>(tcn.mt, r), P.kb);
             for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
                 if (F::STAGE_W) {
                     // this block's raw bytes were copied to shared memory by the loader warp
                     mbar_wait(&full_w[ab % WS], (ab / WS) & 1, abort_flag);
-                    F::load_staged(cur, w_row + (ab % WS) * W_STAGE_BYTES, h);
+                    if constexpr (F::HALF_TILES)
+                        F::load_half_tile(cur, w_row + (ab % WS) * W_STAGE_BYTES, r & 7, h);
+                    else
+                        F::load_staged(cur, w_row + (ab % WS) * W_STAGE_BYTES, h);
                 } else if (blk + 1 < tc.kb1) {
                     F::load(nxt, rowc, blk + 1, h);
                 } else if (have_n) {
                     F::load(nxt, rown, tcn.kb0, h);
                 }
                 typename F::Ctx ctx;
-                F::begin(cur, ctx);
+                F::begin(cur, ctx, h);
                 if (h == 0) s_dw[ab & 7][r] = F::scale_of(F::hdr_of(cur));  // read by the epilogue when it drains this block
                 // Handing the stage back to the loader.  The staged words must have ARRIVED in registers first: the
                 // loads are plain shared-memory loads, their results are not needed until the emits below, and an
@@ -777,34 +786,31 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                     const uint32_t dep = __reduce_or_sync(0xffffffffu, F::staged_words(cur)) & P.zero;
                     if (lane == 0) mbar_arrive(&empty_w[dep]);
                 }
-#pragma unroll
-                for (int pr = 0; pr < 2; ++pr, ita += 2) {
-                    // Slabs go to tensor memory in pairs; the ring holds A_PAIRS pairs (Q4_K: two blocks).  The barriers
-                    // go by (block parity, pair) -- each has ONE waiting MMA warp that sees every phase, so a parity
-                    // wait is never ambiguous -- while the TMEM slot is the pair index modulo the ring size: before
-                    // writing it, wait for the MMAs of the block that used it last.
-                    const uint32_t bidx = 2 * (ab & 1) + pr, slot = bidx % F::A_PAIRS;
-                    if (ab >= F::A_PAIRS / 2) {
-                        const uint32_t abp = ab - F::A_PAIRS / 2;
-                        mbar_wait_relaxed(&empty_a[2 * (abp & 1) + pr], (abp >> 1) & 1, abort_flag);
-                    }
-                    tc5_fence_after_sync();
-                    F::emit(2 * pr, cur, ctx, ta_lane + (uint32_t)(2 * slot * F::A_COLS), h);
-                    F::emit(2 * pr + 1, cur, ctx, ta_lane + (uint32_t)((2 * slot + 1) * F::A_COLS), h);
-                    if (F::HAS_MIN && pr == 1) {
-                        // weight side of the min term, handed over with the second pair.  Its slot was last read by
-                        // the min MMAs of block ab - 2, issued before the commit whose completion the wait above saw.
-                        F::emit_min(cur, ctx, smem_min_a + (size_t)(ab & 1) * G_TILE_BYTES + min_row_off, h, r & 7);
-                        fence_proxy_async_smem();
-                    }
-                    tmem_st_wait();
-                    tc5_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&full_a[bidx]);
+                // The pair goes to tensor memory; the ring holds A_PAIRS pairs (Q4_K: two blocks).  The barriers
+                // go by (block parity, pair) -- each has ONE waiting MMA warp that sees every phase, so a parity
+                // wait is never ambiguous -- while the TMEM slot is the pair index modulo the ring size: before
+                // writing it, wait for the MMAs of the block that used it last.
+                const uint32_t bidx = 2 * (ab & 1) + h, slot = bidx % F::A_PAIRS;
+                if (ab >= F::A_PAIRS / 2) {
+                    const uint32_t abp = ab - F::A_PAIRS / 2;
+                    mbar_wait_relaxed(&empty_a[2 * (abp & 1) + h], (abp >> 1) & 1, abort_flag);
                 }
-                if (F::STAGE_W && WS > 1) {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty_w[ab % WS]);
+                tc5_fence_after_sync();
+                F::emit(0, cur, ctx, ta_lane + (uint32_t)(2 * slot * F::A_COLS));
+                F::emit(1, cur, ctx, ta_lane + (uint32_t)((2 * slot + 1) * F::A_COLS));
+                if (F::HAS_MIN) {
+                    // weight side of the min term.  Its slot was last read by the min MMAs of block ab - 2, issued
+                    // before the commit of that block's second pair.
+                    if (h == 0 && ab >= 2) mbar_wait_relaxed(&empty_a[2 * (ab & 1) + 1], ((ab - 2) >> 1) & 1, abort_flag);
+                    F::emit_min(cur, ctx, smem_min_a + (size_t)(ab & 1) * G_TILE_BYTES + min_row_off, h, r & 7);
+                    fence_proxy_async_smem();
+                }
+                tmem_st_wait();
+                tc5_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&full_a[bidx]);
+                    if (F::STAGE_W && WS > 1) mbar_arrive(&empty_w[ab % WS]);
                 }
                 if (!F::STAGE_W) cur = nxt;
             }
@@ -820,7 +826,43 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         // be skewed against each other and neighbouring lanes, which alternate between them, share banks two by
         // two).  Two blocks ahead the same boxes are requested into L2, so the copy into the one-block-deep stage
         // finds them there.
-        if (F::STAGE_W) {
+        if constexpr (F::HALF_TILES) {
+            // half-tile blocks of the repacked layout: one bulk copy per 8 tile rows, lane i < 16 copies half-tile i
+            // (gate_up: W1 and W3 half-tiles alternate); two blocks ahead the same bytes are requested into L2
+            uint32_t ab = 0;
+            TileCoord tc, tcn;
+            long long tile = blockIdx.x;
+            bool have = decode_tile<TN>(tile, s_offs, P.E, P.m_tiles, P.ksplit, P.kb, tc);
+            constexpr int HT_BYTES = 8 * F::W_ROW_BYTES;  // a half-tile over one 256-block
+            const bool active = lane < G_TILE_M / 8, is_w3 = GATE_UP && (lane & 1);
+            auto src_of = [&](const TileCoord& c) {
+                const int ht = GATE_UP ? c.mt * 8 + (lane >> 1) : c.mt * 16 + lane;
+                return (is_w3 ? P.wb.p[c.e] : P.wa.p[c.e]) + (size_t)ht * P.kb * HT_BYTES;
+            };
+            const uint8_t* src = have && active ? src_of(tc) : nullptr;
+            while (have) {
+                const bool have_n = decode_tile<TN>(tile + gridDim.x, s_offs, P.E, P.m_tiles, P.ksplit, P.kb, tcn);
+                const uint8_t* src_n = have_n && active ? src_of(tcn) : nullptr;
+                for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
+                    const uint32_t ws = ab % WS;
+                    if (ab >= (uint32_t)WS) mbar_wait(&empty_w[ws], ((ab / WS) - 1) & 1, abort_flag);
+                    if (lane == 0) mbar_expect_tx(&full_w[ws], G_TILE_M * F::W_ROW_BYTES);
+                    __syncwarp();
+                    if (active && !*abort_flag) {
+                        bulk_g2s(smem_w + ws * W_STAGE_BYTES + lane * HT_BYTES, src + (size_t)blk * HT_BYTES, HT_BYTES, &full_w[ws]);
+                        const bool same = blk + 2 < tc.kb1;
+                        if (same || have_n)
+                            bulk_prefetch_l2(same ? src + (size_t)(blk + 2) * HT_BYTES : src_n + (size_t)(tcn.kb0 + blk + 2 - tc.kb1) * HT_BYTES,
+                                             HT_BYTES);
+                    }
+                    __syncwarp();
+                }
+                tile += gridDim.x;
+                tc = tcn;
+                src = src_n;
+                have = have_n;
+            }
+        } else if constexpr (F::STAGE_W) {
             uint32_t ab = 0;
             long long tile = blockIdx.x;
             TileCoord tc, tcn;
@@ -848,18 +890,18 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                         uint8_t* dst = smem_w + ws * W_STAGE_BYTES;
                         mbar_expect_tx(&full_w[ws], G_TILE_M * F::W_ROW_BYTES);
                         if (GATE_UP) {
-                            tma_load_2d(dst, m0, blk * (F::W_ROW_BYTES / F::W_MAP_ELEM), y0, &full_w[ws]);
-                            tma_load_2d(dst + HALF, m0 + 1, blk * (F::W_ROW_BYTES / F::W_MAP_ELEM), y0, &full_w[ws]);
+                            tma_load_2d(dst, m0, blk * F::W_ROW_BYTES, y0, &full_w[ws]);
+                            tma_load_2d(dst + HALF, m0 + 1, blk * F::W_ROW_BYTES, y0, &full_w[ws]);
                         } else {
-                            tma_load_2d(dst, m0, blk * (F::W_ROW_BYTES / F::W_MAP_ELEM), y0, &full_w[ws]);
-                            tma_load_2d(dst + HALF, m0, blk * (F::W_ROW_BYTES / F::W_MAP_ELEM), y0 + 64, &full_w[ws]);
+                            tma_load_2d(dst, m0, blk * F::W_ROW_BYTES, y0, &full_w[ws]);
+                            tma_load_2d(dst + HALF, m0, blk * F::W_ROW_BYTES, y0 + 64, &full_w[ws]);
                         }
                         // two blocks ahead, possibly in the next tile
                         const bool same = blk + 2 < tc.kb1;
                         if (same || have_n) {
                             const CUtensorMap* mp = same ? m0 : P.wmaps + 2 * tcn.e;
                             const int yp = same ? y0 : (GATE_UP ? tcn.mt * 64 : tcn.mt * 128);
-                            const int xp = (same ? blk + 2 : tcn.kb0 + blk + 2 - tc.kb1) * (F::W_ROW_BYTES / F::W_MAP_ELEM);
+                            const int xp = (same ? blk + 2 : tcn.kb0 + blk + 2 - tc.kb1) * F::W_ROW_BYTES;
                             tma_prefetch_2d(mp, xp, yp);
                             tma_prefetch_2d(GATE_UP ? mp + 1 : mp, xp, GATE_UP ? yp : yp + 64);
                         }
@@ -1014,17 +1056,15 @@ bool make_map_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dt, int
 }
 
 // byte matrix [rows, row_bytes] -> boxes of [box_rows x box_bytes], no swizzle
-bool make_map_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_bytes, uint32_t box_rows,
-                    int elem = 1) {
+bool make_map_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes, uint32_t box_bytes, uint32_t box_rows) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
-    const cuuint64_t dims[2] = {row_bytes / elem, rows};  // elem = 4: counted in 32-bit words (a box dimension holds at most 256 elements)
+    const cuuint64_t dims[2] = {row_bytes, rows};
     const cuuint64_t strides[1] = {row_bytes};
-    const cuuint32_t box[2] = {box_bytes / elem, box_rows};
+    const cuuint32_t box[2] = {box_bytes, box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    return fn(map, elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 int g_gemm_sms = -1;
@@ -1056,13 +1096,12 @@ cudaError_t launch_gemm_kernel(cudaStream_t st, const GemmParams& G, const CUten
 
 }  // namespace
 
-size_t prepacked_q80_bytes(int64_t n_rows, int k) { return (size_t)n_rows * (size_t)((k + 255) / 256) * GemmQ80::W_ROW_BYTES; }
+size_t prepacked_q80_bytes(int64_t n_rows, int k) { return (size_t)((n_rows + 7) / 8) * (size_t)((k + 255) / 256) * 2 * Q80_HTB_BYTES; }
 cudaError_t launch_prepack_q80(cudaStream_t st, const void* raw, int64_t n_rows, int k, void* dst) {
-    const int k_pad = (k + 255) / 256 * 256;
-    const int64_t units = n_rows * (k_pad / 256);
-    if (units == 0) return cudaSuccess;
-    prepack_q80_kernel<<<(unsigned)((units + 7) / 8), 256, 0, st>>>(static_cast<const uint8_t*>(raw), n_rows, k, k_pad,
-                                                                 static_cast<uint8_t*>(dst));
+    const int kb = 2 * ((k + 255) / 256);
+    const int64_t grid = (n_rows + 7) / 8 * kb;
+    if (grid == 0) return cudaSuccess;
+    prepack_q80_kernel<<<(unsigned)grid, 288, 0, st>>>(static_cast<const uint8_t*>(raw), n_rows, k, kb, static_cast<uint8_t*>(dst));
     return cudaGetLastError();
 }
 
@@ -1128,16 +1167,15 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     // byte-matrix tensor maps of the raw weight blocks (Q4_K): [n_rows, kb * 144] with boxes of 64 rows x one block,
     // written to the head of the scratch on the stream before the kernel
     CUtensorMap* wmaps_dev = reinterpret_cast<CUtensorMap*>(reinterpret_cast<uint8_t*>(d8t) + align_up((size_t)kb * p_pad * 4, 256));
-    if (dtype == CANDLE_GGML_Q4K || q80) {
-        const int rec = q80 ? GemmQ80::W_ROW_BYTES : Q4K_BYTES, elem = q80 ? GemmQ80::W_MAP_ELEM : 1;
-        const uint64_t n_rows = (uint64_t)N, rb = (uint64_t)kb * rec;
+    if (dtype == CANDLE_GGML_Q4K) {
+        const uint64_t n_rows = (uint64_t)N, rb = (uint64_t)kb * Q4K_BYTES;
         for (int m0 = 0; m0 < 2 * E; m0 += MAPS_PER_CHUNK) {
             MapChunk chunk;
             const int n_maps = std::min(MAPS_PER_CHUNK, 2 * E - m0);
             for (int i = 0; i < n_maps; ++i) {
                 const int e2 = (m0 + i) >> 1;
                 const uint8_t* wp = ((m0 + i) & 1) && gate_up ? wb.p[e2] : wa.p[e2];
-                if (!make_map_bytes(&chunk.m[i], wp, n_rows, rb, rec, 64, elem)) return cudaErrorNotSupported;
+                if (!make_map_bytes(&chunk.m[i], wp, n_rows, rb, Q4K_BYTES, 64)) return cudaErrorNotSupported;
             }
             for (int i = n_maps; i < MAPS_PER_CHUNK; ++i) chunk.m[i] = chunk.m[0];
             e = launch_k(write_maps_kernel, dim3(1), dim3(128), 0, st, chunk, wmaps_dev + m0, n_maps);
