@@ -27,6 +27,7 @@ inline int64_t gemm_min_rows() { return tuning_get(TUNE_GEMM_MIN_ROWS); }
 // expert with a row more than expected took a second, almost empty tile.)  A single-device forward only knows the
 // bound T.
 constexpr int64_t GEMM_MIN_ROWS_EXACT = 32;
+constexpr int64_t QMM_DIRECT_MAX_ROWS = 64;  // the dense Q8_0 product over its repacked copy: decode kernels up to here
 constexpr int64_t QMM_GEMM_MIN_ROWS = 48;  // the dense product: one matrix, rows known exactly
 // Decode-sized batches may split K finely (more parallel items, smaller resident activations);
 // larger batches get four slots, enough for the streaming form's activation rows to fit.
@@ -276,8 +277,8 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     if (total_rows_hint <= 0) total_rows_hint = P;
     const int E = w->n_experts, d = w->d_model, ff = w->d_ff;
     const bool large = b.gemm && max_rows > (rows_exact ? GEMM_MIN_ROWS_EXACT : gemm_min_rows()) && gemm_enabled();
-    const bool use_prepacked = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked && w->dtype_w13 != CANDLE_GGML_Q8_0 &&
-                               w->dtype_w2 != CANDLE_GGML_Q8_0 && max_rows <= std::max<int64_t>(gemm_min_rows(), 64) && !large;
+    const bool use_prepacked = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked &&
+                               max_rows <= std::max<int64_t>(gemm_min_rows(), 64) && !large;
     bool gate_done = false, down_done = false;
     *eo_splits = 1;
     ExpertPtrs q1, q3, q2;
@@ -411,7 +412,8 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     // one token: the router kernel has written the dispatch itself
     if (T > 1) CM_TRY(rc(launch_permute(st, ws.topk_ids, T, k, E, ws.counts, ws.offsets, ws.perm_token, ws.pair_pos, ws.perm_scratch)));
     mark(st, 1);
-    if (!fuse_q) CM_TRY(rc(launch_quantize_act(st, x, T, d, w->dtype_w13, ws.xq, ws.xs, ws.xb)));
+    // (that pass also writes the offsets of the shared expert's one group)
+    if (!fuse_q) CM_TRY(rc(launch_quantize_act(st, x, T, d, w->dtype_w13, ws.xq, ws.xs, ws.xb, nullptr, ws.sh_offsets)));
     mark(st, 2);
     // a token selects an expert at most once: no expert sees more than T rows
     int eo_splits = 1, so_splits = 1;
@@ -423,24 +425,29 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     const float* shared_out = nullptr;
     if (w->d_ff_shared > 0) {
         const int fs = w->d_ff_shared;
-        CM_TRY(rc(launch_single_group(st, ws.sh_offsets, (uint32_t)T)));
+        if (fuse_q) CM_TRY(rc(launch_single_group(st, ws.sh_offsets, (uint32_t)T)));
         ExpertPtrs s1{}, s3{}, s2{};
         s1.p[0] = static_cast<const uint8_t*>(w->shared_w1);
         s3.p[0] = static_cast<const uint8_t*>(w->shared_w3);
         s2.p[0] = static_cast<const uint8_t*>(w->shared_w2);
         if (ws.sxq != ws.xq)
             CM_TRY(rc(launch_quantize_act(st, x, T, d, w->dtype_shared13, ws.sxq, ws.sxs, ws.sxb)));
-        // large batches over repacked Q8_0 copies: the tensor-core GEMM with one group holding every row
-        const bool sh_gemm = ws.gemm && T > gemm_min_rows() && gemm_enabled() && w->dtype_shared13 == CANDLE_GGML_Q8_0 &&
-                             w->dtype_shared2 == CANDLE_GGML_Q8_0 && w->shared_w1_prepacked && w->shared_w3_prepacked &&
-                             w->shared_w2_prepacked;
+        // over repacked Q8_0 copies: the decode kernels, and for large batches the tensor-core GEMM, with one group
+        // holding every row
+        const bool sh_packed = w->dtype_shared13 == CANDLE_GGML_Q8_0 && w->dtype_shared2 == CANDLE_GGML_Q8_0 &&
+                               w->shared_w1_prepacked && w->shared_w3_prepacked && w->shared_w2_prepacked;
+        const bool sh_gemm = sh_packed && ws.gemm && T > gemm_min_rows() && gemm_enabled();
+        const bool sh_direct = sh_packed && !sh_gemm && T <= std::max<int64_t>(gemm_min_rows(), 64);
         bool sh_done = false;
-        if (sh_gemm) {
+        if (sh_gemm || sh_direct) {
             ExpertPtrs r1{}, r3{};
             r1.p[0] = static_cast<const uint8_t*>(w->shared_w1_prepacked);
             r3.p[0] = static_cast<const uint8_t*>(w->shared_w3_prepacked);
-            const cudaError_t ce = launch_expert_gemm(st, true, r1, r3, CANDLE_GGML_Q8_0, true, 1, d, fs, ws.sh_offsets, nullptr, T, T,
-                                                      ws.sxq, ws.sxs, ws.sxb, ws.shidden, ws.gemm);
+            const cudaError_t ce =
+                sh_gemm ? launch_expert_gemm(st, true, r1, r3, CANDLE_GGML_Q8_0, true, 1, d, fs, ws.sh_offsets, nullptr, T, T, ws.sxq,
+                                             ws.sxs, ws.sxb, ws.shidden, ws.gemm)
+                        : launch_expert_direct(st, true, r1, r3, CANDLE_GGML_Q8_0, 1, d, fs, ws.sh_offsets, nullptr, T, ws.sxq, ws.sxs,
+                                               ws.sxb, ws.shidden, nullptr, 0, 1, 0, T);
             if (ce == cudaSuccess)
                 sh_done = true;
             else if (ce != cudaErrorNotSupported)
@@ -451,12 +458,14 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
                                              ws.sxs, ws.sxb, ws.shidden)));
         CM_TRY(rc(launch_quantize_act(st, ws.shidden, T, fs, w->dtype_shared2, ws.shq, ws.shs, ws.shb)));
         sh_done = false;
-        if (sh_gemm) {
+        if (sh_gemm || sh_direct) {
             ExpertPtrs r2{};
             r2.p[0] = static_cast<const uint8_t*>(w->shared_w2_prepacked);
-            const cudaError_t ce = launch_expert_gemm(st, false, r2, r2, CANDLE_GGML_Q8_0, true, 1, fs, d, ws.sh_offsets, nullptr, T, T,
-                                                      ws.shq, ws.shs, ws.shb, ws.so, ws.gemm, k_split_slots(T), &so_splits,
-                                                      T * (int64_t)d);
+            const cudaError_t ce =
+                sh_gemm ? launch_expert_gemm(st, false, r2, r2, CANDLE_GGML_Q8_0, true, 1, fs, d, ws.sh_offsets, nullptr, T, T, ws.shq,
+                                             ws.shs, ws.shb, ws.so, ws.gemm, k_split_slots(T), &so_splits, T * (int64_t)d)
+                        : launch_expert_direct(st, false, r2, r2, CANDLE_GGML_Q8_0, 1, fs, d, ws.sh_offsets, nullptr, T, ws.shq,
+                                               ws.shs, ws.shb, ws.so, &so_splits, T * (int64_t)d, k_split_slots(T), 1, T);
             if (ce == cudaSuccess)
                 sh_done = true;
             else if (ce != cudaErrorNotSupported)
@@ -845,9 +854,19 @@ int candle_moe_qmatmul(void* stream, const void* w, const void* w_prepacked, int
     int splits = 1;
     bool done = false;
     const bool large = ws.gemm && gemm_enabled();
-    // The decode kernels over the repacked copy are not used here: with a single group their tiles are too few and
+    // The decode kernels over the repacked copy of a k-quant are not used here: with a single group their tiles are too few and
     // too short, and the streaming form over the GGUF blocks is faster (measured, [4096, 4096] Q4_K / [32000, 4096]
     // Q6_K: 1 row 10.8 / 44.5 us against 17.2 / 46.2; 8 rows 13.5 / 48.6 against 17.7 / 60.1).
+    if (dtype == CANDLE_GGML_Q8_0 && w_prepacked && rows <= QMM_DIRECT_MAX_ROWS) {
+        const cudaError_t ce = launch_expert_direct(st, false, pp, pp, dtype, 1, k, n, ws.offsets, nullptr, rows, ws.xq, ws.xs, ws.xb,
+                                                    dst, &splits, stride, ws.slots, 1, rows);
+        if (ce == cudaSuccess)
+            done = true;
+        else if (ce != cudaErrorNotSupported)
+            return (int)ce;
+        else
+            splits = 1;
+    }
     if (!done && large) {
         const bool rp = dtype == CANDLE_GGML_Q6K && w_prepacked;
         const cudaError_t ce = launch_expert_gemm(st, false, rp ? pp : pw, rp ? pp : pw, dtype, rp, 1, k, n, ws.offsets, nullptr,

@@ -53,6 +53,8 @@ struct ActArgs {
 // ------------------------------------------------------------------------------------------------
 struct DirQ4K {
     static constexpr int HTB = Q4K_HTB_BYTES;
+    static constexpr int BLK = 256, SC_PER_BLOCK = 1;  // elements of a K-block, activation scales per K-block
+    static constexpr int TWO_TILES_COST = 11;          // issued instructions of a K-block for two position tiles, one being 8
     static constexpr int BS_PER_BLOCK = 8;
     __device__ static __forceinline__ int bs_value(const int16_t* bs16, int i) { return (int)bs16[2 * i] + (int)bs16[2 * i + 1]; }
     __device__ static __forceinline__ void bs_split(int v, uint8_t& hi, uint8_t& lo) {
@@ -143,6 +145,7 @@ struct DirQ4K {
 // ------------------------------------------------------------------------------------------------
 struct DirQ6K {
     static constexpr int HTB = Q6K_HTB_BYTES;
+    static constexpr int BLK = 256, SC_PER_BLOCK = 1, TWO_TILES_COST = 11;
     static constexpr int BS_PER_BLOCK = 16;
     __device__ static __forceinline__ int bs_value(const int16_t* bs16, int i) { return (int)bs16[i]; }
     __device__ static __forceinline__ void bs_split(int v, uint8_t& hi, uint8_t& lo) {
@@ -250,6 +253,66 @@ struct DirQ6K {
     }
 };
 
+// ------------------------------------------------------------------------------------------------
+// Q8_0 (repacked by prepack_q80_kernel: 8 rows x 128 elements, 1088 bytes).  A K-block here is 128 elements = four Q8_0
+// blocks, each one m16n8k32 MMA whose integer result is scaled by d_w * d_a in f32 like vec_dot (k_quants.rs:650-668).
+// Rows are zero-padded past K; the walk ends with the last K-block that holds elements.
+// HBM-bound: a K-block of a 16-row tile is 2176 bytes and about 60 issued instructions per position tile, well inside the
+// 370 issue slots its bytes take at the copy peak.  128 elements rather than 256 keep a four-deep ring of every warp beside
+// the activations (139 KB against 278).  Measured on 60 experts [1408, 2048], top-4, shared expert of 5632, 16 rows: the
+// block 502 -> 161 us (the row-per-warp kernels over the GGUF bytes before; 404 MB).
+struct DirQ80 {
+    static constexpr int HTB = Q80_HTB_BYTES;
+    static constexpr int BLK = 128, SC_PER_BLOCK = 4;
+    static constexpr int TWO_TILES_COST = 9;  // 17 bytes per weight pair and one MMA per block: the copies bound it either way
+    static constexpr int BS_PER_BLOCK = 0;  // no offset term: no block sums
+    struct Frag {
+        uint4 qa[2], qb[2];  // per 64 elements: {block 0 k 0-15, k 16-31, block 1 k 0-15, k 16-31} of rows g and g + 8
+        uint2 dA, dB;        // four f16 scales each
+    };
+    __device__ static __forceinline__ void load(Frag& F, uint32_t hta, int lane) {
+        const int g = lane >> 2;
+        const uint32_t bq = hta + 16 * chunk_pos(g, lane & 3), bd = hta + 8 * g;
+        F.qa[0] = lds128_o<0>(bq);
+        F.qa[1] = lds128_o<512>(bq);
+        F.qb[0] = lds128_o<HTB>(bq);
+        F.qb[1] = lds128_o<HTB + 512>(bq);
+        F.dA = lds64_o<1024>(bd);
+        F.dB = lds64_o<HTB + 1024>(bd);
+    }
+    template <int NT, int NTL>
+    __device__ static __forceinline__ void compute(const Frag& F, const ActArgs& A, int, uint64_t (&fp)[NT][2]) {
+        const uint32_t dA[2] = {F.dA.x, F.dA.y}, dB[2] = {F.dB.x, F.dB.y};
+        static_for<2>([&](auto Uc) {
+            constexpr int u = decltype(Uc)::value;
+            uint64_t wA[2], wB[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float a = half_bits_to_float((uint16_t)(i ? dA[u] >> 16 : dA[u] & 0xffffu));
+                const float b = half_bits_to_float((uint16_t)(i ? dB[u] >> 16 : dB[u] & 0xffffu));
+                wA[i] = f32x2_pack(a, a);
+                wB[i] = f32x2_pack(b, b);
+            }
+            const uint32_t a0[4] = {F.qa[u].x, F.qb[u].x, F.qa[u].y, F.qb[u].y};
+            const uint32_t a1[4] = {F.qa[u].z, F.qb[u].z, F.qa[u].w, F.qb[u].w};
+            static_for<NTL>([&](auto Nc) {
+                constexpr int nt = decltype(Nc)::value;
+                uint32_t b[4];
+                ldmatrix_x4_o<64 * u>(b, A.act_blk + nt * A.act_stride8);
+                int p[4], q[4];
+                mma_s8_k32_z(p, a0, b[0], b[1]);
+                mma_s8_k32_z(q, a1, b[2], b[3]);
+                const uint2 s0 = lds64_o<(2 * u) * 32 * NT + 32 * nt>(A.sc_blk), s1 = lds64_o<(2 * u + 1) * 32 * NT + 32 * nt>(A.sc_blk);
+                const uint64_t d0 = f32x2_pack_bits(s0.x, s0.y), d1 = f32x2_pack_bits(s1.x, s1.y);
+                fp[nt][0] = f32x2_fma(f32x2_mul(d0, wA[0]), f32x2_pack((float)p[0], (float)p[1]), fp[nt][0]);
+                fp[nt][1] = f32x2_fma(f32x2_mul(d0, wB[0]), f32x2_pack((float)p[2], (float)p[3]), fp[nt][1]);
+                fp[nt][0] = f32x2_fma(f32x2_mul(d1, wA[1]), f32x2_pack((float)q[0], (float)q[1]), fp[nt][0]);
+                fp[nt][1] = f32x2_fma(f32x2_mul(d1, wB[1]), f32x2_pack((float)q[2], (float)q[3]), fp[nt][1]);
+            });
+        });
+    }
+};
+
 struct DirectParams {
     ExpertPtrs wa, wb;  // prepacked matrices
     const uint32_t* offsets;
@@ -260,6 +323,7 @@ struct DirectParams {
     float* out;
     int64_t out_split_stride;
     int E, K, N, kb, splits, MT;
+    int kb_stride;      // K-blocks a half-tile is stored with (Q8_0 copies are padded)
     int blk_start[9];  // split s covers blocks [blk_start[s], blk_start[s + 1])
     int act_stride;
     uint32_t off_act, off_scale, off_bs, off_ring, off_part;
@@ -267,11 +331,11 @@ struct DirectParams {
 
 // DEPTH = ring slots per warp (DEPTH - 1 blocks in flight while one is multiplied)
 template <class F, bool GATE_UP, int NT, int DEPTH>
-// The one-position-tile Q4_K kernels are held to 96 registers (a bound of 608 threads; they are launched with 512,
-// and Q6_K would spill): the
+// The one-position-tile Q4_K and Q8_0 kernels are held to 96 registers (a bound of 608 threads; they are launched with
+// 512, and Q6_K would spill): the
 // registers a CTA leaves free let the CTAs of the next kernel on the stream become resident and run their
 // prologue under programmatic dependent launch while this one drains.
-__global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB_BYTES ? 608 : DIRECT_THREADS, 1) expert_direct_kernel(const __grid_constant__ DirectParams P) {
+__global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIRECT_THREADS, 1) expert_direct_kernel(const __grid_constant__ DirectParams P) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint32_t s_offs[CANDLE_MOE_MAX_EXPERTS + 1];
     __shared__ int s_rows[16];
@@ -293,6 +357,7 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB_BYTES ? 608 : DIR
     const uint32_t act_lane = smem_u32(act) + (lane & 7) * P.act_stride + 16 * (lane >> 3);
     const uint32_t sc_lane = smem_u32(act_scale) + 8 * (lane & 3);
     const uint32_t bs_lane = smem_u32(bs) + (lane >> 2) * BSB + (BSB == 8 ? 4 * (lane & 1) : 4 * (lane & 3));
+    constexpr int SCB = F::SC_PER_BLOCK, BLK = F::BLK;
     constexpr int SLOT_BYTES = 2 * F::HTB;       // both half-tile blocks of one K-block
     constexpr int VEC_PER_HT = F::HTB / 16;      // 16-byte vectors per half-tile block
     const uint32_t ring = smem_u32(smem + P.off_ring) + (uint32_t)warp * (DEPTH * SLOT_BYTES);
@@ -300,9 +365,9 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB_BYTES ? 608 : DIR
 
     // Cost-balanced contiguous share of the (token group, split, tile) sequence.  Cost = blocks streamed, weighted
     // by what a block costs to multiply: a group of more than eight rows takes two position tiles per block, which
-    // is 11 : 8 in issued instructions against a group of up to eight.
+    // is TWO_TILES_COST : 8 against a group of up to eight.
     const int tiles = P.N / TILE_N;
-    auto group_weight = [](uint32_t rows) { return (NT > 1 && rows > 8) ? 11 : 8; };
+    auto group_weight = [](uint32_t rows) { return (NT > 1 && rows > 8) ? F::TWO_TILES_COST : 8; };
     long long ctot = 0;
     for (int i = 0; i < P.E; ++i) {
         const uint32_t cnt = s_offs[i + 1] - s_offs[i];
@@ -310,7 +375,7 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB_BYTES ? 608 : DIR
     }
     const long long lo = ctot * blockIdx.x / gridDim.x, hi = ctot * (blockIdx.x + 1) / gridDim.x;
     if (lo >= hi) return;
-    const size_t ht_stride = (size_t)P.kb * F::HTB;  // bytes of one half-tile over the whole K
+    const size_t ht_stride = (size_t)P.kb_stride * F::HTB;  // bytes of one half-tile over the whole K
 
     long long acc = 0;  // cost of the groups before the current one
     for (int e = 0; e < P.E && acc < hi; ++e) {
@@ -343,30 +408,36 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB_BYTES ? 608 : DIR
             }
             __syncthreads();
             {
-                const int vec_per_row = nblk * 16;
+                const int vec_per_row = nblk * (BLK / 16), k0 = blk0 * BLK;
 #pragma unroll 4
                 for (int idx = tid; idx < MT * vec_per_row; idx += DIRECT_THREADS) {
                     const int j = idx / vec_per_row, v = idx - j * vec_per_row;
                     const int row = s_rows[j];
                     int4 val = make_int4(0, 0, 0, 0);
-                    if (row >= 0) val = *reinterpret_cast<const int4*>(P.aq + (int64_t)row * P.K + (int64_t)blk0 * 256 + 16 * v);
+                    // (Q8_0: K is a multiple of 32 and may end inside the last K-block)
+                    if (row >= 0 && (BLK == 256 || k0 + 16 * v < P.K))
+                        val = *reinterpret_cast<const int4*>(P.aq + (int64_t)row * P.K + k0 + 16 * v);
                     *reinterpret_cast<int4*>(act + j * P.act_stride + 16 * v) = val;
                 }
-                for (int idx = tid; idx < MT * nblk; idx += DIRECT_THREADS) {
-                    const int j = idx / nblk, bb = idx - j * nblk;
+                const int sc_per_row = nblk * SCB, sc_k = SCB == 1 ? P.kb : P.K / 32;  // scales per row: in this range, in all
+                for (int idx = tid; idx < MT * sc_per_row; idx += DIRECT_THREADS) {
+                    const int j = idx / sc_per_row, bb = idx - j * sc_per_row;
                     const int row = s_rows[j];
-                    act_scale[bb * MT + j] = row >= 0 ? P.ascale[(int64_t)row * P.kb + blk0 + bb] : 0.f;
+                    const bool in = row >= 0 && (SCB == 1 || blk0 * SCB + bb < sc_k);
+                    act_scale[bb * MT + j] = in ? P.ascale[(int64_t)row * sc_k + blk0 * SCB + bb] : 0.f;
                 }
-                const int per_row = nblk * F::BS_PER_BLOCK;
-                for (int idx = tid; idx < MT * per_row; idx += DIRECT_THREADS) {
-                    const int j = idx / per_row, bb = idx - j * per_row;
-                    const int row = s_rows[j];
-                    const int v = row >= 0 ? F::bs_value(P.absum + (int64_t)row * (P.K / 16) + blk0 * 16, bb) : 0;
-                    uint8_t h8, l8;
-                    F::bs_split(v, h8, l8);
-                    const int blk = bb / BSB, i = bb - blk * BSB;
-                    bs[((2 * blk) * MT + j) * BSB + i] = h8;
-                    bs[((2 * blk + 1) * MT + j) * BSB + i] = l8;
+                if constexpr (BSB > 0) {
+                    const int per_row = nblk * F::BS_PER_BLOCK;
+                    for (int idx = tid; idx < MT * per_row; idx += DIRECT_THREADS) {
+                        const int j = idx / per_row, bb = idx - j * per_row;
+                        const int row = s_rows[j];
+                        const int v = row >= 0 ? F::bs_value(P.absum + (int64_t)row * (P.K / 16) + blk0 * 16, bb) : 0;
+                        uint8_t h8, l8;
+                        F::bs_split(v, h8, l8);
+                        const int blk = bb / BSB, i = bb - blk * BSB;
+                        bs[((2 * blk) * MT + j) * BSB + i] = h8;
+                        bs[((2 * blk + 1) * MT + j) * BSB + i] = l8;
+                    }
                 }
             }
             __syncthreads();
@@ -491,8 +562,8 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB == Q4K_HTB_BYTES ? 608 : DIR
                     const uint32_t slot = ring + (uint32_t)(j % DEPTH) * SLOT_BYTES;
                     F::load(cur, slot, lane);
                     const int bk = b0 + j;
-                    A.act_blk = act_lane + bk * 256;
-                    A.sc_blk = sc_lane + bk * (4 * MT);
+                    A.act_blk = act_lane + bk * BLK;
+                    A.sc_blk = sc_lane + bk * (4 * MT * SCB);
                     A.bs_blk = bs_lane + bk * (2 * MT * BSB);
                     if (NT == 1 || ntiles == 1)
                         F::template compute<NT, 1>(cur, A, lane, fp);
@@ -623,9 +694,10 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
                                  int64_t max_rows_per_expert, const int8_t* aq, const float* ascale,
                                  const int16_t* absum, float* out, int* n_splits_out, int64_t split_stride,
                                  int max_splits, int max_active_experts, int64_t total_rows) {
-    if (dtype != CANDLE_GGML_Q4K && dtype != CANDLE_GGML_Q6K) return cudaErrorNotSupported;
+    const bool q80 = dtype == CANDLE_GGML_Q8_0;
+    if (dtype != CANDLE_GGML_Q4K && dtype != CANDLE_GGML_Q6K && !q80) return cudaErrorNotSupported;
     const int tile_n = gate_up ? 8 : 16;
-    if (N % tile_n != 0 || K % 256 != 0) return cudaErrorNotSupported;
+    if (N % tile_n != 0 || K % (q80 ? 32 : 256) != 0) return cudaErrorNotSupported;
     if (g_dir_max_smem < 0) {
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
@@ -635,7 +707,7 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
         e = cudaDeviceGetAttribute(&g_dir_sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
     }
-    const int kb = K / 256;
+    const int blk = q80 ? DirQ80::BLK : 256, kb = (K + blk - 1) / blk;
     // One position tile (8 rows per group) or two (16).  An expert with more rows than a group holds is walked once
     // per group.  When the caller's bound allows more than 8 rows but the experts hold about 3 or fewer on average
     // (total_rows known), practically every expert fits one 8-row group and the one-tile kernel is the cheaper
@@ -644,7 +716,7 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
     const bool few_rows = total_rows > 0 && total_rows <= 3 * (int64_t)E;
     const int NT = max_rows_per_expert <= 8 || few_rows ? 1 : 2;
     const int MT = 8 * NT;
-    const int bs_per_block = dtype == CANDLE_GGML_Q4K ? 8 : 16;
+    const int bs_per_block = q80 ? 0 : (dtype == CANDLE_GGML_Q4K ? 8 : 16);
     DirectParams P{};
     P.wa = wa;
     P.wb = wb;
@@ -668,13 +740,13 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
             off += bytes;
             return o;
         };
-        P.act_stride = ks_blocks * 256 + 16;
+        P.act_stride = ks_blocks * blk + 16;
         P.off_act = take((uint32_t)MT * P.act_stride);
-        P.off_scale = take((uint32_t)MT * ks_blocks * 4);
+        P.off_scale = take((uint32_t)MT * ks_blocks * 4 * (q80 ? DirQ80::SC_PER_BLOCK : 1));
         P.off_bs = take((uint32_t)2 * MT * ks_blocks * bs_per_block);
-        // per-warp rings of DEPTH K-blocks: 4 slots for Q4_K (2368 B each), 3 for Q6_K (3360 B each)
-        const int depth = dtype == CANDLE_GGML_Q4K ? 4 : 3;
-        const uint32_t slot_bytes = 2u * (dtype == CANDLE_GGML_Q4K ? Q4K_HTB_BYTES : Q6K_HTB_BYTES);
+        // per-warp rings of DEPTH K-blocks: 4 slots for Q4_K (2368 B each) and Q8_0 (2176 B), 3 for Q6_K (3360 B)
+        const int depth = dtype == CANDLE_GGML_Q6K ? 3 : 4;
+        const uint32_t slot_bytes = 2u * (q80 ? Q80_HTB_BYTES : (dtype == CANDLE_GGML_Q4K ? Q4K_HTB_BYTES : Q6K_HTB_BYTES));
         P.off_ring = take((uint32_t)DIRECT_WARPS * depth * slot_bytes);
         P.off_part = NT == 1 ? take((uint32_t)DIRECT_WARPS * 512u) : 0u;
         if ((int)off > g_dir_max_smem - 1024) continue;
@@ -697,8 +769,13 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
         P.K = K;
         P.N = N;
         P.kb = kb;
+        P.kb_stride = q80 ? (K + 255) / 256 * 2 : kb;
         P.MT = MT;
         if (n_splits_out) *n_splits_out = splits;
+        if (q80) {
+            if (gate_up) return NT == 1 ? launch_dir<DirQ80, true, 1, 4>(st, P, off) : launch_dir<DirQ80, true, 2, 4>(st, P, off);
+            return NT == 1 ? launch_dir<DirQ80, false, 1, 4>(st, P, off) : launch_dir<DirQ80, false, 2, 4>(st, P, off);
+        }
         if (dtype == CANDLE_GGML_Q4K) {
             if (gate_up) return NT == 1 ? launch_dir<DirQ4K, true, 1, 4>(st, P, off) : launch_dir<DirQ4K, true, 2, 4>(st, P, off);
             return NT == 1 ? launch_dir<DirQ4K, false, 1, 4>(st, P, off) : launch_dir<DirQ4K, false, 2, 4>(st, P, off);
