@@ -859,7 +859,7 @@ int candle_moe_qmatmul(void* stream, const void* w, const void* w_prepacked, int
     // Q6_K: 1 row 10.8 / 44.5 us against 17.2 / 46.2; 8 rows 13.5 / 48.6 against 17.7 / 60.1).
     if (dtype == CANDLE_GGML_Q8_0 && w_prepacked && rows <= QMM_DIRECT_MAX_ROWS) {
         const cudaError_t ce = launch_expert_direct(st, false, pp, pp, dtype, 1, k, n, ws.offsets, nullptr, rows, ws.xq, ws.xs, ws.xb,
-                                                    dst, &splits, stride, ws.slots, 1, rows);
+                                                    dst, &splits, stride, ws.slots, 1, rows, out);
         if (ce == cudaSuccess)
             done = true;
         else if (ce != cudaErrorNotSupported)
@@ -870,7 +870,7 @@ int candle_moe_qmatmul(void* stream, const void* w, const void* w_prepacked, int
     if (!done && large) {
         const bool rp = dtype == CANDLE_GGML_Q6K && w_prepacked;
         const cudaError_t ce = launch_expert_gemm(st, false, rp ? pp : pw, rp ? pp : pw, dtype, rp, 1, k, n, ws.offsets, nullptr,
-                                                  rows, rows, ws.xq, ws.xs, ws.xb, dst, ws.gemm, ws.slots, &splits, stride);
+                                                  rows, rows, ws.xq, ws.xs, ws.xb, dst, ws.gemm, ws.slots, &splits, stride, out);
         if (ce == cudaSuccess)
             done = true;
         else if (ce != cudaErrorNotSupported)
@@ -880,8 +880,10 @@ int candle_moe_qmatmul(void* stream, const void* w, const void* w_prepacked, int
     }
     if (!done)
         CM_TRY(rc(launch_grouped_down(st, pw, dtype, 1, n, k, ws.offsets, rows, ws.xq, ws.xs, ws.xb, dst, stride, ws.slots,
-                                      &splits)));
-    if (ws.eo) return rc(launch_ep_scatter(st, ws.eo, splits, stride, nullptr, rows, n, out));
+                                      &splits, out)));
+    // partial sums only when K was split: an unsplit product has written `out` itself (one launch fewer: [6144, 4096] Q4_K,
+    // 1 row 21.1 -> 18.7 us, [32000, 4096] Q6_K, 32 rows 76.5 -> 73.0 us)
+    if (splits > 1) return rc(launch_ep_scatter(st, ws.eo, splits, stride, nullptr, rows, n, out));
     return CANDLE_MOE_OK;
 }
 

@@ -185,10 +185,13 @@ cudaError_t launch_grouped_gate_up(cudaStream_t st, const ExpertPtrs& w1, const 
                                    const int8_t* xq, const float* xs, const int16_t* xb, float* hidden);
 // `max_rows` bounds the rows of any single expert.  `out` may receive up to `max_splits` partial
 // results (K-splits) spaced `split_stride` floats apart; *n_splits says how many were written and
-// the caller (the combine kernel) adds them in split order.
+// the caller (the combine kernel) adds them in split order.  out_whole (may be null; here and in the other launchers):
+// where the result goes instead of `out` when K is not split, so that a caller whose result needs no more than the sum of
+// the partials has nothing left to do.
 cudaError_t launch_grouped_down(cudaStream_t st, const ExpertPtrs& w2, int dtype, int E, int d, int ff,
                                 const uint32_t* offsets, int64_t max_rows, const int8_t* hq, const float* hs,
-                                const int16_t* hb, float* out, int64_t split_stride, int max_splits, int* n_splits);
+                                const int16_t* hb, float* out, int64_t split_stride, int max_splits, int* n_splits,
+                                float* out_whole = nullptr);
 cudaError_t launch_combine(cudaStream_t st, const float* expert_out, int n_splits, int64_t split_stride,
                            const uint32_t* ids, const float* w, const uint32_t* pair_pos, int64_t T, int k, int d,
                            const float* shared_out, int shared_splits, int64_t shared_split_stride, const float* x,
@@ -199,7 +202,7 @@ cudaError_t launch_expert_stream(cudaStream_t st, bool gate_up, const ExpertPtrs
                                  int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of,
                                  int64_t max_rows_per_expert, const int8_t* aq, const float* ascale,
                                  const int16_t* absum, float* out, int* n_splits_out, int64_t split_stride,
-                                 int max_splits);
+                                 int max_splits, float* out_whole = nullptr);
 // prepacked-weight (register-fragment order) form for decode-sized batches
 size_t prepacked_bytes(int dtype, int64_t n_rows, int k);
 cudaError_t launch_prepack(cudaStream_t st, int dtype, const void* raw, int64_t n_rows, int k, void* dst);
@@ -207,7 +210,7 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
                                  int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of,
                                  int64_t max_rows_per_expert, const int8_t* aq, const float* ascale,
                                  const int16_t* absum, float* out, int* n_splits_out, int64_t split_stride,
-                                 int max_splits, int max_active_experts = 0, int64_t total_rows = 0);
+                                 int max_splits, int max_active_experts = 0, int64_t total_rows = 0, float* out_whole = nullptr);
 // large-batch grouped GEMM on tcgen05 / TMEM: Q4_K in GGUF layout (repacked = false), Q6_K in the repacked
 // layout (repacked = true); `scratch` of expert_gemm_scratch_bytes(P, K) bytes
 size_t expert_gemm_scratch_bytes(int64_t P, int K, int parts = 1);  // parts = 2: the exact Q8_0 gate_up operand
@@ -217,7 +220,8 @@ cudaError_t launch_prepack_q80(cudaStream_t st, const void* raw, int64_t n_rows,
 cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int dtype,
                                bool repacked, int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of, int64_t P,
                                int64_t max_rows, const int8_t* aq, const float* ascale, const int16_t* absum, float* out,
-                               void* scratch, int max_splits = 1, int* n_splits_out = nullptr, int64_t split_stride = 0);
+                               void* scratch, int max_splits = 1, int* n_splits_out = nullptr, int64_t split_stride = 0,
+                               float* out_whole = nullptr);
 // Q8_0 grouped products for many rows per expert (expert_q80.cu); cudaErrorNotSupported for other shapes
 cudaError_t launch_expert_q80(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int E, int K, int N,
                               const uint32_t* offsets, const uint32_t* row_of, const int8_t* aq, const float* ascale, float* out);

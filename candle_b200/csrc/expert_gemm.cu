@@ -1119,7 +1119,7 @@ size_t expert_gemm_scratch_bytes(int64_t P, int K, int parts) {
 cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int dtype,
                                bool repacked, int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of, int64_t P,
                                int64_t max_rows, const int8_t* aq, const float* ascale, const int16_t* absum, float* out,
-                               void* scratch, int max_splits, int* n_splits_out, int64_t split_stride) {
+                               void* scratch, int max_splits, int* n_splits_out, int64_t split_stride, float* out_whole) {
     if (n_splits_out) *n_splits_out = 1;
     if (!scratch) return cudaErrorNotSupported;
     int tn = max_rows <= 32 ? 32 : (max_rows <= 64 ? 64 : 128);  // position tile, from the bound / hint on an expert's rows
@@ -1189,7 +1189,6 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     G.wb = wb;
     G.offsets = offsets;
     G.d8t = d8t;
-    G.out = out;
     G.E = E;
     G.K = K;
     G.N = N;
@@ -1208,6 +1207,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         *n_splits_out = ksplit;
     }
     G.ksplit = ksplit;
+    G.out = ksplit == 1 && out_whole ? out_whole : out;
     G.zero = 0;
     G.split_stride = split_stride;
     e = stream_status_ptr(&G.status);

@@ -231,14 +231,16 @@ cudaError_t launch_grouped_gate_up(cudaStream_t st, const ExpertPtrs& w1, const 
 
 cudaError_t launch_grouped_down(cudaStream_t st, const ExpertPtrs& w2, int dtype, int E, int d, int ff,
                                 const uint32_t* offsets, int64_t max_rows, const int8_t* hq, const float* hs,
-                                const int16_t* hb, float* out, int64_t split_stride, int max_splits, int* n_splits) {
+                                const int16_t* hb, float* out, int64_t split_stride, int max_splits, int* n_splits,
+                                float* out_whole) {
     if (n_splits) *n_splits = 1;
     if (!force_rows() && max_rows <= stream_max_rows()) {
         const cudaError_t e = launch_expert_stream(st, false, w2, w2, dtype, E, ff, d, offsets, nullptr, max_rows, hq, hs,
-                                                   hb, out, n_splits, split_stride, max_splits);
+                                                   hb, out, n_splits, split_stride, max_splits, out_whole);
         if (e != cudaErrorNotSupported) return e;
         if (n_splits) *n_splits = 1;
     }
+    if (out_whole) out = out_whole;
     if (!force_rows() && dtype == CANDLE_GGML_Q8_0 && max_rows > Q80_TILE_MIN_ROWS) {
         const cudaError_t e = launch_expert_q80(st, false, w2, w2, E, ff, d, offsets, nullptr, hq, hs, out);
         if (e != cudaErrorNotSupported) return e;

@@ -622,7 +622,7 @@ cudaError_t launch_expert_stream(cudaStream_t st, bool gate_up, const ExpertPtrs
                                  int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of,
                                  int64_t max_rows_per_expert, const int8_t* aq, const float* ascale,
                                  const int16_t* absum, float* out, int* n_splits_out, int64_t split_stride,
-                                 int max_splits) {
+                                 int max_splits, float* out_whole) {
     if (dtype != CANDLE_GGML_Q4K && dtype != CANDLE_GGML_Q6K) return cudaErrorNotSupported;
     const int tile_n = gate_up ? 8 : 16;
     if (N % tile_n != 0 || K % 256 != 0) return cudaErrorNotSupported;
@@ -683,7 +683,7 @@ cudaError_t launch_expert_stream(cudaStream_t st, bool gate_up, const ExpertPtrs
         P.aq = aq;
         P.ascale = ascale;
         P.absum = absum;
-        P.out = out;
+        P.out = splits == 1 && out_whole ? out_whole : out;
         P.out_split_stride = split_stride;
         P.E = E;
         P.K = K;
