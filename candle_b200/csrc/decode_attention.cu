@@ -7,7 +7,11 @@
 // reads its chunk of K once for all the query heads of the group, keeps the scores in shared memory, then reads its
 // chunk of V once; a second small kernel merges the chunks' partial softmax sums (the usual split-softmax algebra:
 // only the order of f32 additions differs from a one-pass softmax).  f32 throughout, like the reference.
+#include <algorithm>
+
 #include "common.cuh"
+#include "stream_common.cuh"
+#include "tc5_common.cuh"
 
 namespace cmoe {
 
@@ -200,6 +204,221 @@ decode_attention_chunk_kernel(const float* __restrict__ q, const float* __restri
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// The same chunk of work for rows of 128 floats and four query heads per kv head, as a pipeline.  HBM-bound: K and V are
+// read once, and what the general kernel above loses is the time in which a CTA has no loads in flight (its barriers
+// between the K pass, the softmax and the V pass).  Here every warp runs a ring of its own of bulk copies -- a tile is 8
+// positions of K and the same 8 of V, 4 KB each, three tiles deep, which continues into the CTA's next chunk -- and an
+// online softmax, so that a warp meets the others only once per chunk.
+//   scores   a lane holds dims 4 l .. 4 l + 3 of the row and of the four queries: 32 partial dot products per tile, which
+//            31 shuffles (halving the number of values a lane carries) turn into ONE score per lane, lane = 4 p + g
+//   softmax  running maximum per head (3 shuffles), one exponential per lane; the weights go back to all lanes through
+//            32 floats of shared memory
+//   V        o[g][dims of the lane] += w[p][g] * v[p][dims], packed pairs
+// Measured, 32 sequences, 8 kv heads, 4096 positions (1.07 GB of cache; 164 us at 6.5 TB/s), as part of a one-layer decode
+// step: step 619 -> 566 us, of which 5 us belong to the projections.
+// ------------------------------------------------------------------------------------------------
+constexpr int RING_WARPS = 4, RING_THREADS = 32 * RING_WARPS, RING_TILE = 8, RING_DEPTH = 3, RING_D = 128, RING_G = 4;
+constexpr int RING_HALF_BYTES = RING_TILE * RING_D * 4, RING_SMEM = RING_WARPS * RING_DEPTH * 2 * RING_HALF_BYTES;
+static_assert(RING_TILE * RING_G == 32, "one score per lane");
+
+__global__ void __launch_bounds__(RING_THREADS, 2)
+decode_attention_ring_kernel(const float* __restrict__ q, const float* __restrict__ kc, const float* __restrict__ vc,
+                             int64_t max_seq, int n_ctx, float scale, int chunk, int n_chunks, int n_units, float* __restrict__ partial,
+                             int* status, uint32_t zero) {
+    extern __shared__ __align__(128) uint8_t ring[];
+    __shared__ uint64_t full[RING_WARPS][RING_DEPTH];
+    __shared__ __align__(16) float s_w[RING_WARPS][32];
+    __shared__ __align__(16) float s_alpha[RING_WARPS][RING_G];
+    __shared__ float s_m[RING_WARPS][RING_G], s_l[RING_WARPS][RING_G];
+    __shared__ __align__(16) float s_o[RING_WARPS][RING_G][RING_D];
+    __shared__ int s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    pdl_trigger();
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int w = 0; w < RING_WARPS; ++w)
+            for (int i = 0; i < RING_DEPTH; ++i) mbar_init(&full[w][i], 1);
+        fence_barrier_init();
+    }
+    __syncthreads();
+    pdl_wait();
+    volatile int* abort_flag = &s_abort;
+    const uint32_t my_ring = smem_u32(ring) + (uint32_t)warp * (RING_DEPTH * 2 * RING_HALF_BYTES);
+    uint8_t* my_ring_p = ring + warp * (RING_DEPTH * 2 * RING_HALF_BYTES);
+
+    // a unit is one chunk of one (sequence, kv head); this warp takes its tiles warp, warp + RING_WARPS, ...
+    struct Cursor {
+        int unit, tile, n_tiles, np;
+        int64_t row0;  // first cache row of the unit
+    };
+    auto open = [&](Cursor& c) {  // the warp's first tile of unit c.unit, or of a later one if it has none there
+        while (c.unit < n_units) {
+            const int ch = c.unit % n_chunks, bk = c.unit / n_chunks;
+            c.np = min(chunk, n_ctx - ch * chunk);
+            c.n_tiles = (c.np + RING_TILE - 1) / RING_TILE;
+            c.row0 = (int64_t)bk * max_seq + (int64_t)ch * chunk;
+            c.tile = warp;
+            if (c.tile < c.n_tiles) return;
+            c.unit += gridDim.x;
+        }
+    };
+    Cursor pf;  // what to request next
+    pf.unit = blockIdx.x;
+    open(pf);
+    uint32_t n_req = 0, n_use = 0;
+    auto request = [&](uint32_t dep) {  // dep: 0, known only once the slot's old contents have arrived in registers
+        if (pf.unit >= n_units) return;
+        const uint32_t s = n_req % RING_DEPTH + dep;
+        if (lane == 0 && !*abort_flag) {
+            const uint32_t bytes = (uint32_t)min(RING_TILE, pf.np - pf.tile * RING_TILE) * (RING_D * 4);
+            const int64_t row = pf.row0 + pf.tile * RING_TILE;
+            mbar_expect_tx(&full[warp][s], 2 * bytes);
+            bulk_g2s(my_ring_p + s * 2 * RING_HALF_BYTES, kc + row * RING_D, bytes, &full[warp][s]);
+            bulk_g2s(my_ring_p + s * 2 * RING_HALF_BYTES + RING_HALF_BYTES, vc + row * RING_D, bytes, &full[warp][s]);
+        }
+        ++n_req;
+        pf.tile += RING_WARPS;
+        if (pf.tile >= pf.n_tiles) {
+            pf.unit += gridDim.x;
+            open(pf);
+        }
+    };
+    for (int i = 0; i < RING_DEPTH; ++i) request(0);
+
+    for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
+        const int ch = unit % n_chunks, bk = unit / n_chunks, np = min(chunk, n_ctx - ch * chunk);
+        const int n_tiles = (np + RING_TILE - 1) / RING_TILE;
+        uint64_t q2[RING_G][2];  // the queries at this lane's dims, as pairs
+#pragma unroll
+        for (int g = 0; g < RING_G; ++g) {
+            const float4 v = reinterpret_cast<const float4*>(q + ((int64_t)bk * RING_G + g) * RING_D)[lane];
+            q2[g][0] = f32x2_pack(v.x, v.y);
+            q2[g][1] = f32x2_pack(v.z, v.w);
+        }
+        uint64_t o2[RING_G][2];
+#pragma unroll
+        for (int g = 0; g < RING_G; ++g) o2[g][0] = o2[g][1] = 0ull;
+        float m = -INFINITY, l = 0.f;  // of head lane & 3: the maximum (same in all its lanes), this lane's share of the sum
+        for (int tile = warp; tile < n_tiles; tile += RING_WARPS, ++n_use) {
+            const uint32_t s = n_use % RING_DEPTH;
+            mbar_wait(&full[warp][s], (n_use / RING_DEPTH) & 1, abort_flag);
+            const int n = min(RING_TILE, np - tile * RING_TILE);
+            const uint32_t kaddr = my_ring + s * 2 * RING_HALF_BYTES + 16 * lane, vaddr = kaddr + RING_HALF_BYTES;
+            float part[32];  // [4 p + g]
+#pragma unroll
+            for (int p = 0; p < RING_TILE; ++p) {
+                const uint4 kv = lds128(kaddr + p * (RING_D * 4));
+                const uint64_t k0 = f32x2_pack_bits(kv.x, kv.y), k1 = f32x2_pack_bits(kv.z, kv.w);
+#pragma unroll
+                for (int g = 0; g < RING_G; ++g) {
+                    float a, b;
+                    f32x2_unpack(f32x2_fma(q2[g][1], k1, f32x2_mul(q2[g][0], k0)), a, b);
+                    part[4 * p + g] = a + b;
+                }
+            }
+            // after step i a lane carries the values whose index agrees with its lane number in the bits done so far
+            static_for<5>([&](auto Ic) {
+                constexpr int half = 16 >> decltype(Ic)::value;
+                const bool up = lane & half;
+#pragma unroll
+                for (int j = 0; j < half; ++j) {
+                    const float give = up ? part[j] : part[j + half], keep = up ? part[j + half] : part[j];
+                    part[j] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+                }
+            });
+            const float score = (lane >> 2) < n ? part[0] * scale : -INFINITY;
+            float mt = score;
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o));
+            const float m_new = fmaxf(m, mt);
+            // a maximum of -inf (every score so far is -inf) must not turn the weights into NaN: exp(-inf - 0) is 0
+            const float m_ref = m_new == -INFINITY ? 0.f : m_new;
+            const float alpha = expf(m - m_ref), w = expf(score - m_ref);
+            m = m_new;
+            l = fmaf(l, alpha, w);
+            s_w[warp][lane] = w;
+            if (lane < RING_G) s_alpha[warp][lane] = alpha;
+            __syncwarp();
+            uint32_t arrived = 0;
+            const float4 al = *reinterpret_cast<const float4*>(s_alpha[warp]);
+            const float a4[4] = {al.x, al.y, al.z, al.w};
+#pragma unroll
+            for (int g = 0; g < RING_G; ++g) {
+                const uint64_t a2 = f32x2_pack(a4[g], a4[g]);
+                o2[g][0] = f32x2_mul(o2[g][0], a2);
+                o2[g][1] = f32x2_mul(o2[g][1], a2);
+            }
+#pragma unroll
+            for (int p = 0; p < RING_TILE; ++p) {
+                if (p < n) {  // rows past the end of the context were not copied
+                    const uint4 vv = lds128(vaddr + p * (RING_D * 4));
+                    arrived |= vv.x;
+                    const uint64_t v0 = f32x2_pack_bits(vv.x, vv.y), v1 = f32x2_pack_bits(vv.z, vv.w);
+                    const float4 wv = *reinterpret_cast<const float4*>(&s_w[warp][4 * p]);
+                    const float w4[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+                    for (int g = 0; g < RING_G; ++g) {
+                        const uint64_t w2 = f32x2_pack(w4[g], w4[g]);
+                        o2[g][0] = f32x2_fma(w2, v0, o2[g][0]);
+                        o2[g][1] = f32x2_fma(w2, v1, o2[g][1]);
+                    }
+                }
+            }
+            // The slot may be refilled when every lane HAS its rows of V (K went into the scores): the address of the
+            // refill depends on a word of each load (`zero` is 0 at run time), so it cannot be issued before.
+            request(__reduce_or_sync(0xffffffffu, arrived) & zero);
+        }
+        // ---- the warps of the chunk meet ----
+#pragma unroll
+        for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (lane < RING_G) {
+            s_m[warp][lane] = m;
+            s_l[warp][lane] = l;
+        }
+#pragma unroll
+        for (int g = 0; g < RING_G; ++g) {
+            float4 v;
+            f32x2_unpack(o2[g][0], v.x, v.y);
+            f32x2_unpack(o2[g][1], v.z, v.w);
+            *reinterpret_cast<float4*>(&s_o[warp][g][4 * lane]) = v;
+        }
+        __syncthreads();
+        float* out = partial + (int64_t)unit * RING_G * (RING_D + 2);
+        {
+            const int g = warp;  // RING_WARPS == RING_G: a warp finishes one head
+            float M = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < RING_WARPS; ++w) M = fmaxf(M, s_m[w][g]);
+            const float M_ref = M == -INFINITY ? 0.f : M;
+            float L = 0.f, r[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int w = 0; w < RING_WARPS; ++w) {
+                const float f = expf(s_m[w][g] - M_ref);
+                const float4 v = *reinterpret_cast<const float4*>(&s_o[w][g][4 * lane]);
+                L = fmaf(f, s_l[w][g], L);
+                r[0] = fmaf(f, v.x, r[0]);
+                r[1] = fmaf(f, v.y, r[1]);
+                r[2] = fmaf(f, v.z, r[2]);
+                r[3] = fmaf(f, v.w, r[3]);
+            }
+            float* og = out + g * (RING_D + 2);
+            if (lane == 0) {
+                og[0] = M;
+                og[1] = L;
+            }
+            reinterpret_cast<float2*>(og + 2)[2 * lane] = make_float2(r[0], r[1]);
+            reinterpret_cast<float2*>(og + 2)[2 * lane + 1] = make_float2(r[2], r[3]);
+        }
+        __syncthreads();
+    }
+    // nothing of this CTA's copies may be in flight when it leaves (only after a wait that gave up)
+    if (lane == 0)
+        for (; n_use < n_req; ++n_use) mbar_wait(&full[warp][n_use % RING_DEPTH], (n_use / RING_DEPTH) & 1, abort_flag);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_abort) atomicOr(status, 1);
+}
+
 // y[b, head, :] = sum_c exp(m_c - M) o_c / sum_c exp(m_c - M) l_c, chunks in order
 template <int D, int G>
 __global__ void __launch_bounds__(D)
@@ -221,14 +440,44 @@ decode_attention_merge_kernel(const float* __restrict__ partial, int n_kv, int n
     y[((int64_t)b * n_kv * G + head) * D + dim] = num / den;
 }
 
+// Positions per unit of the ring kernel: ATT_CHUNK, halved (down to 64, two tiles per warp) while the units do not give every
+// CTA two: a single sequence of 4096 positions has 64 units of 512 for 296 CTAs.
+constexpr int RING_MIN_CHUNK = 64, RING_MIN_UNITS = 592;
+int ring_chunk(int64_t pairs, int n_ctx) {
+    int chunk = ATT_CHUNK;
+    while (chunk > RING_MIN_CHUNK && pairs * ((n_ctx + chunk - 1) / chunk) < RING_MIN_UNITS) chunk /= 2;
+    return chunk;
+}
+
+cudaError_t launch_ring(cudaStream_t st, const float* q, const float* kc, const float* vc, int B, int n_kv, int64_t max_seq, int n_ctx,
+                        float scale, float* y, float* partial) {
+    int dev = 0, sms = 0;
+    int* status = nullptr;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = stream_status_ptr(&status);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_SMEM);
+    if (e != cudaSuccess) return e;
+    const int chunk = ring_chunk((int64_t)B * n_kv, n_ctx), n_chunks = (n_ctx + chunk - 1) / chunk, n_units = B * n_kv * n_chunks;
+    e = launch_k(decode_attention_ring_kernel, dim3(std::min(n_units, 2 * sms)), dim3(RING_THREADS), (size_t)RING_SMEM, st, q, kc, vc,
+                 max_seq, n_ctx, scale, chunk, n_chunks, n_units, partial, status, 0u);
+    if (e != cudaSuccess) return e;
+    return launch_k(decode_attention_merge_kernel<RING_D, RING_G>, dim3(n_kv * RING_G, B), dim3(RING_D), 0, st, (const float*)partial, n_kv,
+                    n_chunks, y);
+}
+
 template <int D, int G>
 cudaError_t launch_att(cudaStream_t st, const float* q, const float* kc, const float* vc, int B, int n_kv, int64_t max_seq, int n_ctx,
                        float scale, float* y, float* partial) {
-    const int n_chunks = (n_ctx + ATT_CHUNK - 1) / ATT_CHUNK;
-    cudaError_t e = launch_k(decode_attention_chunk_kernel<D, G>, dim3(n_chunks, n_kv, B), dim3(ATT_THREADS), 0, st, q, kc, vc, n_kv,
-                             max_seq, n_ctx, scale, n_chunks, partial);
-    if (e != cudaSuccess) return e;
-    return launch_k(decode_attention_merge_kernel<D, G>, dim3(n_kv * G, B), dim3(D), 0, st, (const float*)partial, n_kv, n_chunks, y);
+    if constexpr (D == RING_D && G == RING_G) {
+        return launch_ring(st, q, kc, vc, B, n_kv, max_seq, n_ctx, scale, y, partial);
+    } else {
+        const int n_chunks = (n_ctx + ATT_CHUNK - 1) / ATT_CHUNK;
+        cudaError_t e = launch_k(decode_attention_chunk_kernel<D, G>, dim3(n_chunks, n_kv, B), dim3(ATT_THREADS), 0, st, q, kc, vc, n_kv,
+                                 max_seq, n_ctx, scale, n_chunks, partial);
+        if (e != cudaSuccess) return e;
+        return launch_k(decode_attention_merge_kernel<D, G>, dim3(n_kv * G, B), dim3(D), 0, st, (const float*)partial, n_kv, n_chunks, y);
+    }
 }
 
 }  // namespace
@@ -279,8 +528,14 @@ cudaError_t launch_rope_kv_append(cudaStream_t st, const float* qkv, int64_t row
 }
 
 size_t decode_attention_workspace_bytes(int B, int n_head, int head_dim, int n_ctx) {
-    const size_t n_chunks = (size_t)(n_ctx + ATT_CHUNK - 1) / ATT_CHUNK;
-    return (size_t)B * n_head * n_chunks * (head_dim + 2) * sizeof(float);
+    size_t rows = (size_t)B * ((n_ctx + ATT_CHUNK - 1) / ATT_CHUNK);  // chunks of all sequences
+    if (head_dim == RING_D && n_head % RING_G == 0) {
+        // A bound for every batch up to B and context up to n_ctx: a chunk below ATT_CHUNK means that twice its length gave
+        // fewer than RING_MIN_UNITS units, so that there are fewer than 2 RING_MIN_UNITS + B n_kv of them.
+        const size_t small = (size_t)2 * RING_MIN_UNITS / (n_head / RING_G) + B;
+        rows = std::max(rows, std::min((size_t)B * ((n_ctx + RING_MIN_CHUNK - 1) / RING_MIN_CHUNK), small));
+    }
+    return rows * n_head * (head_dim + 2) * sizeof(float);
 }
 
 cudaError_t launch_decode_attention(cudaStream_t st, const float* q, const float* kc, const float* vc, int B, int n_head, int n_kv,
