@@ -1204,7 +1204,12 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         const int64_t rows_per = std::max<int64_t>(1, std::min<int64_t>(max_rows, P));
         const int64_t items = (int64_t)G.m_tiles * std::max<int64_t>(1, std::min<int64_t>(E, (P + rows_per - 1) / rows_per)) *
                               ((rows_per + tn - 1) / tn);
-        while (ksplit * 2 <= max_splits && kb % (ksplit * 2) == 0 && items * ksplit < 2 * (int64_t)g_gemm_sms) ksplit *= 2;
+        // Time in units of an unsplit item: whole waves of items over the SMs.  A split has to shorten that by enough: partial
+        // sums cost a little in a consumer that reads the result anyway (0.92), a kernel and their traffic where an unsplit
+        // result is final (0.75: [32000, 4096] at 32 rows is 250 items, two waves whether split in two or not).
+        const auto waves = [&](int ks) { return (double)((items * ks + g_gemm_sms - 1) / g_gemm_sms) / ks; };
+        for (int ks = 2; ks <= max_splits && kb % ks == 0; ks *= 2)
+            if (waves(ks) < (out_whole ? 0.75 : 0.92) * waves(ksplit)) ksplit = ks;
         *n_splits_out = ksplit;
     }
     G.ksplit = ksplit;
