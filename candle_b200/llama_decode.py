@@ -225,8 +225,20 @@ class DecodeStep:
         for li in range(self.cfg.n_layer):
             x = self.attention(li, x, index_pos)
             x = self.ffn(li, x)
-        x = rms_norm(x, self.norm, self.cfg.rms_eps)
-        return self.output.forward(x)
+        return self.output.forward(self._final_norm(x))
+
+    def _final_norm(self, x: torch.Tensor) -> torch.Tensor:
+        if self.attention_impl != "library":
+            return rms_norm(x, self.norm, self.cfg.rms_eps)
+        from . import _lib
+        from .quantized import _stream_ptr
+        x = x.contiguous()
+        h = torch.empty_like(x)
+        with torch.cuda.device(self.device):
+            _lib.check("candle_moe_rmsnorm",
+                       _lib.load().candle_moe_rmsnorm(_stream_ptr(self.device), x.data_ptr(), self.norm.data_ptr(), self.cfg.rms_eps,
+                                                      x.shape[0], self.cfg.d_model, h.data_ptr()))
+        return h
 
     # -- accounting ----------------------------------------------------------------------------------------
     def bytes_per_step(self, index_pos: int) -> dict:
