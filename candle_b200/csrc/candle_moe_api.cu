@@ -376,7 +376,7 @@ EpWorkspace ep_layout(const candle_moe_weights_t* w, int64_t P, void* base_) {
 extern "C" {
 
 static int forward_impl(void* stream, const candle_moe_weights_t* w, const float* x, int64_t T, float* y, void* workspace,
-                        size_t workspace_bytes, const float* residual) {
+                        size_t workspace_bytes, const float* residual, const float* norm_w = nullptr, float eps = 0.f) {
     CM_TRY(check_weights(w));
     if (!x || !y || !w->router) return CANDLE_MOE_E_NULL;
     if (T < 0 || T > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
@@ -407,7 +407,7 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     }
     CM_TRY(rc(launch_router_topk(st, x, w->router, w->router_bias, T, d, E, k, w->renorm, ws.topk_ids, ws.topk_w,
                                  fuse_q ? ws.xq : nullptr, fuse_q ? ws.xs : nullptr, fuse_q ? ws.xb : nullptr,
-                                 T == 1 ? ws.counts : nullptr, ws.offsets, ws.perm_token, ws.pair_pos)));
+                                 T == 1 ? ws.counts : nullptr, ws.offsets, ws.perm_token, ws.pair_pos, norm_w, eps)));
     mark(st, 0);
     // one token: the router kernel has written the dispatch itself
     if (T > 1) CM_TRY(rc(launch_permute(st, ws.topk_ids, T, k, E, ws.counts, ws.offsets, ws.perm_token, ws.pair_pos, ws.perm_scratch)));
@@ -511,6 +511,9 @@ int candle_moe_ffn_layer(void* stream, const candle_moe_weights_t* w, const floa
     const size_t inner = layout(w, T, nullptr).total;
     const size_t need = inner + align_up((size_t)T * w->d_model * sizeof(float), 256);
     if (workspace_bytes < need) return CANDLE_MOE_E_WORKSPACE;
+    // k-quant experts and no shared expert: nothing but the router kernel reads the normalised rows
+    if (router_fuses_norm(T, w->d_model) && w->dtype_w13 != CANDLE_GGML_Q8_0 && w->d_ff_shared == 0)
+        return forward_impl(stream, w, x, T, y, workspace, inner, x, norm_weight, eps);
     float* xn = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + inner);
     CM_TRY(rc(launch_rmsnorm((cudaStream_t)stream, x, norm_weight, eps, T, w->d_model, xn)));
     return forward_impl(stream, w, xn, T, y, workspace, inner, x);

@@ -161,7 +161,9 @@ cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
 cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* router, const float* bias, int64_t T,
                                int d, int E, int k, int renorm, uint32_t* ids, float* w, int8_t* qs = nullptr,
                                float* scales = nullptr, int16_t* bsums = nullptr, uint32_t* counts = nullptr,
-                               uint32_t* offsets = nullptr, uint32_t* perm_token = nullptr, uint32_t* pair_pos = nullptr);
+                               uint32_t* offsets = nullptr, uint32_t* perm_token = nullptr, uint32_t* pair_pos = nullptr,
+                               const float* norm_w = nullptr, float eps = 0.f);
+bool router_fuses_norm(int64_t T, int d);  // norm_w may be given: the router sees (and quantizes) the normalised rows
 // scratch (may be null): permute_scratch_words(T * k, E) words; with it, large batches are sorted by many CTAs
 size_t permute_scratch_words(int64_t n_pairs, int E);
 cudaError_t launch_permute(cudaStream_t st, const uint32_t* ids, int64_t T, int k, int E, uint32_t* counts,

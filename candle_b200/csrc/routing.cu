@@ -43,10 +43,8 @@ bool tuning_set(int key, int64_t value) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// Router (+ activation quantization).  One CTA of 1024 threads per token: for d = 4096 every thread
-// issues its single 128-bit load of x and its 8 loads of the router rows at once, so the whole
-// product costs about one memory latency; partial sums meet through warp shuffles and shared
-// memory in a fixed order.  Warp 0 then does the softmax over all E experts and k rounds of arg-max
+// Router (+ activation quantization).  One CTA per token; partial sums meet through warp shuffles and shared memory in a
+// fixed order.  Warp 0 then does the softmax over all E experts and k rounds of arg-max
 // with "lower expert id wins a tie", which is what a stable descending sort followed by take(k)
 // yields (candle-transformers/src/models/quantized_llama.rs:162-179).  Meanwhile the other warps
 // quantize the same row of x the Q8K way for the expert products (one pass over x instead of two
@@ -137,10 +135,131 @@ __device__ __forceinline__ void softmax_topk_warp(const float* s_logits, int lan
     }
 }
 
-// Few tokens: 1024 threads per token (the whole product in one round of loads).  Many tokens: 256 threads per token,
-// so that eight CTAs share an SM and their load rounds overlap.  The two sizes add the partial sums in different
-// orders (last-bit differences of the logits, as between any two f32 dot-product orders).
-template <int ROUTER_THREADS>
+// Single token (the step of one-sequence decoding): its k experts are distinct, so the dispatch is their ascending order
+// and needs no pass of its own.  Run by one warp whose every lane holds the selection.
+__device__ __forceinline__ void dispatch_one_token(const int (&sel_e)[CANDLE_MOE_MAX_TOPK], int lane, int E, int k,
+                                                   uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets,
+                                                   uint32_t* __restrict__ perm_token, uint32_t* __restrict__ pair_pos) {
+    for (int e = lane; e < E; e += 32) {
+        uint32_t hit = 0, below = 0;
+#pragma unroll
+        for (int r = 0; r < CANDLE_MOE_MAX_TOPK; ++r) {
+            if (r < k) {
+                hit += sel_e[r] == e;
+                below += sel_e[r] < e;
+            }
+        }
+        counts[e] = hit;
+        offsets[e] = below;
+    }
+    if (lane == 0) offsets[E] = (uint32_t)k;
+#pragma unroll
+    for (int r = 0; r < CANDLE_MOE_MAX_TOPK; ++r) {
+        if (r < k && lane == r) {
+            uint32_t pos = 0;
+#pragma unroll
+            for (int r2 = 0; r2 < CANDLE_MOE_MAX_TOPK; ++r2) pos += (r2 < k && sel_e[r2] < sel_e[r]);
+            perm_token[pos] = 0u;
+            pair_pos[r] = pos;
+        }
+    }
+}
+
+// Few tokens (up to 64): 1024 threads per token, latency-bound.  The row passes through shared memory once, with the
+// layer's RmsNorm applied on the way where the caller asks for it (norm_w; one launch fewer), and every warp owns whole
+// dot products: expert e, or for few experts one of `parts` pieces of it, so that all loads of a round are in flight at
+// once and one reduction per expert and warp is left.  (Eight experts at a time across all warps, eight reductions per
+// warp and two barriers per round, was 7.9 us for 8 experts of 4096 and 29.2 us for 60 experts of 2048, 16
+// rows; this form 8.9 us with the norm, which was another 4.5 us, and 11.5 us.)
+// Before the wait for the previous kernel the first CTA asks for the router's rows in L2: a prefetch returns no data, so
+// it does not matter what that kernel still writes.
+template <bool NORM>
+__global__ void __launch_bounds__(1024)
+router_topk_small_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps, const float* __restrict__ wg,
+                         const float* __restrict__ bias, int d, int E, int parts, int k, int renorm, uint32_t* __restrict__ ids,
+                         float* __restrict__ wout, int8_t* __restrict__ qs, float* __restrict__ scales, int16_t* __restrict__ bsums,
+                         uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets, uint32_t* __restrict__ perm_token,
+                         uint32_t* __restrict__ pair_pos) {
+    extern __shared__ __align__(16) float s_x[];  // [d]
+    __shared__ float s_part[8][CANDLE_MOE_MAX_EXPERTS];
+    __shared__ float s_logits[CANDLE_MOE_MAX_EXPERTS];
+    __shared__ float s_red[32];
+    const int64_t t = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d4 = d >> 2;
+    pdl_trigger();
+    if (t == 0)
+        for (int64_t i = tid; i < (int64_t)E * d / 32; i += 1024) asm volatile("prefetch.global.L2 [%0];" ::"l"(wg + 32 * i));
+    pdl_wait();
+    const float4* xr = reinterpret_cast<const float4*>(x + t * (int64_t)d);
+    float4* sx4 = reinterpret_cast<float4*>(s_x);
+    if (NORM) {
+        float ss = 0.f;
+        for (int i = tid; i < d4; i += 1024) {
+            const float4 v = xr[i];
+            sx4[i] = v;
+            ss = fmaf(v.x, v.x, ss);
+            ss = fmaf(v.y, v.y, ss);
+            ss = fmaf(v.z, v.z, ss);
+            ss = fmaf(v.w, v.w, ss);
+        }
+        ss = warp_sum(ss);
+        if (lane == 0) s_red[warp] = ss;
+        __syncthreads();
+        const float m = sqrtf(warp_sum(s_red[lane]) / (float)d + eps);  // every warp adds the 32 sums in the same order
+        for (int i = tid; i < d4; i += 1024) {  // the elements this thread wrote
+            const float4 v = sx4[i], a = reinterpret_cast<const float4*>(norm_w)[i];
+            sx4[i] = make_float4(__fmul_rn(__fdiv_rn(v.x, m), a.x), __fmul_rn(__fdiv_rn(v.y, m), a.y),
+                                 __fmul_rn(__fdiv_rn(v.z, m), a.z), __fmul_rn(__fdiv_rn(v.w, m), a.w));
+        }
+    } else {
+        for (int i = tid; i < d4; i += 1024) sx4[i] = xr[i];
+    }
+    __syncthreads();
+    // unit u = (expert, part); part p covers float4s [p d4 / parts, (p + 1) d4 / parts)
+    for (int u = warp; u < E * parts; u += 32) {
+        const int e = u / parts, p = u - e * parts;
+        const int i1 = d4 * (p + 1) / parts;
+        const float4* wr = reinterpret_cast<const float4*>(wg + (int64_t)e * d);
+        float acc = 0.f;
+#pragma unroll 8
+        for (int i = d4 * p / parts + lane; i < i1; i += 32) {
+            const float4 wv = wr[i], xv = sx4[i];
+            acc = fmaf(xv.x, wv.x, acc);
+            acc = fmaf(xv.y, wv.y, acc);
+            acc = fmaf(xv.z, wv.z, acc);
+            acc = fmaf(xv.w, wv.w, acc);
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) s_part[p][e] = acc;
+    }
+    __syncthreads();
+    if (warp != 0) {
+        // warps 1.. quantize the row (each 256-element block by one warp)
+        if (qs) {
+            const int nb = d >> 8;
+            for (int b = warp - 1; b < nb; b += 31)
+                quantize_q8k_block(s_x + b * 256, lane, qs + t * (int64_t)d + b * 256, scales + t * nb + b, bsums + (t * nb + b) * 16);
+        }
+        return;
+    }
+    for (int e = lane; e < E; e += 32) {
+        float v = 0.f;
+        for (int p = 0; p < parts; ++p) v += s_part[p][e];
+        if (bias) v += bias[e];
+        s_logits[e] = v;
+    }
+    __syncwarp();
+    float sel_p[CANDLE_MOE_MAX_TOPK];
+    int sel_e[CANDLE_MOE_MAX_TOPK];
+    softmax_topk_warp(s_logits, lane, E, k, renorm, ids + t * k, wout + t * k, sel_p, sel_e);
+    if (counts) dispatch_one_token(sel_e, lane, E, k, counts, offsets, perm_token, pair_pos);
+}
+constexpr int ROUTER_SMALL_TOKENS = 64, ROUTER_SMALL_MAX_D = 10240;  // the row in 40 KB of shared memory
+
+// Many tokens (and rows too long for the form above): 256 threads per token, so that eight CTAs share an SM and their
+// load rounds overlap.  The forms add the partial sums in different orders (last-bit differences of the logits, as between
+// any two f32 dot-product orders).
+constexpr int ROUTER_THREADS = 256;
 __global__ void __launch_bounds__(ROUTER_THREADS)
 router_topk_kernel(const float* __restrict__ x, const float* __restrict__ wg, const float* __restrict__ bias,
                    int d, int E, int k, int renorm, uint32_t* __restrict__ ids, float* __restrict__ wout,
@@ -203,33 +322,7 @@ router_topk_kernel(const float* __restrict__ x, const float* __restrict__ wg, co
     float sel_p[CANDLE_MOE_MAX_TOPK];
     int sel_e[CANDLE_MOE_MAX_TOPK];
     softmax_topk_warp(s_logits, lane, E, k, renorm, ids + t * k, wout + t * k, sel_p, sel_e);
-    // A single token (the step of one-sequence decoding): its k experts are distinct, so the dispatch is their
-    // ascending order and needs no pass of its own.  Every lane holds the selection.
-    if (counts) {
-        for (int e = lane; e < E; e += 32) {
-            uint32_t hit = 0, below = 0;
-#pragma unroll
-            for (int r = 0; r < CANDLE_MOE_MAX_TOPK; ++r) {
-                if (r < k) {
-                    hit += sel_e[r] == e;
-                    below += sel_e[r] < e;
-                }
-            }
-            counts[e] = hit;
-            offsets[e] = below;
-        }
-        if (lane == 0) offsets[E] = (uint32_t)k;
-#pragma unroll
-        for (int r = 0; r < CANDLE_MOE_MAX_TOPK; ++r) {
-            if (r < k && lane == r) {
-                uint32_t pos = 0;
-#pragma unroll
-                for (int r2 = 0; r2 < CANDLE_MOE_MAX_TOPK; ++r2) pos += (r2 < k && sel_e[r2] < sel_e[r]);
-                perm_token[pos] = 0u;
-                pair_pos[r] = pos;
-            }
-        }
-    }
+    if (counts) dispatch_one_token(sel_e, lane, E, k, counts, offsets, perm_token, pair_pos);
 }
 
 // Many tokens and many experts (prefill of a fine-grained layer): the router product as a tiled f32 GEMM.  The
@@ -317,19 +410,27 @@ router_topk_tiled_kernel(const float* __restrict__ x, const float* __restrict__ 
     }
 }
 
+// the fused norm is there only where the small form runs
+bool router_fuses_norm(int64_t T, int d) { return T <= ROUTER_SMALL_TOKENS && d <= ROUTER_SMALL_MAX_D; }
+
 cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* router, const float* bias, int64_t T,
                                int d, int E, int k, int renorm, uint32_t* ids, float* w, int8_t* qs, float* scales,
-                               int16_t* bsums, uint32_t* counts, uint32_t* offsets, uint32_t* perm_token, uint32_t* pair_pos) {
+                               int16_t* bsums, uint32_t* counts, uint32_t* offsets, uint32_t* perm_token, uint32_t* pair_pos,
+                               const float* norm_w, float eps) {
     if (T == 0) return cudaSuccess;
     if (counts && (T != 1 || !offsets || !perm_token || !pair_pos)) return cudaErrorInvalidValue;  // single-token dispatch only
+    if (T <= ROUTER_SMALL_TOKENS && d <= ROUTER_SMALL_MAX_D) {
+        const int parts = E <= 4 ? 8 : (E <= 8 ? 4 : (E <= 16 ? 2 : 1));
+        auto kfn = norm_w ? router_topk_small_kernel<true> : router_topk_small_kernel<false>;
+        return launch_k(kfn, dim3((unsigned)T), dim3(1024), (size_t)d * sizeof(float), st, x, norm_w, eps, router, bias, d, E, parts, k,
+                        renorm, ids, w, qs, scales, bsums, counts, offsets, perm_token, pair_pos);
+    }
+    if (norm_w) return cudaErrorInvalidValue;
     if (T >= 512 && E >= 16 && !qs && !counts && d % RT_KC == 0)
         return launch_k(router_topk_tiled_kernel, dim3((unsigned)((T + RT_TOK - 1) / RT_TOK)), dim3(256), 0, st, x, router, bias, T, d, E, k,
                         renorm, ids, w);
-    if (T > 64)
-        return launch_k(router_topk_kernel<256>, dim3((unsigned)T), dim3(256), 0, st, x, router, bias, d, E, k, renorm, ids, w, qs,
-                        scales, bsums, counts, offsets, perm_token, pair_pos);
-    return launch_k(router_topk_kernel<1024>, dim3((unsigned)T), dim3(1024), 0, st, x, router, bias, d, E, k, renorm, ids, w, qs,
-                    scales, bsums, counts, offsets, perm_token, pair_pos);
+    return launch_k(router_topk_kernel, dim3((unsigned)T), dim3(ROUTER_THREADS), 0, st, x, router, bias, d, E, k, renorm, ids, w, qs, scales,
+                    bsums, counts, offsets, perm_token, pair_pos);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -1,0 +1,53 @@
+"""The small-batch router (whole dot products per warp, optional norm, single-token dispatch) at the edges of its rule, and
+the operand preparation that quantizes f32 rows itself against the two-pass form."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,k", [(1, 1), (4, 2), (5, 3), (8, 2), (9, 4), (16, 8), (17, 2), (33, 4), (128, 8)])
+def test_router_at_the_edges_of_its_forms(orc, torch_cuda, E, k):
+    torch = torch_cuda
+    from candle_b200 import _lib
+    # rows of few float4s, of an odd number, the longest of the small form and one beyond; the last count takes the other form
+    for d in (4, 36, 1028, 10240, 10244):
+        for T in (1, 64, 65) if d <= 1028 else (3,):
+            rng = np.random.default_rng(E + d + T)
+            x = rng.standard_normal((T, d), dtype=np.float32)
+            wg = rng.standard_normal((E, d), dtype=np.float32) * np.float32(0.05)
+            probs, ids_ref, w_ref = orc.router_topk(x, wg, k, True, None)
+            xd, wd = torch.from_numpy(x).cuda(), torch.from_numpy(wg).cuda()
+            ids = torch.empty((T, k), dtype=torch.int32, device="cuda")
+            w = torch.empty((T, k), dtype=torch.float32, device="cuda")
+            assert _lib.load().candle_moe_router_topk(torch.cuda.current_stream().cuda_stream, xd.data_ptr(), wd.data_ptr(), None, T, d, E, k,
+                                                      1, ids.data_ptr(), w.data_ptr()) == 0
+            got = ids.cpu().numpy().astype(np.uint32)
+            H.check_routing(probs, ids_ref, got)
+            same = (ids_ref == got).all(axis=1)
+            # logits are sums of d products in another order: d 2^-24 relative to the largest term bounds them loosely
+            assert np.allclose(w.cpu().numpy()[same], w_ref[same], rtol=5e-5, atol=1e-7), (d, T)
+
+
+@pytest.mark.parametrize("T", [1, 2, 64, 65])
+def test_layer_equals_norm_block_residual_in_three_steps(orc, torch_cuda, T):
+    torch = torch_cuda
+    from candle_b200 import _lib
+    cfg = dict(d=1024, ff=1024, E=8, k=2, dt13=orc.Q4K, dt2=orc.Q6K, renorm=True)
+    blk, _ = H.random_device_block(orc, torch, cfg, seed=T)
+    blk.prepack()
+    x = torch.from_numpy(orc.make_activations(T, T, 1024)).cuda() * 3
+    nw = 1.0 + 0.1 * torch.randn(1024, generator=torch.Generator(device="cuda").manual_seed(T), device="cuda")
+    xn = torch.empty_like(x)
+    assert _lib.load().candle_moe_rmsnorm(torch.cuda.current_stream().cuda_stream, x.data_ptr(), nw.data_ptr(), 1e-5, T, 1024, xn.data_ptr()) == 0
+    want = blk.forward(xn) + x
+    ids = blk.last_routing(T)[0]
+    y = blk.forward_layer(x, nw, 1e-5)
+    same = (ids == blk.last_routing(T)[0]).all(dim=1).cuda()
+    assert int((~same).sum()) <= 1  # a near tie may fall either way
+    # the norm's sum of squares is added in another order: last bits of the rows, now and then a step of an int8 value
+    assert H.rel_l2((y - x)[same].cpu().numpy(), (want - x)[same].cpu().numpy()) <= H.REL_L2_TOL
