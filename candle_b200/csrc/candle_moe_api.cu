@@ -315,7 +315,11 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
         CM_TRY(rc(launch_grouped_gate_up(st, p1, p3, w->dtype_w13, E, d, ff, offsets, row_of, max_rows, xq, xs, xb,
                                          b.hidden)));
     if (marks) mark(st, 3);
-    CM_TRY(rc(launch_quantize_act(st, b.hidden, P, ff, w->dtype_w2, b.hq, b.hs, b.hb, row_limit)));
+    // The down product on the GEMM quantizes the hidden rows while it prepares its operand (not with a device-side row
+    // limit: the operand is prepared for all P rows)
+    const bool rp2 = (w->dtype_w2 == CANDLE_GGML_Q6K || w->dtype_w2 == CANDLE_GGML_Q8_0) && w->w2_prepacked;
+    const bool fuse_h = large && !row_limit && expert_gemm_takes(false, w->dtype_w2, rp2, ff, d, P);
+    if (!fuse_h) CM_TRY(rc(launch_quantize_act(st, b.hidden, P, ff, w->dtype_w2, b.hq, b.hs, b.hb, row_limit)));
     if (marks) mark(st, 4);
     if (use_prepacked) {
         const cudaError_t ce = launch_expert_direct(st, false, q2, q2, w->dtype_w2, E, ff, d, offsets, nullptr, max_rows, b.hq,
@@ -328,16 +332,15 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
             *eo_splits = 1;
     }
     if (!down_done && large) {
-        const bool rp = (w->dtype_w2 == CANDLE_GGML_Q6K || w->dtype_w2 == CANDLE_GGML_Q8_0) && w->w2_prepacked;
         ExpertPtrs g2 = p2;
-        if (rp) CM_TRY(fill_ptrs(w->w2_prepacked, E, g2));
-        const cudaError_t ce = launch_expert_gemm(st, false, g2, g2, w->dtype_w2, rp, E, ff, d, offsets, nullptr, P, tile_rows,
-                                                  b.hq, b.hs, b.hb, b.eo, b.gemm, slots, eo_splits, P * d);
-        if (ce == cudaSuccess) {
+        if (rp2) CM_TRY(fill_ptrs(w->w2_prepacked, E, g2));
+        const cudaError_t ce = launch_expert_gemm(st, false, g2, g2, w->dtype_w2, rp2, E, ff, d, offsets, nullptr, P, tile_rows,
+                                                  b.hq, b.hs, b.hb, b.eo, b.gemm, slots, eo_splits, P * d, nullptr,
+                                                  fuse_h ? b.hidden : nullptr);
+        if (ce == cudaSuccess)
             down_done = true;
-        } else if (ce != cudaErrorNotSupported) {
+        else if (ce != cudaErrorNotSupported || fuse_h)
             return (int)ce;
-        }
     }
     if (!down_done)
         CM_TRY(rc(launch_grouped_down(st, p2, w->dtype_w2, E, d, ff, offsets, max_rows, b.hq, b.hs, b.hb, b.eo, P * d, slots,
@@ -456,19 +459,21 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
         if (!sh_done)
             CM_TRY(rc(launch_grouped_gate_up(st, s1, s3, w->dtype_shared13, 1, d, fs, ws.sh_offsets, nullptr, T, ws.sxq,
                                              ws.sxs, ws.sxb, ws.shidden)));
-        CM_TRY(rc(launch_quantize_act(st, ws.shidden, T, fs, w->dtype_shared2, ws.shq, ws.shs, ws.shb)));
+        const bool fuse_sh = sh_gemm && expert_gemm_takes(false, CANDLE_GGML_Q8_0, true, fs, d, T);
+        if (!fuse_sh) CM_TRY(rc(launch_quantize_act(st, ws.shidden, T, fs, w->dtype_shared2, ws.shq, ws.shs, ws.shb)));
         sh_done = false;
         if (sh_gemm || sh_direct) {
             ExpertPtrs r2{};
             r2.p[0] = static_cast<const uint8_t*>(w->shared_w2_prepacked);
             const cudaError_t ce =
                 sh_gemm ? launch_expert_gemm(st, false, r2, r2, CANDLE_GGML_Q8_0, true, 1, fs, d, ws.sh_offsets, nullptr, T, T, ws.shq,
-                                             ws.shs, ws.shb, ws.so, ws.gemm, k_split_slots(T), &so_splits, T * (int64_t)d)
+                                             ws.shs, ws.shb, ws.so, ws.gemm, k_split_slots(T), &so_splits, T * (int64_t)d, nullptr,
+                                             fuse_sh ? ws.shidden : nullptr)
                         : launch_expert_direct(st, false, r2, r2, CANDLE_GGML_Q8_0, 1, fs, d, ws.sh_offsets, nullptr, T, ws.shq,
                                                ws.shs, ws.shb, ws.so, &so_splits, T * (int64_t)d, k_split_slots(T), 1, T);
             if (ce == cudaSuccess)
                 sh_done = true;
-            else if (ce != cudaErrorNotSupported)
+            else if (ce != cudaErrorNotSupported || fuse_sh)
                 return (int)ce;
             else
                 so_splits = 1;
@@ -850,13 +855,15 @@ int candle_moe_qmatmul(void* stream, const void* w, const void* w_prepacked, int
     ExpertPtrs pw{}, pp{};
     pw.p[0] = static_cast<const uint8_t*>(w);
     pp.p[0] = static_cast<const uint8_t*>(w_prepacked);
-    // the quantizer also writes the offsets of the one group that holds every row
-    CM_TRY(rc(launch_quantize_act(st, x, rows, k, dtype, ws.xq, ws.xs, ws.xb, nullptr, ws.offsets)));
+    const bool rp = dtype == CANDLE_GGML_Q6K && w_prepacked;
+    const bool large = ws.gemm && gemm_enabled() && expert_gemm_takes(false, dtype, rp, k, n, rows);
+    // the quantizer -- with the GEMM the preparation of its operand -- also writes the offsets of the one group that holds
+    // every row
+    if (!large) CM_TRY(rc(launch_quantize_act(st, x, rows, k, dtype, ws.xq, ws.xs, ws.xb, nullptr, ws.offsets)));
     float* dst = ws.eo ? ws.eo : out;
     const int64_t stride = rows * (int64_t)n;
     int splits = 1;
     bool done = false;
-    const bool large = ws.gemm && gemm_enabled();
     // The decode kernels over the repacked copy of a k-quant are not used here: with a single group their tiles are too few and
     // too short, and the streaming form over the GGUF blocks is faster (measured, [4096, 4096] Q4_K / [32000, 4096]
     // Q6_K: 1 row 10.8 / 44.5 us against 17.2 / 46.2; 8 rows 13.5 / 48.6 against 17.7 / 60.1).
@@ -870,16 +877,10 @@ int candle_moe_qmatmul(void* stream, const void* w, const void* w_prepacked, int
         else
             splits = 1;
     }
-    if (!done && large) {
-        const bool rp = dtype == CANDLE_GGML_Q6K && w_prepacked;
-        const cudaError_t ce = launch_expert_gemm(st, false, rp ? pp : pw, rp ? pp : pw, dtype, rp, 1, k, n, ws.offsets, nullptr,
-                                                  rows, rows, ws.xq, ws.xs, ws.xb, dst, ws.gemm, ws.slots, &splits, stride, out);
-        if (ce == cudaSuccess)
-            done = true;
-        else if (ce != cudaErrorNotSupported)
-            return (int)ce;
-        else
-            splits = 1;
+    if (large) {
+        CM_TRY(rc(launch_expert_gemm(st, false, rp ? pp : pw, rp ? pp : pw, dtype, rp, 1, k, n, ws.offsets, nullptr, rows, rows, ws.xq,
+                                     ws.xs, ws.xb, dst, ws.gemm, ws.slots, &splits, stride, out, x, ws.offsets)));
+        done = true;
     }
     if (!done)
         CM_TRY(rc(launch_grouped_down(st, pw, dtype, 1, n, k, ws.offsets, rows, ws.xq, ws.xs, ws.xb, dst, stride, ws.slots,

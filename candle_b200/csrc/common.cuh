@@ -68,10 +68,9 @@ __device__ __forceinline__ void q4k_scale_min(int j, const uint8_t* q, int& sc, 
 // BlockQ8K::from_float (candle-core/src/quantized/k_quants.rs:1819-1856) for one 256-element block
 // by one warp, 8 consecutive elements per lane.  `max` is the signed value of the first element with
 // the largest magnitude; IEEE division, roundf = round half away from zero like f32::round.
-__device__ __forceinline__ void quantize_q8k_block(const float* __restrict__ xblk, int lane, int8_t* __restrict__ qs,
-                                                   float* __restrict__ scale, int16_t* __restrict__ bsums) {
-    const float4* src = reinterpret_cast<const float4*>(xblk) + lane * 2;
-    const float4 a = src[0], b = src[1];
+// From the lane's eight elements a, b: the rounded values as floats in q and the block's scale in d.  Where 1 / d overflows (a
+// block of denormals) d is 0 and a q may be infinite.
+__device__ __forceinline__ void quantize_q8k_values(const float4& a, const float4& b, float (&q)[8], float& d) {
     const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     float amax = 0.f, mx = 0.f;
 #pragma unroll
@@ -87,18 +86,25 @@ __device__ __forceinline__ void quantize_q8k_block(const float* __restrict__ xbl
     const uint32_t mine = __float_as_uint(amax), top = __reduce_max_sync(0xffffffffu, mine);
     mx = __shfl_sync(0xffffffffu, mx, __ffs(__ballot_sync(0xffffffffu, mine == top)) - 1);
     amax = __uint_as_float(top);
-    int q[8];
-    float d;
     if (amax == 0.f) {
         d = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = 0;
+        for (int i = 0; i < 8; ++i) q[i] = 0.f;
     } else {
         const float iscale = __fdiv_rn(-128.0f, mx);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = (int)fminf(roundf(__fmul_rn(iscale, v[i])), 127.f);
+        for (int i = 0; i < 8; ++i) q[i] = fminf(roundf(__fmul_rn(iscale, v[i])), 127.f);
         d = __fdiv_rn(1.0f, iscale);
     }
+}
+__device__ __forceinline__ void quantize_q8k_block(const float* __restrict__ xblk, int lane, int8_t* __restrict__ qs,
+                                                   float* __restrict__ scale, int16_t* __restrict__ bsums) {
+    const float4* src = reinterpret_cast<const float4*>(xblk) + lane * 2;
+    float qf[8], d;
+    quantize_q8k_values(src[0], src[1], qf, d);
+    int q[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = (int)qf[i];
     int s = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) s += q[i];
@@ -215,7 +221,10 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
                                bool repacked, int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of, int64_t P,
                                int64_t max_rows, const int8_t* aq, const float* ascale, const int16_t* absum, float* out,
                                void* scratch, int max_splits = 1, int* n_splits_out = nullptr, int64_t split_stride = 0,
-                               float* out_whole = nullptr);
+                               float* out_whole = nullptr, const float* x_f32 = nullptr, uint32_t* single_group = nullptr);
+// whether launch_expert_gemm takes the product (given scratch).  Its x_f32: the f32 rows in grouped order instead of their
+// quantization (aq, ascale, absum are then not read); single_group: as in launch_quantize_act, with x_f32 only
+bool expert_gemm_takes(bool gate_up, int dtype, bool repacked, int K, int N, int64_t P);
 // Q8_0 grouped products for many rows per expert (expert_q80.cu); cudaErrorNotSupported for other shapes
 cudaError_t launch_expert_q80(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int E, int K, int N,
                               const uint32_t* offsets, const uint32_t* row_of, const int8_t* aq, const float* ascale, float* out);

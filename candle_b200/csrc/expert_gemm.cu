@@ -156,6 +156,121 @@ prep_gemm_b_q80_kernel(const int8_t* __restrict__ aq, const float* __restrict__ 
     if (lane == 0) d8t[(int64_t)blk * P_pad + p] = exact ? 1.0f / 64.0f : 1.0f;
 }
 
+// The two preparations straight from f32 rows that lie in grouped order already (hidden rows before the down product, the
+// rows of a dense product): the activation quantization of quantize_act.cu -- the same values bit for bit -- and the
+// operand in one pass, so that the int8 rows neither travel to memory and back nor cost a launch.  A warp takes PREP_UNITS
+// (row, 256-block) units, loads first; rows at or past P are zeros.  The rounded values stay floats (they are integers of at
+// most 128): no conversion to int and back.  HBM-bound: 4 bytes read and 2 (Q8_0 exact: 4) written per element.
+// Measured: 4096 hidden rows of 14336 (Q6_K down) 60.9 + 41.7 us in two passes, 64.5 us in one; 16384 rows of 1408 (Q8_0 down)
+// 20.5 + 22.3 us against 28.1; one unit per warp and integer conversions took 82 us for the first.
+constexpr int PREP_UNITS = 2;
+__global__ void __launch_bounds__(256)
+prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, __half* __restrict__ bf16, float* __restrict__ bmin,
+                         float* __restrict__ d8t, uint32_t* __restrict__ single_group) {
+    pdl_trigger();
+    pdl_wait();
+    if (single_group && blockIdx.x == 0 && threadIdx.x < 2) single_group[threadIdx.x] = threadIdx.x ? (uint32_t)P : 0u;
+    const int kb = K >> 8;
+    const int lane = threadIdx.x & 31;
+    const int64_t n_units = (int64_t)P_pad * kb;
+    const int64_t unit0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * PREP_UNITS;  // (p, block)
+    int p[PREP_UNITS], blk[PREP_UNITS];
+    float4 a[PREP_UNITS], b[PREP_UNITS];
+#pragma unroll
+    for (int u = 0; u < PREP_UNITS; ++u) {
+        p[u] = (int)((unit0 + u) / kb);
+        blk[u] = (int)(unit0 + u - (int64_t)p[u] * kb);
+        a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);  // zeros quantize to zeros with scale 0
+        if (p[u] < P) {
+            const float4* src = reinterpret_cast<const float4*>(x + (int64_t)p[u] * K + blk[u] * 256) + lane * 2;
+            a[u] = src[0];
+            b[u] = src[1];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < PREP_UNITS; ++u) {
+        if (unit0 + u >= n_units) return;
+        float q[8], d8;
+        quantize_q8k_values(a[u], b[u], q, d8);
+        if (d8 == 0.f) {  // zeros, or a block of denormals: what the int8 row would hold
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] = (float)(int8_t)(int)q[i];
+        }
+        __half2 h[4] = {__floats2half2_rn(q[0], q[2]), __floats2half2_rn(q[1], q[3]), __floats2half2_rn(q[4], q[6]), __floats2half2_rn(q[5], q[7])};
+        *reinterpret_cast<uint4*>(bf16 + (int64_t)p[u] * K + blk[u] * 256 + lane * 8) = *reinterpret_cast<uint4*>(h);
+        if (bmin) {
+            float s = 0.f;  // sums of integers of at most 128: exact
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s += q[i];
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);  // 32 elements = four lanes
+            const int j = lane & 7, part = lane >> 3;  // the words of prep_gemm_b_kernel
+            const float bv = __shfl_sync(0xffffffffu, s, 4 * j), b1 = tf32_head(bv), b2 = bv - b1;
+            bmin[((int64_t)p[u] * kb + blk[u]) * 32 + lane] = part == 2 ? b2 : (part == 3 ? 0.f : b1);
+        }
+        if (lane == 0) d8t[(int64_t)blk[u] * P_pad + p[u]] = d8;
+    }
+}
+
+__global__ void __launch_bounds__(256)
+prep_gemm_f32_q80_kernel(const float* __restrict__ x, int P, int P_pad, int K, int K_pad, int exact, __half* __restrict__ bf16,
+                         float* __restrict__ d8t, uint32_t* __restrict__ single_group) {
+    pdl_trigger();
+    pdl_wait();
+    if (single_group && blockIdx.x == 0 && threadIdx.x < 2) single_group[threadIdx.x] = threadIdx.x ? (uint32_t)P : 0u;
+    const int kb = K_pad >> 8;
+    const int lane = threadIdx.x & 31;
+    const int64_t n_units = (int64_t)P_pad * kb;
+    const int64_t unit0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * PREP_UNITS;  // (p, block of 256)
+    int p[PREP_UNITS], blk[PREP_UNITS];
+    float4 a[PREP_UNITS], b[PREP_UNITS];
+#pragma unroll
+    for (int u = 0; u < PREP_UNITS; ++u) {
+        p[u] = (int)((unit0 + u) / kb);
+        blk[u] = (int)(unit0 + u - (int64_t)p[u] * kb);
+        a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int k0 = blk[u] * 256 + lane * 8;
+        if (p[u] < P && k0 < K) {  // K is a multiple of 32: whole groups of four lanes
+            const float4* src = reinterpret_cast<const float4*>(x + (int64_t)p[u] * K + k0);
+            a[u] = src[0];
+            b[u] = src[1];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < PREP_UNITS; ++u) {
+        if (unit0 + u >= n_units) return;
+        const float v[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
+        float amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        const float d = __fdiv_rn(amax, 127.0f);
+        const float id = d != 0.f ? __fdiv_rn(1.0f, d) : 0.f;
+        const float df = __fmul_rn(__half2float(__float2half_rn(d)), exact ? 64.0f : 1.0f);  // a power of two: exact
+        float t[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)  // exact in f32: 8 x 11 bits
+            t[i] = __fmul_rn(fmaxf(fminf(roundf(__fmul_rn(v[i], id)), 127.f), -128.f), df);
+        __half2 h[4] = {__floats2half2_rn(t[0], t[2]), __floats2half2_rn(t[1], t[3]), __floats2half2_rn(t[4], t[6]), __floats2half2_rn(t[5], t[7])};
+        if (exact) {
+            __half2 g[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int i0 = (i >> 1) * 4 + (i & 1);
+                const float2 f = __half22float2(h[i]);
+                g[i] = __floats2half2_rn(__fsub_rn(t[i0], f.x), __fsub_rn(t[i0 + 2], f.y));
+            }
+            __half* dst = bf16 + (int64_t)p[u] * (2 * K_pad) + blk[u] * 512 + lane * 8;
+            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(h);
+            *reinterpret_cast<uint4*>(dst + 256) = *reinterpret_cast<uint4*>(g);
+        } else {
+            *reinterpret_cast<uint4*>(bf16 + (int64_t)p[u] * K_pad + blk[u] * 256 + lane * 8) = *reinterpret_cast<uint4*>(h);
+        }
+        if (lane == 0) d8t[(int64_t)blk[u] * P_pad + p[u]] = exact ? 1.0f / 64.0f : 1.0f;
+    }
+}
+
 // Q8_0 GGUF rows [n][K / 32 blocks of 34 bytes] -> [ceil(n / 8)][2 * ceil(K / 256)][1088]: 8 rows x 128 elements, two
 // 512-byte regions of 64 elements (chunk_pos order, a chunk of row g holds the words at 4 t, 16 + 4 t, 32 + 4 t, 48 + 4 t)
 // and [8 rows][4] f16 scales; zeros past K and past n.  The pieces the decode kernels' fragments and the GEMM's
@@ -1114,18 +1229,24 @@ size_t expert_gemm_scratch_bytes(int64_t P, int K, int parts) {
            sizeof(CUtensorMap) * 2 * CANDLE_MOE_MAX_EXPERTS;
 }
 
+bool expert_gemm_takes(bool gate_up, int dtype, bool repacked, int K, int N, int64_t P) {
+    const bool q80 = dtype == CANDLE_GGML_Q8_0 && repacked;
+    if (!((dtype == CANDLE_GGML_Q4K && !repacked) || (dtype == CANDLE_GGML_Q6K && repacked) || q80)) return false;
+    return K % (q80 ? 32 : 256) == 0 && N % (gate_up ? 64 : 128) == 0 && P > 0 && P <= (1 << 30) && encode_tiled_fn() != nullptr;
+}
+
 // Takes Q4_K weights in GGUF layout (repacked = false), Q6_K weights in the repacked layout of the decode kernels
 // and Q8_0 weights in the layout of prepack_q80_kernel (repacked = true); cudaErrorNotSupported for every other
 // shape / dtype / layout.
 cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int dtype,
                                bool repacked, int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of, int64_t P,
                                int64_t max_rows, const int8_t* aq, const float* ascale, const int16_t* absum, float* out,
-                               void* scratch, int max_splits, int* n_splits_out, int64_t split_stride, float* out_whole) {
+                               void* scratch, int max_splits, int* n_splits_out, int64_t split_stride, float* out_whole,
+                               const float* x_f32, uint32_t* single_group) {
     if (n_splits_out) *n_splits_out = 1;
-    if (!scratch) return cudaErrorNotSupported;
+    if (!scratch || !expert_gemm_takes(gate_up, dtype, repacked, K, N, P) || (x_f32 && row_of)) return cudaErrorNotSupported;
     int tn = max_rows <= 32 ? 32 : (max_rows <= 64 ? 64 : 128);  // position tile, from the bound / hint on an expert's rows
     const bool q80 = dtype == CANDLE_GGML_Q8_0 && repacked;
-    if (!((dtype == CANDLE_GGML_Q4K && !repacked) || (dtype == CANDLE_GGML_Q6K && repacked) || q80)) return cudaErrorNotSupported;
     // Q8_0: the DOWN product runs with operands that carry the block scales rounded to fp16 (a few 1e-4 relative on a
     // product), which a final product tolerates.  The gate_up product does not: its f32 hidden rows are re-quantized to
     // int8 before W2, and a relative difference of 1e-4 from the reference's hidden values already moves a few per cent
@@ -1135,8 +1256,6 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     const int parts = q80x ? 2 : 1;
     const int K_in = K;
     if (q80) K = (K + 255) / 256 * 256;  // the repacked rows and the fp16 operand are padded with zeros
-    if (K_in % (q80 ? 32 : 256) != 0 || N % (gate_up ? 64 : 128) != 0 || P <= 0 || P > (1 << 30)) return cudaErrorNotSupported;
-    if (!encode_tiled_fn()) return cudaErrorNotSupported;
     if (g_gemm_sms < 0) {
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
@@ -1153,10 +1272,19 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     const bool has_min = dtype == CANDLE_GGML_Q4K;
 
     const int64_t units = p_pad * kb;
-    cudaError_t e = q80 ? launch_k(prep_gemm_b_q80_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, st, aq, ascale, row_of,
-                                   (int)P, (int)p_pad, K_in, K, q80x ? 1 : 0, bf16, d8t)
-                        : launch_k(prep_gemm_b_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, st, aq, ascale, absum,
-                                   row_of, (int)P, (int)p_pad, K, bf16, has_min ? bmin : (float*)nullptr, d8t);
+    const int64_t per_cta = 8 * (x_f32 ? PREP_UNITS : 1);
+    const dim3 prep_grid((unsigned)((units + per_cta - 1) / per_cta));
+    cudaError_t e;
+    if (x_f32)
+        e = q80 ? launch_k(prep_gemm_f32_q80_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K_in, K, q80x ? 1 : 0, bf16,
+                           d8t, single_group)
+                : launch_k(prep_gemm_f32_q8k_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K, bf16,
+                           has_min ? bmin : (float*)nullptr, d8t, single_group);
+    else
+        e = q80 ? launch_k(prep_gemm_b_q80_kernel, prep_grid, dim3(256), 0, st, aq, ascale, row_of, (int)P, (int)p_pad, K_in, K,
+                           q80x ? 1 : 0, bf16, d8t)
+                : launch_k(prep_gemm_b_kernel, prep_grid, dim3(256), 0, st, aq, ascale, absum, row_of, (int)P, (int)p_pad, K, bf16,
+                           has_min ? bmin : (float*)nullptr, d8t);
     if (e != cudaSuccess) return e;
 
     CUtensorMap map_b, map_bs;

@@ -51,3 +51,43 @@ def test_layer_equals_norm_block_residual_in_three_steps(orc, torch_cuda, T):
     assert int((~same).sum()) <= 1  # a near tie may fall either way
     # the norm's sum of squares is added in another order: last bits of the rows, now and then a step of an int8 value
     assert H.rel_l2((y - x)[same].cpu().numpy(), (want - x)[same].cpu().numpy()) <= H.REL_L2_TOL
+
+
+@pytest.mark.parametrize("name,k,n,rows", [("Q4K", 256, 128, 49), ("Q4K", 1024, 256, 130), ("Q6K", 512, 128, 65), ("Q6K", 1024, 384, 257)])
+def test_gemm_operand_from_f32_rows(orc, torch_cuda, name, k, n, rows):
+    """The dense product quantizes its rows while it prepares the operand: rows of every size, rows and blocks of zeros."""
+    torch = torch_cuda
+    from candle_b200 import GgmlDType, QMatMul, QTensor
+    dt = getattr(orc, name)
+    rng = np.random.default_rng(k + n + rows)
+    x = rng.standard_normal((rows, k), dtype=np.float32) * np.exp2(rng.integers(-20, 20, (rows, 1))).astype(np.float32)
+    x[3] = 0.0
+    x[5, 256 * (k // 256 - 1):] = 0.0
+    wq = orc.quantize(dt, rng.standard_normal((n, k), dtype=np.float32) * np.float32(0.02))
+    mm = QMatMul.from_qtensor(QTensor.from_blocks(wq, GgmlDType(dt), (n, k))).prepack()
+    got = mm.forward(torch.from_numpy(x).cuda()).cpu().numpy()
+    ref = orc.matmul(dt, x, wq, n)
+    assert np.array_equal(got[3], np.zeros(n, np.float32))
+    # the same integers; f32 sums in another order: row by row, as the rows differ in size
+    for r in range(rows):
+        if r != 3 and not (k == 256 and r == 5):
+            assert H.rel_l2(got[r], ref[r]) < 1e-5, r
+
+
+@pytest.mark.parametrize("T,d,ff,fs", [(97, 256, 384, 128), (130, 512, 1408, 640), (513, 1024, 160, 384)])
+def test_q80_large_batch_with_the_fused_operand(orc, torch_cuda, T, d, ff, fs):
+    """Hidden rows whose length ends inside a 256-block (routed) and not (shared); against the form without repacked copies."""
+    torch = torch_cuda
+    from candle_b200 import _lib
+    cfg = dict(d=d, ff=ff, E=4, k=2, dt13=orc.Q8_0, dt2=orc.Q8_0, renorm=True, ff_shared=fs)
+    blk, _ = H.random_device_block(orc, torch, cfg, seed=T)
+    x = torch.from_numpy(orc.make_activations(T, T, d)).cuda()
+    want = blk.forward(x).clone()
+    blk.prepack()
+    blk._ws, blk._ws_tokens = None, 0  # with the copies the large batch needs more scratch
+    y = blk.forward(x).clone()
+    assert torch.equal(y, blk.forward(x))
+    v = C.c_int32(-1)
+    assert _lib.load().candle_moe_device_status(C.byref(v)) == 0 and v.value == 0
+    loose = 1.0 if ff >= 1024 else 2.0
+    assert H.rel_l2(y.cpu().numpy(), want.cpu().numpy()) <= loose * H.REL_L2_TOL
