@@ -35,6 +35,16 @@ struct ExpertBufs {
     void* gemm;     // scratch of the large-batch GEMM (may be null)
 };
 
+// The shared expert's products beside the routed ones (run_experts takes them where the decode kernels do): what each needs,
+// its hidden rows and their quantization, and how far run_experts came.
+struct SharedRun {
+    SharedGroup gate, down;
+    float* hidden;
+    int8_t* hq;
+    float* hs;
+    bool gate_done = false, quantized = false, down_done = false;
+};
+
 // The routed experts over P rows grouped by expert (device offsets [E + 1]).  `max_rows` picks the kernels: a bound
 // on the rows of one expert, or (rows_exact) the actual / expected largest count -- every kernel is correct for any
 // count, the choice only matters for speed.  `row_limit` (device, may be null): actual number of rows when P is a
@@ -42,7 +52,7 @@ struct ExpertBufs {
 int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs& p1, const ExpertPtrs& p3,
                 const ExpertPtrs& p2, int64_t max_rows, int64_t P, const uint32_t* offsets, const uint32_t* row_of,
                 const int8_t* xq, const float* xs, const int16_t* xb, const ExpertBufs& b, int slots, int* eo_splits,
-                bool marks, bool rows_exact, const uint32_t* row_limit, int64_t total_rows_hint);
+                bool marks, bool rows_exact, const uint32_t* row_limit, int64_t total_rows_hint, SharedRun* shared = nullptr);
 
 // Scratch of the expert-parallel local phase for up to P rows
 struct EpWorkspace {

@@ -273,7 +273,7 @@ namespace cmoe {
 int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs& p1, const ExpertPtrs& p3,
                 const ExpertPtrs& p2, int64_t max_rows, int64_t P, const uint32_t* offsets, const uint32_t* row_of,
                 const int8_t* xq, const float* xs, const int16_t* xb, const ExpertBufs& b, int slots, int* eo_splits,
-                bool marks, bool rows_exact, const uint32_t* row_limit, int64_t total_rows_hint) {
+                bool marks, bool rows_exact, const uint32_t* row_limit, int64_t total_rows_hint, SharedRun* shared) {
     if (total_rows_hint <= 0) total_rows_hint = P;
     const int E = w->n_experts, d = w->d_model, ff = w->d_ff;
     const bool large = b.gemm && max_rows > (rows_exact ? GEMM_MIN_ROWS_EXACT : gemm_min_rows()) && gemm_enabled();
@@ -286,8 +286,14 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
         CM_TRY(fill_ptrs(w->w1_prepacked, E, q1));
         CM_TRY(fill_ptrs(w->w3_prepacked, E, q3));
         CM_TRY(fill_ptrs(w->w2_prepacked, E, q2));
-        const cudaError_t ce = launch_expert_direct(st, true, q1, q3, w->dtype_w13, E, d, ff, offsets, row_of, max_rows, xq,
-                                                    xs, xb, b.hidden, nullptr, 0, 1, 0, total_rows_hint);
+        cudaError_t ce = cudaErrorNotSupported;
+        const SharedGroup* const tries[2] = {shared ? &shared->gate : nullptr, nullptr};  // with the shared expert, or without
+        for (const SharedGroup* sg : tries) {
+            if (ce != cudaErrorNotSupported) break;
+            ce = launch_expert_direct(st, true, q1, q3, w->dtype_w13, E, d, ff, offsets, row_of, max_rows, xq, xs, xb, b.hidden, nullptr,
+                                      0, 1, 0, total_rows_hint, nullptr, sg);
+            if (ce == cudaSuccess && sg) shared->gate_done = true;
+        }
         if (ce == cudaSuccess)
             gate_done = true;
         else if (ce != cudaErrorNotSupported)
@@ -320,10 +326,20 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     const bool rp2 = (w->dtype_w2 == CANDLE_GGML_Q6K || w->dtype_w2 == CANDLE_GGML_Q8_0) && w->w2_prepacked;
     const bool fuse_h = large && !row_limit && expert_gemm_takes(false, w->dtype_w2, rp2, ff, d, P);
     if (!fuse_h) CM_TRY(rc(launch_quantize_act(st, b.hidden, P, ff, w->dtype_w2, b.hq, b.hs, b.hb, row_limit)));
+    if (shared && shared->gate_done) {
+        CM_TRY(rc(launch_quantize_act(st, shared->hidden, shared->gate.rows, shared->gate.N, CANDLE_GGML_Q8_0, shared->hq, shared->hs, nullptr)));
+        shared->quantized = true;
+    }
     if (marks) mark(st, 4);
     if (use_prepacked) {
-        const cudaError_t ce = launch_expert_direct(st, false, q2, q2, w->dtype_w2, E, ff, d, offsets, nullptr, max_rows, b.hq,
-                                                    b.hs, b.hb, b.eo, eo_splits, P * d, slots, (int)(total_rows_hint < E ? total_rows_hint : E), total_rows_hint);
+        cudaError_t ce = cudaErrorNotSupported;
+        const SharedGroup* const tries[2] = {shared && shared->quantized ? &shared->down : nullptr, nullptr};
+        for (const SharedGroup* sg : tries) {
+            if (ce != cudaErrorNotSupported) break;
+            ce = launch_expert_direct(st, false, q2, q2, w->dtype_w2, E, ff, d, offsets, nullptr, max_rows, b.hq, b.hs, b.hb, b.eo, eo_splits,
+                                      P * d, slots, (int)(total_rows_hint < E ? total_rows_hint : E), total_rows_hint, nullptr, sg);
+            if (ce == cudaSuccess && sg) shared->down_done = true;
+        }
         if (ce == cudaSuccess)
             down_done = true;
         else if (ce != cudaErrorNotSupported)
@@ -421,8 +437,24 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     // a token selects an expert at most once: no expert sees more than T rows
     int eo_splits = 1, so_splits = 1;
     const ExpertBufs eb{ws.hidden, ws.hq, ws.hs, ws.hb, ws.eo, ws.gemm};
+    // over repacked Q8_0 copies the shared expert takes the decode kernels -- in the launches of the routed experts where those
+    // are Q8_0 too -- and for large batches the tensor-core GEMM
+    const bool sh_packed = w->d_ff_shared > 0 && w->dtype_shared13 == CANDLE_GGML_Q8_0 && w->dtype_shared2 == CANDLE_GGML_Q8_0 &&
+                           w->shared_w1_prepacked && w->shared_w3_prepacked && w->shared_w2_prepacked;
+    const bool sh_gemm = sh_packed && ws.gemm && T > gemm_min_rows() && gemm_enabled();
+    const bool sh_direct = sh_packed && !sh_gemm && T <= std::max<int64_t>(gemm_min_rows(), 64);
+    SharedRun sr;
+    const bool sh_joins = sh_direct && w->dtype_w13 == CANDLE_GGML_Q8_0 && w->dtype_w2 == CANDLE_GGML_Q8_0 && ws.sxq == ws.xq;
+    if (sh_joins) {
+        const int fs = w->d_ff_shared;
+        sr.gate = {w->shared_w1_prepacked, w->shared_w3_prepacked, T, d, fs, ws.xq, ws.xs, ws.shidden, 0, 1, nullptr};
+        sr.down = {w->shared_w2_prepacked, nullptr, T, fs, d, ws.shq, ws.shs, ws.so, T * (int64_t)d, k_split_slots(T), &so_splits};
+        sr.hidden = ws.shidden;
+        sr.hq = ws.shq;
+        sr.hs = ws.shs;
+    }
     CM_TRY(run_experts(st, w, p1, p3, p2, T, Tk, ws.offsets, ws.perm_token, ws.xq, ws.xs, ws.xb, eb, k_split_slots(T),
-                       &eo_splits, true, false, nullptr, 0));
+                       &eo_splits, true, false, nullptr, 0, sh_joins ? &sr : nullptr));
     mark(st, 5);
 
     const float* shared_out = nullptr;
@@ -435,14 +467,8 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
         s2.p[0] = static_cast<const uint8_t*>(w->shared_w2);
         if (ws.sxq != ws.xq)
             CM_TRY(rc(launch_quantize_act(st, x, T, d, w->dtype_shared13, ws.sxq, ws.sxs, ws.sxb)));
-        // over repacked Q8_0 copies: the decode kernels, and for large batches the tensor-core GEMM, with one group
-        // holding every row
-        const bool sh_packed = w->dtype_shared13 == CANDLE_GGML_Q8_0 && w->dtype_shared2 == CANDLE_GGML_Q8_0 &&
-                               w->shared_w1_prepacked && w->shared_w3_prepacked && w->shared_w2_prepacked;
-        const bool sh_gemm = sh_packed && ws.gemm && T > gemm_min_rows() && gemm_enabled();
-        const bool sh_direct = sh_packed && !sh_gemm && T <= std::max<int64_t>(gemm_min_rows(), 64);
-        bool sh_done = false;
-        if (sh_gemm || sh_direct) {
+        bool sh_done = sr.gate_done;
+        if (!sh_done && (sh_gemm || sh_direct)) {
             ExpertPtrs r1{}, r3{};
             r1.p[0] = static_cast<const uint8_t*>(w->shared_w1_prepacked);
             r3.p[0] = static_cast<const uint8_t*>(w->shared_w3_prepacked);
@@ -460,9 +486,9 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
             CM_TRY(rc(launch_grouped_gate_up(st, s1, s3, w->dtype_shared13, 1, d, fs, ws.sh_offsets, nullptr, T, ws.sxq,
                                              ws.sxs, ws.sxb, ws.shidden)));
         const bool fuse_sh = sh_gemm && expert_gemm_takes(false, CANDLE_GGML_Q8_0, true, fs, d, T);
-        if (!fuse_sh) CM_TRY(rc(launch_quantize_act(st, ws.shidden, T, fs, w->dtype_shared2, ws.shq, ws.shs, ws.shb)));
-        sh_done = false;
-        if (sh_gemm || sh_direct) {
+        if (!fuse_sh && !sr.quantized) CM_TRY(rc(launch_quantize_act(st, ws.shidden, T, fs, w->dtype_shared2, ws.shq, ws.shs, ws.shb)));
+        sh_done = sr.down_done;
+        if (!sh_done && (sh_gemm || sh_direct)) {
             ExpertPtrs r2{};
             r2.p[0] = static_cast<const uint8_t*>(w->shared_w2_prepacked);
             const cudaError_t ce =

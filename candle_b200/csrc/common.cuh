@@ -206,15 +206,28 @@ cudaError_t launch_expert_stream(cudaStream_t st, bool gate_up, const ExpertPtrs
 // prepacked-weight (register-fragment order) form for decode-sized batches
 size_t prepacked_bytes(int dtype, int64_t n_rows, int k);
 cudaError_t launch_prepack(cudaStream_t st, int dtype, const void* raw, int64_t n_rows, int k, void* dst);
+// A matrix (gate_up: a pair) that every row goes through, walked in the launch of the routed experts (Q8_0 only).
+struct SharedGroup {
+    const void *wa, *wb;  // repacked
+    int64_t rows;
+    int K, N;
+    const int8_t* aq;
+    const float* ascale;
+    float* out;
+    int64_t split_stride;
+    int max_splits;
+    int* n_splits_out;
+};
 cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int dtype,
                                  int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of,
                                  int64_t max_rows_per_expert, const int8_t* aq, const float* ascale,
                                  const int16_t* absum, float* out, int* n_splits_out, int64_t split_stride,
-                                 int max_splits, int max_active_experts = 0, int64_t total_rows = 0, float* out_whole = nullptr);
+                                 int max_splits, int max_active_experts = 0, int64_t total_rows = 0, float* out_whole = nullptr,
+                                 const SharedGroup* shared = nullptr);
 // large-batch grouped GEMM on tcgen05 / TMEM: Q4_K in GGUF layout (repacked = false), Q6_K in the repacked
 // layout (repacked = true); `scratch` of expert_gemm_scratch_bytes(P, K) bytes
 size_t expert_gemm_scratch_bytes(int64_t P, int K, int parts = 1);  // parts = 2: the exact Q8_0 gate_up operand
-// Q8_0 rows repacked for the GEMM: [n][ceil(k / 256)][256 int8 | 8 f16 scales]
+// Q8_0 rows repacked for the decode kernels and the GEMM (see Q80_HTB_BYTES)
 size_t prepacked_q80_bytes(int64_t n_rows, int k);
 cudaError_t launch_prepack_q80(cudaStream_t st, const void* raw, int64_t n_rows, int k, void* dst);
 cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int dtype,

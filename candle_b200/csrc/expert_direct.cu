@@ -22,6 +22,8 @@
 //   Q6_K (1680 B): [3][32 lanes][16 B]: u = 0,1: ql words of half u {ql[64u+4t], +16, +32, +48};
 //                  u = 2: qh words {qh[4t], qh[16+4t], qh[32+4t], qh[48+4t]}; scales [8][16] i8; d [8] f16
 // Q4_K grows by 2.8 % (the 12-byte packed scales become 16 bytes); Q6_K keeps its size.
+#include <algorithm>
+
 #include "common.cuh"
 #include "stream_common.cuh"
 #include "tc5_common.cuh"
@@ -327,10 +329,23 @@ struct DirectParams {
     int blk_start[9];  // split s covers blocks [blk_start[s], blk_start[s + 1])
     int act_stride;
     uint32_t off_act, off_scale, off_bs, off_ring, off_part;
+    // one more group over a matrix of another shape (SH kernels): the always-on shared expert beside the routed ones
+    struct {
+        const uint8_t *wa, *wb;
+        const int8_t* aq;
+        const float* ascale;
+        float* out;
+        int64_t out_split_stride;
+        int rows, K, N, kb, kb_stride, splits;
+        int blk_start[9];
+    } sh;
 };
 
 // DEPTH = ring slots per warp (DEPTH - 1 blocks in flight while one is multiplied)
-template <class F, bool GATE_UP, int NT, int DEPTH>
+// SH: the shared expert's group is walked after the experts', in the same launch.  (As launches of its own its two products, 24
+// and 12 MB for 5632 x 2048, took 13.3 and 12.3 us, nearly all of it the fixed cost of a launch.  60 experts, top-4: 1 row 70 ->
+// 64 us, 8 rows 109 -> 100, 16 rows 129 -> 124, 96 rows 229 -> 211; 16 experts, 8 rows 85 -> 72.)
+template <class F, bool GATE_UP, int NT, int DEPTH, bool SH>
 // The one-position-tile Q4_K and Q8_0 kernels are held to 96 registers (a bound of 608 threads; they are launched with
 // 512, and Q6_K would spill): the
 // registers a CTA leaves free let the CTAs of the next kernel on the stream become resident and run their
@@ -366,32 +381,37 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIR
     // Cost-balanced contiguous share of the (token group, split, tile) sequence.  Cost = blocks streamed, weighted
     // by what a block costs to multiply: a group of more than eight rows takes two position tiles per block, which
     // is TWO_TILES_COST : 8 against a group of up to eight.
-    const int tiles = P.N / TILE_N;
     auto group_weight = [](uint32_t rows) { return (NT > 1 && rows > 8) ? F::TWO_TILES_COST : 8; };
     long long ctot = 0;
     for (int i = 0; i < P.E; ++i) {
         const uint32_t cnt = s_offs[i + 1] - s_offs[i];
-        ctot += (long long)tiles * P.kb * ((long long)(cnt / MT) * group_weight(MT) + (cnt % MT ? group_weight(cnt % MT) : 0));
+        ctot += (long long)(P.N / TILE_N) * P.kb * ((long long)(cnt / MT) * group_weight(MT) + (cnt % MT ? group_weight(cnt % MT) : 0));
+    }
+    if (SH) {
+        const uint32_t cnt = (uint32_t)P.sh.rows;
+        ctot += (long long)(P.sh.N / TILE_N) * P.sh.kb * ((long long)(cnt / MT) * group_weight(MT) + (cnt % MT ? group_weight(cnt % MT) : 0));
     }
     const long long lo = ctot * blockIdx.x / gridDim.x, hi = ctot * (blockIdx.x + 1) / gridDim.x;
     if (lo >= hi) return;
-    const size_t ht_stride = (size_t)P.kb_stride * F::HTB;  // bytes of one half-tile over the whole K
 
     long long acc = 0;  // cost of the groups before the current one
-    for (int e = 0; e < P.E && acc < hi; ++e) {
-      const uint32_t cnt = s_offs[e + 1] - s_offs[e];
+    for (int e = 0; e < P.E + (SH ? 1 : 0) && acc < hi; ++e) {
+      const bool sh = SH && e == P.E;
+      const uint32_t e_base = sh ? 0u : s_offs[e], cnt = sh ? (uint32_t)P.sh.rows : s_offs[e + 1] - e_base;
+      const int gN = sh ? P.sh.N : P.N, gK = sh ? P.sh.K : P.K, gkb = sh ? P.sh.kb : P.kb, tiles = gN / TILE_N;
+      const size_t ht_stride = (size_t)(sh ? P.sh.kb_stride : P.kb_stride) * F::HTB;  // bytes of one half-tile over the whole K
       for (uint32_t g0 = 0; g0 < cnt && acc < hi; g0 += MT) {
         const uint32_t rows = min((uint32_t)MT, cnt - g0);
         const int w = group_weight(rows);
-        const long long gcost = (long long)tiles * P.kb * w;
+        const long long gcost = (long long)tiles * gkb * w;
         const long long g_lo = acc;
         acc += gcost;
         if (acc <= lo) continue;
-        const uint32_t p_base = s_offs[e] + g0;
+        const uint32_t p_base = e_base + g0;
         const uint32_t p_end = p_base + rows;
         const int ntiles = (int)(rows + 7) / 8;
-        for (int sp = 0; sp < P.splits; ++sp) {
-            const int blk0 = P.blk_start[sp], nblk = P.blk_start[sp + 1] - blk0;
+        for (int sp = 0; sp < (sh ? P.sh.splits : P.splits); ++sp) {
+            const int blk0 = sh ? P.sh.blk_start[sp] : P.blk_start[sp], nblk = (sh ? P.sh.blk_start[sp + 1] : P.blk_start[sp + 1]) - blk0;
             const long long unit = (long long)nblk * w;  // cost of one tile over this split
             const long long ph_lo = g_lo + (long long)tiles * blk0 * w;
             const long long ph_hi = ph_lo + (long long)tiles * unit;
@@ -404,7 +424,7 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIR
             __syncthreads();
             if (tid < MT) {
                 const uint32_t pp = p_base + tid;
-                s_rows[tid] = pp < p_end ? (P.row_of ? (int)P.row_of[pp] : (int)pp) : -1;
+                s_rows[tid] = pp < p_end ? (!sh && P.row_of ? (int)P.row_of[pp] : (int)pp) : -1;
             }
             __syncthreads();
             {
@@ -415,16 +435,16 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIR
                     const int row = s_rows[j];
                     int4 val = make_int4(0, 0, 0, 0);
                     // (Q8_0: K is a multiple of 32 and may end inside the last K-block)
-                    if (row >= 0 && (BLK == 256 || k0 + 16 * v < P.K))
-                        val = *reinterpret_cast<const int4*>(P.aq + (int64_t)row * P.K + k0 + 16 * v);
+                    if (row >= 0 && (BLK == 256 || k0 + 16 * v < gK))
+                        val = *reinterpret_cast<const int4*>((sh ? P.sh.aq : P.aq) + (int64_t)row * gK + k0 + 16 * v);
                     *reinterpret_cast<int4*>(act + j * P.act_stride + 16 * v) = val;
                 }
-                const int sc_per_row = nblk * SCB, sc_k = SCB == 1 ? P.kb : P.K / 32;  // scales per row: in this range, in all
+                const int sc_per_row = nblk * SCB, sc_k = SCB == 1 ? gkb : gK / 32;  // scales per row: in this range, in all
                 for (int idx = tid; idx < MT * sc_per_row; idx += DIRECT_THREADS) {
                     const int j = idx / sc_per_row, bb = idx - j * sc_per_row;
                     const int row = s_rows[j];
                     const bool in = row >= 0 && (SCB == 1 || blk0 * SCB + bb < sc_k);
-                    act_scale[bb * MT + j] = in ? P.ascale[(int64_t)row * sc_k + blk0 * SCB + bb] : 0.f;
+                    act_scale[bb * MT + j] = in ? (sh ? P.sh.ascale : P.ascale)[(int64_t)row * sc_k + blk0 * SCB + bb] : 0.f;
                 }
                 if constexpr (BSB > 0) {
                     const int per_row = nblk * F::BS_PER_BLOCK;
@@ -478,9 +498,10 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIR
                         const uint32_t p = p_base + nt * 8 + 2 * t + cc;
                         if (p < p_end) {
                             if (GATE_UP) {
-                                P.out[(int64_t)p * P.N + tile * 8 + g] = silu_f(f[cc]) * f[2 + cc];
+                                (sh ? P.sh.out : P.out)[(int64_t)p * gN + tile * 8 + g] = silu_f(f[cc]) * f[2 + cc];
                             } else {
-                                float* o = P.out + (int64_t)sp * P.out_split_stride + (int64_t)p * P.N + tile * 16 + g;
+                                float* o = (sh ? P.sh.out + (int64_t)sp * P.sh.out_split_stride : P.out + (int64_t)sp * P.out_split_stride) +
+                                           (int64_t)p * gN + tile * 16 + g;
                                 o[0] = f[cc];
                                 o[8] = f[2 + cc];
                             }
@@ -520,10 +541,10 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIR
                 const uint8_t* hta;
                 const uint8_t* htb;
                 if (GATE_UP) {
-                    hta = P.wa.p[e] + (size_t)tile * ht_stride + (size_t)(blk0 + b0) * F::HTB;
-                    htb = P.wb.p[e] + (size_t)tile * ht_stride + (size_t)(blk0 + b0) * F::HTB;
+                    hta = (sh ? P.sh.wa : P.wa.p[e]) + (size_t)tile * ht_stride + (size_t)(blk0 + b0) * F::HTB;
+                    htb = (sh ? P.sh.wb : P.wb.p[e]) + (size_t)tile * ht_stride + (size_t)(blk0 + b0) * F::HTB;
                 } else {
-                    hta = P.wa.p[e] + (size_t)(2 * tile) * ht_stride + (size_t)(blk0 + b0) * F::HTB;
+                    hta = (sh ? P.sh.wa : P.wa.p[e]) + (size_t)(2 * tile) * ht_stride + (size_t)(blk0 + b0) * F::HTB;
                     htb = hta + ht_stride;
                 }
 #pragma unroll
@@ -659,9 +680,9 @@ __global__ void __launch_bounds__(384) prepack_q6k_kernel(const uint8_t* __restr
 
 int g_dir_max_smem = -1, g_dir_sms = -1;
 
-template <class F, bool GATE_UP, int NT, int DEPTH>
+template <class F, bool GATE_UP, int NT, int DEPTH, bool SH = false>
 cudaError_t launch_dir(cudaStream_t st, const DirectParams& P, size_t smem_bytes) {
-    auto kfn = expert_direct_kernel<F, GATE_UP, NT, DEPTH>;
+    auto kfn = expert_direct_kernel<F, GATE_UP, NT, DEPTH, SH>;
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     if (e != cudaSuccess) return e;
     return launch_k(kfn, dim3(g_dir_sms), dim3(DIRECT_THREADS), smem_bytes, st, P);
@@ -693,11 +714,13 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
                                  int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of,
                                  int64_t max_rows_per_expert, const int8_t* aq, const float* ascale,
                                  const int16_t* absum, float* out, int* n_splits_out, int64_t split_stride,
-                                 int max_splits, int max_active_experts, int64_t total_rows, float* out_whole) {
+                                 int max_splits, int max_active_experts, int64_t total_rows, float* out_whole,
+                                 const SharedGroup* shared) {
     const bool q80 = dtype == CANDLE_GGML_Q8_0;
     if (dtype != CANDLE_GGML_Q4K && dtype != CANDLE_GGML_Q6K && !q80) return cudaErrorNotSupported;
     const int tile_n = gate_up ? 8 : 16;
     if (N % tile_n != 0 || K % (q80 ? 32 : 256) != 0) return cudaErrorNotSupported;
+    if (shared && (!q80 || shared->N % tile_n != 0 || shared->K % 32 != 0 || shared->rows <= 0)) return cudaErrorNotSupported;
     if (g_dir_max_smem < 0) {
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
@@ -714,6 +737,10 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
     // choice (Mixtral-shaped layer: 145 us at 9 rows against ~200 with two tiles; from 16 rows on the two are equal
     // and beyond 20 the two-tile kernel wins).
     const bool few_rows = total_rows > 0 && total_rows <= 3 * (int64_t)E;
+    // With the shared expert in the launch, whose group holds every row: at up to 16 rows two passes over its matrix cost less
+    // than a second tile (16 rows 124 against 141 us); where the experts would take one tile and the shared group more passes
+    // than that, separate launches are as good or better (60 experts, 24 rows 156 either way, 32 rows 162 against 167 us).
+    if (shared && few_rows && max_rows_per_expert > 8 && shared->rows > 16) return cudaErrorNotSupported;
     const int NT = max_rows_per_expert <= 8 || few_rows ? 1 : 2;
     const int MT = 8 * NT;
     const int bs_per_block = q80 ? 0 : (dtype == CANDLE_GGML_Q4K ? 8 : 16);
@@ -732,7 +759,16 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
     }
     for (int splits = min_splits; splits <= max_splits && splits <= kb; ++splits) {
         if (gate_up && splits > 1) break;
-        const int ks_blocks = (kb + splits - 1) / splits;
+        int ks_blocks = (kb + splits - 1) / splits;
+        // the shared group: its own K splits, no longer than the routed ranges or than 45 KB of activations
+        int sh_kb = 0, sh_splits = 1;
+        if (shared) {
+            sh_kb = (shared->K + blk - 1) / blk;
+            const int room = gate_up ? sh_kb : std::max(ks_blocks, 176 / MT * 2);
+            sh_splits = (sh_kb + room - 1) / room;
+            if (sh_splits > (gate_up ? 1 : std::min(8, shared->max_splits))) return cudaErrorNotSupported;
+            ks_blocks = std::max(ks_blocks, (sh_kb + sh_splits - 1) / sh_splits);
+        }
         uint32_t off = 0;
         auto take = [&](uint32_t bytes) {
             off = (off + 127u) & ~127u;
@@ -772,6 +808,29 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
         P.kb_stride = q80 ? (K + 255) / 256 * 2 : kb;
         P.MT = MT;
         if (n_splits_out) *n_splits_out = splits;
+        if (shared) {
+            P.sh.wa = static_cast<const uint8_t*>(shared->wa);
+            P.sh.wb = static_cast<const uint8_t*>(shared->wb);
+            P.sh.aq = shared->aq;
+            P.sh.ascale = shared->ascale;
+            P.sh.out = shared->out;
+            P.sh.out_split_stride = shared->split_stride;
+            P.sh.rows = (int)shared->rows;
+            P.sh.K = shared->K;
+            P.sh.N = shared->N;
+            P.sh.kb = sh_kb;
+            P.sh.kb_stride = (shared->K + 255) / 256 * 2;
+            P.sh.splits = sh_splits;
+            int at = 0;
+            for (int s = 0; s < sh_splits; ++s) {
+                P.sh.blk_start[s] = at;
+                at += (sh_kb - at + sh_splits - s - 1) / (sh_splits - s);
+            }
+            P.sh.blk_start[sh_splits] = sh_kb;
+            if (shared->n_splits_out) *shared->n_splits_out = sh_splits;
+            if (gate_up) return NT == 1 ? launch_dir<DirQ80, true, 1, 4, true>(st, P, off) : launch_dir<DirQ80, true, 2, 4, true>(st, P, off);
+            return NT == 1 ? launch_dir<DirQ80, false, 1, 4, true>(st, P, off) : launch_dir<DirQ80, false, 2, 4, true>(st, P, off);
+        }
         if (q80) {
             if (gate_up) return NT == 1 ? launch_dir<DirQ80, true, 1, 4>(st, P, off) : launch_dir<DirQ80, true, 2, 4>(st, P, off);
             return NT == 1 ? launch_dir<DirQ80, false, 1, 4>(st, P, off) : launch_dir<DirQ80, false, 2, 4>(st, P, off);
