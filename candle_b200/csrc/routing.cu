@@ -327,85 +327,91 @@ router_topk_kernel(const float* __restrict__ x, const float* __restrict__ wg, co
 
 // Many tokens and many experts (prefill of a fine-grained layer): the router product as a tiled f32 GEMM.  The
 // one-token kernels spend their time in warp reductions -- one per (token, expert) -- which for 60 experts and 4096
-// tokens is most of 0.15 ms.  Here a CTA takes 32 tokens x all experts: x and the router rows pass through shared
-// memory in K chunks of 32 (the next chunk is fetched into registers while this one is multiplied), thread (token t,
-// group g) accumulates token t against experts g, g + 8, ... in registers with no reduction at all, and the eight
-// warps then do the softmax and the selection of four tokens each.  Every logit is a plain sequential f32 sum over K
-// (another order than the one-token kernels': last-bit differences, as between any two f32 dot products).  No fused
-// quantization: used where the activations are quantized by a pass of their own (Q8_0 experts).  Measured (60
-// experts, d = 2048, 4096 tokens): 155 -> 98 us; a variant with 64-wide chunks double-buffered by cp.async took 133 us.
-constexpr int RT_TOK = 32, RT_KC = 32, RT_PAD = 36, RT_EPT = CANDLE_MOE_MAX_EXPERTS / 8;
-__global__ void __launch_bounds__(256)
+// tokens is most of 0.15 ms.  Here a CTA of 128 threads takes 16 tokens x up to 64 experts at a time: x and the router rows
+// pass through shared memory in K chunks of 64 (the next chunk is fetched into registers while this one is multiplied), a
+// thread accumulates 2 tokens x 4 experts in registers, six 128-bit shared loads per 32 multiply-adds, and the four warps
+// then do the softmax and the selection of four tokens each.  Every logit is one sequential f32 sum over K (another order than
+// the one-token kernels': last-bit differences, as between any two f32 dot products).  No fused quantization: used where the
+// activations are quantized by a pass of their own (Q8_0 experts).  Bound by the multiply-adds (15 us for 60 experts,
+// d = 2048, 4096 tokens), the shared loads and the latency of the chunks.  Measured there: one token x eight experts per
+// thread, 32 tokens per CTA of 256 threads (nine shared loads, a CTA per SM) 93 us; this 70 us. (Four K slices per CTA took 47 us, but add a
+// logit in four parts, and near ties then fall the other way more often than one sequential sum lets them.)
+constexpr int RT_TOK = 16, RT_EXP = 64, RT_KC = 64, RT_PAD = RT_KC + 4, RT_THREADS = 128;
+__global__ void __launch_bounds__(RT_THREADS)
 router_topk_tiled_kernel(const float* __restrict__ x, const float* __restrict__ wg, const float* __restrict__ bias,
                          int64_t T, int d, int E, int k, int renorm, uint32_t* __restrict__ ids, float* __restrict__ wout) {
     pdl_trigger();
     pdl_wait();
     __shared__ __align__(16) float s_x[RT_TOK][RT_PAD];
-    __shared__ __align__(16) float s_w[CANDLE_MOE_MAX_EXPERTS][RT_PAD];
-    __shared__ float s_logits[8][CANDLE_MOE_MAX_EXPERTS];
+    __shared__ __align__(16) float s_w[RT_EXP][RT_PAD];
+    __shared__ float s_logits[RT_TOK][CANDLE_MOE_MAX_EXPERTS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t t0 = (int64_t)blockIdx.x * RT_TOK;
-    const int n_ept = (E + 7) / 8;  // experts per thread
-    // loads: thread -> (row tid / 8, float4 tid % 8) of the x chunk; the router chunk takes E * 8 float4, tid, tid + 256, ...
-    const float4* xsrc = reinterpret_cast<const float4*>(x + min(t0 + (tid >> 3), T - 1) * (int64_t)d) + (tid & 7);
-    float acc[RT_EPT];
+    const int tg = lane & 7, eg = warp * 4 + (lane >> 3);  // tokens tg, tg + 8; experts eg + 16 j
+    const int col = tid & 15, row = tid >> 4;              // loads: float4 column, row + 8 i
+    for (int e0 = 0; e0 < E; e0 += RT_EXP) {
+        float acc[2][4];
 #pragma unroll
-    for (int i = 0; i < RT_EPT; ++i) acc[i] = 0.f;
-    const int n_w4 = E * 8;
-    float4 px = xsrc[0], pw[4];
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int u = tid + 256 * i;
-        pw[i] = u < n_w4 ? reinterpret_cast<const float4*>(wg + (int64_t)(u >> 3) * d)[u & 7] : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        // rows past the end repeat the last one (their results are not used); columns past d are not read
+        const float4* px[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) px[i] = reinterpret_cast<const float4*>(x + min(t0 + row + 8 * i, T - 1) * (int64_t)d) + col;
+        float4 vx[2], vw[8];
+        auto fetch = [&](int c) {
+            if (c + 4 * col < d) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) vx[i] = px[i][c >> 2];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    vw[i] = reinterpret_cast<const float4*>(wg + (int64_t)min(e0 + row + 8 * i, E - 1) * d + c)[col];
+            }
+        };
+        fetch(0);
+        for (int c = 0; c < d; c += RT_KC) {
+            __syncthreads();  // the previous chunk has been consumed
+#pragma unroll
+            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(&s_x[row + 8 * i][4 * col]) = vx[i];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(&s_w[row + 8 * i][4 * col]) = vw[i];
+            __syncthreads();
+            if (c + RT_KC < d) fetch(c + RT_KC);  // the next chunk travels while this one is multiplied
+            const int n4 = min(RT_KC, d - c) >> 2;
+#pragma unroll 8
+            for (int k4 = 0; k4 < n4; ++k4) {
+                float4 xv[2], wv[4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) xv[i] = *reinterpret_cast<const float4*>(&s_x[tg + 8 * i][4 * k4]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) wv[j] = *reinterpret_cast<const float4*>(&s_w[eg + 16 * j][4 * k4]);
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]);
+                        acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
+                        acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]);
+                        acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
+                    }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int e = e0 + eg + 16 * j;
+                if (e < E) s_logits[tg + 8 * i][e] = acc[i][j] + (bias ? bias[e] : 0.f);
+            }
     }
-    for (int c = 0; c < d; c += RT_KC) {
-        __syncthreads();  // the previous chunk has been consumed
-        *reinterpret_cast<float4*>(&s_x[tid >> 3][4 * (tid & 7)]) = px;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int u = tid + 256 * i;
-            if (u < n_w4) *reinterpret_cast<float4*>(&s_w[u >> 3][4 * (u & 7)]) = pw[i];
-        }
-        __syncthreads();
-        if (c + RT_KC < d) {  // the next chunk travels while this one is multiplied
-            px = xsrc[(c + RT_KC) >> 2];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int u = tid + 256 * i;
-                if (u < n_w4) pw[i] = reinterpret_cast<const float4*>(wg + (int64_t)(u >> 3) * d + c + RT_KC)[u & 7];
-            }
-        }
-#pragma unroll
-        for (int k4 = 0; k4 < RT_KC / 4; ++k4) {
-            const float4 xv = *reinterpret_cast<const float4*>(&s_x[lane][4 * k4]);
-#pragma unroll
-            for (int i = 0; i < RT_EPT; ++i) {
-                if (i < n_ept) {
-                    const float4 wv = *reinterpret_cast<const float4*>(&s_w[warp + 8 * i][4 * k4]);  // one address per warp
-                    acc[i] = fmaf(xv.x, wv.x, acc[i]);
-                    acc[i] = fmaf(xv.y, wv.y, acc[i]);
-                    acc[i] = fmaf(xv.z, wv.z, acc[i]);
-                    acc[i] = fmaf(xv.w, wv.w, acc[i]);
-                }
-            }
-        }
-    }
-    // four rounds of eight tokens: logits to shared memory, then warp w selects for token 8 * round + w
-    for (int round = 0; round < RT_TOK / 8; ++round) {
-        __syncthreads();
-        if ((lane >> 3) == round) {  // this thread's token is lane: tokens 8 round .. 8 round + 7 in this round
-#pragma unroll
-            for (int i = 0; i < RT_EPT; ++i) {
-                const int e = warp + 8 * i;
-                if (i < n_ept && e < E) s_logits[lane & 7][e] = acc[i] + (bias ? bias[e] : 0.f);
-            }
-        }
-        __syncthreads();
-        const int64_t t = t0 + 8 * round + warp;
+    __syncthreads();
+    for (int i = warp; i < RT_TOK; i += RT_THREADS / 32) {
+        const int64_t t = t0 + i;
         if (t < T) {
             float sel_p[CANDLE_MOE_MAX_TOPK];
             int sel_e[CANDLE_MOE_MAX_TOPK];
-            softmax_topk_warp(s_logits[warp], lane, E, k, renorm, ids + t * k, wout + t * k, sel_p, sel_e);
+            softmax_topk_warp(s_logits[i], lane, E, k, renorm, ids + t * k, wout + t * k, sel_p, sel_e);
         }
     }
 }
@@ -426,9 +432,9 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
                         renorm, ids, w, qs, scales, bsums, counts, offsets, perm_token, pair_pos);
     }
     if (norm_w) return cudaErrorInvalidValue;
-    if (T >= 512 && E >= 16 && !qs && !counts && d % RT_KC == 0)
-        return launch_k(router_topk_tiled_kernel, dim3((unsigned)((T + RT_TOK - 1) / RT_TOK)), dim3(256), 0, st, x, router, bias, T, d, E, k,
-                        renorm, ids, w);
+    if (T >= 512 && E >= 16 && !qs && !counts && d % 32 == 0)
+        return launch_k(router_topk_tiled_kernel, dim3((unsigned)((T + RT_TOK - 1) / RT_TOK)), dim3(RT_THREADS), 0, st, x, router, bias, T, d,
+                        E, k, renorm, ids, w);
     return launch_k(router_topk_kernel, dim3((unsigned)T), dim3(ROUTER_THREADS), 0, st, x, router, bias, d, E, k, renorm, ids, w, qs, scales,
                     bsums, counts, offsets, perm_token, pair_pos);
 }

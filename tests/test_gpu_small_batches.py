@@ -33,6 +33,28 @@ def test_router_at_the_edges_of_its_forms(orc, torch_cuda, E, k):
             assert np.allclose(w.cpu().numpy()[same], w_ref[same], rtol=5e-5, atol=1e-7), (d, T)
 
 
+@pytest.mark.parametrize("E,k", [(16, 2), (60, 4), (64, 8), (65, 3), (128, 8)])
+def test_tiled_router(orc, torch_cuda, E, k):
+    """Many tokens and experts: fewer K chunks than slices, a ragged last token tile, one and two passes over the experts."""
+    torch = torch_cuda
+    from candle_b200 import _lib
+    for d, T in ((32, 512), (96, 513), (1056, 543)):
+        rng = np.random.default_rng(E + d)
+        x = rng.standard_normal((T, d), dtype=np.float32)
+        wg = rng.standard_normal((E, d), dtype=np.float32) * np.float32(0.05)
+        bias = rng.standard_normal(E, dtype=np.float32)
+        probs, ids_ref, w_ref = orc.router_topk(x, wg, k, True, bias)
+        xd, wd, bd = (torch.from_numpy(a).cuda() for a in (x, wg, bias))
+        ids = torch.empty((T, k), dtype=torch.int32, device="cuda")
+        w = torch.empty((T, k), dtype=torch.float32, device="cuda")
+        assert _lib.load().candle_moe_router_topk(torch.cuda.current_stream().cuda_stream, xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), T, d, E,
+                                                  k, 1, ids.data_ptr(), w.data_ptr()) == 0
+        got = ids.cpu().numpy().astype(np.uint32)
+        H.check_routing(probs, ids_ref, got)
+        same = (ids_ref == got).all(axis=1)
+        assert np.allclose(w.cpu().numpy()[same], w_ref[same], rtol=5e-5, atol=1e-7), (d, T)
+
+
 @pytest.mark.parametrize("T", [1, 2, 64, 65])
 def test_layer_equals_norm_block_residual_in_three_steps(orc, torch_cuda, T):
     torch = torch_cuda
