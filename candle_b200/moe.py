@@ -16,7 +16,7 @@ from typing import List, Optional
 import torch
 
 from . import _lib
-from .quantized import GgmlDType, QMatMul, QTensor, _stream_ptr
+from .quantized import GgmlDType, QMatMul, QTensor, _on_device, _stream_ptr
 
 
 @dataclass
@@ -105,8 +105,7 @@ class MlpOrMoe:
 
     def prepack(self) -> "MlpOrMoe":
         """Make the optional repacked copies of every expert matrix (one-time, doubles the weight memory of this
-        block): k-quants for the decode kernels (batches of up to 96 rows) and Q6_K in the large-batch GEMM, Q8_0 for
-        the large-batch GEMM."""
+        block): for the decode kernels (batches of up to 96 rows), and Q6_K and Q8_0 in the large-batch GEMM."""
         def copies(mats):
             # every matrix of the family or none: a shape the repack does not take (CANDLE_MOE_E_SHAPE, e.g. Q6_K rows
             # with an odd number of 256-blocks) leaves the family on its GGUF blocks
@@ -164,7 +163,7 @@ class MlpOrMoe:
         T = x2.shape[0]
         self.reserve(max(T, 1))
         y = out if out is not None else torch.empty_like(x2)
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             st = _lib.load().candle_moe_forward(_stream_ptr(self.device), C.byref(self._cw), x2.data_ptr(), T,
                                                 y.data_ptr(), self._ws_ptr(), self._ws.numel() - 256)
         _lib.check("candle_moe_forward", st)
@@ -188,7 +187,7 @@ class MlpOrMoe:
             self._ws = torch.empty(need.value + 256, dtype=torch.uint8, device=self.device)
             self._ws_tokens = T
         y = torch.empty_like(x2)
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             st = L.candle_moe_ffn_layer(_stream_ptr(self.device), C.byref(self._cw), nw.data_ptr(), float(eps), x2.data_ptr(), T,
                                         y.data_ptr(), self._ws_ptr(), self._ws.numel() - 256)
         _lib.check("candle_moe_ffn_layer", st)

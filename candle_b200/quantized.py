@@ -7,6 +7,7 @@ GGUF blocks, row-major `[n][k / block]`, exactly the bytes `QCudaStorage` keeps
 """
 from __future__ import annotations
 
+import contextlib
 import enum
 from typing import Optional, Tuple
 
@@ -34,6 +35,15 @@ class GgmlDType(enum.IntEnum):
 
 def _stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def _on_device(device: torch.device):
+    """`torch.cuda.device(device)`, or nothing to enter and leave where that device is current already (the call sits on
+    the path of every small product, whose kernels take a few microseconds)."""
+    return _NO_GUARD if device.index is None or device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 class QTensor:
@@ -144,21 +154,21 @@ class QMatMul:
 
     def forward(self, xs: torch.Tensor) -> torch.Tensor:
         """`QMatMul::forward` (mod.rs:533-537) through `candle_moe_qmatmul`."""
-        import ctypes as C
         lib = _lib.load()
         n, k = self.inner.shape()
         if xs.shape[-1] != k:
             raise ValueError(f"shape mismatch in qmatmul: {tuple(xs.shape)} x ({n}, {k})^T")
         if not xs.is_cuda or xs.dtype != torch.float32:
             raise ValueError("QMatMul.forward expects a CUDA f32 tensor")
-        lead = xs.shape[:-1]
-        x2 = xs.reshape(-1, k).contiguous()
+        flat = xs.dim() == 2
+        x2 = xs if flat and xs.is_contiguous() else xs.reshape(-1, k).contiguous()
         rows = x2.shape[0]
         dev, dt = x2.device, int(self.inner.dtype())
         out = torch.empty((rows, n), dtype=torch.float32, device=dev)
         if rows == 0:
-            return out.reshape(*lead, n)
+            return out.reshape(*xs.shape[:-1], n)
         if self._ws is None or rows > self._ws_rows:
+            import ctypes as C
             need = C.c_size_t(0)
             cap = max(rows, 2 * self._ws_rows)
             _lib.check("candle_moe_qmatmul_workspace_bytes", lib.candle_moe_qmatmul_workspace_bytes(dt, cap, n, k, C.byref(need)))
@@ -170,10 +180,10 @@ class QMatMul:
             self._ws_rows = cap
         ws_ptr = (self._ws.data_ptr() + 255) // 256 * 256
         pp = None if self._prepacked is None else self._prepacked.data_ptr()
-        with torch.cuda.device(dev):
+        with _on_device(dev):
             _lib.check("candle_moe_qmatmul",
                        lib.candle_moe_qmatmul(_stream_ptr(dev), self.inner.device_ptr(), pp, dt, n, k, x2.data_ptr(), rows,
                                               out.data_ptr(), ws_ptr, self._ws.numel() - 256))
-        return out.reshape(*lead, n)
+        return out if flat else out.reshape(*xs.shape[:-1], n)
 
     __call__ = forward
