@@ -373,14 +373,18 @@ def block_launches(cfg, T, prepacked, gemm_min_rows):
     gemm = T > gemm_min_rows
     def product(dt, E, takes_gemm):
         if gemm and takes_gemm:
-            return 1 + (maps(E) if dt in (12, 8) else 0) + 1                    # operand preparation, maps, GEMM
+            return 1 + (maps(E) if dt == 12 else 0) + 1                         # operand preparation, maps, GEMM
         return 1
     k13 = cfg["dt13"] == 12 or (prepacked and cfg["dt13"] in (14, 8))
     k2 = cfg["dt2"] == 12 or (prepacked and cfg["dt2"] in (14, 8))
-    n += product(cfg["dt13"], cfg["E"], k13) + 1 + product(cfg["dt2"], cfg["E"], k2) + 1  # gate_up, quantize h, down, combine
+    quantize_h = 0 if gemm and k2 else 1                                        # with the GEMM part of its operand preparation
+    n += product(cfg["dt13"], cfg["E"], k13) + quantize_h + product(cfg["dt2"], cfg["E"], k2) + 1  # gate_up, quantize h, down, combine
     if cfg["ff_shared"]:
         sh = prepacked and q8
-        n += 1 + (0 if q8 else 1) + product(cfg["dt13"], 1, sh) + 1 + product(cfg["dt2"], 1, sh)  # offsets, (x), gate_up, quantize, down
+        if sh and not gemm:
+            n += 1                                                              # its products join the routed launches
+        else:
+            n += (0 if q8 else 2) + product(cfg["dt13"], 1, sh) + (0 if sh else 1) + product(cfg["dt2"], 1, sh)  # (offsets, x), gate_up, quantize, down
     return n
 
 
@@ -927,7 +931,7 @@ def run_c3(args):
             "cpu_baseline": None,
             "e2e": {"value": B * world / (ms_e2e * 1e-3), "unit": "tokens/s", "h2d_bytes_per_step": B * 8,
                     "d2h_bytes_per_step": B * cfg.vocab * 4, "ms_per_step": ms_e2e},
-            "gpu_launches": cfg.n_layer * (1 + 6 + 1 + 2 + 6 + 7) * args.steps,
+            "gpu_launches": (cfg.n_layer * (1 + 2 + 1 + 2 + 2 + 6) + 3) * args.steps,  # norm, qkv, rope, attention, wo, ffn; norm, head
             "finite": bool(torch.isfinite(logits).all()),
             "clocks": clocks,
         }

@@ -85,7 +85,8 @@ typedef struct candle_moe_weights {
     const void* const* w1_prepacked;
     const void* const* w3_prepacked;
     const void* const* w2_prepacked;
-    /* The same for the shared expert (device pointers or NULL; Q8_0 only: large batches then take the tensor-core GEMM). */
+    /* The same for the shared expert (device pointers or NULL; Q8_0 only: small batches then take the
+     * decode kernels, large ones the tensor-core GEMM). */
     const void* shared_w1_prepacked;
     const void* shared_w3_prepacked;
     const void* shared_w2_prepacked;
@@ -361,9 +362,9 @@ CANDLE_MOE_API int candle_moe_decode_attention(void* stream, const float* q, con
 /* One-time repack of a Q4_K / Q6_K matrix [n_rows, k] (n_rows a multiple of 8 -- 16 for w2 --, k a
  * multiple of 256) into the register-fragment order the decode kernels read with coalesced
  * 128-bit loads.  Q4_K grows by 2.8 % (its 12-byte packed 6-bit scales are widened to 16 bytes),
- * Q6_K keeps its size.  A Q8_0 matrix (k a multiple of 32) is repacked for the large-batch tensor-core GEMM instead:
- * per row and 256 elements a 16-byte aligned record of 256 int8 values and 8 f16 scales (the 34-byte GGUF blocks are
- * only 2-byte aligned), rows padded with zero records to a multiple of 256 elements (+6 %, more for short rows).
+ * Q6_K keeps its size.  A Q8_0 matrix (k a multiple of 32) is repacked the same way for the decode kernels and the
+ * large-batch tensor-core GEMM: per 8 rows and 128 elements 1024 bytes of quants and 64 of f16 scales (the 34-byte GGUF
+ * blocks are only 2-byte aligned), rows padded with zeros to a multiple of 256 elements.
  * No counterpart in the reference, whose kernels read the GGUF layout
  * directly (candle-kernels/src/quantized.cu:2626-2698); optional here as well.
  *   candle_moe_prepacked_bytes: size of the destination buffer (0 bytes = shape or dtype not supported)
