@@ -369,7 +369,7 @@ def block_launches(cfg, T, prepacked, gemm_min_rows):
     q8 = cfg["dt13"] == 8
     pairs = T * cfg["k"]
     n = 1 + (0 if T == 1 else (3 if pairs > 2048 else 1)) + (1 if q8 else 0)  # router (+ x quantization fused unless Q8_0), dispatch
-    maps = lambda E: (2 * E + 15) // 16                                        # tensor-map copies, 16 maps per launch
+    maps = lambda E: (2 * E + 15) // 16 - 1                                    # tensor-map copies beyond the 16 of the preparation
     gemm = T > gemm_min_rows
     def product(dt, E, takes_gemm):
         if gemm and takes_gemm:

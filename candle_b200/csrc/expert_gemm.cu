@@ -57,6 +57,27 @@ constexpr int G_TMEM_COLS = 512;
 constexpr int G_TM_MAIN = 0;    // + 128 * buffer
 constexpr int G_TM_A = 256;     // weight operand ring: columns 256..511
 
+// Tensor maps of the weight matrices reach device memory as kernel PARAMETERS -- of the operand preparation that runs before the
+// GEMM anyway, and of a small copy kernel for what does not fit there -- never
+// from host memory on the stream: a copy node recorded while a stream is being captured into a CUDA graph reads
+// its host source again at every replay, long after the array it pointed to has gone.
+constexpr int MAPS_PER_CHUNK = 16;
+struct MapChunk {
+    CUtensorMap m[MAPS_PER_CHUNK];
+    CUtensorMap* dst;
+    int n;  // 0: none
+};
+__device__ __forceinline__ void write_maps(const MapChunk& c) {  // by one CTA, after the previous user of the scratch has finished
+    const uint4* src = reinterpret_cast<const uint4*>(c.m);
+    uint4* d = reinterpret_cast<uint4*>(c.dst);
+    for (int i = threadIdx.x; i < c.n * (int)(sizeof(CUtensorMap) / 16); i += blockDim.x) d[i] = src[i];
+}
+__global__ void __launch_bounds__(128) write_maps_kernel(const __grid_constant__ MapChunk c) {
+    pdl_trigger();
+    pdl_wait();
+    write_maps(c);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Operand preparation: the int8 activation rows in grouped order as fp16 (B operand), the block scales
 // transposed to [block][position], and the activation side of the Q4_K min term (below).
@@ -79,9 +100,10 @@ __device__ __forceinline__ float tf32_head(float v) { return __uint_as_float((__
 __global__ void __launch_bounds__(256)
 prep_gemm_b_kernel(const int8_t* __restrict__ aq, const float* __restrict__ ascale, const int16_t* __restrict__ absum,
                    const uint32_t* __restrict__ row_of, int P, int P_pad, int K, __half* __restrict__ bf16,
-                   float* __restrict__ bmin, float* __restrict__ d8t) {
+                   float* __restrict__ bmin, float* __restrict__ d8t, const __grid_constant__ MapChunk maps) {
     pdl_trigger();
     pdl_wait();
+    if (blockIdx.x == 0) write_maps(maps);
     const int kb = K >> 8;
     const int lane = threadIdx.x & 31;
     const int64_t unit = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // (p, block)
@@ -166,9 +188,10 @@ prep_gemm_b_q80_kernel(const int8_t* __restrict__ aq, const float* __restrict__ 
 constexpr int PREP_UNITS = 2;
 __global__ void __launch_bounds__(256)
 prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, __half* __restrict__ bf16, float* __restrict__ bmin,
-                         float* __restrict__ d8t, uint32_t* __restrict__ single_group) {
+                         float* __restrict__ d8t, uint32_t* __restrict__ single_group, const __grid_constant__ MapChunk maps) {
     pdl_trigger();
     pdl_wait();
+    if (blockIdx.x == 0) write_maps(maps);
     if (single_group && blockIdx.x == 0 && threadIdx.x < 2) single_group[threadIdx.x] = threadIdx.x ? (uint32_t)P : 0u;
     const int kb = K >> 8;
     const int lane = threadIdx.x & 31;
@@ -1185,21 +1208,6 @@ bool make_map_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64_t 
 
 int g_gemm_sms = -1;
 
-// Tensor maps of the weight matrices reach device memory as kernel PARAMETERS of a small copy kernel, never
-// from host memory on the stream: a copy node recorded while a stream is being captured into a CUDA graph reads
-// its host source again at every replay, long after the array it pointed to has gone.
-constexpr int MAPS_PER_CHUNK = 16;
-struct MapChunk {
-    CUtensorMap m[MAPS_PER_CHUNK];
-};
-__global__ void __launch_bounds__(128) write_maps_kernel(const __grid_constant__ MapChunk c, CUtensorMap* dst, int n) {
-    pdl_trigger();
-    pdl_wait();  // the previous user of this scratch has finished
-    const uint4* src = reinterpret_cast<const uint4*>(&c);
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    for (int i = threadIdx.x; i < n * (int)(sizeof(CUtensorMap) / 16); i += blockDim.x) d[i] = src[i];
-}
-
 template <class F, bool GATE_UP, int TN>
 cudaError_t launch_gemm_kernel(cudaStream_t st, const GemmParams& G, const CUtensorMap& map_b, const CUtensorMap& map_bs) {
     const int smem_bytes = G_B_STAGES * (4 + (F::HAS_MIN ? 1 : 0)) * (TN * G_SLAB_K * 2) + (F::HAS_MIN ? 2 : 0) * G_TILE_BYTES +
@@ -1271,20 +1279,45 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     float* d8t = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bmin) + align_up((size_t)p_pad * kb * 32 * 4, 256));
     const bool has_min = dtype == CANDLE_GGML_Q4K;
 
+    // byte-matrix tensor maps of the raw weight blocks (Q4_K): [n_rows, kb * 144] with boxes of 64 rows x one block, written to
+    // the scratch on the stream before the kernel: the first chunk by the operand preparation, more (beyond eight experts) by
+    // copy kernels
+    CUtensorMap* wmaps_dev = reinterpret_cast<CUtensorMap*>(reinterpret_cast<uint8_t*>(d8t) + align_up((size_t)kb * p_pad * 4, 256));
+    MapChunk first{};
+    cudaError_t e;
+    if (dtype == CANDLE_GGML_Q4K) {
+        const uint64_t n_rows = (uint64_t)N, rb = (uint64_t)kb * Q4K_BYTES;
+        for (int m0 = 0; m0 < 2 * E; m0 += MAPS_PER_CHUNK) {
+            MapChunk chunk{};
+            chunk.dst = wmaps_dev + m0;
+            chunk.n = std::min(MAPS_PER_CHUNK, 2 * E - m0);
+            for (int i = 0; i < chunk.n; ++i) {
+                const int e2 = (m0 + i) >> 1;
+                const uint8_t* wp = ((m0 + i) & 1) && gate_up ? wb.p[e2] : wa.p[e2];
+                if (!make_map_bytes(&chunk.m[i], wp, n_rows, rb, Q4K_BYTES, 64)) return cudaErrorNotSupported;
+            }
+            if (m0 == 0) {
+                first = chunk;
+            } else {
+                e = launch_k(write_maps_kernel, dim3(1), dim3(128), 0, st, chunk);
+                if (e != cudaSuccess) return e;
+            }
+        }
+    }
+
     const int64_t units = p_pad * kb;
     const int64_t per_cta = 8 * (x_f32 ? PREP_UNITS : 1);
     const dim3 prep_grid((unsigned)((units + per_cta - 1) / per_cta));
-    cudaError_t e;
     if (x_f32)
         e = q80 ? launch_k(prep_gemm_f32_q80_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K_in, K, q80x ? 1 : 0, bf16,
                            d8t, single_group)
                 : launch_k(prep_gemm_f32_q8k_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K, bf16,
-                           has_min ? bmin : (float*)nullptr, d8t, single_group);
+                           has_min ? bmin : (float*)nullptr, d8t, single_group, first);
     else
         e = q80 ? launch_k(prep_gemm_b_q80_kernel, prep_grid, dim3(256), 0, st, aq, ascale, row_of, (int)P, (int)p_pad, K_in, K,
                            q80x ? 1 : 0, bf16, d8t)
                 : launch_k(prep_gemm_b_kernel, prep_grid, dim3(256), 0, st, aq, ascale, absum, row_of, (int)P, (int)p_pad, K, bf16,
-                           has_min ? bmin : (float*)nullptr, d8t);
+                           has_min ? bmin : (float*)nullptr, d8t, first);
     if (e != cudaSuccess) return e;
 
     CUtensorMap map_b, map_bs;
@@ -1292,25 +1325,6 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         return cudaErrorNotSupported;
     if (!make_map_2d(&map_bs, bmin, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)p_pad, (uint64_t)kb * 32, 32, tn))
         return cudaErrorNotSupported;
-
-    // byte-matrix tensor maps of the raw weight blocks (Q4_K): [n_rows, kb * 144] with boxes of 64 rows x one block,
-    // written to the head of the scratch on the stream before the kernel
-    CUtensorMap* wmaps_dev = reinterpret_cast<CUtensorMap*>(reinterpret_cast<uint8_t*>(d8t) + align_up((size_t)kb * p_pad * 4, 256));
-    if (dtype == CANDLE_GGML_Q4K) {
-        const uint64_t n_rows = (uint64_t)N, rb = (uint64_t)kb * Q4K_BYTES;
-        for (int m0 = 0; m0 < 2 * E; m0 += MAPS_PER_CHUNK) {
-            MapChunk chunk;
-            const int n_maps = std::min(MAPS_PER_CHUNK, 2 * E - m0);
-            for (int i = 0; i < n_maps; ++i) {
-                const int e2 = (m0 + i) >> 1;
-                const uint8_t* wp = ((m0 + i) & 1) && gate_up ? wb.p[e2] : wa.p[e2];
-                if (!make_map_bytes(&chunk.m[i], wp, n_rows, rb, Q4K_BYTES, 64)) return cudaErrorNotSupported;
-            }
-            for (int i = n_maps; i < MAPS_PER_CHUNK; ++i) chunk.m[i] = chunk.m[0];
-            e = launch_k(write_maps_kernel, dim3(1), dim3(128), 0, st, chunk, wmaps_dev + m0, n_maps);
-            if (e != cudaSuccess) return e;
-        }
-    }
 
     GemmParams G{};
     G.wmaps = wmaps_dev;

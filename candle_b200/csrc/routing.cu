@@ -334,8 +334,8 @@ router_topk_kernel(const float* __restrict__ x, const float* __restrict__ wg, co
 // the one-token kernels': last-bit differences, as between any two f32 dot products).  No fused quantization: used where the
 // activations are quantized by a pass of their own (Q8_0 experts).  Bound by the multiply-adds (15 us for 60 experts,
 // d = 2048, 4096 tokens), the shared loads and the latency of the chunks.  Measured there: one token x eight experts per
-// thread, 32 tokens per CTA of 256 threads (nine shared loads, a CTA per SM) 93 us; this 70 us. (Four K slices per CTA took 47 us, but add a
-// logit in four parts, and near ties then fall the other way more often than one sequential sum lets them.)
+// thread, 32 tokens per CTA of 256 threads (nine shared loads, a CTA per SM) 93 us; this 70 us.  (Four K slices per CTA took
+// 47 us, but add a logit in four parts: kept as one sum, so that the logits stay what they were bit for bit.)
 constexpr int RT_TOK = 16, RT_EXP = 64, RT_KC = 64, RT_PAD = RT_KC + 4, RT_THREADS = 128;
 __global__ void __launch_bounds__(RT_THREADS)
 router_topk_tiled_kernel(const float* __restrict__ x, const float* __restrict__ wg, const float* __restrict__ bias,
