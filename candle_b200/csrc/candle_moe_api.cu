@@ -440,7 +440,9 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     // over repacked Q8_0 copies the shared expert takes the decode kernels -- in the launches of the routed experts where those
     // are Q8_0 too -- and for large batches the tensor-core GEMM
     const bool sh_packed = w->d_ff_shared > 0 && w->dtype_shared13 == CANDLE_GGML_Q8_0 && w->dtype_shared2 == CANDLE_GGML_Q8_0 &&
-                           w->shared_w1_prepacked && w->shared_w3_prepacked && w->shared_w2_prepacked;
+                           w->shared_w1_prepacked && w->shared_w3_prepacked && w->shared_w2_prepacked &&
+                           !((reinterpret_cast<uintptr_t>(w->shared_w1_prepacked) | reinterpret_cast<uintptr_t>(w->shared_w3_prepacked) |
+                              reinterpret_cast<uintptr_t>(w->shared_w2_prepacked)) & 15);
     const bool sh_gemm = sh_packed && ws.gemm && T > gemm_min_rows() && gemm_enabled();
     const bool sh_direct = sh_packed && !sh_gemm && T <= std::max<int64_t>(gemm_min_rows(), 64);
     SharedRun sr;
@@ -893,7 +895,8 @@ int candle_moe_qmatmul(void* stream, const void* w, const void* w_prepacked, int
     // The decode kernels over the repacked copy of a k-quant are not used here: with a single group their tiles are too few and
     // too short, and the streaming form over the GGUF blocks is faster (measured, [4096, 4096] Q4_K / [32000, 4096]
     // Q6_K: 1 row 10.8 / 44.5 us against 17.2 / 46.2; 8 rows 13.5 / 48.6 against 17.7 / 60.1).
-    if (dtype == CANDLE_GGML_Q8_0 && w_prepacked && rows <= QMM_DIRECT_MAX_ROWS) {
+    // (a copy made by candle_moe_prepack is 16-byte aligned; anything else is left alone)
+    if (dtype == CANDLE_GGML_Q8_0 && w_prepacked && !(reinterpret_cast<uintptr_t>(w_prepacked) & 15) && rows <= QMM_DIRECT_MAX_ROWS) {
         const cudaError_t ce = launch_expert_direct(st, false, pp, pp, dtype, 1, k, n, ws.offsets, nullptr, rows, ws.xq, ws.xs, ws.xb,
                                                     dst, &splits, stride, ws.slots, 1, rows, out);
         if (ce == cudaSuccess)

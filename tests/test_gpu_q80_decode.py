@@ -49,3 +49,17 @@ def test_q80_block_over_the_repacked_copies(orc, torch_cuda, T, d, ff, E, k, fs)
     H.check_routing(orc.router_topk(xs, mw.router, k, False, None)[0], ref.topk_ids, blk.last_routing(T)[0].numpy().astype(np.uint32))
     got = y.cpu().numpy()
     assert H.max_rel(got[same], ref.y[same]) <= loose * H.MAX_REL_TOL and H.rel_l2(got[same], ref.y[same]) <= loose * H.REL_L2_TOL
+
+
+def test_q80_projection_ignores_a_copy_it_cannot_read(orc, torch_cuda):
+    """The decode kernels copy 16-byte vectors: a pointer that candle_moe_prepack cannot have filled is left alone."""
+    torch = torch_cuda
+    from candle_b200 import GgmlDType, QMatMul, QTensor
+    n, k, m = 64, 256, 5
+    rng = np.random.default_rng(1)
+    wq = orc.quantize(orc.Q8_0, rng.standard_normal((n, k), dtype=np.float32) * np.float32(0.02))
+    x = rng.standard_normal((m, k), dtype=np.float32)
+    mm = QMatMul.from_qtensor(QTensor.from_blocks(wq, GgmlDType.Q8_0, (n, k))).prepack()
+    mm._prepacked = torch.cat([torch.zeros(8, dtype=torch.uint8, device="cuda"), mm._prepacked])[8:]
+    assert mm._prepacked.data_ptr() % 16 == 8
+    assert H.rel_l2(mm.forward(torch.from_numpy(x).cuda()).cpu().numpy(), orc.matmul(orc.Q8_0, x, wq, n)) < 1e-6
