@@ -165,7 +165,7 @@ __device__ __forceinline__ void dispatch_one_token(const int (&sel_e)[CANDLE_MOE
     }
 }
 
-// Few tokens (up to 64): 1024 threads per token, latency-bound.  The row passes through shared memory once, with the
+// Few tokens: 1024 threads per token, latency-bound.  The row passes through shared memory once, with the
 // layer's RmsNorm applied on the way where the caller asks for it (norm_w; one launch fewer), and every warp owns whole
 // dot products: expert e, or for few experts one of `parts` pieces of it, so that all loads of a round are in flight at
 // once and one reduction per expert and warp is left.  (Eight experts at a time across all warps, eight reductions per
@@ -254,7 +254,10 @@ router_topk_small_kernel(const float* __restrict__ x, const float* __restrict__ 
     softmax_topk_warp(s_logits, lane, E, k, renorm, ids + t * k, wout + t * k, sel_p, sel_e);
     if (counts) dispatch_one_token(sel_e, lane, E, k, counts, offsets, perm_token, pair_pos);
 }
-constexpr int ROUTER_SMALL_TOKENS = 64, ROUTER_SMALL_MAX_D = 10240;  // the row in 40 KB of shared memory
+constexpr int ROUTER_SMALL_MAX_D = 10240;  // the row in 40 KB of shared memory
+// Up to 64 tokens; rows long enough to keep 1024 threads busy up to 256 (Mixtral-shaped layer, d = 4096: 100 rows 354.8 -> 345.5 us,
+// 140 rows 389 -> 375, 290 rows equal; d = 1024, 257 rows 77 against 86 us the other way round).
+static bool router_small(int64_t T, int d) { return d <= ROUTER_SMALL_MAX_D && (T <= 64 || (d >= 4096 && T <= 256)); }
 
 // Many tokens (and rows too long for the form above): 256 threads per token, so that eight CTAs share an SM and their
 // load rounds overlap.  The forms add the partial sums in different orders (last-bit differences of the logits, as between
@@ -417,7 +420,7 @@ router_topk_tiled_kernel(const float* __restrict__ x, const float* __restrict__ 
 }
 
 // the fused norm is there only where the small form runs
-bool router_fuses_norm(int64_t T, int d) { return T <= ROUTER_SMALL_TOKENS && d <= ROUTER_SMALL_MAX_D; }
+bool router_fuses_norm(int64_t T, int d) { return router_small(T, d); }
 
 cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* router, const float* bias, int64_t T,
                                int d, int E, int k, int renorm, uint32_t* ids, float* w, int8_t* qs, float* scales,
@@ -425,7 +428,7 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
                                const float* norm_w, float eps) {
     if (T == 0) return cudaSuccess;
     if (counts && (T != 1 || !offsets || !perm_token || !pair_pos)) return cudaErrorInvalidValue;  // single-token dispatch only
-    if (T <= ROUTER_SMALL_TOKENS && d <= ROUTER_SMALL_MAX_D) {
+    if (router_small(T, d)) {
         const int parts = E <= 4 ? 8 : (E <= 8 ? 4 : (E <= 16 ? 2 : 1));
         auto kfn = norm_w ? router_topk_small_kernel<true> : router_topk_small_kernel<false>;
         return launch_k(kfn, dim3((unsigned)T), dim3(1024), (size_t)d * sizeof(float), st, x, norm_w, eps, router, bias, d, E, parts, k,
