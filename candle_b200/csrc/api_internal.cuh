@@ -33,6 +33,8 @@ struct ExpertBufs {
     int16_t* hb;
     float* eo;      // [slots][P, d]
     void* gemm;     // scratch of the large-batch GEMM (may be null)
+    uint8_t* repack = nullptr;  // room for one expert's Q6_K matrices repacked on the way (null: that form is not used)
+    void* repack_gemm = nullptr;  // ... and that form's operand scratch
 };
 
 // The shared expert's products beside the routed ones (run_experts takes them where the decode kernels do): what each needs,

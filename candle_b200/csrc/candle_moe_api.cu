@@ -63,10 +63,25 @@ struct Workspace {
     int16_t* shb;
     float* so;  // [T, d]
     void* gemm;  // operand scratch of the large-batch tensor-core GEMM (null for decode-sized T)
-    size_t total;
+    void* repack_gemm;  // large batches over Q6_K without copies: operand scratch of that form (null: not enough workspace for it)
+    uint8_t* repack;    // ... and one expert's repacked matrices
+    size_t total;      // without that form
+    size_t total_ext;  // with it
 };
 
-Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_) {
+constexpr int REPACK_K_SPLITS = 2;
+// Q6_K as the GEMM reads it is the repacked layout.  Without copies a large batch (P rows over E experts) repacks one expert at a
+// time on its way through the GEMM, for shapes the repack takes (as candle_moe_prepack and the GEMM check them).  Against the
+// streaming form, which passes over an expert's weights once per 16 rows, that pays from about six passes on (Q4_K / Q6_K layer of
+// d = 4096, ff = 14336: 25 rows per expert 594 us streaming, 854 repacking; 75 rows 1180 / 979; 512 rows 6183 / 2659; Q6_K layer of
+// d = 2048, ff = 4096: 25 rows 213 / 504, 250 rows 1317 / 710); the streaming form does not take rows that are not 16-byte aligned,
+// and the row-per-warp form is slower at once (d = 1536, ff = 2560, 37 rows per expert 491 / 199 us).
+inline bool repacks_on_the_way(int dtype, bool has_copy, int n, int k, bool gate_up, int64_t P, int E) {
+    return dtype == CANDLE_GGML_Q6K && !has_copy && n % (gate_up ? 64 : 128) == 0 && k % 512 == 0 && (P >= 96 * (int64_t)E || k % 2048 != 0);
+}
+
+// avail: bytes behind base_ (the optional part is handed out only if it fits)
+Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_, size_t avail = 0) {
     uint8_t* base = static_cast<uint8_t*>(base_);
     Workspace ws{};
     size_t off = 0;
@@ -85,6 +100,7 @@ Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_) {
     ws.hq = carve<int8_t>(base, off, Tk * ff);
     ws.hs = carve<float>(base, off, Tk * ff / act_block(w->dtype_w2));
     ws.hb = carve<int16_t>(base, off, Tk * ff / 16);
+    size_t free_at = align_up(off, 256) + REPACK_K_SPLITS * Tk * d * sizeof(float);  // behind the partial outputs of that form
     ws.eo = carve<float>(base, off, Tk * d * k_split_slots(T));
     if (w->d_ff_shared > 0) {
         const size_t fs = w->d_ff_shared;
@@ -103,6 +119,7 @@ Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_) {
         ws.shs = carve<float>(base, off, (size_t)T * fs / act_block(w->dtype_shared2));
         ws.shb = carve<int16_t>(base, off, (size_t)T * fs / 16);
         ws.so = carve<float>(base, off, (size_t)T * d * k_split_slots(T));
+        free_at = off;
     }
     if (T > gemm_min_rows()) {
         // large batches: fp16 activation operand of the tcgen05 GEMM (Q4_K matrices), reused by gate_up and down
@@ -124,6 +141,25 @@ Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_) {
         }
     }
     ws.total = align_up(off, 256);
+    ws.total_ext = ws.total;
+    if (T > gemm_min_rows()) {
+        const bool r13 = repacks_on_the_way(w->dtype_w13, w->w1_prepacked && w->w3_prepacked, w->d_ff, w->d_model, true, (int64_t)Tk, w->n_experts);
+        const bool r2 = repacks_on_the_way(w->dtype_w2, w->w2_prepacked != nullptr, w->d_model, w->d_ff, false, (int64_t)Tk, w->n_experts);
+        if (r13 || r2) {
+            // The partial outputs it does not use and the GEMM's own scratch (the other product's, done or not begun) lie free
+            const size_t at = align_up(free_at, 1024);
+            const size_t operand = align_up(std::max(r13 ? expert_gemm_scratch_bytes((int64_t)Tk, (int)d) : 0,
+                                                     r2 ? expert_gemm_scratch_bytes((int64_t)Tk, (int)ff) : 0), 1024);
+            const size_t matrices = std::max(r13 ? 2 * prepacked_bytes(CANDLE_GGML_Q6K, (int64_t)ff, (int)d) : 0,
+                                             r2 ? prepacked_bytes(CANDLE_GGML_Q6K, (int64_t)d, (int)ff) : 0);
+            ws.total_ext = std::max(ws.total, align_up(at + operand + matrices, 256));
+            if (base && avail >= ws.total_ext) {
+                ws.repack_gemm = base + at;
+                ws.repack = base + at + operand;
+                if (!ws.gemm) ws.gemm = ws.repack_gemm;
+            }
+        }
+    }
     return ws;
 }
 
@@ -193,7 +229,7 @@ int candle_moe_workspace_bytes(const candle_moe_weights_t* w, int64_t max_tokens
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     CM_TRY(check_weights(w));
     if (max_tokens < 0 || max_tokens > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
-    *out_bytes = layout(w, max_tokens, nullptr).total;
+    *out_bytes = layout(w, max_tokens, nullptr).total_ext;
     return CANDLE_MOE_OK;
 }
 
@@ -267,6 +303,27 @@ int candle_moe_grouped_down(void* stream, const void* const* w2, int32_t dtype, 
 }  // extern "C"
 
 namespace cmoe {
+// A large batch over Q6_K experts that have no repacked copies: expert by expert, its matrices are repacked into the workspace and
+// taken through the GEMM (see repacks_on_the_way for when and what it measured).
+static cudaError_t gemm_repacking(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int E, int K, int N,
+                                  const uint32_t* offsets, const uint32_t* row_of, int64_t P, int64_t tile_rows, const int8_t* aq,
+                                  const float* ascale, const int16_t* absum, float* out, const ExpertBufs& b, int* n_splits,
+                                  int64_t split_stride, const float* x_f32) {
+    const size_t bytes = prepacked_bytes(CANDLE_GGML_Q6K, N, K);
+    ExpertPtrs ra{}, rb{};
+    ra.p[0] = b.repack;
+    rb.p[0] = gate_up ? b.repack + bytes : b.repack;
+    for (int e = 0; e < E; ++e) {
+        cudaError_t ce = launch_prepack(st, CANDLE_GGML_Q6K, wa.p[e], N, K, b.repack);
+        if (ce == cudaSuccess && gate_up) ce = launch_prepack(st, CANDLE_GGML_Q6K, wb.p[e], N, K, b.repack + bytes);
+        if (ce == cudaSuccess)
+            ce = launch_expert_gemm(st, gate_up, ra, rb, CANDLE_GGML_Q6K, true, 1, K, N, offsets + e, row_of, P, tile_rows, aq, ascale, absum,
+                                    out, b.repack_gemm, n_splits ? REPACK_K_SPLITS : 1, n_splits, split_stride, nullptr, x_f32, nullptr, e > 0);
+        if (ce != cudaSuccess) return ce == cudaErrorNotSupported && e > 0 ? cudaErrorUnknown : ce;
+    }
+    return cudaSuccess;
+}
+
 // The routed experts over P rows grouped by expert (device offsets [E + 1]); no expert has more than max_rows
 // rows.  Picks, per product, the decode kernels over the repacked copies (max_rows <= 128), the tensor-core GEMM
 // (more than that, scratch present), or the streaming / row forms.  Leaves *eo_splits partial outputs in b.eo.
@@ -310,7 +367,10 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
             CM_TRY(fill_ptrs(w->w1_prepacked, E, g1));
             CM_TRY(fill_ptrs(w->w3_prepacked, E, g3));
         }
-        const cudaError_t ce = launch_expert_gemm(st, true, g1, g3, w->dtype_w13, rp, E, d, ff, offsets, row_of, P, tile_rows, xq,
+        const cudaError_t ce = !rp && b.repack && repacks_on_the_way(w->dtype_w13, false, ff, d, true, P, E)
+                                   ? gemm_repacking(st, true, p1, p3, E, d, ff, offsets, row_of, P, tile_rows, xq, xs, xb, b.hidden, b,
+                                                    nullptr, 0, nullptr)
+                                   : launch_expert_gemm(st, true, g1, g3, w->dtype_w13, rp, E, d, ff, offsets, row_of, P, tile_rows, xq,
                                                   xs, xb, b.hidden, b.gemm);
         if (ce == cudaSuccess)
             gate_done = true;
@@ -324,7 +384,8 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     // The down product on the GEMM quantizes the hidden rows while it prepares its operand (not with a device-side row
     // limit: the operand is prepared for all P rows)
     const bool rp2 = (w->dtype_w2 == CANDLE_GGML_Q6K || w->dtype_w2 == CANDLE_GGML_Q8_0) && w->w2_prepacked;
-    const bool fuse_h = large && !row_limit && expert_gemm_takes(false, w->dtype_w2, rp2, ff, d, P);
+    const bool repack2 = b.repack && repacks_on_the_way(w->dtype_w2, w->w2_prepacked != nullptr, d, ff, false, P, E);
+    const bool fuse_h = large && !row_limit && expert_gemm_takes(false, w->dtype_w2, rp2 || repack2, ff, d, P);
     if (!fuse_h) CM_TRY(rc(launch_quantize_act(st, b.hidden, P, ff, w->dtype_w2, b.hq, b.hs, b.hb, row_limit)));
     if (shared && shared->gate_done) {
         CM_TRY(rc(launch_quantize_act(st, shared->hidden, shared->gate.rows, shared->gate.N, CANDLE_GGML_Q8_0, shared->hq, shared->hs, nullptr)));
@@ -350,7 +411,9 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     if (!down_done && large) {
         ExpertPtrs g2 = p2;
         if (rp2) CM_TRY(fill_ptrs(w->w2_prepacked, E, g2));
-        const cudaError_t ce = launch_expert_gemm(st, false, g2, g2, w->dtype_w2, rp2, E, ff, d, offsets, nullptr, P, tile_rows,
+        const cudaError_t ce = repack2 ? gemm_repacking(st, false, p2, p2, E, ff, d, offsets, nullptr, P, tile_rows, b.hq, b.hs, b.hb, b.eo, b,
+                                                        eo_splits, P * d, fuse_h ? b.hidden : nullptr)
+                               : launch_expert_gemm(st, false, g2, g2, w->dtype_w2, rp2, E, ff, d, offsets, nullptr, P, tile_rows,
                                                   b.hq, b.hs, b.hb, b.eo, b.gemm, slots, eo_splits, P * d, nullptr,
                                                   fuse_h ? b.hidden : nullptr);
         if (ce == cudaSuccess)
@@ -404,7 +467,7 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     if ((reinterpret_cast<uintptr_t>(workspace) & 255) || (reinterpret_cast<uintptr_t>(x) & 15) ||
         (reinterpret_cast<uintptr_t>(y) & 15) || (reinterpret_cast<uintptr_t>(w->router) & 15))
         return CANDLE_MOE_E_ALIGN;
-    const Workspace ws = layout(w, T, workspace);
+    const Workspace ws = layout(w, T, workspace, workspace_bytes);
     if (workspace_bytes < ws.total) return CANDLE_MOE_E_WORKSPACE;
     const int E = w->n_experts, k = w->top_k, d = w->d_model;
     ExpertPtrs p1, p3, p2;
@@ -436,7 +499,7 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     mark(st, 2);
     // a token selects an expert at most once: no expert sees more than T rows
     int eo_splits = 1, so_splits = 1;
-    const ExpertBufs eb{ws.hidden, ws.hq, ws.hs, ws.hb, ws.eo, ws.gemm};
+    const ExpertBufs eb{ws.hidden, ws.hq, ws.hs, ws.hb, ws.eo, ws.gemm, ws.repack, ws.repack_gemm};
     // over repacked Q8_0 copies the shared expert takes the decode kernels -- in the launches of the routed experts where those
     // are Q8_0 too -- and for large batches the tensor-core GEMM
     const bool sh_packed = w->d_ff_shared > 0 && w->dtype_shared13 == CANDLE_GGML_Q8_0 && w->dtype_shared2 == CANDLE_GGML_Q8_0 &&
@@ -527,7 +590,7 @@ int candle_moe_ffn_layer_workspace_bytes(const candle_moe_weights_t* w, int64_t 
     CM_TRY(check_weights(w));
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     if (T < 0 || T > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
-    *out_bytes = layout(w, T, nullptr).total + align_up((size_t)T * w->d_model * sizeof(float), 256);
+    *out_bytes = layout(w, T, nullptr).total_ext + align_up((size_t)T * w->d_model * sizeof(float), 256);
     return CANDLE_MOE_OK;
 }
 
@@ -541,9 +604,10 @@ int candle_moe_ffn_layer(void* stream, const candle_moe_weights_t* w, const floa
     if ((reinterpret_cast<uintptr_t>(workspace) & 255) || (reinterpret_cast<uintptr_t>(x) & 15) ||
         (reinterpret_cast<uintptr_t>(norm_weight) & 15))
         return CANDLE_MOE_E_ALIGN;
-    const size_t inner = layout(w, T, nullptr).total;
-    const size_t need = inner + align_up((size_t)T * w->d_model * sizeof(float), 256);
-    if (workspace_bytes < need) return CANDLE_MOE_E_WORKSPACE;
+    const Workspace plan = layout(w, T, nullptr);
+    const size_t norm_bytes = align_up((size_t)T * w->d_model * sizeof(float), 256);
+    if (workspace_bytes < plan.total + norm_bytes) return CANDLE_MOE_E_WORKSPACE;
+    const size_t inner = workspace_bytes >= plan.total_ext + norm_bytes ? plan.total_ext : plan.total;
     // k-quant experts and no shared expert: nothing but the router kernel reads the normalised rows
     if (router_fuses_norm(T, w->d_model) && w->dtype_w13 != CANDLE_GGML_Q8_0 && w->d_ff_shared == 0)
         return forward_impl(stream, w, x, T, y, workspace, inner, x, norm_weight, eps);
@@ -607,8 +671,9 @@ int static_scratch_ptr(void** out) {
 }  // namespace
 
 int candle_moe_forward_static(void* stream, const candle_moe_weights_t* w, const float* x, int64_t T, float* y) {
-    size_t need = 0;
-    CM_TRY(candle_moe_workspace_bytes(w, T, &need));
+    CM_TRY(check_weights(w));
+    if (T < 0 || T > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
+    const size_t need = layout(w, T, nullptr).total;
     if (need > (size_t)CANDLE_MOE_STATIC_SCRATCH_BYTES) return CANDLE_MOE_E_STATIC_SCRATCH;
     void* scratch = nullptr;
     CM_TRY(static_scratch_ptr(&scratch));

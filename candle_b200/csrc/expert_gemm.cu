@@ -1236,7 +1236,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
                                bool repacked, int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of, int64_t P,
                                int64_t max_rows, const int8_t* aq, const float* ascale, const int16_t* absum, float* out,
                                void* scratch, int max_splits, int* n_splits_out, int64_t split_stride, float* out_whole,
-                               const float* x_f32, uint32_t* single_group) {
+                               const float* x_f32, uint32_t* single_group, bool operand_ready) {
     if (n_splits_out) *n_splits_out = 1;
     if (!scratch || !expert_gemm_takes(gate_up, dtype, repacked, K, N, P) || (x_f32 && row_of)) return cudaErrorNotSupported;
     int tn = max_rows <= 32 ? 32 : (max_rows <= 64 ? 64 : 128);  // position tile, from the bound / hint on an expert's rows
@@ -1294,7 +1294,9 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     const int64_t units = p_pad * kb;
     const int64_t per_cta = 8 * (x_f32 ? PREP_UNITS : 1);
     const dim3 prep_grid((unsigned)((units + per_cta - 1) / per_cta));
-    if (x_f32)
+    if (operand_ready)  // an earlier call prepared the same rows in the same scratch (and wrote the maps, which Q4_K alone has)
+        e = dtype == CANDLE_GGML_Q4K ? cudaErrorInvalidValue : cudaSuccess;
+    else if (x_f32)
         e = q80 ? launch_k(prep_gemm_f32_q80_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K_in, K, q80x ? 1 : 0, bf16,
                            d8t, single_group)
                 : launch_k(prep_gemm_f32_q8k_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K, bf16,
