@@ -448,60 +448,7 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
 // each warp owns experts warp, warp+32, ... and walks the pair list 32 at a time with a ballot, first
 // to count, then (after an exclusive scan over experts) to place.
 // ------------------------------------------------------------------------------------------------
-// Up to PERMUTE_SMEM pairs the ids are brought to shared memory first, one or two loads per thread: the walk of a warp is then a
-// chain of shared loads instead of one of trips to L2, twice (514 pairs 7.2 -> 6.3 us, 64 pairs 3.3 -> 3.0 us).
-constexpr int PERMUTE_THREADS = 1024, PERMUTE_SMEM = 2048;
-
-template <class Ids>
-__device__ __forceinline__ void permute_walk(const Ids& id_of, int64_t n_pairs, int k, int E, uint32_t* s_count, uint32_t* s_off,
-                                             uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets,
-                                             uint32_t* __restrict__ perm_token, uint32_t* __restrict__ pair_pos) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = PERMUTE_THREADS / 32;
-    for (int e = warp; e < E; e += n_warps) {
-        uint32_t c = 0;
-#pragma unroll 4
-        for (int64_t i0 = 0; i0 < n_pairs; i0 += 32) {
-            const int64_t i = i0 + lane;
-            const bool hit = i < n_pairs && id_of(i) == (uint32_t)e;
-            c += __popc(__ballot_sync(0xffffffffu, hit));
-        }
-        if (lane == 0) s_count[e] = c;
-    }
-    __syncthreads();
-    if (warp == 0) {  // exclusive scan over the experts, 32 at a time
-        uint32_t run = 0;
-        for (int e0 = 0; e0 < E; e0 += 32) {
-            const uint32_t c = e0 + lane < E ? s_count[e0 + lane] : 0u;
-            uint32_t v = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += u;
-            }
-            if (e0 + lane < E) s_off[e0 + lane] = run + v - c;
-            run += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) s_off[E] = run;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < E; e += PERMUTE_THREADS) counts[e] = s_count[e];
-    for (int e = threadIdx.x; e <= E; e += PERMUTE_THREADS) offsets[e] = s_off[e];
-    for (int e = warp; e < E; e += n_warps) {
-        uint32_t base = s_off[e];
-#pragma unroll 4
-        for (int64_t i0 = 0; i0 < n_pairs; i0 += 32) {
-            const int64_t i = i0 + lane;
-            const bool hit = i < n_pairs && id_of(i) == (uint32_t)e;
-            const uint32_t m = __ballot_sync(0xffffffffu, hit);
-            if (hit) {
-                const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
-                perm_token[pos] = (uint32_t)(i / k);
-                pair_pos[i] = pos;
-            }
-            base += __popc(m);
-        }
-    }
-}
+constexpr int PERMUTE_THREADS = 1024;
 
 __global__ void __launch_bounds__(PERMUTE_THREADS)
 permute_kernel(const uint32_t* __restrict__ ids, int64_t n_pairs, int k, int E, uint32_t* __restrict__ counts,
@@ -510,13 +457,41 @@ permute_kernel(const uint32_t* __restrict__ ids, int64_t n_pairs, int k, int E, 
     pdl_wait();
     __shared__ uint32_t s_count[CANDLE_MOE_MAX_EXPERTS];
     __shared__ uint32_t s_off[CANDLE_MOE_MAX_EXPERTS + 1];
-    __shared__ uint32_t s_ids[PERMUTE_SMEM];
-    if (n_pairs <= PERMUTE_SMEM) {
-        for (int i = threadIdx.x; i < (int)n_pairs; i += PERMUTE_THREADS) s_ids[i] = ids[i];
-        __syncthreads();
-        permute_walk([&](int64_t i) { return s_ids[i]; }, n_pairs, k, E, s_count, s_off, counts, offsets, perm_token, pair_pos);
-    } else {
-        permute_walk([&](int64_t i) { return ids[i]; }, n_pairs, k, E, s_count, s_off, counts, offsets, perm_token, pair_pos);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = PERMUTE_THREADS / 32;
+    for (int e = warp; e < E; e += n_warps) {
+        uint32_t c = 0;
+        for (int64_t i0 = 0; i0 < n_pairs; i0 += 32) {
+            const int64_t i = i0 + lane;
+            const bool hit = i < n_pairs && ids[i] == (uint32_t)e;
+            c += __popc(__ballot_sync(0xffffffffu, hit));
+        }
+        if (lane == 0) s_count[e] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t run = 0;
+        for (int e = 0; e < E; ++e) {
+            s_off[e] = run;
+            run += s_count[e];
+        }
+        s_off[E] = run;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += PERMUTE_THREADS) counts[e] = s_count[e];
+    for (int e = threadIdx.x; e <= E; e += PERMUTE_THREADS) offsets[e] = s_off[e];
+    for (int e = warp; e < E; e += n_warps) {
+        uint32_t base = s_off[e];
+        for (int64_t i0 = 0; i0 < n_pairs; i0 += 32) {
+            const int64_t i = i0 + lane;
+            const bool hit = i < n_pairs && ids[i] == (uint32_t)e;
+            const uint32_t m = __ballot_sync(0xffffffffu, hit);
+            if (hit) {
+                const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
+                perm_token[pos] = (uint32_t)(i / k);
+                pair_pos[i] = pos;
+            }
+            base += __popc(m);
+        }
     }
 }
 
