@@ -924,7 +924,10 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                 // with a kernel parameter that is zero at run time): the arrive cannot be issued before those words
                 // exist.  (Released after the emits instead, a ring of two stages gave a copy less than the time of one
                 // block's emits: all-Q8_0 layer of 60 experts, 4096 rows, gate_up 562 -> 531 us, shared down 136 -> 125 us.)
-                if (F::STAGE_W) {
+                // A ring of three or four stages (narrow position tiles) has that time, and there the reduction costs more than it
+                // gives: released after the emits (nothing reads the stage later than that, whatever the order of the
+                // instructions), gate_up of the Mixtral-shaped layer at 100 rows takes 201 us, released here 212.
+                if (F::STAGE_W && WS <= 2) {
                     const uint32_t dep = __reduce_or_sync(0xffffffffu, F::staged_words(cur)) & P.zero;
                     if (lane == 0) mbar_arrive(&empty_w[ab % WS + dep]);
                 }
@@ -950,7 +953,10 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                 tmem_st_wait();
                 tc5_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&full_a[bidx]);
+                if (lane == 0) {
+                    mbar_arrive(&full_a[bidx]);
+                    if (F::STAGE_W && WS > 2) mbar_arrive(&empty_w[ab % WS]);
+                }
                 if (!F::STAGE_W) cur = nxt;
             }
             tile += gridDim.x;
