@@ -165,6 +165,19 @@ __device__ __forceinline__ void dispatch_one_token(const int (&sel_e)[CANDLE_MOE
     }
 }
 
+__device__ __forceinline__ void add4(float4& a, const float4& b) {
+    a.x += b.x;
+    a.y += b.y;
+    a.z += b.z;
+    a.w += b.w;
+}
+__device__ __forceinline__ void fma4(float4& s, const float4& a, const float4& b) {
+    s.x = fmaf(a.x, b.x, s.x);
+    s.y = fmaf(a.y, b.y, s.y);
+    s.z = fmaf(a.z, b.z, s.z);
+    s.w = fmaf(a.w, b.w, s.w);
+}
+
 // Few tokens: 1024 threads per token, latency-bound.  The row passes through shared memory once, with the
 // layer's RmsNorm applied on the way where the caller asks for it (norm_w; one launch fewer), and every warp owns whole
 // dot products: expert e, or for few experts one of `parts` pieces of it, so that all loads of a round are in flight at
@@ -220,15 +233,22 @@ router_topk_small_kernel(const float* __restrict__ x, const float* __restrict__ 
         const int e = u / parts, p = u - e * parts;
         const int i1 = d4 * (p + 1) / parts;
         const float4* wr = reinterpret_cast<const float4*>(wg + (int64_t)e * d);
-        float acc = 0.f;
-#pragma unroll 8
-        for (int i = d4 * p / parts + lane; i < i1; i += 32) {
-            const float4 wv = wr[i], xv = sx4[i];
-            acc = fmaf(xv.x, wv.x, acc);
-            acc = fmaf(xv.y, wv.y, acc);
-            acc = fmaf(xv.z, wv.z, acc);
-            acc = fmaf(xv.w, wv.w, acc);
+        // a lane's elements are added in runs of eight per component of the float4s, runs and components on their own: ten terms
+        // in a row at most, where one sum over all of them had 256 for d = 8192 (root mean square error of a logit, 60 experts,
+        // 64 rows of 8192: 5.4e-7 -> 2.3e-7, eight experts of 4096 1.8e-7 -> 1.5e-7; the time is the same)
+        float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
+        int i = d4 * p / parts + lane;
+        for (; i + 7 * 32 < i1; i += 8 * 32) {
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) fma4(s, sx4[i + 32 * j], wr[i + 32 * j]);
+            add4(tot, s);
         }
+        float4 rest = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (; i < i1; i += 32) fma4(rest, sx4[i], wr[i]);
+        add4(tot, rest);
+        float acc = (tot.x + tot.y) + (tot.z + tot.w);
         acc = warp_sum(acc);
         if (lane == 0) s_part[p][e] = acc;
     }
@@ -620,12 +640,6 @@ cudaError_t launch_single_group(cudaStream_t st, uint32_t* offsets, uint32_t row
 // ------------------------------------------------------------------------------------------------
 constexpr int COMBINE_THREADS = 256;
 
-__device__ __forceinline__ void add4(float4& a, const float4& b) {
-    a.x += b.x;
-    a.y += b.y;
-    a.z += b.z;
-    a.w += b.w;
-}
 // sum of the partials p, p + stride, ... (n of them) of one float4, in split order, BATCH loads in flight
 template <int BATCH>
 __device__ __forceinline__ float4 sum_partials(const float4* __restrict__ p, int64_t stride4, int n) {
