@@ -71,6 +71,7 @@ struct EpWorkspace {
 EpWorkspace ep_layout(const candle_moe_weights_t* w, int64_t P, void* base);
 // K-split partial outputs the local phase may use for P rows over E local experts: eight while the rows are few
 // (decode-sized steps, where splitting K is what fills the SMs), four beyond
-inline int ep_eo_slots(int64_t P, int E) { return (P <= 64 * (int64_t)E || P <= 2048) ? MAX_K_SPLITS : 4; }
+inline int64_t ep_many_slot_rows(int E) { return 64 * (int64_t)E > 2048 ? 64 * (int64_t)E : 2048; }
+inline int ep_eo_slots(int64_t P, int E) { return P <= ep_many_slot_rows(E) ? MAX_K_SPLITS : 4; }
 
 }  // namespace cmoe

@@ -32,6 +32,9 @@ constexpr int64_t QMM_GEMM_MIN_ROWS = 48;  // the dense product: one matrix, row
 // Decode-sized batches may split K finely (more parallel items, smaller resident activations);
 // larger batches get four slots, enough for the streaming form's activation rows to fit.
 inline int k_split_slots(int64_t T) { return T <= gemm_min_rows() ? MAX_K_SPLITS : 4; }
+// A workspace for up to T rows serves smaller batches too: the scratch grows with the rows except at this step (8 slots -> 4),
+// so the larger of the sizes for T and for this many rows holds every batch up to T.
+inline int64_t small_rows(int64_t T) { return std::min(T, std::max<int64_t>(0, gemm_min_rows())); }
 
 struct Workspace {
     // routing
@@ -229,7 +232,7 @@ int candle_moe_workspace_bytes(const candle_moe_weights_t* w, int64_t max_tokens
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     CM_TRY(check_weights(w));
     if (max_tokens < 0 || max_tokens > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
-    *out_bytes = layout(w, max_tokens, nullptr).total_ext;
+    *out_bytes = std::max(layout(w, max_tokens, nullptr).total_ext, layout(w, small_rows(max_tokens), nullptr).total_ext);
     return CANDLE_MOE_OK;
 }
 
@@ -590,7 +593,8 @@ int candle_moe_ffn_layer_workspace_bytes(const candle_moe_weights_t* w, int64_t 
     CM_TRY(check_weights(w));
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     if (T < 0 || T > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
-    *out_bytes = layout(w, T, nullptr).total_ext + align_up((size_t)T * w->d_model * sizeof(float), 256);
+    const auto need = [&](int64_t rows) { return layout(w, rows, nullptr).total_ext + align_up((size_t)rows * w->d_model * sizeof(float), 256); };
+    *out_bytes = std::max(need(T), need(small_rows(T)));
     return CANDLE_MOE_OK;
 }
 
@@ -850,7 +854,9 @@ int candle_moe_ep_workspace_bytes(const candle_moe_weights_t* w, int64_t max_row
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     if (max_rows_total < 0 || max_rows_total > (int64_t)1 << 26) return CANDLE_MOE_E_SHAPE;
     if (w->dtype_w13 == CANDLE_GGML_Q8_0 || w->dtype_w2 == CANDLE_GGML_Q8_0) return CANDLE_MOE_E_DTYPE;
-    *out_bytes = ep_layout(w, max_rows_total, nullptr).total;
+    // as small_rows: the slots of the partial outputs fall from 8 to 4 behind this many rows
+    const int64_t few = std::min(max_rows_total, ep_many_slot_rows(w->n_experts));
+    *out_bytes = std::max(ep_layout(w, max_rows_total, nullptr).total, ep_layout(w, few, nullptr).total);
     return CANDLE_MOE_OK;
 }
 

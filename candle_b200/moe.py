@@ -132,6 +132,7 @@ class MlpOrMoe:
             if sh is not None:
                 self._cw.shared_w1_prepacked, self._cw.shared_w3_prepacked, self._cw.shared_w2_prepacked = (
                     t.data_ptr() for t in sh)
+        self._ws, self._ws_tokens = None, 0  # with the copies a batch may need more scratch than before
         return self
 
     @property

@@ -53,6 +53,27 @@ def test_workspace_query_is_host_only_and_monotonic(lib):
     assert sizes[-1] < 2048 * 2 * (14336 * 6 + 4096 * 20) + (1 << 20)
 
 
+@pytest.mark.parametrize("kw", [{}, {"copies": True}, {"dtype_w13": 14}, {"dtype_w13": 8, "dtype_w2": 8, "n_experts": 60, "top_k": 4, "d_ff": 1408,
+                                                                         "d_model": 2048, "d_ff_shared": 5632, "dtype_shared13": 8, "dtype_shared2": 8}])
+def test_a_workspace_for_many_rows_holds_every_smaller_batch(lib, kw):
+    """Around the row counts where the number of partial outputs falls (96 rows; expert parallelism 2048, 64 per expert)."""
+    L, kw = lib.load(), dict(kw)
+    table = (C.c_void_p * 128)(*[4096] * 128)
+    if kw.pop("copies", False):
+        kw.update(w1_prepacked=table, w3_prepacked=table, w2_prepacked=table)
+    w, out = _weights(lib, **kw), C.c_size_t(0)
+    for query, rows in ((L.candle_moe_workspace_bytes, (1, 31, 95, 96, 97, 100, 191, 193, 400, 2000, 4096)),
+                        (L.candle_moe_ffn_layer_workspace_bytes, (1, 95, 96, 97, 130, 500)),
+                        (L.candle_moe_ep_workspace_bytes, (1, 32, 33, 511, 513, 2047, 2048, 2049, 3000, 3841, 5000))):
+        if query is L.candle_moe_ep_workspace_bytes and w.dtype_w13 == 8:
+            continue
+        sizes = []
+        for T in rows:
+            assert query(C.byref(w), T, C.byref(out)) == 0
+            sizes.append(out.value)
+        assert sizes == sorted(sizes), query.__name__
+
+
 @pytest.mark.parametrize("field,value,code", [
     ("d_model", 4000, -2),        # not a multiple of 256 for Q4K
     ("d_ff", 100, -2),

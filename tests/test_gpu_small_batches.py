@@ -127,7 +127,6 @@ def test_q80_large_batch_with_the_fused_operand(orc, torch_cuda, T, d, ff, fs):
     x = torch.from_numpy(orc.make_activations(T, T, d)).cuda()
     want = blk.forward(x).clone()
     blk.prepack()
-    blk._ws, blk._ws_tokens = None, 0  # with the copies the large batch needs more scratch
     y = blk.forward(x).clone()
     assert torch.equal(y, blk.forward(x))
     v = C.c_int32(-1)
@@ -171,3 +170,24 @@ def test_large_batch_over_q6k_without_copies(orc, torch_cuda, w13, w2, T, d, ff,
     assert H.rel_l2(y2.cpu().numpy(), y.cpu().numpy()) <= loose * H.REL_L2_TOL
     v = C.c_int32(-1)
     assert L.candle_moe_device_status(C.byref(v)) == 0 and v.value == 0
+
+
+@pytest.mark.parametrize("w13,w2,fs", [("Q4K", "Q6K", 0), ("Q8_0", "Q8_0", 640)])
+def test_one_block_takes_batches_in_any_order(orc, torch_cuda, w13, w2, fs):
+    """A block keeps its scratch: a batch just above the decode kernels' range, one just inside it (whose partial outputs
+    need more), and both again after the repacked copies have been made."""
+    torch = torch_cuda
+    cfg = dict(d=1024, ff=512, E=8, k=2, dt13=getattr(orc, w13), dt2=getattr(orc, w2), renorm=True, ff_shared=fs)
+    blk, _ = H.random_device_block(orc, torch, cfg, seed=1)
+    x = torch.from_numpy(orc.make_activations(1, 400, 1024)).cuda()
+    nw = torch.ones(1024, device="cuda")
+    first = {}
+    for step in range(2):
+        for T in (97, 96, 400, 95):
+            y = blk.forward(x[:T]).clone()
+            blk.forward_layer(x[:T], nw, 1e-5)
+            assert torch.equal(blk.forward(x[:T]), y), (step, T)
+            # other kernels after the copies: the same integers, other f32 orders
+            assert step == 0 or H.rel_l2(y.cpu().numpy(), first[T].cpu().numpy()) <= 2 * H.REL_L2_TOL, T
+            first.setdefault(T, y)
+        blk.prepack()
