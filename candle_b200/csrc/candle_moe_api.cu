@@ -73,14 +73,24 @@ struct Workspace {
 };
 
 constexpr int REPACK_K_SPLITS = 2;
-// Q6_K as the GEMM reads it is the repacked layout.  Without copies a large batch (P rows over E experts) repacks one expert at a
-// time on its way through the GEMM, for shapes the repack takes (as candle_moe_prepack and the GEMM check them).  Against the
-// streaming form, which passes over an expert's weights once per 16 rows, that pays from about six passes on (Q4_K / Q6_K layer of
-// d = 4096, ff = 14336: 25 rows per expert 594 us streaming, 854 repacking; 75 rows 1180 / 979; 512 rows 6183 / 2659; Q6_K layer of
-// d = 2048, ff = 4096: 25 rows 213 / 504, 250 rows 1317 / 710); the streaming form does not take rows that are not 16-byte aligned,
-// and the row-per-warp form is slower at once (d = 1536, ff = 2560, 37 rows per expert 491 / 199 us).
+// Q6_K as the GEMM reads it is the repacked layout.  Without copies a large batch (P rows over E experts) can repack one expert
+// at a time on its way through the GEMM, for shapes the repack takes (as candle_moe_prepack and the GEMM check them).  Two or
+// three launches per expert, one after the other and each over one matrix: worth it only where the other forms pass over an
+// expert's weights long enough.  Microseconds per expert, W = its weights in millions, r = its rows on average, fitted to the
+// shapes below: repacking 5 per launch + W / 0.8 + r W / 190; streaming r W / 34 (it takes rows of whole 16 bytes, k a
+// multiple of 2048); row-per-warp r W / 3 + 1.1 r / E (the latency of a row, which few small experts do not hide).  Taken with a
+// margin of 1.15 for what the fit misses.
+// Whole layers (both products Q6_K unless said otherwise), other form / repacking, us -- d = 1536, ff = 1536, 60 experts: 6 rows per expert 954 /
+// 2145, 13 rows 1762 / 2153, 27 rows 3385 / 2412; d = 512, ff = 1024, 128 experts, 1.5 rows 234 / 3017; d = 1536, ff = 768, 128
+// experts, 25 rows 3483 / 3741, 50 rows 6811 / 5288; d = 1536, ff = 2560, 8 experts, 24 rows 730 / 350; streaming: d = 2048,
+// ff = 4096, 8 experts, 100 rows 592 / 604, 200 rows 1070 / 662; d = 2048, ff = 2048, 60 experts, 107 rows 2380 / 3480; d = 4096,
+// ff = 14336, 8 experts, Q4_K gate_up, 75 rows 1177 / 979, 100 rows 1454 / 1177, 500 rows 6128 / 2669.
 inline bool repacks_on_the_way(int dtype, bool has_copy, int n, int k, bool gate_up, int64_t P, int E) {
-    return dtype == CANDLE_GGML_Q6K && !has_copy && n % (gate_up ? 64 : 128) == 0 && k % 512 == 0 && (P >= 96 * (int64_t)E || k % 2048 != 0);
+    if (dtype != CANDLE_GGML_Q6K || has_copy || n % (gate_up ? 64 : 128) || k % 512 || tuning_get(TUNE_FORCE_ROWS)) return false;
+    const double weights = 1e-6 * n * k * (gate_up ? 2 : 1), work = weights * (double)P / E;
+    const double repacking = 5.0 * (gate_up ? 3 : 2) + weights / 0.8 + work / 190.0;
+    const double other = k % 2048 == 0 ? work / 34.0 : work / 3.0 + 1.1 * (double)P / E / E;
+    return other > 1.15 * repacking;
 }
 
 // avail: bytes behind base_ (the optional part is handed out only if it fits)
