@@ -132,7 +132,7 @@ class MlpOrMoe:
             if sh is not None:
                 self._cw.shared_w1_prepacked, self._cw.shared_w3_prepacked, self._cw.shared_w2_prepacked = (
                     t.data_ptr() for t in sh)
-        self._ws, self._ws_tokens = None, 0  # with the copies a batch may need more scratch than before
+        self._ws_tokens = 0  # with the copies a batch may need more scratch (the present one still holds the last routing)
         return self
 
     @property
