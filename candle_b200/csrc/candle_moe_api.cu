@@ -331,7 +331,7 @@ static cudaError_t gemm_repacking(cudaStream_t st, bool gate_up, const ExpertPtr
         if (ce == cudaSuccess && gate_up) ce = launch_prepack(st, CANDLE_GGML_Q6K, wb.p[e], N, K, b.repack + bytes);
         if (ce == cudaSuccess)
             ce = launch_expert_gemm(st, gate_up, ra, rb, CANDLE_GGML_Q6K, true, 1, K, N, offsets + e, row_of, P, tile_rows, aq, ascale, absum,
-                                    out, b.repack_gemm, n_splits ? REPACK_K_SPLITS : 1, n_splits, split_stride, nullptr, x_f32, nullptr, e > 0);
+                                    out, b.repack_gemm, n_splits ? REPACK_K_SPLITS : 1, n_splits, split_stride, nullptr, x_f32, nullptr, e > 0, true);
         if (ce != cudaSuccess) return ce == cudaErrorNotSupported && e > 0 ? cudaErrorUnknown : ce;
     }
     return cudaSuccess;

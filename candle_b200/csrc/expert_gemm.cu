@@ -365,6 +365,7 @@ __device__ __forceinline__ uint32_t w4(const uint4& v, int i) { return i == 0 ? 
 // are slab s, low nibbles k = 0..31, high nibbles k = 32..63.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ4K {
+    static constexpr bool EXACT_GATE = false;
     static constexpr bool HAS_MIN = true;
     static constexpr int A_COLS = 32, A_PARTS = 1, A_PAIRS = 4;  // 8 slabs of 32 columns: two blocks in flight
     static constexpr int B_PARTS = 1;
@@ -462,6 +463,7 @@ struct GemmQ4K {
 // 16 (q - 32), times ceil(sc/2)/16 and floor(sc/2)/16 gives the two exact operand parts.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ6K {
+    static constexpr bool EXACT_GATE = false;
     static constexpr bool HAS_MIN = false;
     static constexpr int A_COLS = 64, A_PARTS = 2, A_PAIRS = 2;  // 4 slabs of 64 columns (two operand parts each)
     static constexpr int B_PARTS = 1;
@@ -538,6 +540,15 @@ struct GemmQ6K {
     __device__ static __forceinline__ float scale_of(uint32_t hdr) { return half_bits_to_float((uint16_t)hdr); }
 };
 
+// Matrices without copies, repacked on their way (candle_moe_api.cu).  The forms that take such a layer otherwise gate with expf and
+// an exact division (silu_f); the hidden rows are quantized to int8 again, where a difference in the last bit can become a
+// step, so this one does the same: largest relative error of a gate 2.4e-7 (8.1e-7 with __expf and an approximate division), of
+// the hidden rows against 64-bit arithmetic 0.98-1.01e-7 (streaming form 0.98-1.01e-7, row-per-warp form 1.2-1.5e-7, without
+// the exact gate 1.01-1.05e-7).  It costs 3-6 % of a layer of small matrices (8 experts of 1536 x 2560, 400 rows: 457 -> 470 us).
+struct GemmQ6KOnTheWay : GemmQ6K {
+    static constexpr bool EXACT_GATE = true;
+};
+
 // ------------------------------------------------------------------------------------------------
 // Q8_0, repacked layout (prepack_q80_kernel): half-tile blocks of 8 rows x 128 elements, two of them per 256-block, rows
 // padded with zeros to a multiple of 256 elements.  The reference multiplies per 32-element
@@ -550,6 +561,7 @@ struct GemmQ6K {
 // Half h of a 256-block is its half-tile block h; word cw of chunk t of region s holds elements 16 cw + 4 t .. + 3.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ80 {
+    static constexpr bool EXACT_GATE = false;
     static constexpr bool HAS_MIN = false;
     static constexpr int A_COLS = 32, A_PARTS = 1, A_PAIRS = 4;
     static constexpr int B_PARTS = 1;
@@ -861,7 +873,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                     const float recv = __shfl_xor_sync(0xffffffffu, up ? acc[c] : acc[c + CH / 2], 8);
                     const float gv = up ? recv : acc[c], uv = up ? acc[c + CH / 2] : recv;
                     const uint32_t p = pc0 + c + (up ? CH / 2 : 0);
-                    if (p < tc.p_end) out_k[(size_t)p * P.N + n] = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
+                    if (p < tc.p_end) out_k[(size_t)p * P.N + n] = (F::EXACT_GATE ? silu_f(gv) : __fdividef(gv, 1.0f + __expf(-gv))) * uv;
                 }
             } else {
 #pragma unroll
@@ -1242,7 +1254,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
                                bool repacked, int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of, int64_t P,
                                int64_t max_rows, const int8_t* aq, const float* ascale, const int16_t* absum, float* out,
                                void* scratch, int max_splits, int* n_splits_out, int64_t split_stride, float* out_whole,
-                               const float* x_f32, uint32_t* single_group, bool operand_ready) {
+                               const float* x_f32, uint32_t* single_group, bool operand_ready, bool exact_gate) {
     if (n_splits_out) *n_splits_out = 1;
     if (!scratch || !expert_gemm_takes(gate_up, dtype, repacked, K, N, P) || (x_f32 && row_of)) return cudaErrorNotSupported;
     int tn = max_rows <= 32 ? 32 : (max_rows <= 64 ? 64 : 128);  // position tile, from the bound / hint on an expert's rows
@@ -1370,6 +1382,11 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         if (tn == 32) return launch_gemm_kernel<GemmQ80, false, 32>(st, G, map_b, map_bs);
         if (tn == 64) return launch_gemm_kernel<GemmQ80, false, 64>(st, G, map_b, map_bs);
         return launch_gemm_kernel<GemmQ80, false, 128>(st, G, map_b, map_bs);
+    }
+    if (gate_up && exact_gate) {
+        if (tn == 32) return launch_gemm_kernel<GemmQ6KOnTheWay, true, 32>(st, G, map_b, map_bs);
+        if (tn == 64) return launch_gemm_kernel<GemmQ6KOnTheWay, true, 64>(st, G, map_b, map_bs);
+        return launch_gemm_kernel<GemmQ6KOnTheWay, true, 128>(st, G, map_b, map_bs);
     }
     if (tn == 32)
         return gate_up ? launch_gemm_kernel<GemmQ6K, true, 32>(st, G, map_b, map_bs) : launch_gemm_kernel<GemmQ6K, false, 32>(st, G, map_b, map_bs);

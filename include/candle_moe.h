@@ -110,8 +110,10 @@ CANDLE_MOE_API int candle_moe_get_tuning(int32_t key, int64_t* value);
 /* Library identification: returns a static string "candle_moe_sm100 <version>". */
 CANDLE_MOE_API const char* candle_moe_version(void);
 
-/* Bytes of scratch that candle_moe_forward needs for up to max_tokens rows (for large batches over Q6_K matrices without
- * repacked copies with room for one expert's, which a smaller workspace does without, at less speed).  Replaces the
+/* Bytes of scratch that candle_moe_forward needs for up to max_tokens rows.  For some large batches over Q6_K matrices without
+ * repacked copies that includes room for one expert's copies; a workspace without it is taken too and such a batch then
+ * runs on another kernel form, at less speed: its f32 sums go in another order, which through the int8 quantization of
+ * the hidden rows shows as a relative L2 of up to 1e-4 between the two, as it does between batch sizes.  Replaces the
  * per-call allocations of the reference block (dev.alloc in candle-core/src/quantized/cuda.rs:253,
  * 321 and the zeros_like/index_add copies of quantized_llama.rs:184,202). */
 CANDLE_MOE_API int candle_moe_workspace_bytes(const candle_moe_weights_t* w, int64_t max_tokens, size_t* out_bytes);

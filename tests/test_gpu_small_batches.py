@@ -191,3 +191,35 @@ def test_one_block_takes_batches_in_any_order(orc, torch_cuda, w13, w2, fs):
             assert step == 0 or H.rel_l2(y.cpu().numpy(), first[T].cpu().numpy()) <= 2 * H.REL_L2_TOL, T
             first.setdefault(T, y)
         blk.prepack()
+
+
+def test_gate_of_repacked_q6k_is_the_exact_one(orc, torch_cuda):
+    """Q6_K gate_up repacked on its way: silu as the forms for other batch sizes compute it (expf, an exact division), since the
+    hidden rows are quantized again.  Operands whose sums are exact in f32 (scales are powers of two, integers small), so that
+    only the gate rounds: expf one unit in the last place, the sum and the division half a unit each, two units of 2^-23 in all."""
+    torch = torch_cuda
+    from candle_b200 import GgmlDType, Mlp, MlpOrMoe, QMatMul, QTensor
+    d, ff, T = 512, 512, 400
+
+    def q6k(n, k, sc, m):
+        b = np.zeros((n, k // 256, 210), np.uint8)  # ql[128], qh[64], scales[16], d
+        q = (m + 32).astype(np.uint8)[:, None, None]
+        b[..., :128] = (q & 15) * 17
+        b[..., 128:192] = (q >> 4) * 85
+        b[..., 192:208] = sc.astype(np.uint8)[:, None, None]
+        b[..., 208:210] = np.frombuffer(np.float16(2.0 ** -14).tobytes(), np.uint8)
+        return QTensor.from_blocks(b.reshape(-1), GgmlDType.Q6K, (n, k))
+
+    i = np.arange(ff)
+    sc, m = 1 + i % 127, np.array([-32, -29, -23, 31])[i // 128]
+    w1, w3 = q6k(ff, d, sc, m), q6k(ff, d, np.full(ff, 16), np.full(ff, 16))
+    w2 = q6k(d, ff, np.full(d, 1), np.full(d, 1))
+    blk = MlpOrMoe.moe(1, torch.zeros((1, d), device="cuda"), [Mlp(QMatMul(w1), QMatMul(w2), QMatMul(w3))])
+    blk.forward(torch.full((T, d), 0.125, device="cuda"))
+    gate = sc * m * (512 * 2.0 ** -14 * 0.125)  # -15.9 .. 15.4; the other product is 1
+    want = torch.from_numpy(gate / (1 + np.exp(-gate))).cuda()
+    words = blk._ws[blk._ws_ptr() - blk._ws.data_ptr():].view(torch.float32)
+    at = [o for o in range(0, words.numel() - T * ff, 64) if torch.allclose(words[o:o + ff].double(), want, rtol=1e-4, atol=0)][:1]
+    assert at, "the hidden rows were not found in the scratch"
+    got = words[at[0]:at[0] + T * ff].reshape(T, ff).double()
+    assert float(((got - want) / want).abs().max()) <= 2.01 * 2 ** -23
