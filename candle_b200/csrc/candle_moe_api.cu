@@ -32,9 +32,6 @@ constexpr int64_t QMM_GEMM_MIN_ROWS = 48;  // the dense product: one matrix, row
 // Decode-sized batches may split K finely (more parallel items, smaller resident activations);
 // larger batches get four slots, enough for the streaming form's activation rows to fit.
 inline int k_split_slots(int64_t T) { return T <= gemm_min_rows() ? MAX_K_SPLITS : 4; }
-// A workspace for up to T rows serves smaller batches too: the scratch grows with the rows except at this step (8 slots -> 4),
-// so the larger of the sizes for T and for this many rows holds every batch up to T.
-inline int64_t small_rows(int64_t T) { return std::min(T, std::max<int64_t>(0, gemm_min_rows())); }
 
 struct Workspace {
     // routing
@@ -72,7 +69,10 @@ struct Workspace {
     size_t total_ext;  // with it
 };
 
-constexpr int REPACK_K_SPLITS = 2;
+constexpr int REPACK_MAX_RUN = 12;  // see gemm_repacking
+// partial outputs of that form: the room behind them is its own
+constexpr int64_t REPACK_MANY_SLOT_ROWS = 2048;
+inline int repack_slots(int64_t P) { return P <= REPACK_MANY_SLOT_ROWS ? 4 : 2; }
 // Q6_K as the GEMM reads it is the repacked layout.  Without copies a large batch (P rows over E experts) can repack one expert
 // at a time on its way through the GEMM, for shapes the repack takes (as candle_moe_prepack and the GEMM check them).  Two or
 // three launches per expert, one after the other and each over one matrix: worth it only where the other forms pass over an
@@ -113,7 +113,7 @@ Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_, size_t a
     ws.hq = carve<int8_t>(base, off, Tk * ff);
     ws.hs = carve<float>(base, off, Tk * ff / act_block(w->dtype_w2));
     ws.hb = carve<int16_t>(base, off, Tk * ff / 16);
-    size_t free_at = align_up(off, 256) + REPACK_K_SPLITS * Tk * d * sizeof(float);  // behind the partial outputs of that form
+    size_t free_at = align_up(off, 256) + repack_slots((int64_t)Tk) * Tk * d * sizeof(float);
     ws.eo = carve<float>(base, off, Tk * d * k_split_slots(T));
     if (w->d_ff_shared > 0) {
         const size_t fs = w->d_ff_shared;
@@ -174,6 +174,14 @@ Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_, size_t a
         }
     }
     return ws;
+}
+
+// A workspace for up to T rows serves smaller batches too: its size grows with the rows except where the partial outputs become
+// fewer (behind gemm_min_rows() rows; REPACK_MANY_SLOT_ROWS selections), so the largest of these holds every batch up to T.
+template <class Bytes>
+size_t for_every_batch(const candle_moe_weights_t* w, int64_t T, Bytes bytes) {
+    const int64_t few = std::max<int64_t>(0, gemm_min_rows());
+    return std::max({bytes(T), bytes(std::min(T, few)), bytes(std::min(T, REPACK_MANY_SLOT_ROWS / w->top_k))});
 }
 
 }  // namespace
@@ -242,7 +250,7 @@ int candle_moe_workspace_bytes(const candle_moe_weights_t* w, int64_t max_tokens
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     CM_TRY(check_weights(w));
     if (max_tokens < 0 || max_tokens > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
-    *out_bytes = std::max(layout(w, max_tokens, nullptr).total_ext, layout(w, small_rows(max_tokens), nullptr).total_ext);
+    *out_bytes = for_every_batch(w, max_tokens, [&](int64_t rows) { return layout(w, rows, nullptr).total_ext; });
     return CANDLE_MOE_OK;
 }
 
@@ -317,7 +325,11 @@ int candle_moe_grouped_down(void* stream, const void* const* w2, int32_t dtype, 
 
 namespace cmoe {
 // A large batch over Q6_K experts that have no repacked copies: expert by expert, its matrices are repacked into the workspace and
-// taken through the GEMM (see repacks_on_the_way for when and what it measured).
+// taken through the GEMM (see repacks_on_the_way for when and what it measured).  K of the down product is split until no f32 sum
+// runs over more than twelve blocks, as far as the slots go (two for more than 2048 rows, whose partial outputs weigh most):
+// the forms that take the layer otherwise add in many short runs.  (Relative error against 64-bit arithmetic on the same int8
+// rows, K = 14336: unsplit 1.38e-7, four splits 0.84e-7, streaming 0.72e-7; K = 4096 0.78 / 0.65 / 0.62e-7; row-per-warp K = 2560
+// 0.89, here 0.58e-7.  Up to 4 % of a layer's time.)
 static cudaError_t gemm_repacking(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int E, int K, int N,
                                   const uint32_t* offsets, const uint32_t* row_of, int64_t P, int64_t tile_rows, const int8_t* aq,
                                   const float* ascale, const int16_t* absum, float* out, const ExpertBufs& b, int* n_splits,
@@ -331,7 +343,8 @@ static cudaError_t gemm_repacking(cudaStream_t st, bool gate_up, const ExpertPtr
         if (ce == cudaSuccess && gate_up) ce = launch_prepack(st, CANDLE_GGML_Q6K, wb.p[e], N, K, b.repack + bytes);
         if (ce == cudaSuccess)
             ce = launch_expert_gemm(st, gate_up, ra, rb, CANDLE_GGML_Q6K, true, 1, K, N, offsets + e, row_of, P, tile_rows, aq, ascale, absum,
-                                    out, b.repack_gemm, n_splits ? REPACK_K_SPLITS : 1, n_splits, split_stride, nullptr, x_f32, nullptr, e > 0, true);
+                                    out, b.repack_gemm, n_splits ? repack_slots(P) : 1, n_splits, split_stride, nullptr, x_f32, nullptr, e > 0, true,
+                                    REPACK_MAX_RUN);
         if (ce != cudaSuccess) return ce == cudaErrorNotSupported && e > 0 ? cudaErrorUnknown : ce;
     }
     return cudaSuccess;
@@ -604,7 +617,7 @@ int candle_moe_ffn_layer_workspace_bytes(const candle_moe_weights_t* w, int64_t 
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     if (T < 0 || T > (int64_t)1 << 24) return CANDLE_MOE_E_SHAPE;
     const auto need = [&](int64_t rows) { return layout(w, rows, nullptr).total_ext + align_up((size_t)rows * w->d_model * sizeof(float), 256); };
-    *out_bytes = std::max(need(T), need(small_rows(T)));
+    *out_bytes = for_every_batch(w, T, need);
     return CANDLE_MOE_OK;
 }
 
@@ -864,7 +877,7 @@ int candle_moe_ep_workspace_bytes(const candle_moe_weights_t* w, int64_t max_row
     if (!out_bytes) return CANDLE_MOE_E_NULL;
     if (max_rows_total < 0 || max_rows_total > (int64_t)1 << 26) return CANDLE_MOE_E_SHAPE;
     if (w->dtype_w13 == CANDLE_GGML_Q8_0 || w->dtype_w2 == CANDLE_GGML_Q8_0) return CANDLE_MOE_E_DTYPE;
-    // as small_rows: the slots of the partial outputs fall from 8 to 4 behind this many rows
+    // as for_every_batch: the slots of the partial outputs fall from 8 to 4 behind this many rows
     const int64_t few = std::min(max_rows_total, ep_many_slot_rows(w->n_experts));
     *out_bytes = std::max(ep_layout(w, max_rows_total, nullptr).total, ep_layout(w, few, nullptr).total);
     return CANDLE_MOE_OK;

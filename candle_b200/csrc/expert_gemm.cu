@@ -1254,7 +1254,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
                                bool repacked, int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of, int64_t P,
                                int64_t max_rows, const int8_t* aq, const float* ascale, const int16_t* absum, float* out,
                                void* scratch, int max_splits, int* n_splits_out, int64_t split_stride, float* out_whole,
-                               const float* x_f32, uint32_t* single_group, bool operand_ready, bool exact_gate) {
+                               const float* x_f32, uint32_t* single_group, bool operand_ready, bool exact_gate, int max_run) {
     if (n_splits_out) *n_splits_out = 1;
     if (!scratch || !expert_gemm_takes(gate_up, dtype, repacked, K, N, P) || (x_f32 && row_of)) return cudaErrorNotSupported;
     int tn = max_rows <= 32 ? 32 : (max_rows <= 64 ? 64 : 128);  // position tile, from the bound / hint on an expert's rows
@@ -1358,6 +1358,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         const auto waves = [&](int ks) { return (double)((items * ks + g_gemm_sms - 1) / g_gemm_sms) / ks; };
         for (int ks = 2; ks <= max_splits && kb % ks == 0; ks *= 2)
             if (waves(ks) < (out_whole ? 0.75 : 0.92) * waves(ksplit)) ksplit = ks;
+        while (max_run && kb / ksplit > max_run && ksplit * 2 <= max_splits && kb % (ksplit * 2) == 0) ksplit *= 2;
         *n_splits_out = ksplit;
     }
     G.ksplit = ksplit;

@@ -56,14 +56,15 @@ def test_workspace_query_is_host_only_and_monotonic(lib):
 @pytest.mark.parametrize("kw", [{}, {"copies": True}, {"dtype_w13": 14}, {"dtype_w13": 8, "dtype_w2": 8, "n_experts": 60, "top_k": 4, "d_ff": 1408,
                                                                          "d_model": 2048, "d_ff_shared": 5632, "dtype_shared13": 8, "dtype_shared2": 8}])
 def test_a_workspace_for_many_rows_holds_every_smaller_batch(lib, kw):
-    """Around the row counts where the number of partial outputs falls (96 rows; expert parallelism 2048, 64 per expert)."""
+    """Around the row counts where the number of partial outputs falls (96 rows; 2048 selections where Q6_K is repacked on
+    its way; expert parallelism 2048, 64 per expert)."""
     L, kw = lib.load(), dict(kw)
     table = (C.c_void_p * 128)(*[4096] * 128)
     if kw.pop("copies", False):
         kw.update(w1_prepacked=table, w3_prepacked=table, w2_prepacked=table)
     w, out = _weights(lib, **kw), C.c_size_t(0)
-    for query, rows in ((L.candle_moe_workspace_bytes, (1, 31, 95, 96, 97, 100, 191, 193, 400, 2000, 4096)),
-                        (L.candle_moe_ffn_layer_workspace_bytes, (1, 95, 96, 97, 130, 500)),
+    for query, rows in ((L.candle_moe_workspace_bytes, (1, 31, 95, 96, 97, 100, 191, 193, 400, 511, 513, 1023, 1024, 1025, 1100, 2000, 4096)),
+                        (L.candle_moe_ffn_layer_workspace_bytes, (1, 95, 96, 97, 130, 500, 1024, 1025)),
                         (L.candle_moe_ep_workspace_bytes, (1, 32, 33, 511, 513, 2047, 2048, 2049, 3000, 3841, 5000))):
         if query is L.candle_moe_ep_workspace_bytes and w.dtype_w13 == 8:
             continue
@@ -94,12 +95,14 @@ def _smallest_workspace(lib, w, T):
     (4, 2, 4096, 6144, 400, True),     # instead of the streaming form
     (60, 2, 1536, 1536, 200, False),   # 7 rows each: five launches per expert cost more than the rows do
     (60, 1, 1536, 1536, 200, False),
+    (60, 4, 1536, 1536, 400, True),    # 27 rows each
     (128, 2, 512, 1024, 400, False),   # 640 launches
+    (60, 4, 2048, 2048, 1600, False),  # the streaming form passes over small matrices faster than they are repacked
     (8, 2, 4096, 6144, 240, False),    # 60 rows each: the streaming form passes over a matrix four times in less
 ])
 def test_q6k_without_copies_is_repacked_only_where_the_rows_pay_for_it(lib, E, k, d, ff, T, taken):
-    """Whether a batch asks for room for one expert's repacked matrices: shapes in which that is more than the room of the partial
-    outputs that the form does not use, and row counts whose own size is not below that of a smaller batch."""
+    """Whether a batch asks for room for one expert's repacked matrices (row counts whose own size is not below that of a
+    smaller batch)."""
     w = _weights(lib, dtype_w13=14, dtype_w2=14, n_experts=E, top_k=k, d_model=d, d_ff=ff, router=4096)
     out = C.c_size_t(0)
     assert lib.load().candle_moe_workspace_bytes(C.byref(w), T, C.byref(out)) == 0

@@ -193,6 +193,17 @@ def test_one_block_takes_batches_in_any_order(orc, torch_cuda, w13, w2, fs):
         blk.prepack()
 
 
+def _hidden_rows(torch, blk, first, T):
+    """The hidden rows a call left in the block's scratch, found by the first of them."""
+    words, ff = blk._ws[blk._ws_ptr() - blk._ws.data_ptr():].view(torch.float32), first.numel()
+    tol = 1e-4 * float(first.abs().max())
+    starts = ((words[:words.numel() - T * ff:64].double() - first[0].double()).abs() <= tol).nonzero()[:, 0].tolist()
+    for o in (64 * i for i in starts):
+        if torch.allclose(words[o:o + ff].double(), first.double(), rtol=0, atol=tol):
+            return words[o:o + T * ff].reshape(T, ff)
+    raise AssertionError("the hidden rows were not found in the scratch")
+
+
 def test_gate_of_repacked_q6k_is_the_exact_one(orc, torch_cuda):
     """Q6_K gate_up repacked on its way: silu as the forms for other batch sizes compute it (expf, an exact division), since the
     hidden rows are quantized again.  Operands whose sums are exact in f32 (scales are powers of two, integers small), so that
@@ -218,8 +229,34 @@ def test_gate_of_repacked_q6k_is_the_exact_one(orc, torch_cuda):
     blk.forward(torch.full((T, d), 0.125, device="cuda"))
     gate = sc * m * (512 * 2.0 ** -14 * 0.125)  # -15.9 .. 15.4; the other product is 1
     want = torch.from_numpy(gate / (1 + np.exp(-gate))).cuda()
-    words = blk._ws[blk._ws_ptr() - blk._ws.data_ptr():].view(torch.float32)
-    at = [o for o in range(0, words.numel() - T * ff, 64) if torch.allclose(words[o:o + ff].double(), want, rtol=1e-4, atol=0)][:1]
-    assert at, "the hidden rows were not found in the scratch"
-    got = words[at[0]:at[0] + T * ff].reshape(T, ff).double()
+    got = _hidden_rows(torch, blk, want, T).double()
     assert float(((got - want) / want).abs().max()) <= 2.01 * 2 ** -23
+
+
+def test_down_product_of_repacked_q6k_adds_short_runs(orc, torch_cuda):
+    """The down product of 14336 columns repacked on its way, against 64-bit arithmetic on the same int8 rows.  56 block sums in
+    a row are off by about 2^-24 sqrt(56 / 6) of the sum's size (1.8e-7 with nothing else, 1.4e-7 measured), four runs of 14 and
+    their sum by 2^-24 sqrt((14 + 2 * 4) / 6) = 1.1e-7, less where the terms differ in size."""
+    torch = torch_cuda
+    from candle_b200 import GgmlDType, Mlp, MlpOrMoe, QMatMul, QTensor, _lib
+    d, ff, T = 4096, 14336, 500
+    g = torch.Generator(device="cuda").manual_seed(1)
+    mk = lambda n, k, t: QTensor.quantize(torch.randn((n, k), generator=g, device="cuda") * 0.02, t)
+    w1, w3, w2 = mk(ff, d, GgmlDType.Q4K), mk(ff, d, GgmlDType.Q4K), mk(d, ff, GgmlDType.Q6K)
+    blk = MlpOrMoe.moe(1, torch.zeros((1, d), device="cuda"), [Mlp(QMatMul(w1), QMatMul(w2), QMatMul(w3))])
+    x = torch.randn((T, d), generator=g, device="cuda")
+    y = blk.forward(x)
+
+    def int8_rows(v):
+        rows, k = v.shape
+        q = torch.empty((rows, k), dtype=torch.int8, device="cuda")
+        s, bs = torch.empty((rows, k // 256), device="cuda"), torch.empty((rows, k // 16), dtype=torch.int16, device="cuda")
+        assert _lib.load().candle_moe_quantize_act(torch.cuda.current_stream().cuda_stream, v.data_ptr(), rows, k, int(GgmlDType.Q6K), q.data_ptr(),
+                                                   s.data_ptr(), bs.data_ptr()) == 0
+        return (q.double().reshape(rows, -1, 256) * s.double()[..., None]).reshape(rows, k)
+
+    x0 = int8_rows(x[:1].contiguous())
+    gate, up = x0 @ w1.dequantize().double().T, x0 @ w3.dequantize().double().T
+    hidden = _hidden_rows(torch, blk, (gate / (1 + torch.exp(-gate)) * up)[0], T)
+    ref = int8_rows(hidden.contiguous()) @ w2.dequantize().double().T
+    assert float((y.double() - ref).norm() / ref.norm()) < 1.1e-7
