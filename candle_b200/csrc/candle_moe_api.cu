@@ -360,15 +360,20 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     if (total_rows_hint <= 0) total_rows_hint = P;
     const int E = w->n_experts, d = w->d_model, ff = w->d_ff;
     const bool large = b.gemm && max_rows > (rows_exact ? GEMM_MIN_ROWS_EXACT : gemm_min_rows()) && gemm_enabled();
-    const bool use_prepacked = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked &&
-                               max_rows <= std::max<int64_t>(gemm_min_rows(), 64) && !large;
+    bool use_prepacked = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked &&
+                         max_rows <= std::max<int64_t>(gemm_min_rows(), 64) && !large;
     bool gate_done = false, down_done = false;
     *eo_splits = 1;
     ExpertPtrs q1, q3, q2;
     if (use_prepacked) {
-        CM_TRY(fill_ptrs(w->w1_prepacked, E, q1));
-        CM_TRY(fill_ptrs(w->w3_prepacked, E, q3));
-        CM_TRY(fill_ptrs(w->w2_prepacked, E, q2));
+        int st_copies = fill_ptrs(w->w1_prepacked, E, q1);
+        if (st_copies == CANDLE_MOE_OK) st_copies = fill_ptrs(w->w3_prepacked, E, q3);
+        if (st_copies == CANDLE_MOE_OK) st_copies = fill_ptrs(w->w2_prepacked, E, q2);
+        // tables with a missing or misaligned entry: an error for k-quants, left alone with Q8_0 matrices (which need no copies here)
+        if (st_copies != CANDLE_MOE_OK && w->dtype_w13 != CANDLE_GGML_Q8_0 && w->dtype_w2 != CANDLE_GGML_Q8_0) return st_copies;
+        use_prepacked = st_copies == CANDLE_MOE_OK;
+    }
+    if (use_prepacked) {
         cudaError_t ce = cudaErrorNotSupported;
         const SharedGroup* const tries[2] = {shared ? &shared->gate : nullptr, nullptr};  // with the shared expert, or without
         for (const SharedGroup* sg : tries) {

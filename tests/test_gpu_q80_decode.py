@@ -63,3 +63,24 @@ def test_q80_projection_ignores_a_copy_it_cannot_read(orc, torch_cuda):
     mm._prepacked = torch.cat([torch.zeros(8, dtype=torch.uint8, device="cuda"), mm._prepacked])[8:]
     assert mm._prepacked.data_ptr() % 16 == 8
     assert H.rel_l2(mm.forward(torch.from_numpy(x).cuda()).cpu().numpy(), orc.matmul(orc.Q8_0, x, wq, n)) < 1e-6
+
+
+@pytest.mark.parametrize("w13,w2", [("Q8_0", "Q8_0"), ("Q4K", "Q8_0"), ("Q4K", "Q6K")])
+def test_tables_with_a_hole(orc, torch_cuda, w13, w2):
+    """Copies for some experts only: a decode-sized batch with Q8_0 matrices runs on the GGUF blocks, bit for bit as without
+    tables; k-quants refuse such tables."""
+    torch = torch_cuda
+    from candle_b200 import _lib
+    cfg = dict(d=512, ff=512, E=4, k=2, dt13=getattr(orc, w13), dt2=getattr(orc, w2), renorm=True)
+    blk, _ = H.random_device_block(orc, torch, cfg, seed=3)
+    x = torch.from_numpy(orc.make_activations(3, 9, 512)).cuda()
+    plain = blk.forward(x).clone()
+    blk.prepack()
+    for value in (None, blk._p2[2] + 8):
+        blk._p2[2] = value
+        if w2 == "Q8_0":
+            assert torch.equal(blk.forward(x), plain)
+        else:
+            with pytest.raises(_lib.CandleMoeError) as e:
+                blk.forward(x)
+            assert e.value.status == (-1 if value is None else -5)
