@@ -32,6 +32,7 @@
 // sit in neighbouring lanes and meet with one shuffle.
 // Every mbarrier wait is bounded (see stream_common.cuh); nothing here uses cluster multicast.
 #include <algorithm>
+#include <cmath>
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
 
@@ -1349,15 +1350,27 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     // outputs are summed by whoever consumes them (combine, or the expert-parallel scatter)
     int ksplit = 1;
     if (!gate_up && n_splits_out && max_splits > 1) {
-        const int64_t rows_per = std::max<int64_t>(1, std::min<int64_t>(max_rows, P));
-        const int64_t items = (int64_t)G.m_tiles * std::max<int64_t>(1, std::min<int64_t>(E, (P + rows_per - 1) / rows_per)) *
-                              ((rows_per + tn - 1) / tn);
-        // Time in units of an unsplit item: whole waves of items over the SMs.  A split has to shorten that by enough: partial
-        // sums cost a little in a consumer that reads the result anyway (0.92), a kernel and their traffic where an unsplit
-        // result is final (0.75: [32000, 4096] at 32 rows is 250 items, two waves whether split in two or not).
-        const auto waves = [&](int ks) { return (double)((items * ks + g_gemm_sms - 1) / g_gemm_sms) / ks; };
+        // Position tiles of all experts: of its rows where there is one expert, else expected (in whole tiles) of rows scattered
+        // around their average like independent draws
+        double tiles = (double)((std::min<int64_t>(max_rows, P) + tn - 1) / tn);
+        if (E > 1) {
+            const double experts = (double)std::min<int64_t>(E, P), avg = std::min((double)P / E, (double)max_rows);
+            double extra = 0.0;  // tiles of an expert beyond its first
+            for (double m = tn; m < avg + 4.0 * std::sqrt(avg) + 1.0; m += tn) extra += 0.5 * std::erfc((m + 0.5 - avg) / std::sqrt(2.0 * avg));
+            tiles = std::floor(experts * (1.0 + extra));
+        }
+        const int64_t items = G.m_tiles * (int64_t)tiles;
+        // Time in blocks: whole waves of items over the SMs, an item being its blocks and a turn-over (the accumulators are
+        // stored and a new tile begins) of about one block for 32-wide tiles, one and a half for 64, three and a half for 128.
+        // A split has to shorten that by enough: partial sums cost a little in a consumer that reads the result anyway
+        // (0.95), a kernel and their traffic where an unsplit result is final (0.75: [32000, 4096] at 32 rows is 250 items, two
+        // waves whether split in two or not).  By waves alone, without the turn-over, sums of few blocks were split: 16 experts,
+        // top-8, d = 2048, ff = 1024 (four blocks), 1000 rows 288 -> 399 us, now 283; 32 experts, top-4, d = 1536, ff = 2048, 800 rows 257
+        // -> 206; 8 experts, d = 4096, ff = 4096, 257 rows 205 -> 187.
+        const double turn = tn == 32 ? 1.0 : (tn == 64 ? 1.5 : 3.5);
+        const auto time = [&](int ks) { return (double)((items * ks + g_gemm_sms - 1) / g_gemm_sms) * ((double)kb / ks + turn); };
         for (int ks = 2; ks <= max_splits && kb % ks == 0; ks *= 2)
-            if (waves(ks) < (out_whole ? 0.75 : 0.92) * waves(ksplit)) ksplit = ks;
+            if (time(ks) < (out_whole ? 0.75 : 0.95) * time(ksplit)) ksplit = ks;
         while (max_run && kb / ksplit > max_run && ksplit * 2 <= max_splits && kb % (ksplit * 2) == 0) ksplit *= 2;
         *n_splits_out = ksplit;
     }

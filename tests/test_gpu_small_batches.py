@@ -260,3 +260,19 @@ def test_down_product_of_repacked_q6k_adds_short_runs(orc, torch_cuda):
     hidden = _hidden_rows(torch, blk, (gate / (1 + torch.exp(-gate)) * up)[0], T)
     ref = int8_rows(hidden.contiguous()) @ w2.dequantize().double().T
     assert float((y.double() - ref).norm() / ref.norm()) < 1.1e-7
+
+
+@pytest.mark.parametrize("T,E,k,d,ff,slots", [(200, 16, 8, 1024, 1024, 1), (300, 8, 8, 512, 512, 1), (130, 8, 2, 1024, 3584, 2)])
+def test_sums_of_few_blocks_are_not_split(orc, torch_cuda, T, E, k, d, ff, slots):
+    """How many partial outputs the down product on the GEMM leaves: none beyond the first where K has a few blocks and the tiles
+    fill the device, two where they do not.  Read from the scratch, which is filled with a pattern before the call."""
+    torch = torch_cuda
+    cfg = dict(d=d, ff=ff, E=E, k=k, dt13=orc.Q4K, dt2=orc.Q4K, renorm=True)
+    blk, _ = H.random_device_block(orc, torch, cfg, seed=2)
+    x = torch.from_numpy(orc.make_activations(2, T, d)).cuda()
+    blk.reserve(T)
+    blk._ws.fill_(255)
+    blk.forward(x)
+    untouched = int((blk._ws[blk._ws_ptr() - blk._ws.data_ptr():].view(torch.int32) == -1).sum())
+    int8_rows = T * k * ff * (1 + 4 / 256 + 2 / 16) / 4  # of the hidden rows: not written where the operand's preparation quantizes
+    assert 4 - slots <= (untouched - int8_rows) / (T * k * d) < 4.9 - slots
