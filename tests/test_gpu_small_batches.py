@@ -276,3 +276,23 @@ def test_sums_of_few_blocks_are_not_split(orc, torch_cuda, T, E, k, d, ff, slots
     untouched = int((blk._ws[blk._ws_ptr() - blk._ws.data_ptr():].view(torch.int32) == -1).sum())
     int8_rows = T * k * ff * (1 + 4 / 256 + 2 / 16) / 4  # of the hidden rows: not written where the operand's preparation quantizes
     assert 4 - slots <= (untouched - int8_rows) / (T * k * d) < 4.9 - slots
+
+
+@pytest.mark.parametrize("rows", [32, 64])
+def test_narrow_gemm_tiles_add_in_runs(orc, torch_cuda, rows):
+    """A dense Q6_K product of 4096 columns on the GEMM with K unsplit, against 64-bit arithmetic on the same int8 rows: 16 block
+    sums in a row were off by 7.8e-8, two runs of eight are by 6.5e-8 (2^-24 sqrt(n / 6) and what the rounding of the scales
+    adds: 0.6 of 2^-24 for n = 1)."""
+    torch = torch_cuda
+    from candle_b200 import GgmlDType, QMatMul, QTensor, _lib
+    n, k = 12800, 4096
+    g = torch.Generator(device="cuda").manual_seed(4)
+    w = QTensor.quantize(torch.randn((n, k), generator=g, device="cuda") * 0.02, GgmlDType.Q6K)
+    x = torch.randn((rows, k), generator=g, device="cuda")
+    q = torch.empty((rows, k), dtype=torch.int8, device="cuda")
+    s, bs = torch.empty((rows, k // 256), device="cuda"), torch.empty((rows, k // 16), dtype=torch.int16, device="cuda")
+    assert _lib.load().candle_moe_quantize_act(torch.cuda.current_stream().cuda_stream, x.data_ptr(), rows, k, int(GgmlDType.Q6K), q.data_ptr(),
+                                               s.data_ptr(), bs.data_ptr()) == 0
+    ref = (q.double().reshape(rows, -1, 256) * s.double()[..., None]).reshape(rows, k) @ w.dequantize().double().T
+    y = QMatMul(w).prepack().forward(x)
+    assert float((y.double() - ref).norm() / ref.norm()) < 7.1e-8
