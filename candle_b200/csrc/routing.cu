@@ -279,10 +279,10 @@ constexpr int ROUTER_SMALL_MAX_D = 10240;  // the row in 40 KB of shared memory
 // 140 rows 389 -> 375, 290 rows equal; d = 1024, 257 rows 77 against 86 us the other way round).
 static bool router_small(int64_t T, int d) { return d <= ROUTER_SMALL_MAX_D && (T <= 64 || (d >= 4096 && T <= 256)); }
 
-// Many tokens (and rows too long for the form above): 256 threads per token, so that eight CTAs share an SM and their
-// load rounds overlap.  The forms add the partial sums in different orders (last-bit differences of the logits, as between
-// any two f32 dot-product orders).
-constexpr int ROUTER_THREADS = 256;
+// Many tokens: 256 threads per token, so that eight CTAs share an SM and their load rounds overlap.  Few tokens with rows too
+// long for the form above: 1024 threads (d = 16384, 60 experts, 16 rows 61 -> 44 us, two experts 10.0 -> 6.8).  The forms add
+// the partial sums in different orders (last-bit differences of the logits, as between any two f32 dot-product orders).
+template <int ROUTER_THREADS>
 __global__ void __launch_bounds__(ROUTER_THREADS)
 router_topk_kernel(const float* __restrict__ x, const float* __restrict__ wg, const float* __restrict__ bias,
                    int d, int E, int k, int renorm, uint32_t* __restrict__ ids, float* __restrict__ wout,
@@ -458,8 +458,8 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
     if (T >= 512 && E >= 16 && !qs && !counts && d % 32 == 0)
         return launch_k(router_topk_tiled_kernel, dim3((unsigned)((T + RT_TOK - 1) / RT_TOK)), dim3(RT_THREADS), 0, st, x, router, bias, T, d,
                         E, k, renorm, ids, w);
-    return launch_k(router_topk_kernel, dim3((unsigned)T), dim3(ROUTER_THREADS), 0, st, x, router, bias, d, E, k, renorm, ids, w, qs, scales,
-                    bsums, counts, offsets, perm_token, pair_pos);
+    return launch_k(T > 64 ? router_topk_kernel<256> : router_topk_kernel<1024>, dim3((unsigned)T), dim3(T > 64 ? 256 : 1024), 0, st, x, router,
+                    bias, d, E, k, renorm, ids, w, qs, scales, bsums, counts, offsets, perm_token, pair_pos);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -33,12 +33,13 @@ def test_router_at_the_edges_of_its_forms(orc, torch_cuda, E, k):
             assert np.allclose(w.cpu().numpy()[same], w_ref[same], rtol=5e-5, atol=1e-7), (d, T)
 
 
-@pytest.mark.parametrize("E,d", [(8, 4096), (60, 1024), (60, 4096), (60, 8192), (128, 10240)])
+@pytest.mark.parametrize("E,d", [(8, 4096), (60, 1024), (60, 4096), (60, 8192), (128, 10240), (60, 32768)])
 def test_router_logits_are_as_exact_as_short_sums(torch_cuda, E, d):
-    """The logits of the small form against 64-bit arithmetic.  Sums of n terms of random sign in a row are off by about
+    """The logits of the forms for few rows against 64-bit arithmetic.  Sums of n terms of random sign in a row are off by about
     2^-24 sqrt(n / 6) of the root of their sum of squares (which here is the size of the sum): 2.3 units of 2^-24 for 32 terms, 6.5
     for 256, while runs of ten, four components and a tree over 32 lanes stay near 2^-24 sqrt((10 + 2 * 7) / 6) = 2.  The
-    softmax's own rounding of a probability adds about one."""
+    softmax's own rounding of a probability adds about one.  (Longer rows than the small form takes have 32
+    terms in a row and a sum over 32 warps.)"""
     torch = torch_cuda
     from candle_b200 import _lib
     T, k = 64, 8
@@ -51,7 +52,7 @@ def test_router_logits_are_as_exact_as_short_sums(torch_cuda, E, d):
                                               ids.data_ptr(), w.data_ptr()) == 0
     ref = torch.softmax(x.double() @ wg.double().T, -1).gather(1, ids.long())
     err = torch.log(w.double()) - torch.log(ref)  # of a logit, with that of the row's normaliser
-    assert float(err.pow(2).mean().sqrt()) < 3.0 * 2 ** -24
+    assert float(err.pow(2).mean().sqrt()) < (3.0 if d <= 10240 else 4.0) * 2 ** -24
 
 
 @pytest.mark.parametrize("E,k", [(16, 2), (60, 4), (64, 8), (65, 3), (128, 8)])
