@@ -275,12 +275,21 @@ router_topk_small_kernel(const float* __restrict__ x, const float* __restrict__ 
     if (counts) dispatch_one_token(sel_e, lane, E, k, counts, offsets, perm_token, pair_pos);
 }
 constexpr int ROUTER_SMALL_MAX_D = 10240;  // the row in 40 KB of shared memory
-// Up to 64 tokens; rows long enough to keep 1024 threads busy up to 256 (Mixtral-shaped layer, d = 4096: 100 rows 354.8 -> 345.5 us,
-// 140 rows 389 -> 375, 290 rows equal; d = 1024, 257 rows 77 against 86 us the other way round).
-static bool router_small(int64_t T, int d) { return d <= ROUTER_SMALL_MAX_D && (T <= 64 || (d >= 4096 && T <= 256)); }
+// Up to 64 tokens; rows long enough to keep 1024 threads busy up to 256 with the norm on the way (Mixtral-shaped layer, d = 4096:
+// 100 rows 354.8 -> 345.5 us, 140 rows 389 -> 375, 290 rows equal; d = 1024, 257 rows 77 against 86 us the other way round), without
+// it as far as that is no slower: beyond one CTA per SM only with many experts (router alone, other form / this, 200 rows of 4096:
+// 8 experts 6.8 / 10.5 us, 16 10.3 / 12.7, 32 16.7 / 16.6, 64 31.6 / 26.2; 100 rows: 8 experts 5.8 / 5.8, 16 8.4 / 6.9), and not for
+// the one round of five to eight experts that the other form makes of a few rows (16 rows, 8 experts: d = 4096 5.4 / 5.7, 8192
+// 6.4 / 7.0; two experts 5.0 / 4.8, 16 experts 7.6 / 6.9).
+constexpr int ROUTER_SMALL_WAVE = 148, ROUTER_SMALL_MANY_EXPERTS = 32;
+static bool router_small(int64_t T, int d, int E, bool norm) {
+    if (d > ROUTER_SMALL_MAX_D || T > (d >= 4096 ? 256 : 64)) return false;
+    if (norm) return true;
+    return T <= 64 ? E <= 4 || E > 8 : T <= ROUTER_SMALL_WAVE || E >= ROUTER_SMALL_MANY_EXPERTS;
+}
 
-// Many tokens: 256 threads per token, so that eight CTAs share an SM and their load rounds overlap.  Few tokens with rows too
-// long for the form above: 1024 threads (d = 16384, 60 experts, 16 rows 61 -> 44 us, two experts 10.0 -> 6.8).  The forms add
+// Many tokens: 256 threads per token, so that eight CTAs share an SM and their load rounds overlap.  Few tokens that the form
+// above does not take: 1024 threads (d = 16384, 60 experts, 16 rows 61 -> 44 us, two experts 10.0 -> 6.8).  The forms add
 // the partial sums in different orders (last-bit differences of the logits, as between any two f32 dot-product orders).
 template <int ROUTER_THREADS>
 __global__ void __launch_bounds__(ROUTER_THREADS)
@@ -440,7 +449,7 @@ router_topk_tiled_kernel(const float* __restrict__ x, const float* __restrict__ 
 }
 
 // the fused norm is there only where the small form runs
-bool router_fuses_norm(int64_t T, int d) { return router_small(T, d); }
+bool router_fuses_norm(int64_t T, int d) { return router_small(T, d, 1, true); }
 
 cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* router, const float* bias, int64_t T,
                                int d, int E, int k, int renorm, uint32_t* ids, float* w, int8_t* qs, float* scales,
@@ -448,7 +457,7 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
                                const float* norm_w, float eps) {
     if (T == 0) return cudaSuccess;
     if (counts && (T != 1 || !offsets || !perm_token || !pair_pos)) return cudaErrorInvalidValue;  // single-token dispatch only
-    if (router_small(T, d)) {
+    if (router_small(T, d, E, norm_w != nullptr)) {
         const int parts = E <= 4 ? 8 : (E <= 8 ? 4 : (E <= 16 ? 2 : 1));
         auto kfn = norm_w ? router_topk_small_kernel<true> : router_topk_small_kernel<false>;
         return launch_k(kfn, dim3((unsigned)T), dim3(1024), (size_t)d * sizeof(float), st, x, norm_w, eps, router, bias, d, E, parts, k,

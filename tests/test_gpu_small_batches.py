@@ -16,7 +16,7 @@ def test_router_at_the_edges_of_its_forms(orc, torch_cuda, E, k):
     from candle_b200 import _lib
     # rows of few float4s, of an odd number, the longest of the small form and one beyond; the last count takes the other form
     for d in (4, 36, 1028, 4096, 10240, 10244):
-        for T in (1, 64, 65) if d <= 1028 else (256, 257) if d == 4096 and E in (8, 17) else (3,):
+        for T in (1, 64, 65) if d <= 1028 else (148, 149, 256, 257) if d == 4096 and E in (8, 17, 33) else (3,):
             rng = np.random.default_rng(E + d + T)
             x = rng.standard_normal((T, d), dtype=np.float32)
             wg = rng.standard_normal((E, d), dtype=np.float32) * np.float32(0.05)
