@@ -359,19 +359,24 @@ router_topk_kernel(const float* __restrict__ x, const float* __restrict__ wg, co
 
 // Many tokens and many experts (prefill of a fine-grained layer): the router product as a tiled f32 GEMM.  The
 // one-token kernels spend their time in warp reductions -- one per (token, expert) -- which for 60 experts and 4096
-// tokens is most of 0.15 ms.  Here a CTA of 128 threads takes 16 tokens x up to 64 experts at a time: x and the router rows
+// tokens is most of 0.15 ms.  Here a CTA of 128 threads takes 16 tokens x all experts (64, 96 or 128): x and the router rows
 // pass through shared memory in K chunks of 64 (the next chunk is fetched into registers while this one is multiplied), a
-// thread accumulates 2 tokens x 4 experts in registers, six 128-bit shared loads per 32 multiply-adds, and the four warps
+// thread accumulates 2 tokens x 4 (6, 8) experts in registers, six 128-bit shared loads per 32 multiply-adds, and the four warps
 // then do the softmax and the selection of four tokens each.  Every logit is one sequential f32 sum over K (another order than
 // the one-token kernels': last-bit differences, as between any two f32 dot products).  No fused quantization: used where the
 // activations are quantized by a pass of their own (Q8_0 experts).  Bound by the multiply-adds (15 us for 60 experts,
 // d = 2048, 4096 tokens), the shared loads and the latency of the chunks.  Measured there: one token x eight experts per
 // thread, 32 tokens per CTA of 256 threads (nine shared loads, a CTA per SM) 93 us; this 70 us.  (Four K slices per CTA took
 // 47 us, but add a logit in four parts: kept as one sum, so that the logits stay what they were bit for bit.)
-constexpr int RT_TOK = 16, RT_EXP = 64, RT_KC = 64, RT_PAD = RT_KC + 4, RT_THREADS = 128;
-__global__ void __launch_bounds__(RT_THREADS)
+// NJ experts per thread: 16 NJ experts, as few as hold them all (65 experts, 4096 tokens of 2048: two passes of 64 205 us, one
+// of 96 140).  MIN_CTAS: four CTAs per SM where their registers allow it; with eight experts per thread three of them do more
+// (128 experts, 4096 tokens 135 against 196 us), unless the CTAs then make a second wave (8192 tokens 231 against 198).
+constexpr int RT_TOK = 16, RT_KC = 64, RT_PAD = RT_KC + 4, RT_THREADS = 128;
+template <int NJ, int MIN_CTAS>
+__global__ void __launch_bounds__(RT_THREADS, MIN_CTAS)
 router_topk_tiled_kernel(const float* __restrict__ x, const float* __restrict__ wg, const float* __restrict__ bias,
                          int64_t T, int d, int E, int k, int renorm, uint32_t* __restrict__ ids, float* __restrict__ wout) {
+    constexpr int RT_EXP = 16 * NJ;
     pdl_trigger();
     pdl_wait();
     __shared__ __align__(16) float s_x[RT_TOK][RT_PAD];
@@ -381,62 +386,60 @@ router_topk_tiled_kernel(const float* __restrict__ x, const float* __restrict__ 
     const int64_t t0 = (int64_t)blockIdx.x * RT_TOK;
     const int tg = lane & 7, eg = warp * 4 + (lane >> 3);  // tokens tg, tg + 8; experts eg + 16 j
     const int col = tid & 15, row = tid >> 4;              // loads: float4 column, row + 8 i
-    for (int e0 = 0; e0 < E; e0 += RT_EXP) {
-        float acc[2][4];
+    float acc[2][NJ];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-        // rows past the end repeat the last one (their results are not used); columns past d are not read
-        const float4* px[2];
+        for (int j = 0; j < NJ; ++j) acc[i][j] = 0.f;
+    // rows past the end repeat the last one (their results are not used); columns past d are not read
+    const float4* px[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) px[i] = reinterpret_cast<const float4*>(x + min(t0 + row + 8 * i, T - 1) * (int64_t)d) + col;
-        float4 vx[2], vw[8];
-        auto fetch = [&](int c) {
-            if (c + 4 * col < d) {
+    for (int i = 0; i < 2; ++i) px[i] = reinterpret_cast<const float4*>(x + min(t0 + row + 8 * i, T - 1) * (int64_t)d) + col;
+    float4 vx[2], vw[2 * NJ];
+    auto fetch = [&](int c) {
+        if (c + 4 * col < d) {
 #pragma unroll
-                for (int i = 0; i < 2; ++i) vx[i] = px[i][c >> 2];
+            for (int i = 0; i < 2; ++i) vx[i] = px[i][c >> 2];
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    vw[i] = reinterpret_cast<const float4*>(wg + (int64_t)min(e0 + row + 8 * i, E - 1) * d + c)[col];
-            }
-        };
-        fetch(0);
-        for (int c = 0; c < d; c += RT_KC) {
-            __syncthreads();  // the previous chunk has been consumed
-#pragma unroll
-            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(&s_x[row + 8 * i][4 * col]) = vx[i];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(&s_w[row + 8 * i][4 * col]) = vw[i];
-            __syncthreads();
-            if (c + RT_KC < d) fetch(c + RT_KC);  // the next chunk travels while this one is multiplied
-            const int n4 = min(RT_KC, d - c) >> 2;
-#pragma unroll 8
-            for (int k4 = 0; k4 < n4; ++k4) {
-                float4 xv[2], wv[4];
-#pragma unroll
-                for (int i = 0; i < 2; ++i) xv[i] = *reinterpret_cast<const float4*>(&s_x[tg + 8 * i][4 * k4]);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) wv[j] = *reinterpret_cast<const float4*>(&s_w[eg + 16 * j][4 * k4]);
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]);
-                        acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
-                        acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]);
-                        acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
-                    }
-            }
+            for (int i = 0; i < 2 * NJ; ++i)
+                vw[i] = reinterpret_cast<const float4*>(wg + (int64_t)min(row + 8 * i, E - 1) * d + c)[col];
         }
+    };
+    fetch(0);
+    for (int c = 0; c < d; c += RT_KC) {
+        __syncthreads();  // the previous chunk has been consumed
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(&s_x[row + 8 * i][4 * col]) = vx[i];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int e = e0 + eg + 16 * j;
-                if (e < E) s_logits[tg + 8 * i][e] = acc[i][j] + (bias ? bias[e] : 0.f);
-            }
+        for (int i = 0; i < 2 * NJ; ++i) *reinterpret_cast<float4*>(&s_w[row + 8 * i][4 * col]) = vw[i];
+        __syncthreads();
+        if (c + RT_KC < d) fetch(c + RT_KC);  // the next chunk travels while this one is multiplied
+        const int n4 = min(RT_KC, d - c) >> 2;
+#pragma unroll 8
+        for (int k4 = 0; k4 < n4; ++k4) {
+            float4 xv[2], wv[NJ];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) xv[i] = *reinterpret_cast<const float4*>(&s_x[tg + 8 * i][4 * k4]);
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) wv[j] = *reinterpret_cast<const float4*>(&s_w[eg + 16 * j][4 * k4]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
+                }
+        }
     }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const int e = eg + 16 * j;
+            if (e < E) s_logits[tg + 8 * i][e] = acc[i][j] + (bias ? bias[e] : 0.f);
+        }
     __syncthreads();
     for (int i = warp; i < RT_TOK; i += RT_THREADS / 32) {
         const int64_t t = t0 + i;
@@ -464,9 +467,14 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
                         renorm, ids, w, qs, scales, bsums, counts, offsets, perm_token, pair_pos);
     }
     if (norm_w) return cudaErrorInvalidValue;
-    if (T >= 512 && E >= 16 && !qs && !counts && d % 32 == 0)
-        return launch_k(router_topk_tiled_kernel, dim3((unsigned)((T + RT_TOK - 1) / RT_TOK)), dim3(RT_THREADS), 0, st, x, router, bias, T, d,
-                        E, k, renorm, ids, w);
+    if (T >= 512 && E >= 16 && !qs && !counts && d % 32 == 0) {
+        const int64_t ctas = (T + RT_TOK - 1) / RT_TOK;
+        auto kfn = E <= 64                           ? router_topk_tiled_kernel<4, 4>
+                   : E <= 96                         ? router_topk_tiled_kernel<6, 4>
+                   : ctas > 3 * 148 && ctas <= 4 * 148 ? router_topk_tiled_kernel<8, 4>
+                                                     : router_topk_tiled_kernel<8, 3>;
+        return launch_k(kfn, dim3((unsigned)ctas), dim3(RT_THREADS), 0, st, x, router, bias, T, d, E, k, renorm, ids, w);
+    }
     return launch_k(T > 64 ? router_topk_kernel<256> : router_topk_kernel<1024>, dim3((unsigned)T), dim3(T > 64 ? 256 : 1024), 0, st, x, router,
                     bias, d, E, k, renorm, ids, w, qs, scales, bsums, counts, offsets, perm_token, pair_pos);
 }

@@ -55,12 +55,13 @@ def test_router_logits_are_as_exact_as_short_sums(torch_cuda, E, d):
     assert float(err.pow(2).mean().sqrt()) < (3.0 if d <= 10240 else 4.0) * 2 ** -24
 
 
-@pytest.mark.parametrize("E,k", [(16, 2), (60, 4), (64, 8), (65, 3), (128, 8)])
+@pytest.mark.parametrize("E,k", [(16, 2), (60, 4), (64, 8), (65, 3), (96, 6), (97, 2), (128, 8)])
 def test_tiled_router(orc, torch_cuda, E, k):
-    """Many tokens and experts: fewer K chunks than slices, a ragged last token tile, one and two passes over the experts."""
+    """Many tokens and experts: rows of half a K chunk, of one and a half and of a ragged last one, a ragged last token tile,
+    four, six and eight experts per thread."""
     torch = torch_cuda
     from candle_b200 import _lib
-    for d, T in ((32, 512), (96, 513), (1056, 543)):
+    for d, T in ((32, 512), (96, 513), (1056, 543), (64, 7105)):
         rng = np.random.default_rng(E + d)
         x = rng.standard_normal((T, d), dtype=np.float32)
         wg = rng.standard_normal((E, d), dtype=np.float32) * np.float32(0.05)
