@@ -266,7 +266,7 @@ decode_attention_ring_kernel(const float* __restrict__ q, const float* __restric
     Cursor pf;  // what to request next
     pf.unit = blockIdx.x;
     open(pf);
-    uint32_t n_req = 0, n_use = 0;
+    uint32_t n_req = 0, n_use = 0, n_issued = 0;  // n_issued: lane 0's; equal to n_req until the abort flag is seen
     auto request = [&](uint32_t dep) {  // dep: 0, known only once the slot's old contents have arrived in registers
         if (pf.unit >= n_units) return;
         const uint32_t s = n_req % RING_DEPTH + dep;
@@ -276,6 +276,7 @@ decode_attention_ring_kernel(const float* __restrict__ q, const float* __restric
             mbar_expect_tx(&full[warp][s], 2 * bytes);
             bulk_g2s(my_ring_p + s * 2 * RING_HALF_BYTES, kc + row * RING_D, bytes, &full[warp][s]);
             bulk_g2s(my_ring_p + s * 2 * RING_HALF_BYTES + RING_HALF_BYTES, vc + row * RING_D, bytes, &full[warp][s]);
+            n_issued = n_req + 1;
         }
         ++n_req;
         pf.tile += RING_WARPS;
@@ -416,9 +417,11 @@ decode_attention_ring_kernel(const float* __restrict__ q, const float* __restric
         }
         __syncthreads();
     }
-    // nothing of this CTA's copies may be in flight when it leaves (only after a wait that gave up)
-    if (lane == 0)
-        for (; n_use < n_req; ++n_use) mbar_wait(&full[warp][n_use % RING_DEPTH], (n_use / RING_DEPTH) & 1, abort_flag);
+    // Nothing of this CTA's copies may be in flight when it leaves.  Without the abort flag every one has been waited for; with it
+    // the last ones issued (at most one per slot) may not have been.
+    if (lane == 0 && *abort_flag)
+        for (uint32_t i = n_issued > RING_DEPTH ? n_issued - RING_DEPTH : 0; i < n_issued; ++i)
+            mbar_drain(&full[warp][i % RING_DEPTH], (i / RING_DEPTH) & 1);
     __syncthreads();
     if (threadIdx.x == 0 && s_abort) atomicOr(status, 1);
 }

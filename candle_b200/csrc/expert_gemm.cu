@@ -1181,6 +1181,10 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
     }
     tc5_fence_before_sync();
     __syncthreads();
+    // After a wait that gave up, copies and MMAs of this CTA may still be under way (the issuing warps have run through their
+    // remaining blocks): give them time, some microseconds each at most, before the shared and tensor memory go
+    if (s_abort)
+        for (int i = 0; i < 5000; ++i) __nanosleep(1000);
     if (warp == G_WARP_TMA) {
         tc5_fence_after_sync();
         tmem_dealloc(tmem_base, G_TMEM_COLS);

@@ -438,12 +438,12 @@ __global__ void __launch_bounds__(32 * (1 + CW), 1) expert_stream_kernel(const _
                              &full_bar[s]);
             }
         }
-        // do not leave while copies into this CTA's shared memory may still be in flight
+        // do not leave while copies into this CTA's shared memory may still be in flight (also after a wait that gave up)
         if (lane == 0) {
             const uint32_t n = it < (uint32_t)P.stages ? it : (uint32_t)P.stages;
             for (uint32_t j = 0; j < n; ++j) {
                 const uint32_t last = it - 1 - j;
-                mbar_wait(&full_bar[last % P.stages], (last / P.stages) & 1, abort_flag);
+                mbar_drain(&full_bar[last % P.stages], (last / P.stages) & 1);
             }
         }
     } else {
@@ -723,19 +723,39 @@ cudaError_t reset_stream_status() {
 }
 
 namespace {
-// Waits on a barrier that nothing completes: the bounded wait gives up after `limit` polls and the kernel returns.
+// Waits on a barrier that nothing completes: the bounded wait gives up after `limit` polls.  A copy issued beside it must have
+// arrived, abort flag or not, when its drain returns; then the kernel returns.
+constexpr int SELFTEST_WORDS = 2048;
+__device__ __align__(16) uint32_t g_selftest_src[SELFTEST_WORDS];
 __global__ void selftest_wait_kernel(int limit, int* status) {
-    __shared__ uint64_t bar;
-    __shared__ int s_abort;
+    __shared__ uint64_t bar, copied;
+    __shared__ int s_abort, s_bad;
+    __shared__ __align__(16) uint32_t dst[SELFTEST_WORDS];
+    for (int i = threadIdx.x; i < SELFTEST_WORDS; i += blockDim.x) {
+        g_selftest_src[i] = 0x9e3779b9u * (i + 1);
+        dst[i] = 0;
+    }
     if (threadIdx.x == 0) {
-        s_abort = 0;
+        s_abort = s_bad = 0;
         mbar_init(&bar, 1);
+        mbar_init(&copied, 1);
         fence_barrier_init();
     }
+    __threadfence();
     __syncthreads();
     mbar_wait(&bar, 0, &s_abort, limit);
     __syncthreads();
-    if (threadIdx.x == 0 && s_abort) atomicOr(status, 1);
+    if (threadIdx.x == 0) {
+        asm volatile("fence.proxy.async;" ::: "memory");  // the words above were written by ordinary stores
+        mbar_expect_tx(&copied, sizeof(dst));
+        bulk_g2s(dst, g_selftest_src, sizeof(dst), &copied);
+    }
+    __syncthreads();
+    const bool arrived = mbar_drain(&copied, 0);
+    for (int i = threadIdx.x; i < SELFTEST_WORDS; i += blockDim.x)
+        if (!arrived || dst[i] != 0x9e3779b9u * (i + 1)) s_bad = 1;
+    __syncthreads();
+    if (threadIdx.x == 0 && s_abort) atomicOr(status, s_bad ? 1 | 1 << 8 : 1);
 }
 }  // namespace
 

@@ -60,6 +60,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     *abort_flag = 1;
     return false;
 }
+// After a wait that gave up: a copy that was issued completes this phase, whatever the abort flag says, so its CTA must not
+// leave before (bounded, as every wait: a phase whose copies were never issued runs into the limit).
+__device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity, int limit = SPIN_LIMIT) {
+    for (int i = 0; i < limit; ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        __nanosleep(20);
+    }
+    return false;
+}
 // The same wait for warps that run ahead of their consumer (producers waiting for a free stage): they sleep
 // between polls so that their polling does not take issue slots from the warps that work.  (try_wait with a
 // suspend-time hint is no alternative: it is expanded into exactly such a loop.)

@@ -394,8 +394,9 @@ CANDLE_MOE_API int candle_moe_grouped_down_prepacked(void* stream, const void* c
  * received slot header fails its checks.  candle_moe_device_status synchronises the device and returns the
  * accumulated flags in *flags (0 = healthy); candle_moe_device_status_reset clears them.
  * candle_moe_selftest_bounded_wait enqueues a one-CTA kernel that waits, with the library's own wait primitive and
- * the given poll limit, on a barrier that nothing ever completes: the wait runs out, the kernel raises bit 0 and
- * returns -- the way to see the give-up path work without a stuck copy.
+ * the given poll limit, on a barrier that nothing ever completes: the wait runs out, the kernel raises bit 0 (and
+ * bit 8 if a copy issued beside it had not arrived after its own bounded wait) and returns -- the way to see the give-up
+ * path work without a stuck copy.
  * No counterpart in the reference (its kernels do not wait on asynchronous copies). */
 CANDLE_MOE_API int candle_moe_device_status(int32_t* flags);
 CANDLE_MOE_API int candle_moe_device_status_reset(void);
