@@ -347,7 +347,7 @@ struct DirectParams {
 // 64 us, 8 rows 109 -> 100, 16 rows 129 -> 124, 96 rows 229 -> 211; 16 experts, 8 rows 85 -> 72.)
 template <class F, bool GATE_UP, int NT, int DEPTH, bool SH>
 // The one-position-tile Q4_K and Q8_0 kernels are held to 96 registers (a bound of 608 threads; they are launched with
-// 512, and Q6_K would spill): the
+// 512; they fit but for 8 bytes of the Q8_0 down product with a shared group, Q6_K needs 128): the
 // registers a CTA leaves free let the CTAs of the next kernel on the stream become resident and run their
 // prologue under programmatic dependent launch while this one drains.
 __global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIRECT_THREADS, 1) expert_direct_kernel(const __grid_constant__ DirectParams P) {
@@ -399,7 +399,9 @@ __global__ void __launch_bounds__(NT == 1 && F::HTB != Q6K_HTB_BYTES ? 608 : DIR
       const bool sh = SH && e == P.E;
       const uint32_t e_base = sh ? 0u : s_offs[e], cnt = sh ? (uint32_t)P.sh.rows : s_offs[e + 1] - e_base;
       const int gN = sh ? P.sh.N : P.N, gK = sh ? P.sh.K : P.K, gkb = sh ? P.sh.kb : P.kb, tiles = gN / TILE_N;
-      const size_t ht_stride = (size_t)(sh ? P.sh.kb_stride : P.kb_stride) * F::HTB;  // bytes of one half-tile over the whole K
+      // bytes of one half-tile over the whole K (only Q8_0 copies are padded; a second value to keep made the one-tile k-quant
+      // kernels spill, up to 32 bytes, and left out of the two-tile ones it made those spill)
+      const size_t ht_stride = (size_t)(BLK == 256 && NT == 1 ? P.kb : (sh ? P.sh.kb_stride : P.kb_stride)) * F::HTB;
       for (uint32_t g0 = 0; g0 < cnt && acc < hi; g0 += MT) {
         const uint32_t rows = min((uint32_t)MT, cnt - g0);
         const int w = group_weight(rows);
