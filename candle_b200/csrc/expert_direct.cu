@@ -266,7 +266,9 @@ struct DirQ6K {
 struct DirQ80 {
     static constexpr int HTB = Q80_HTB_BYTES;
     static constexpr int BLK = 128, SC_PER_BLOCK = 4;
-    static constexpr int TWO_TILES_COST = 9;  // 17 bytes per weight pair and one MMA per block: the copies bound it either way
+    // as for the k-quants, although fewer instructions are issued here (60 experts and a shared one, 48 / 64 / 96 rows: cost 8 187 /
+    // 192 / 215 us, 9 178 / 188 / 211, 11 171 / 177 / 206; 16 experts, 32 rows 85 / 83 / 81; 8 of 4096 x 8192, 64 rows 254 / 260 / 268)
+    static constexpr int TWO_TILES_COST = 11;
     static constexpr int BS_PER_BLOCK = 0;  // no offset term: no block sums
     struct Frag {
         uint4 qa[2], qb[2];  // per 64 elements: {block 0 k 0-15, k 16-31, block 1 k 0-15, k 16-31} of rows g and g + 8
