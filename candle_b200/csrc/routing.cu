@@ -275,16 +275,17 @@ router_topk_small_kernel(const float* __restrict__ x, const float* __restrict__ 
     if (counts) dispatch_one_token(sel_e, lane, E, k, counts, offsets, perm_token, pair_pos);
 }
 constexpr int ROUTER_SMALL_MAX_D = 10240;  // the row in 40 KB of shared memory
-// Up to 64 tokens; rows long enough to keep 1024 threads busy up to 256 with the norm on the way (Mixtral-shaped layer, d = 4096:
-// 100 rows 354.8 -> 345.5 us, 140 rows 389 -> 375, 290 rows equal; d = 1024, 257 rows 77 against 86 us the other way round), without
-// it as far as that is no slower: beyond one CTA per SM only with many experts (router alone, other form / this, 200 rows of 4096:
-// 8 experts 6.8 / 10.5 us, 16 10.3 / 12.7, 32 16.7 / 16.6, 64 31.6 / 26.2; 100 rows: 8 experts 5.8 / 5.8, 16 8.4 / 6.9), and not for
-// the one round of five to eight experts that the other form makes of a few rows (16 rows, 8 experts: d = 4096 5.4 / 5.7, 8192
-// 6.4 / 7.0; two experts 5.0 / 4.8, 16 experts 7.6 / 6.9).
+// Up to 64 tokens; rows long enough to keep 1024 threads busy up to 256 (Mixtral-shaped layer, d = 4096: 100 rows 354.8 -> 345.5 us,
+// 140 rows 389 -> 375, 290 rows equal; d = 1024, 257 rows 77 against 86 us the other way round).  That holds inside the block, where
+// this form asks for the router's rows in L2 while the kernel before it still runs; a router called on its own keeps the other
+// forms where they are faster: beyond one CTA per SM except with many experts (other form / this, 200 rows of 4096: 8 experts
+// 6.8 / 10.5 us, 16 10.3 / 12.7, 32 16.7 / 16.6, 64 31.6 / 26.2; 100 rows: 8 experts 5.8 / 5.8, 16 8.4 / 6.9), and for the one round of five
+// to eight experts that the other form makes of a few rows (16 rows, 8 experts: d = 4096 5.4 / 5.7, 8192 6.4 / 7.0, but the block
+// of 4096 x 14336 at one row 76.2 / 75.3; two experts 5.0 / 4.8, 16 experts 7.6 / 6.9).
 constexpr int ROUTER_SMALL_WAVE = 148, ROUTER_SMALL_MANY_EXPERTS = 32;
-static bool router_small(int64_t T, int d, int E, bool norm) {
+static bool router_small(int64_t T, int d, int E, bool in_block) {
     if (d > ROUTER_SMALL_MAX_D || T > (d >= 4096 ? 256 : 64)) return false;
-    if (norm) return true;
+    if (in_block) return true;
     return T <= 64 ? E <= 4 || E > 8 : T <= ROUTER_SMALL_WAVE || E >= ROUTER_SMALL_MANY_EXPERTS;
 }
 
@@ -460,7 +461,7 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
                                const float* norm_w, float eps) {
     if (T == 0) return cudaSuccess;
     if (counts && (T != 1 || !offsets || !perm_token || !pair_pos)) return cudaErrorInvalidValue;  // single-token dispatch only
-    if (router_small(T, d, E, norm_w != nullptr)) {
+    if (router_small(T, d, E, norm_w || offsets)) {  // (only the block hands over where the dispatch goes)
         const int parts = E <= 4 ? 8 : (E <= 8 ? 4 : (E <= 16 ? 2 : 1));
         auto kfn = norm_w ? router_topk_small_kernel<true> : router_topk_small_kernel<false>;
         return launch_k(kfn, dim3((unsigned)T), dim3(1024), (size_t)d * sizeof(float), st, x, norm_w, eps, router, bias, d, E, parts, k,
