@@ -469,8 +469,9 @@ decode_attention_merge_kernel(const float* __restrict__ partial, int n_kv, int n
 }
 
 // Positions per unit of the ring kernel: ATT_CHUNK, halved (down to 64, two tiles per warp) while the units do not give every
-// CTA two: a single sequence of 4096 positions has 64 units of 512 for 296 CTAs.
-constexpr int RING_MIN_CHUNK = 64, RING_MIN_UNITS = 592;
+// CTA two: a single sequence of 4096 positions has 64 units of 512 for 296 CTAs, two per SM of a B200.  (The workspace bound
+// rests on the constant; the device is not asked on the way: a step over a context of 16 is 6.5 us, all host time.)
+constexpr int RING_MIN_CHUNK = 64, RING_CTAS = 2 * 148, RING_MIN_UNITS = 2 * RING_CTAS;
 int ring_chunk(int64_t pairs, int n_ctx) {
     int chunk = ATT_CHUNK;
     while (chunk > RING_MIN_CHUNK && pairs * ((n_ctx + chunk - 1) / chunk) < RING_MIN_UNITS) chunk /= 2;
@@ -479,15 +480,12 @@ int ring_chunk(int64_t pairs, int n_ctx) {
 
 cudaError_t launch_ring(cudaStream_t st, const float* q, const float* kc, const float* vc, int B, int n_kv, int64_t max_seq, int n_ctx,
                         float scale, float* y, float* partial) {
-    int dev = 0, sms = 0;
     int* status = nullptr;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = stream_status_ptr(&status);
+    cudaError_t e = stream_status_ptr(&status);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(decode_attention_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_SMEM);
     if (e != cudaSuccess) return e;
     const int chunk = ring_chunk((int64_t)B * n_kv, n_ctx), n_chunks = (n_ctx + chunk - 1) / chunk, n_units = B * n_kv * n_chunks;
-    e = launch_k(decode_attention_ring_kernel, dim3(std::min(n_units, 2 * sms)), dim3(RING_THREADS), (size_t)RING_SMEM, st, q, kc, vc,
+    e = launch_k(decode_attention_ring_kernel, dim3(std::min(n_units, RING_CTAS)), dim3(RING_THREADS), (size_t)RING_SMEM, st, q, kc, vc,
                  max_seq, n_ctx, scale, chunk, n_chunks, n_units, partial, status, 0u);
     if (e != cudaSuccess) return e;
     return launch_k(decode_attention_merge_kernel<RING_D, RING_G>, dim3(n_kv * RING_G, B), dim3(RING_D), 0, st, (const float*)partial, n_kv,
