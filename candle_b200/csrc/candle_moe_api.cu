@@ -27,7 +27,10 @@ inline int64_t gemm_min_rows() { return tuning_get(TUNE_GEMM_MIN_ROWS); }
 // expert with a row more than expected took a second, almost empty tile.)  A single-device forward only knows the
 // bound T.
 constexpr int64_t GEMM_MIN_ROWS_EXACT = 32;
-constexpr int64_t QMM_DIRECT_MAX_ROWS = 64;  // the dense Q8_0 product over its repacked copy: decode kernels up to here
+// The dense Q8_0 product over its repacked copy: decode kernels up to the rows that split K ([32000, 4096], int8 tiles or rows / decode
+// kernels: 8 rows 309 / 37 us, 32 235 / 55, 48 172 / 85, 64 130 / 92; [2048, 4096] 64 rows 42.6 / 19.8, [1024, 512] 22.2 / 15.2;
+// faster in all of 300 sizes from 1024 to 32000 by 512 to 4096).  Every sixteen rows are one more pass over the copy.
+constexpr int64_t QMM_DIRECT_MAX_ROWS = 64;
 constexpr int64_t QMM_GEMM_MIN_ROWS = 48;  // the dense product: one matrix, rows known exactly
 // Decode-sized batches may split K finely (more parallel items, smaller resident activations);
 // larger batches get four slots, enough for the streaming form's activation rows to fit.
