@@ -110,3 +110,22 @@ def random_device_block(orc, torch, cfg, seed=0, device="cuda"):
         mw.sw1, mw.sw3, mw.sw2 = host(s.feed_forward_w1), host(s.feed_forward_w3), host(s.feed_forward_w2)
         mw.shared_gate = kw["shared_expert_gate"].cpu().numpy()
     return blk, mw
+
+
+def smallest_workspace(lib, w, T):
+    """The smallest size that candle_moe_forward takes for T rows: without expert tables its answer changes from E_WORKSPACE (-4) to
+    E_NULL (-1) there, before anything is launched."""
+    import ctypes as C
+    w = type(w).from_buffer_copy(w)
+    w.w1, w.router = None, 4096
+
+    def refused(n):
+        st = lib.load().candle_moe_forward(None, C.byref(w), 4096, T, 4096, 4096, n)
+        assert st in (-1, -4), st
+        return st == -4
+
+    lo, hi = 0, 1 << 40
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if refused(mid) else (lo, mid)
+    return hi

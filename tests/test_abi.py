@@ -6,6 +6,8 @@ import re
 
 import pytest
 
+from tests import helpers as H
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -75,20 +77,6 @@ def test_a_workspace_for_many_rows_holds_every_smaller_batch(lib, kw):
         assert sizes == sorted(sizes), query.__name__
 
 
-def _smallest_workspace(lib, w, T):
-    """The smallest size that candle_moe_forward takes: the answer changes from E_WORKSPACE to E_NULL (no expert tables), before
-    anything is launched."""
-    def refused(n):
-        st = lib.load().candle_moe_forward(None, C.byref(w), 4096, T, 4096, 4096, n)
-        assert st in (-1, -4), st
-        return st == -4
-    lo, hi = 0, 1 << 40
-    while hi - lo > 1:
-        mid = (lo + hi) // 2
-        lo, hi = (mid, hi) if refused(mid) else (lo, mid)
-    return hi
-
-
 @pytest.mark.parametrize("E,k,d,ff,T,taken", [
     (8, 2, 1536, 2560, 200, True),     # 50 rows per expert, 3.9 million weights a matrix
     (16, 2, 2560, 5120, 200, True),
@@ -106,7 +94,7 @@ def test_q6k_without_copies_is_repacked_only_where_the_rows_pay_for_it(lib, E, k
     w = _weights(lib, dtype_w13=14, dtype_w2=14, n_experts=E, top_k=k, d_model=d, d_ff=ff, router=4096)
     out = C.c_size_t(0)
     assert lib.load().candle_moe_workspace_bytes(C.byref(w), T, C.byref(out)) == 0
-    assert (out.value > _smallest_workspace(lib, w, T)) == taken
+    assert (out.value > H.smallest_workspace(lib, w, T)) == taken
 
 
 @pytest.mark.parametrize("field,value,code", [
