@@ -239,7 +239,7 @@ inline void mark(cudaStream_t st, int stage_done) {
 
 extern "C" {
 
-const char* candle_moe_version(void) { return "candle_moe_sm100 0.1"; }
+const char* candle_moe_version(void) { return "candle_moe_sm100 0.2"; }
 
 int candle_moe_set_tuning(int32_t key, int64_t value) { return tuning_set(key, value) ? CANDLE_MOE_OK : CANDLE_MOE_E_SHAPE; }
 int candle_moe_get_tuning(int32_t key, int64_t* value) {

@@ -6,13 +6,12 @@ runtime.  What runs where:
 
 * this library (C ABI): every quantized product -- wq / wk / wv (as one product over their concatenated rows) / wo and
   the lm head through `QMatMul.forward` (`candle_moe_qmatmul`) --, and with `attention="library"` the rest of the
-  attention half: `attention_norm` (`candle_moe_rmsnorm`), rotary embedding + cache append
+  attention half: `attention_norm` (`candle_moe_rmsnorm`, also the final norm), rotary embedding + cache append
   (`candle_moe_rope_kv_append`), the attention over the cache (`candle_moe_decode_attention`); the FFN half of each layer (`ffn_norm` -> MoE block -> `+ residual`) as one call
   (`candle_moe_ffn_layer`), or, with the experts sharded over ranks, `ExpertParallelMoe.forward` between a PyTorch
   RmsNorm and residual add;
-* stock PyTorch ops, with the reference's arithmetic: token embedding lookup, the final norm, the residual add of the
-  attention half, and, with `attention="pytorch"`, the whole glue of the attention half: RmsNorm
-  (candle-nn/src/ops.rs:504-514), interleaved rotary embedding (`rope_i`, candle-nn/src/rotary_emb.rs:53-66, tables of
+* stock PyTorch ops, with the reference's arithmetic: token embedding lookup, the residual add of the attention half,
+  and, with `attention="pytorch"`, the whole glue of the attention half and the final norm: RmsNorm (candle-nn/src/ops.rs:504-514), interleaved rotary embedding (`rope_i`, candle-nn/src/rotary_emb.rs:53-66, tables of
   quantized_llama.rs:410-427), the f32 KV cache append (candle-nn/src/kv_cache.rs:143-164) and the attention itself as
   the reference's `standard_attention` (quantized_llama.rs:303-317: q k^T / sqrt(head_dim), softmax, times v, grouped
   heads instead of a materialised `repeat_kv`).

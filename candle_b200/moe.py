@@ -197,7 +197,9 @@ class MlpOrMoe:
     STAGES = ("router_topk", "permute", "quantize_x", "gate_up", "quantize_h", "down", "shared_expert", "combine")
 
     def forward_timed(self, xs: torch.Tensor):
-        """One forward with CUDA events between its launches: (y, {stage: milliseconds})."""
+        """One forward with CUDA events between its launches: (y, {stage: milliseconds}).  Work that a kernel does on the way
+        counts where it runs: with the GEMM the hidden rows are quantized in "down" ("quantize_h" is then next to nothing), and a
+        Q8_0 shared expert that joins the routed launches counts in "gate_up", "quantize_h" and "down"."""
         x2 = xs.reshape(-1, self.d_model).contiguous()
         T = x2.shape[0]
         self.reserve(max(T, 1))

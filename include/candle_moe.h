@@ -193,8 +193,9 @@ CANDLE_MOE_API int candle_moe_ffn_layer(void* stream, const candle_moe_weights_t
 /* candle_moe_forward with CUDA events recorded on `stream` between its launches; synchronises the
  * stream and writes the device time of each stage in milliseconds to stage_ms[8]:
  * {router (+ fused quantization of x), dispatch, separate quantization of x, gate_up, quantization
- * of the hidden rows, down, shared expert, combine}.  For measurement only (it creates and destroys
- * events); plays the part of the tracing spans around `QMatMul::forward` in the reference
+ * of the hidden rows, down, shared expert, combine}.  Work that a kernel does on the way counts where it runs: the GEMM's
+ * down product quantizes the hidden rows itself, and the products of a Q8_0 shared expert with copies join the routed
+ * experts' launches for small batches.  For measurement only (it creates and destroys events); plays the part of the tracing spans around `QMatMul::forward` in the reference
  * (candle-transformers/src/models/quantized_llama.rs:97-115). */
 CANDLE_MOE_API int candle_moe_forward_timed(void* stream, const candle_moe_weights_t* w, const float* x, int64_t T,
                                             float* y, void* workspace, size_t workspace_bytes, float* stage_ms);
