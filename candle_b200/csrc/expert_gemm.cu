@@ -1378,9 +1378,11 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         double tiles = (double)((std::min<int64_t>(max_rows, P) + tn - 1) / tn);
         if (E > 1) {
             const double experts = (double)std::min<int64_t>(E, P), avg = std::min((double)P / E, (double)max_rows);
-            double extra = 0.0;  // tiles of an expert beyond its first
-            for (double m = tn; m < avg + 4.0 * std::sqrt(avg) + 1.0; m += tn) extra += 0.5 * std::erfc((m + 0.5 - avg) / std::sqrt(2.0 * avg));
-            tiles = std::floor(experts * (1.0 + extra));
+            // tiles of an expert beyond its first: those that nearly every expert fills, and the likely ones beyond
+            const double spread = 4.0 * std::sqrt(avg) + 1.0, sure = std::max(1.0, std::floor((avg - spread) / tn));
+            double extra = sure - 1.0;
+            for (double m = sure * tn; m < avg + spread; m += tn) extra += 0.5 * std::erfc((m + 0.5 - avg) / std::sqrt(2.0 * avg));
+            tiles = std::floor(experts * (1.0 + extra) + 0.1);
         }
         const int64_t items = G.m_tiles * (int64_t)tiles;
         // Time in blocks: whole waves of items over the SMs, an item being its blocks and a turn-over (the accumulators are
@@ -1388,7 +1390,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         // A split has to shorten that by enough: partial sums cost a little in a consumer that reads the result anyway
         // (0.95), a kernel and their traffic where an unsplit result is final (0.75: [32000, 4096] at 32 rows is 250 items, two
         // waves whether split in two or not).  By waves alone, without the turn-over, sums of few blocks were split: 16 experts,
-        // top-8, d = 2048, ff = 1024 (four blocks), 1000 rows 288 -> 399 us, now 283; 32 experts, top-4, d = 1536, ff = 2048, 800 rows 257
+        // top-8, d = 2048, ff = 1024 (four blocks), 1000 rows 288 -> 399 us, now 267; 32 experts, top-4, d = 1536, ff = 2048, 800 rows 257
         // -> 206; 8 experts, d = 4096, ff = 4096, 257 rows 205 -> 187; ff = 14336, 100 rows 359 -> 365 (in runs, see the epilogue).
         const double turn = tn == 32 ? 1.0 : (tn == 64 ? 1.5 : 3.5);
         const auto time = [&](int ks) { return (double)((items * ks + g_gemm_sms - 1) / g_gemm_sms) * ((double)kb / ks + turn); };

@@ -176,6 +176,25 @@ def test_large_batch_over_q6k_without_copies(orc, torch_cuda, w13, w2, T, d, ff,
     assert L.candle_moe_device_status(C.byref(v)) == 0 and v.value == 0
 
 
+@pytest.mark.parametrize("w13,w2,T,d,ff,E", [("Q4K", "Q6K", 97, 512, 1024, 8), ("Q6K", "Q6K", 300, 1024, 1536, 4), ("Q6K", "Q4K", 130, 512, 512, 3),
+                                             ("Q6K", "Q6K", 97, 1536, 512, 8), ("Q6K", "Q6K", 640, 2048, 512, 4)])
+def test_q6k_without_copies_on_either_side_of_the_rule(orc, torch_cuda, w13, w2, T, d, ff, E):
+    """Layers of which the rule takes both products, one or none for the GEMM."""
+    torch = torch_cuda
+    cfg = dict(d=d, ff=ff, E=E, k=2, dt13=getattr(orc, w13), dt2=getattr(orc, w2), renorm=True)
+    blk, mw = H.random_device_block(orc, torch, cfg, seed=T)
+    x = torch.from_numpy(orc.make_activations(T, T, d)).cuda()
+    xs = x.cpu().numpy()
+    ref = orc.moe_forward(mw, xs)
+    y = blk.forward(x).clone()
+    assert torch.equal(y, blk.forward(x))
+    ids = blk.last_routing(T)[0].numpy().astype(np.uint32)
+    H.check_routing(orc.router_topk(xs, mw.router, 2, True, None)[0], ref.topk_ids, ids)
+    same = (ref.topk_ids == ids).all(axis=1)
+    loose = 1.0 if ff >= 1024 else 2.0
+    assert H.rel_l2(y.cpu().numpy()[same], ref.y[same]) <= loose * H.REL_L2_TOL
+
+
 @pytest.mark.parametrize("w13,w2,fs", [("Q4K", "Q6K", 0), ("Q8_0", "Q8_0", 640)])
 def test_one_block_takes_batches_in_any_order(orc, torch_cuda, w13, w2, fs):
     """A block keeps its scratch: a batch just above the decode kernels' range, one just inside it (whose partial outputs
