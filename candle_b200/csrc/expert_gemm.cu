@@ -45,9 +45,10 @@ namespace {
 
 constexpr int G_TILE_M = 128, G_SLAB_K = 64;  // the position tile (N) is a template parameter: 128, or 32 for small batches
 constexpr int G_PAD_ROWS = 128;                // zero rows after the last position, so that no box leaves the buffers
-constexpr int G_W_STAGES_MAX = 4;  // raw weight blocks in flight per CTA (narrow position tiles leave room for a deep ring)
+constexpr int G_W_STAGES_MAX = 6;  // raw weight blocks in flight per CTA (narrow position tiles leave room for a deep ring)
 constexpr int G_B_STAGES = 2;   // in shared memory, one 256-wide block each (four slabs + the min-term box for Q4_K)
-constexpr int G_TILE_BYTES = G_TILE_M * G_SLAB_K * 2;  // one [128 x 64] fp16 (or [128 x 32] tf32) operand tile, 16 KB
+constexpr int G_MIN_K = 16;     // min term of Q4_K: floats per row and block, two K steps of tf32 (64-byte rows, 64-byte swizzle)
+constexpr int G_MIN_A_BYTES = G_TILE_M * G_MIN_K * 4;
 constexpr int G_EPI_WARPS = 8, G_DQ_WARPS = 8;
 // Warp roles.  The MMA and TMA warps take the highest indices: measured, their short instruction streams
 // are served far better there than at the lowest ones (1.75x on the whole kernel).
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(128) write_maps_kernel(const __grid_constant__
 // as the integer main sum M: three more K=8 steps per block, kind::tf32 (fp32 exponent range, 10-bit
 // mantissa).  rho_j (fp32) is split into tf32 terms r1 + r2 (to 2^-23), the integer bsum32 (at most 32 * 127,
 // 12 bits) exactly into b1 + b2; the steps are r1 b1 + r2 b1 + r1 b2.  Per (position, block) the buffer holds
-// 32 floats [b1 (8) | b1 (8) | b2 (8) | 0 (8)], matched by [r1 | r2 | r1 | -] on the weight side.  The main
+// 16 floats [b1 (8) | b2 (8)], matched by [r1 | r2] on the weight side.  The main
 // sum stays an exact integer until these last three steps; what they add in error is of the order of the
 // reference's own f32 rounding (2^-23 of the min term).
 // ---------------------------------------------------------------------------------------------
@@ -125,15 +126,15 @@ prep_gemm_b_kernel(const int8_t* __restrict__ aq, const float* __restrict__ asca
         o = *reinterpret_cast<uint4*>(h);
         d8 = ascale[row * kb + blk];
         if (bmin) {
-            const int j = lane & 7, part = lane >> 3;  // word: part 0, 1 = b1_j; part 2 = b2_j; part 3 = 0
+            const int j = lane & 7;  // word j: b1_j, word 8 + j: b2_j
             const int16_t* bs = absum + row * (K / 16) + blk * 16 + 2 * j;
             const float bv = (float)((int)bs[0] + (int)bs[1]);
             const float b1 = tf32_head(bv), b2 = bv - b1;  // exact: |bv| < 4096, so b2 is -1, 0 or 1
-            bm = part == 2 ? b2 : (part == 3 ? 0.f : b1);
+            bm = lane < 8 ? b1 : b2;
         }
     }
     *reinterpret_cast<uint4*>(bf16 + (int64_t)p * K + blk * 256 + lane * 8) = o;
-    if (bmin) bmin[((int64_t)p * kb + blk) * 32 + lane] = bm;
+    if (bmin && lane < G_MIN_K) bmin[((int64_t)p * kb + blk) * G_MIN_K + lane] = bm;
     if (lane == 0) d8t[(int64_t)blk * P_pad + p] = d8;
 }
 
@@ -229,9 +230,9 @@ prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, _
             for (int i = 0; i < 8; ++i) s += q[i];
             s += __shfl_xor_sync(0xffffffffu, s, 1);
             s += __shfl_xor_sync(0xffffffffu, s, 2);  // 32 elements = four lanes
-            const int j = lane & 7, part = lane >> 3;  // the words of prep_gemm_b_kernel
+            const int j = lane & 7;  // the words of prep_gemm_b_kernel
             const float bv = __shfl_sync(0xffffffffu, s, 4 * j), b1 = tf32_head(bv), b2 = bv - b1;
-            bmin[((int64_t)p[u] * kb + blk[u]) * 32 + lane] = part == 2 ? b2 : (part == 3 ? 0.f : b1);
+            if (lane < G_MIN_K) bmin[((int64_t)p[u] * kb + blk[u]) * G_MIN_K + lane] = lane < 8 ? b1 : b2;
         }
         if (lane == 0) d8t[(int64_t)blk[u] * P_pad + p[u]] = d8;
     }
@@ -374,7 +375,7 @@ struct GemmQ4K {
     static constexpr bool STAGE_W = true;      // raw blocks of the tile pass through shared memory
     static constexpr bool HALF_TILES = false;  // ... as rows of GGUF blocks (tensor-map boxes)
     static constexpr int W_ROW_BYTES = Q4K_BYTES;
-    static constexpr int W_STAGES_WIDE = 1;    // staged blocks that fit beside 128-wide activation stages
+    static constexpr int W_STAGES_WIDE = 3;    // staged blocks that fit beside 128-wide activation stages
     struct Row {};
     struct Pre {
         uint4 hdr, q[4];
@@ -438,7 +439,7 @@ struct GemmQ4K {
         tmem_st32(ta, o);
     }
     // weight side of the min term (see prep_gemm_b_kernel): -rho_j = -dmin m_j / d split into tf32 terms.  One
-    // row is 32 floats [r1 (8) | r2 (8) | r1 (8) | unused]; half h writes its four values of each.  2^23 + m as float
+    // row is 16 floats [r1 (8) | r2 (8)]; half h writes its four values of each.  2^23 + m as float
     // bits is 0x4B000000 | m.
     __device__ static __forceinline__ void emit_min(const Pre& pr, const Ctx& c, uint8_t* arow, int h, int sw) {
         const float ratio = -__fdividef(half_bits_to_float((uint16_t)(pr.hdr.x >> 16)), scale_of(pr.hdr.x));
@@ -452,7 +453,6 @@ struct GemmQ4K {
         }
         *reinterpret_cast<uint4*>(arow + ((h ^ sw) << 4)) = make_uint4(r1[0], r1[1], r1[2], r1[3]);
         *reinterpret_cast<uint4*>(arow + (((2 + h) ^ sw) << 4)) = make_uint4(r2[0], r2[1], r2[2], r2[3]);
-        *reinterpret_cast<uint4*>(arow + (((4 + h) ^ sw) << 4)) = make_uint4(r1[0], r1[1], r1[2], r1[3]);
     }
 };
 
@@ -671,10 +671,15 @@ struct GemmQ80X : GemmQ80 {
     }
 };
 
+// one activation stage: a 256-wide block (four slabs) or the half of one with two operand parts, + the min-term box
+template <class F, int TN>
+__host__ __device__ constexpr int b_stage_bytes() {
+    return 4 * (TN * G_SLAB_K * 2) + (F::HAS_MIN ? TN * G_MIN_K * 4 : 0);
+}
 // raw weight blocks staged per CTA (see the kernel): what fits beside the activation stages
 template <class F, int TN>
 __host__ __device__ constexpr int w_stages() {
-    return !F::STAGE_W ? 1 : (TN <= 32 ? 4 : (TN <= 64 ? (F::B_PARTS == 2 ? 4 : 3) : F::W_STAGES_WIDE));
+    return !F::STAGE_W ? 1 : (TN <= 64 ? (F::HALF_TILES ? 4 : 6) : F::W_STAGES_WIDE);
 }
 
 // weight row of tile row r: gate_up tiles hold 8 rows of W1, then the same 8 rows of W3, and so on (64 rows of each)
@@ -757,14 +762,15 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
     // refilled for the next block as soon as its own pair's MMAs are done; the same shared memory then takes
     // 128-wide position tiles.
     constexpr bool B_HALF = F::B_PARTS == 2;
-    constexpr int G_STAGE_BYTES = (4 + (F::HAS_MIN ? 1 : 0)) * B_TILE;
+    constexpr int G_STAGE_BYTES = b_stage_bytes<F, TN>();
     uint8_t* smem_min_a = smem + G_B_STAGES * G_STAGE_BYTES;  // Q4_K: 2 slots of the min operand (weights side)
-    // staged raw blocks of the tile rows: a ring of WS blocks.  With 128-wide position tiles the activation stages
-    // leave room for one block only (the L2 prefetch ahead of it has to do); narrower tiles take a deeper ring, so
-    // that the copy of block b + WS - 1 is in flight while block b is unpacked.
+    // staged raw blocks of the tile rows: a ring of WS blocks, so that the copy of block b + WS - 1 is in flight while
+    // block b is unpacked.  (Q4_K, 128-wide position tiles: one block and requests into L2 ahead of it, with a min-term box
+    // of 32 floats per row, against three blocks beside 16 floats: 2048 rows 2470 -> 2422 us, 8 small experts at 257
+    // rows 78.0 -> 75.0, [4096, 4096] at 777 rows 53.9 -> 52.9.)
     constexpr int WS = w_stages<F, TN>();
     constexpr int W_STAGE_BYTES = G_TILE_M * F::W_ROW_BYTES;
-    uint8_t* smem_w = smem_min_a + (F::HAS_MIN ? 2 : 0) * G_TILE_BYTES;
+    uint8_t* smem_w = smem_min_a + (F::HAS_MIN ? 2 : 0) * G_MIN_A_BYTES;
     for (int i = threadIdx.x; i <= P.E; i += G_THREADS) s_offs[i] = P.offsets[i];
     if (threadIdx.x == 0) {
         s_abort = 0;
@@ -921,7 +927,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         const int quarter = warp & 3, h = (warp - G_WARP_DQ0) >> 2;
         const int r = 32 * quarter + lane;
         const uint32_t ta_lane = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)G_TM_A;
-        const uint32_t min_row_off = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
+        const uint32_t min_row_off = (uint32_t)(r * G_MIN_K * 4);
         uint32_t ab = 0;
         TileCoord tc, tcn;
         bool have = walk.next(tc);
@@ -990,7 +996,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                     // weight side of the min term.  Its slot was last read by the min MMAs of block ab - 2, issued
                     // before the commit of that block's second pair.
                     if (h == 0 && ab >= 2) mbar_wait_relaxed(&empty_a[2 * (ab & 1) + 1], ((ab - 2) >> 1) & 1, abort_flag);
-                    F::emit_min(cur, ctx, smem_min_a + (size_t)(ab & 1) * G_TILE_BYTES + min_row_off, h, r & 7);
+                    F::emit_min(cur, ctx, smem_min_a + (size_t)(ab & 1) * G_MIN_A_BYTES + min_row_off, h, (r >> 1) & 3);
                     fence_proxy_async_smem();
                 }
                 tmem_st_wait();
@@ -1011,8 +1017,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         // One TMA box per matrix and block: [64 or 128 rows x 144 bytes] of the byte matrix [n_rows, row_bytes]
         // (gate_up: the W1 rows, then the W3 rows; a TMA destination must be 128-byte aligned, so the halves cannot
         // be skewed against each other and neighbouring lanes, which alternate between them, share banks two by
-        // two).  Two blocks ahead the same boxes are requested into L2, so the copy into the one-block-deep stage
-        // finds them there.
+        // two).
         if constexpr (F::HALF_TILES) {
             // half-tile blocks of the repacked layout: one bulk copy per 8 tile rows, lane i < 16 copies half-tile i
             // (gate_up: W1 and W3 half-tiles alternate).  No requests into L2 ahead: the CTAs of a weight tile's position tiles
@@ -1037,22 +1042,17 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
             }
         } else if constexpr (F::STAGE_W) {
             uint32_t ab = 0;
-            TileCoord tc, tcn;
-            bool have = walk.next(tc);
+            int fenced = -1;
+            TileCoord tc;
             constexpr int HALF = G_TILE_M / 2 * F::W_ROW_BYTES;  // 9216
-            while (have) {
-                const bool have_n = walk.next(tcn);
+            while (walk.next(tc)) {
                 const CUtensorMap* m0 = P.wmaps + 2 * tc.e;
-                // the maps were written by a kernel earlier on the stream: fence each once, before its first use by
-                // this warp -- the current expert's on the first tile, the next expert's one tile ahead, because the
-                // prefetches reach into it (every lane fences: any may be elected)
-                if (ab == 0) {
+                // the maps were written by a kernel earlier on the stream: fence an expert's once, before their first use by this
+                // warp (every lane fences: any may be elected)
+                if (fenced != tc.e) {
+                    fenced = tc.e;
                     tensormap_fence_acquire(m0);
                     if (GATE_UP) tensormap_fence_acquire(m0 + 1);
-                }
-                if (have_n && tcn.e != tc.e) {
-                    tensormap_fence_acquire(P.wmaps + 2 * tcn.e);
-                    if (GATE_UP) tensormap_fence_acquire(P.wmaps + 2 * tcn.e + 1);
                 }
                 const int y0 = GATE_UP ? tc.mt * 64 : tc.mt * 128;
                 for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
@@ -1068,20 +1068,9 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                             tma_load_2d(dst, m0, blk * F::W_ROW_BYTES, y0, &full_w[ws]);
                             tma_load_2d(dst + HALF, m0, blk * F::W_ROW_BYTES, y0 + 64, &full_w[ws]);
                         }
-                        // two blocks ahead, possibly in the next tile
-                        const bool same = blk + 2 < tc.kb1;
-                        if (same || have_n) {
-                            const CUtensorMap* mp = same ? m0 : P.wmaps + 2 * tcn.e;
-                            const int yp = same ? y0 : (GATE_UP ? tcn.mt * 64 : tcn.mt * 128);
-                            const int xp = (same ? blk + 2 : tcn.kb0 + blk + 2 - tc.kb1) * F::W_ROW_BYTES;
-                            tma_prefetch_2d(mp, xp, yp);
-                            tma_prefetch_2d(GATE_UP ? mp + 1 : mp, xp, GATE_UP ? yp : yp + 64);
-                        }
                     }
                     __syncwarp();
                 }
-                tc = tcn;
-                have = have_n;
             }
         }
     } else if (warp == G_WARP_TMA) {
@@ -1117,7 +1106,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
 #pragma unroll
                     for (int s4 = 0; s4 < 4; ++s4)
                         tma_load_2d(dst + s4 * B_TILE, &map_b, blk * 256 + s4 * 64, (int)tc.p0, &full_b[st]);
-                    if (F::HAS_MIN) tma_load_2d(dst + 4 * B_TILE, &map_bs, blk * 32, (int)tc.p0, &full_b[st]);
+                    if (F::HAS_MIN) tma_load_2d(dst + 4 * B_TILE, &map_bs, blk * G_MIN_K, (int)tc.p0, &full_b[st]);
                 }
                 __syncwarp();
             }
@@ -1129,7 +1118,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         TileCoord tc;
         const uint32_t a_base = tmem_base + (uint32_t)G_TM_A;
         const uint64_t b_desc0 = umma_desc_sw128(smem_u32(smem));
-        const uint64_t ma_desc0 = umma_desc_sw128(smem_u32(smem_min_a));
+        const uint64_t ma_desc0 = umma_desc_sw64(smem_u32(smem_min_a)), mb_desc0 = umma_desc_sw64(smem_u32(smem) + 4 * B_TILE);
         bool rdy_a = false, rdy_b = false;
         while (walk.next(tc)) {
             // The last position tile of an expert is rarely full: its MMAs run N = the rows it holds, rounded up to 16
@@ -1171,9 +1160,10 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                         }
                         if (pr == 1 && F::HAS_MIN) {
                             // the min term joins the same accumulator: three tf32 steps, last in the block
-                            const uint64_t da = ma_desc0 + (uint64_t)(buf * (G_TILE_BYTES >> 4)), dm = db + (uint64_t)(4 * (B_TILE >> 4));
-#pragma unroll
-                            for (int k = 0; k < 3; ++k) umma_tf32(d_main, da + 2 * k, dm + 2 * k, idesc_tf32, true);
+                            const uint64_t da = ma_desc0 + (uint64_t)(buf * (G_MIN_A_BYTES >> 4)), dm = mb_desc0 + (uint64_t)(buf * (G_STAGE_BYTES >> 4));
+                            umma_tf32(d_main, da, dm, idesc_tf32, true);      // r1 b1
+                            umma_tf32(d_main, da + 2, dm, idesc_tf32, true);  // r2 b1
+                            umma_tf32(d_main, da, dm + 2, idesc_tf32, true);  // r1 b2
                         }
                         umma_commit(&empty_a[bidx]);  // the stages may be refilled once these MMAs have read them
                         if (B_HALF) umma_commit(&empty_b[pr]);
@@ -1217,9 +1207,9 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// row-major matrix [rows, cols] -> boxes of [box_rows x box_cols] (128 bytes wide), 128-byte swizzle
+// row-major matrix [rows, cols] -> boxes of [box_rows x box_cols], as wide as the swizzle (128 or 64 bytes)
 bool make_map_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t rows, uint64_t cols,
-                 uint32_t box_cols, uint32_t box_rows) {
+                 uint32_t box_cols, uint32_t box_rows, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {cols, rows};
@@ -1227,7 +1217,7 @@ bool make_map_2d(CUtensorMap* map, const void* base, CUtensorMapDataType dt, int
     const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     return fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // byte matrix [rows, row_bytes] -> boxes of [box_rows x box_bytes], no swizzle
@@ -1246,7 +1236,7 @@ int g_gemm_sms = -1;
 
 template <class F, bool GATE_UP, int TN>
 cudaError_t launch_gemm_kernel(cudaStream_t st, const GemmParams& G, const CUtensorMap& map_b, const CUtensorMap& map_bs) {
-    const int smem_bytes = G_B_STAGES * (4 + (F::HAS_MIN ? 1 : 0)) * (TN * G_SLAB_K * 2) + (F::HAS_MIN ? 2 : 0) * G_TILE_BYTES +
+    const int smem_bytes = G_B_STAGES * b_stage_bytes<F, TN>() + (F::HAS_MIN ? 2 : 0) * G_MIN_A_BYTES +
                            (F::STAGE_W ? w_stages<F, TN>() * G_TILE_M * F::W_ROW_BYTES : 0) + 1024 /* alignment slack */;
     auto kfn = expert_gemm_kernel<F, GATE_UP, TN>;
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
@@ -1269,7 +1259,7 @@ cudaError_t launch_prepack_q80(cudaStream_t st, const void* raw, int64_t n_rows,
 size_t expert_gemm_scratch_bytes(int64_t P, int K, int parts) {
     K = (K + 255) / 256 * 256;  // Q8_0 rows are padded to whole 256-element blocks
     const size_t p_pad = (size_t)P + G_PAD_ROWS, kb = (size_t)K / 256;
-    return align_up(p_pad * K * 2 * parts, 256) + align_up(p_pad * kb * 64 * 2, 256) + align_up(kb * p_pad * 4, 256) +
+    return align_up(p_pad * K * 2 * parts, 256) + align_up(p_pad * kb * G_MIN_K * 4, 256) + align_up(kb * p_pad * 4, 256) +
            sizeof(CUtensorMap) * 2 * CANDLE_MOE_MAX_EXPERTS;
 }
 
@@ -1312,7 +1302,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     uint8_t* base = static_cast<uint8_t*>(scratch);
     __half* bf16 = reinterpret_cast<__half*>(base);
     float* bmin = reinterpret_cast<float*>(base + align_up((size_t)p_pad * K * 2 * parts, 256));
-    float* d8t = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bmin) + align_up((size_t)p_pad * kb * 32 * 4, 256));
+    float* d8t = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bmin) + align_up((size_t)p_pad * kb * G_MIN_K * 4, 256));
     const bool has_min = dtype == CANDLE_GGML_Q4K;
 
     // byte-matrix tensor maps of the raw weight blocks (Q4_K): [n_rows, kb * 144] with boxes of 64 rows x one block, written to
@@ -1361,7 +1351,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     CUtensorMap map_b, map_bs;
     if (!make_map_2d(&map_b, bf16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)p_pad, (uint64_t)K * parts, G_SLAB_K, tn))
         return cudaErrorNotSupported;
-    if (!make_map_2d(&map_bs, bmin, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)p_pad, (uint64_t)kb * 32, 32, tn))
+    if (!make_map_2d(&map_bs, bmin, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)p_pad, (uint64_t)kb * G_MIN_K, G_MIN_K, tn, CU_TENSOR_MAP_SWIZZLE_64B))
         return cudaErrorNotSupported;
 
     GemmParams G{};

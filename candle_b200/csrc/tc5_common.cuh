@@ -116,6 +116,16 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;                        // layout: SWIZZLE_128B
     return d;
 }
+// Rows of 64 bytes with 64-byte swizzle: 8-row atoms of 512 B, the tile base 512-byte aligned.
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;  // layout: SWIZZLE_64B
+    return d;
+}
 // Instruction descriptor for kind::f16: A and B fp16, both K-major, D fp32, tile M x N.
 __host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N) {
     return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
@@ -161,14 +171,10 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
         ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
-// the same box requested into L2 only (no shared-memory destination, no completion)
 // Orders this thread's later uses of a tensor map through the tensor-map proxy after writes to the map's 128
 // bytes that are already visible to it through the generic proxy (another kernel wrote the map to global memory).
 __device__ __forceinline__ void tensormap_fence_acquire(const void* map) {
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 // generic-proxy writes to shared memory become visible to the async proxy (UMMA / TMA)
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
