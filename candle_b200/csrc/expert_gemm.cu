@@ -2,34 +2,37 @@
 // in tensor memory.
 //
 // out[p, n] = W_e[n, :] . act[row(p), :] for all grouped positions p of every expert, as a grouped GEMM
-// over tiles of 128 weight rows x 128 grouped positions.  The integers are the reference's
+// over tiles of 128 weight rows x 128 (64, 32) grouped positions.  The integers are the reference's
 // (candle-core/src/quantized/k_quants.rs:1205-1285 Q4_K, :1520-1600 Q6_K): activations are the int8
-// Q8K rows, and the weight operand holds (sub-block scale) x (quant), both exact in fp16, multiplied by
-// `tcgen05.mma kind::f16` with fp32 accumulation in tensor memory -- exact while a 256-element block's
-// sum stays below 2^24, which it does by a wide margin for real data.  After every 256-element block
+// Q8K rows, and the weight operand holds (sub-block scale) x (quant).  After every 256-element block
 // the accumulator is drained and scaled by d_w(row, block) * d8(position, block) on the CUDA cores.
-//   Q4_K: operand sc_j * q (at most 63 * 15); the min term joins the same accumulator as three tf32
-//         steps per block against dmin / d (see prep_gemm_b_kernel).
-//   Q6_K: sc_j * (q - 32) reaches 4096 and is not always an fp16 integer, so the int8 scale is split
-//         into ceil(sc/2) + floor(sc/2) and the slab is multiplied twice (each half at most 32 * 64 =
-//         2048: exact).  Reads the repacked layout of the decode kernels (16-byte aligned pieces; the
+//   Q4_K: fp16 operand sc_j * q (at most 63 * 15, exact), `tcgen05.mma kind::f16`, fp32 accumulation in tensor memory
+//         -- exact while a block's sum stays below 2^24, which it does by a wide margin for real data; the min
+//         term joins the same accumulator as three tf32 steps per block against dmin / d (see prep_gemm_b_kernel).
+//   Q6_K: sc_j * (q - 32) reaches 4096 and is not always an fp16 integer: two int8 planes, `kind::i8`, int32
+//         accumulation (exact).  Reads the repacked layout of the decode kernels (16-byte aligned pieces; the
 //         210-byte GGUF blocks are only 2-byte aligned).
+//   Q8_0: see GemmQ80 and GemmQ80X.
 //
-// One CTA per SM, persistent over tiles, warp-specialised (20 warps, five warpgroups):
-//   warps 0-7   epilogue: drain TMEM (tcgen05.ld, next load in flight) once per block, scale, keep 64
-//               columns per thread in registers (128 registers per thread, taken from the last
-//               warpgroup with setmaxnreg); at the end of a tile apply the SiLU gate and store
-//   warps 8-15  unpack the weight nibbles of [128 rows x 64 k] to fp16 x scale with one HFMA2 per two
-//               elements and store them straight into TENSOR MEMORY (tcgen05.st): the A operand never
-//               touches shared memory, whose bandwidth the B operand needs
-//   warp  18    TMA: the activation operand, [128 positions x 64 k] fp16 boxes, 128-byte swizzle; one
-//               stage is a whole 256-wide block (four boxes + the min-term box), two stages
-//   warp  19    issues the MMAs (A from TMEM, B from shared memory) and commits to mbarriers; the whole
-//               warp walks the loop with warp-uniform operands, one elected lane issues
-// Tensor memory: two main accumulators (2 x 128 columns: the MMAs of block b+1 overlap the drain of
-// block b) and a 256-column ring of weight-operand slabs, handed over in pairs.  gate_up interleaves
-// rows of W1 and W3 (tile row 2i = W1 row, 2i+1 = W3 row) so the two factors of silu(w1 x) * (w3 x)
-// sit in neighbouring lanes and meet with one shuffle.
+// One CTA per SM, persistent over tiles, warp-specialised:
+//   4 or 8 warps  epilogue: drain TMEM once per block, scale, keep CH columns per thread in registers (taken from
+//                 the last warpgroup with setmaxnreg); at the end of a tile apply the SiLU gate and store
+//   8 warps       unpack: two groups take the blocks in turn, a thread a weight row; the operand goes straight into
+//                 TENSOR MEMORY (tcgen05.st) and never touches shared memory, whose bandwidth the B operand needs
+//   4 warps       raw weight blocks -> shared memory; activation scales of the drain; TMA of the activation operand
+//                 (128-byte swizzle, half a 256-wide block per stage); MMA issue (A from TMEM, B from shared memory)
+// Everything goes through short rings of mbarriers: weight stages, pairs of weight slabs with their activation stage, two
+// accumulators (the MMAs of block b+1 overlap the drain of block b).  gate_up interleaves rows of W1 and W3 so that the two
+// factors of silu(w1 x) * (w3 x) sit in neighbouring lanes and meet with one shuffle.
+//
+// What bounds it: not one unit but the kernel's instruction streams.  Narrow tiles (a Mixtral-shaped layer at 100 rows, gate_up)
+// took the same 0.9 us per 128 x 256 block with the unpack's arithmetic, the drain's arithmetic, most of the MMAs and half of
+// the operand copies taken out: the MMA warp walked its few dozen instructions per pair of slabs at several clocks each beside
+// busy warps, behind an instruction cache that 60-90 KB of code -- every wait written out with its give-up path at every place
+// -- did not fit.  Hence constant ring addresses, waits of a few instructions (mbar_wait_tight), no tile search in the unpack
+// warps, one barrier per pair for both operands, masks fused with the fp16 magic number (field).  Layers, before -> after: Mixtral-shaped,
+// 100 rows 388 -> 315 us, 2048 rows 2471 -> 2079; 8 small experts from GGUF blocks, 257 rows 79.4 -> 72.3; 60 Q8_0 experts,
+// 4096 rows 1776 -> 1710; [32000, 4096] Q6_K at 32 rows 49.4 -> 44.4, [4096, 4096] Q4_K at 777 rows 53.8 -> 48.7.
 // Every mbarrier wait is bounded (see stream_common.cuh); nothing here uses cluster multicast.
 #include <algorithm>
 #include <cmath>
@@ -45,20 +48,12 @@ namespace {
 
 constexpr int G_TILE_M = 128, G_SLAB_K = 64;  // the position tile (N) is a template parameter: 128, or 32 for small batches
 constexpr int G_PAD_ROWS = 128;                // zero rows after the last position, so that no box leaves the buffers
-constexpr int G_W_STAGES_MAX = 6;  // raw weight blocks in flight per CTA (narrow position tiles leave room for a deep ring)
-constexpr int G_B_STAGES = 2;   // in shared memory, one 256-wide block each (four slabs + the min-term box for Q4_K)
+// Barriers of the weight stages go by the stage's number modulo this, not by the slot it stands for: each then belongs to one
+// group of unpack warps, which sees every phase of it (a parity wait cannot tell phase k from phase k - 2).
+constexpr int G_W_BARS = 8;
 constexpr int G_MIN_K = 16;     // min term of Q4_K: floats per row and block, two K steps of tf32 (64-byte rows, 64-byte swizzle)
-constexpr int G_MIN_A_BYTES = G_TILE_M * G_MIN_K * 4;
-constexpr int G_EPI_WARPS = 8, G_DQ_WARPS = 8;
-// Warp roles.  The MMA and TMA warps take the highest indices: measured, their short instruction streams
-// are served far better there than at the lowest ones (1.75x on the whole kernel).
-constexpr int G_WARP_EPI0 = 0, G_WARP_DQ0 = G_WARP_EPI0 + G_EPI_WARPS, G_WARP_LOAD = 16, G_WARP_TMA = 18, G_WARP_MMA = 19;
-constexpr int G_THREADS = 32 * 20;  // five warpgroups: 2 epilogue, 2 unpack, 1 with the TMA and MMA warps (+ 2 idle)
-constexpr int G_REGS_EPI = 128, G_REGS_MISC = 32;  // budgets after the trade: 2 * 128 + 2 * 96 + 32 = 5 * 96, the launch allocation
 constexpr int G_TMEM_COLS = 512;
 constexpr int G_RUN = 8;  // blocks that narrow tiles add in a row
-constexpr int G_TM_MAIN = 0;    // + 128 * buffer
-constexpr int G_TM_A = 256;     // weight operand ring: columns 256..511
 
 // Tensor maps of the weight matrices reach device memory as kernel PARAMETERS -- of the operand preparation that runs before the
 // GEMM anyway, and of a small copy kernel for what does not fit there -- never
@@ -100,6 +95,34 @@ __global__ void __launch_bounds__(128) write_maps_kernel(const __grid_constant__
 // nearest value with a 10-bit mantissa (the 13 low bits of the fp32 container zero)
 __device__ __forceinline__ float tf32_head(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
 
+// four integers of at most 128 as bytes: 2^23 + 2^22 + v has v in its low bits
+__device__ __forceinline__ uint32_t pack_s8(float a, float b, float c, float d) {
+    const uint32_t ab = __byte_perm(__float_as_uint(a + 12582912.f), __float_as_uint(b + 12582912.f), 0x0040);
+    const uint32_t cd = __byte_perm(__float_as_uint(c + 12582912.f), __float_as_uint(d + 12582912.f), 0x0040);
+    return __byte_perm(ab, cd, 0x5410);
+}
+// Q6_K: the int8 rows themselves, in grouped order
+__global__ void __launch_bounds__(256)
+prep_gemm_i8_kernel(const int8_t* __restrict__ aq, const float* __restrict__ ascale, const uint32_t* __restrict__ row_of, int P, int P_pad,
+                    int K, int8_t* __restrict__ b8, float* __restrict__ d8t) {
+    pdl_trigger();
+    pdl_wait();
+    const int kb = K >> 8;
+    const int lane = threadIdx.x & 31;
+    const int64_t unit = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // (p, block)
+    if (unit >= (int64_t)P_pad * kb) return;
+    const int p = (int)(unit / kb), blk = (int)(unit - (int64_t)p * kb);
+    uint2 v = make_uint2(0, 0);
+    float d8 = 0.f;
+    if (p < P) {
+        const int64_t row = row_of ? (int64_t)row_of[p] : (int64_t)p;
+        v = *reinterpret_cast<const uint2*>(aq + row * K + blk * 256 + lane * 8);
+        d8 = ascale[row * kb + blk];
+    }
+    *reinterpret_cast<uint2*>(b8 + (int64_t)p * K + blk * 256 + lane * 8) = v;
+    if (lane == 0) d8t[(int64_t)blk * P_pad + p] = d8;
+}
+
 __global__ void __launch_bounds__(256)
 prep_gemm_b_kernel(const int8_t* __restrict__ aq, const float* __restrict__ ascale, const int16_t* __restrict__ absum,
                    const uint32_t* __restrict__ row_of, int P, int P_pad, int K, __half* __restrict__ bf16,
@@ -125,16 +148,14 @@ prep_gemm_b_kernel(const int8_t* __restrict__ aq, const float* __restrict__ asca
         h[3] = __halves2half2(__int2half_rn(b[5]), __int2half_rn(b[7]));
         o = *reinterpret_cast<uint4*>(h);
         d8 = ascale[row * kb + blk];
-        if (bmin) {
-            const int j = lane & 7;  // word j: b1_j, word 8 + j: b2_j
-            const int16_t* bs = absum + row * (K / 16) + blk * 16 + 2 * j;
-            const float bv = (float)((int)bs[0] + (int)bs[1]);
-            const float b1 = tf32_head(bv), b2 = bv - b1;  // exact: |bv| < 4096, so b2 is -1, 0 or 1
-            bm = lane < 8 ? b1 : b2;
-        }
+        const int j = lane & 7;  // word j: b1_j, word 8 + j: b2_j
+        const int16_t* bs = absum + row * (K / 16) + blk * 16 + 2 * j;
+        const float bv = (float)((int)bs[0] + (int)bs[1]);
+        const float b1 = tf32_head(bv), b2 = bv - b1;  // exact: |bv| < 4096, so b2 is -1, 0 or 1
+        bm = lane < 8 ? b1 : b2;
     }
     *reinterpret_cast<uint4*>(bf16 + (int64_t)p * K + blk * 256 + lane * 8) = o;
-    if (bmin && lane < G_MIN_K) bmin[((int64_t)p * kb + blk) * G_MIN_K + lane] = bm;
+    if (lane < G_MIN_K) bmin[((int64_t)p * kb + blk) * G_MIN_K + lane] = bm;
     if (lane == 0) d8t[(int64_t)blk * P_pad + p] = d8;
 }
 
@@ -190,7 +211,7 @@ prep_gemm_b_q80_kernel(const int8_t* __restrict__ aq, const float* __restrict__ 
 // 20.5 + 22.3 us against 28.1; one unit per warp and integer conversions took 82 us for the first.
 constexpr int PREP_UNITS = 2;
 __global__ void __launch_bounds__(256)
-prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, __half* __restrict__ bf16, float* __restrict__ bmin,
+prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, int8_t* __restrict__ b8, __half* __restrict__ bf16, float* __restrict__ bmin,
                          float* __restrict__ d8t, uint32_t* __restrict__ single_group, const __grid_constant__ MapChunk maps) {
     pdl_trigger();
     pdl_wait();
@@ -222,9 +243,14 @@ prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, _
 #pragma unroll
             for (int i = 0; i < 8; ++i) q[i] = (float)(int8_t)(int)q[i];
         }
-        __half2 h[4] = {__floats2half2_rn(q[0], q[2]), __floats2half2_rn(q[1], q[3]), __floats2half2_rn(q[4], q[6]), __floats2half2_rn(q[5], q[7])};
-        *reinterpret_cast<uint4*>(bf16 + (int64_t)p[u] * K + blk[u] * 256 + lane * 8) = *reinterpret_cast<uint4*>(h);
-        if (bmin) {
+        if (b8) {  // Q6_K: as int8
+            uint2 o;
+            o.x = pack_s8(q[0], q[1], q[2], q[3]);
+            o.y = pack_s8(q[4], q[5], q[6], q[7]);
+            *reinterpret_cast<uint2*>(b8 + (int64_t)p[u] * K + blk[u] * 256 + lane * 8) = o;
+        } else {
+            __half2 h[4] = {__floats2half2_rn(q[0], q[2]), __floats2half2_rn(q[1], q[3]), __floats2half2_rn(q[4], q[6]), __floats2half2_rn(q[5], q[7])};
+            *reinterpret_cast<uint4*>(bf16 + (int64_t)p[u] * K + blk[u] * 256 + lane * 8) = *reinterpret_cast<uint4*>(h);
             float s = 0.f;  // sums of integers of at most 128: exact
 #pragma unroll
             for (int i = 0; i < 8; ++i) s += q[i];
@@ -344,7 +370,7 @@ struct GemmParams {
     int m_tiles;                  // tiles along the weight rows (N / 64 for gate_up, N / 128 for down)
     int ksplit;                   // K splits (down only): partial outputs out + ks * split_stride, summed by the caller
     long long split_stride;
-    uint32_t zero;                // 0 at run time, unknown to the compiler (see the release of a weight stage in the kernel)
+    uint32_t magic;               // 0x64006400 (see field)
 };
 
 __device__ __forceinline__ __half2 h2_bits(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
@@ -355,104 +381,94 @@ __device__ __forceinline__ __half2 byte_magic2(uint32_t w, int b) {
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0x64646464u), "r"(0x4040u | (uint32_t)b | ((uint32_t)b << 8)));
     return h2_bits(r);
 }
-__device__ __forceinline__ uint4 ldg128(const uint8_t* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
+// (w & MASK) | magic in one operation: fields of the bytes of w dropped into the mantissa of 1024 (magic = 0x64006400, from a
+// register that the compiler knows nothing about: as constants, mask and magic take an operation each)
+template <uint32_t MASK>
+__device__ __forceinline__ __half2 field(uint32_t w, uint32_t magic) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(magic));
+    return h2_bits(r);
+}
+template <uint32_t MASK>
+__device__ __forceinline__ uint32_t or_field(uint32_t v, uint32_t w) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "n"(MASK), "r"(v));
+    return r;
+}
 __device__ __forceinline__ uint32_t w4(const uint4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
 
 // ------------------------------------------------------------------------------------------------
-// The unpack formats.  An unpack thread owns (tile row, K half h): elements 128 h .. 128 h + 127 of every 256-block,
-// i.e. slabs 2h and 2h + 1 of 64 elements, handed over as one pair.  (Splitting a row's bytes between two threads inside
-// every slab instead made both decode the same scales.)  A slab is 32 TMEM columns of two elements each; element k of
-// the slab belongs to column k / 2, inside a group of four in the order (0, 2), (1, 3).
+// The unpack formats.  An unpack thread owns a tile row of a 256-block and goes through it in two halves: elements 128 h ..
+// 128 h + 127, i.e. slabs 2h and 2h + 1 of 64 elements, handed over as one pair.  A slab is 32 TMEM columns of two
+// elements each (A_PARTS times); element k of the slab belongs to column k / 2, inside a group of four in the order (0, 2),
+// (1, 3).  All formats read raw blocks that were staged in shared memory (`row`: the thread's place in a stage).
 //
 // Q4_K, GGUF layout (144-byte blocks: d, dmin, 12 scale bytes, 128 nibble bytes): bytes 32 s .. 32 s + 31 of the nibbles
 // are slab s, low nibbles k = 0..31, high nibbles k = 32..63.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ4K {
-    static constexpr bool EXACT_GATE = false;
-    static constexpr bool HAS_MIN = true;
-    static constexpr int A_COLS = 32, A_PARTS = 1, A_PAIRS = 4;  // 8 slabs of 32 columns: two blocks in flight
-    static constexpr int B_PARTS = 1;
-    static constexpr bool STAGE_W = true;      // raw blocks of the tile pass through shared memory
-    static constexpr bool HALF_TILES = false;  // ... as rows of GGUF blocks (tensor-map boxes)
-    static constexpr int W_ROW_BYTES = Q4K_BYTES;
-    static constexpr int W_STAGES_WIDE = 3;    // staged blocks that fit beside 128-wide activation stages
-    struct Row {};
-    struct Pre {
-        uint4 hdr, q[4];
-    };
-    __device__ static __forceinline__ void load(Pre&, const Row&, int, int) {}
-    __device__ static __forceinline__ Row row(const uint8_t*, int, int) { return Row{}; }
-    // this thread's pieces of the staged row (rows are 36 words apart: the eight lanes of a 16-byte load phase cover all
-    // 32 banks once)
-    __device__ static __forceinline__ void load_staged(Pre& pr, uint32_t row_addr, int h) {
-        pr.hdr = lds128_o<0>(row_addr);
-        const uint32_t rb = row_addr + 64 * h;
-        pr.q[0] = lds128_o<16>(rb);
-        pr.q[1] = lds128_o<32>(rb);
-        pr.q[2] = lds128_o<48>(rb);
-        pr.q[3] = lds128_o<64>(rb);
-    }
-    // one word of every vector load_staged fetched: a value that exists only when all of them have arrived
-    __device__ static __forceinline__ uint32_t staged_words(const Pre& pr) {
-        return pr.hdr.x | pr.q[0].x | pr.q[1].x | pr.q[2].x | pr.q[3].x;
-    }
-    // d (low half) and dmin (high half) of the block, fp16 bits
-    __device__ static __forceinline__ uint32_t hdr_of(const Pre& pr) { return pr.hdr.x; }
+    static constexpr bool EXACT_GATE = false, I8 = false, HAS_MIN = true;
+    static constexpr int A_PARTS = 1, B_PARTS = 1;
+    static constexpr bool HALF_TILES = false;  // staged as rows of GGUF blocks (tensor-map boxes)
+    static constexpr int W_UNITS = 1;          // stages per 256-block
+    static constexpr int W_UNIT_BYTES = G_TILE_M * Q4K_BYTES;
     struct Ctx {
-        uint32_t sc, mn;  // 6-bit scales / mins of this half's sub-blocks 4h .. 4h + 3 as bytes (utils.rs:50-60)
+        uint32_t dd;            // d (low half) and dmin (high half), fp16 bits
+        uint32_t sc[2], mn[2];  // 6-bit scales / mins of the sub-blocks as bytes (utils.rs:50-60)
     };
-    __device__ static __forceinline__ void begin(const Pre& pr, Ctx& c, int h) {
-        const uint32_t s0 = pr.hdr.y, s1 = pr.hdr.z, s2 = pr.hdr.w;
-        if (h == 0) {
-            c.sc = s0 & 0x3f3f3f3fu;
-            c.mn = s1 & 0x3f3f3f3fu;
-        } else {
-            c.sc = (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
-            c.mn = ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4);
-        }
-        if ((pr.hdr.x & 0x7fffu) == 0) c.sc = 0;  // d = 0: the block is its min term alone (see scale_of)
+    // (rows are 36 words apart: the eight lanes of a 16-byte load phase cover all 32 banks once)
+    __device__ static __forceinline__ void begin(Ctx& c, uint32_t row, int) {
+        const uint4 hdr = lds128_o<0>(row);
+        const uint32_t s0 = hdr.y, s1 = hdr.z, s2 = hdr.w;
+        c.dd = hdr.x;
+        c.sc[0] = s0 & 0x3f3f3f3fu;
+        c.mn[0] = s1 & 0x3f3f3f3fu;
+        c.sc[1] = (s2 & 0x0f0f0f0fu) | (((s0 >> 6) & 0x03030303u) << 4);
+        c.mn[1] = ((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4);
+        if ((hdr.x & 0x7fffu) == 0) c.sc[0] = c.sc[1] = 0;  // d = 0: the block is its min term alone (see scale_of)
     }
     // The epilogue multiplies the block's accumulator by d; a block with d = 0 (and no main sum, above) is
     // scaled by dmin instead so that its min term survives, or by 1 if both are zero.
-    __device__ static __forceinline__ float scale_of(uint32_t hdr) {
-        const uint32_t hb = (hdr & 0x7fffu) ? (hdr & 0xffffu) : (((hdr >> 16) & 0x7fffu) ? (hdr >> 16) : 0x3c00u);
+    __device__ static __forceinline__ float scale_of(const Ctx& c) {
+        const uint32_t hb = (c.dd & 0x7fffu) ? (c.dd & 0xffffu) : (((c.dd >> 16) & 0x7fffu) ? (c.dd >> 16) : 0x3c00u);
         return half_bits_to_float((uint16_t)hb);
     }
-    // slab s of this half = sub-blocks 2s (low nibbles) and 2s + 1 (high nibbles) of the half.  0x6400 | n is 1024 + n
+    // slab s of half h = sub-blocks 2s (low nibbles) and 2s + 1 (high nibbles) of the half.  0x6400 | n is 1024 + n
     // and fma(1024 + n, sc, -1024 sc) rounds the exact n * sc once; 0x6400 | (n << 4) is 1024 + 16 n and
     // fma(1024 + 16 n, sc / 16, -64 sc) does the same for a nibble left in the high half of its byte.
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx& c, uint32_t ta) {
+    __device__ static __forceinline__ void emit(const Ctx& c, uint32_t row, int, int h, uint32_t magic, uint32_t ta) {
         const __half2 k1024 = __float2half2_rn(1024.f);
-        const __half2 scl = __hsub2(byte_magic2(c.sc, 2 * s), k1024);
-        const __half2 sch = __hsub2(byte_magic2(c.sc, 2 * s + 1), k1024);
-        const __half2 offl = __hmul2(scl, __float2half2_rn(-1024.f));
-        const __half2 sch16 = __hmul2(sch, __float2half2_rn(0.0625f)), offh = __hmul2(sch, __float2half2_rn(-64.f));
-        uint32_t o[32];
+        const uint32_t scs = h ? c.sc[1] : c.sc[0], a = row + 64 * h;
+        const uint4 q[4] = {lds128_o<16>(a), lds128_o<32>(a), lds128_o<48>(a), lds128_o<64>(a)};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t x = w4(pr.q[2 * s + (i >> 2)], i & 3), y = x >> 8;  // bytes (0, 2) and (1, 3) of the four
-            o[2 * i] = bits_h2(__hfma2(h2_bits((x & 0x000F000Fu) | 0x64006400u), scl, offl));
-            o[2 * i + 1] = bits_h2(__hfma2(h2_bits((y & 0x000F000Fu) | 0x64006400u), scl, offl));
-            o[16 + 2 * i] = bits_h2(__hfma2(h2_bits((x & 0x00F000F0u) | 0x64006400u), sch16, offh));
-            o[16 + 2 * i + 1] = bits_h2(__hfma2(h2_bits((y & 0x00F000F0u) | 0x64006400u), sch16, offh));
+        for (int s = 0; s < 2; ++s) {
+            const __half2 scl = __hsub2(byte_magic2(scs, 2 * s), k1024);
+            const __half2 sch = __hsub2(byte_magic2(scs, 2 * s + 1), k1024);
+            const __half2 offl = __hmul2(scl, __float2half2_rn(-1024.f));
+            const __half2 sch16 = __hmul2(sch, __float2half2_rn(0.0625f)), offh = __hmul2(sch, __float2half2_rn(-64.f));
+            uint32_t o[32];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t x = w4(q[2 * s + (i >> 2)], i & 3), y = x >> 8;  // bytes (0, 2) and (1, 3) of the four
+                o[2 * i] = bits_h2(__hfma2(field<0x000F000Fu>(x, magic), scl, offl));
+                o[2 * i + 1] = bits_h2(__hfma2(field<0x000F000Fu>(y, magic), scl, offl));
+                o[16 + 2 * i] = bits_h2(__hfma2(field<0x00F000F0u>(x, magic), sch16, offh));
+                o[16 + 2 * i + 1] = bits_h2(__hfma2(field<0x00F000F0u>(y, magic), sch16, offh));
+            }
+            tmem_st32(ta + 32 * s, o);
         }
-        tmem_st32(ta, o);
     }
-    // weight side of the min term (see prep_gemm_b_kernel): -rho_j = -dmin m_j / d split into tf32 terms.  One
-    // row is 16 floats [r1 (8) | r2 (8)]; half h writes its four values of each.  2^23 + m as float
-    // bits is 0x4B000000 | m.
-    __device__ static __forceinline__ void emit_min(const Pre& pr, const Ctx& c, uint8_t* arow, int h, int sw) {
-        const float ratio = -__fdividef(half_bits_to_float((uint16_t)(pr.hdr.x >> 16)), scale_of(pr.hdr.x));
-        uint32_t r1[4], r2[4];
+    // weight side of the min term (see prep_gemm_b_kernel): -rho_j = -dmin m_j / d split into tf32 terms [r1 (8) | r2 (8)].
+    // 2^23 + m as float bits is 0x4B000000 | m.
+    __device__ static __forceinline__ void min_operand(const Ctx& c, uint32_t (&r)[16]) {
+        const float ratio = -__fdividef(half_bits_to_float((uint16_t)(c.dd >> 16)), scale_of(c));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float mf = __uint_as_float(__byte_perm(c.mn, 0x4B000000u, 0x7650 | j)) - 8388608.f;
+        for (int j = 0; j < 8; ++j) {
+            const float mf = __uint_as_float(__byte_perm(c.mn[j >> 2], 0x4B000000u, 0x7650 | (j & 3))) - 8388608.f;
             const float a = __fmul_rn(ratio, mf), a1 = tf32_head(a);
-            r1[j] = __float_as_uint(a1);
-            r2[j] = __float_as_uint(tf32_head(__fsub_rn(a, a1)));
+            r[j] = __float_as_uint(a1);
+            r[8 + j] = __float_as_uint(tf32_head(__fsub_rn(a, a1)));
         }
-        *reinterpret_cast<uint4*>(arow + ((h ^ sw) << 4)) = make_uint4(r1[0], r1[1], r1[2], r1[3]);
-        *reinterpret_cast<uint4*>(arow + (((2 + h) ^ sw) << 4)) = make_uint4(r2[0], r2[1], r2[2], r2[3]);
     }
 };
 
@@ -461,85 +477,61 @@ struct GemmQ4K {
 // high bit pairs 512, 128 scales, 8 d; a row's four 16-byte chunks t of a 512-byte region lie in chunk_pos order).  Word
 // cw of chunk t of half h holds elements k0 = 16 cw + 4 t .. + 3 of the half's two slabs (low nibbles: first slab, high
 // nibbles: second), words 2h, 2h + 1 of chunk t of the third region their high bit pairs.
-// The quant is placed at mantissa bits 4..9 (0x6400 | q << 4 = 1024 + 16 q); minus 1536 leaves
-// 16 (q - 32), times ceil(sc/2)/16 and floor(sc/2)/16 gives the two exact operand parts.
+// sc * (q - 32) reaches 4096, two bits more than an fp16 operand holds: it is multiplied as int8, in two planes
+// p = 256 hi + lo (lo unsigned) with an int32 accumulator each, put together again when a block is drained.  The sums are
+// exact, int8 steps run at twice the rate of fp16 ones, and the activation operand is the int8 row itself.  (As two fp16
+// operands -- the scale in halves, or the low and the high bits of the quant -- the products took the tensor pipe twice the time
+// and the unpack 600-690 clocks per 128 x 128 weights, 560 this way.)
 // ------------------------------------------------------------------------------------------------
 struct GemmQ6K {
-    static constexpr bool EXACT_GATE = false;
-    static constexpr bool HAS_MIN = false;
-    static constexpr int A_COLS = 64, A_PARTS = 2, A_PAIRS = 2;  // 4 slabs of 64 columns (two operand parts each)
-    static constexpr int B_PARTS = 1;
-    static constexpr bool STAGE_W = false;
-    static constexpr bool HALF_TILES = false;
-    static constexpr int W_ROW_BYTES = 0;
-    static constexpr int W_STAGES_WIDE = 1;
-    struct Row {
-        const uint8_t* p;  // half-tile block 0 of the row's group of 8
-        int g;
+    static constexpr bool EXACT_GATE = false, I8 = true, HAS_MIN = false;
+    static constexpr int A_PARTS = 1, B_PARTS = 1;
+    static constexpr bool HALF_TILES = true;  // staged as half-tile blocks, one bulk copy per 8 rows
+    static constexpr int W_UNITS = 1;
+    static constexpr int W_UNIT_BYTES = G_TILE_M / 8 * Q6K_HTB_BYTES;
+    struct Ctx {
+        float d;
     };
-    __device__ static __forceinline__ Row row(const uint8_t* w, int n, int kb) {
-        return Row{w + (size_t)(n >> 3) * kb * Q6K_HTB_BYTES, n & 7};
-    }
-    struct Pre {
+    __device__ static __forceinline__ void begin(Ctx& c, uint32_t row, int g) { c.d = half_bits_to_float((uint16_t)lds16(row + 1664 + 2 * g)); }
+    __device__ static __forceinline__ float scale_of(const Ctx& c) { return c.d; }
+    // columns of a pair: [lo: slab 0 (16) | slab 1 (16) | hi: slab 0 | slab 1], element k of a slab in column k / 4
+    __device__ static __forceinline__ void emit(const Ctx&, uint32_t row, int g, int h, uint32_t, uint32_t ta) {
+        const uint2 scw = lds64_o<1536>(row + 16 * g + 8 * h);
         uint4 ql[4];
-        uint2 qh[4], sc;
-        uint32_t d;  // fp16 bits
-    };
-    __device__ static __forceinline__ uint32_t hdr_of(const Pre& pr) { return pr.d; }
-    __device__ static __forceinline__ void load_staged(Pre&, uint32_t, int) {}
-    __device__ static __forceinline__ uint32_t staged_words(const Pre&) { return 0u; }
-    __device__ static __forceinline__ void load(Pre& pr, const Row& r, int blk, int h) {
-        const uint8_t* b = r.p + (size_t)blk * Q6K_HTB_BYTES;
+        uint2 qh[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            const int c = 16 * chunk_pos(r.g, t);
-            pr.ql[t] = ldg128(b + 512 * h + c);
-            pr.qh[t] = __ldg(reinterpret_cast<const uint2*>(b + 1024 + c + 8 * h));
+            const uint32_t c = row + 16 * chunk_pos(g, t);
+            ql[t] = lds128_o<0>(c + 512 * h);
+            qh[t] = lds64_o<1024>(c + 8 * h);
         }
-        pr.sc = __ldg(reinterpret_cast<const uint2*>(b + 1536 + 16 * r.g + 8 * h));
-        pr.d = (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(b + 1664 + 2 * r.g));
-    }
-    struct Ctx {
-        uint32_t xc[2], xh[2];  // per scale byte: ceil(sc/2) + 64 and floor(sc/2) + 64
-    };
-    __device__ static __forceinline__ void begin(const Pre& pr, Ctx& c, int) {
-        const uint32_t w[2] = {pr.sc.x, pr.sc.y};
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint32_t x = w[i] ^ 0x80808080u;  // sc + 128 per byte
-            c.xh[i] = (x >> 1) & 0x7f7f7f7fu;
-            c.xc[i] = c.xh[i] + (x & 0x01010101u);
-        }
-    }
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx& c, uint32_t ta) {
-        const __half2 k16th = __float2half2_rn(0.0625f), km68 = __float2half2_rn(-68.f), km1536 = __float2half2_rn(-1536.f);
+        for (int s = 0; s < 2; ++s) {
 #pragma unroll
-        for (int cw = 0; cw < 4; ++cw) {
-            // (1024 + x) / 16 - 68 = (x - 64) / 16: the half scale over 16; c = -1536 m, so that
-            // fma(1024 + 16 q, m, c) = (q - 32) * (half scale), an integer of at most 2048: exact
-            const __half2 m1 = __hfma2(byte_magic2(c.xc[s], cw), k16th, km68);
-            const __half2 m2 = __hfma2(byte_magic2(c.xh[s], cw), k16th, km68);
-            const __half2 c1 = __hmul2(m1, km1536), c2 = __hmul2(m2, km1536);
-            const int bq = 2 * ((cw >> 1) + 2 * s);  // bit position of this quarter's pair in the qh byte
-            uint32_t o1[8], o2[8];
+            for (int c2 = 0; c2 < 2; ++c2) {
+                uint32_t lo[8], hi[8];
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const uint32_t qlw = w4(pr.ql[t], cw), qhw = (cw & 1) ? pr.qh[t].y : pr.qh[t].x;
-                const uint32_t a02 = s ? qlw : (qlw << 4), a13 = s ? (qlw >> 8) : (qlw >> 4);
-                const uint32_t b02 = qhw << (8 - bq), b13 = qhw >> bq;
-                const __half2 v02 = h2_bits(((a02 & 0x00F000F0u) | 0x64006400u) | (b02 & 0x03000300u));
-                const __half2 v13 = h2_bits(((a13 & 0x00F000F0u) | 0x64006400u) | (b13 & 0x03000300u));
-                o1[2 * t] = bits_h2(__hfma2(v02, m1, c1));
-                o1[2 * t + 1] = bits_h2(__hfma2(v13, m1, c1));
-                o2[2 * t] = bits_h2(__hfma2(v02, m2, c2));
-                o2[2 * t + 1] = bits_h2(__hfma2(v13, m2, c2));
+                for (int cx = 0; cx < 2; ++cx) {
+                    const int cw = 2 * c2 + cx, sc = (int)(int8_t)((s ? scw.y : scw.x) >> (8 * cw));
+                    // 32768 - 32 sc in both halves: the biased products are positive, nothing is borrowed
+                    const uint32_t bias = 0x80008000u - (uint32_t)(sc * 0x00200020);
+                    const int bq = 2 * ((cw >> 1) + 2 * s);  // bit position of this quarter's pair in the high-bit byte
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const uint32_t qlw = w4(ql[t], cw), qhw = (cw & 1) ? qh[t].y : qh[t].x;
+                        const uint32_t l = s ? qlw >> 4 : qlw, hb = bq < 4 ? qhw << (4 - bq) : qhw >> (bq - 4);
+                        const uint32_t q = (l & 0x0f0f0f0fu) | (hb & ~0x0f0f0f0fu);  // (two bits above the quant are foreign)
+                        const uint32_t e = (q & 0x003f003fu) * (uint32_t)sc + bias;         // bytes 0, 2: 32768 + sc (q - 32)
+                        const uint32_t o = ((q >> 8) & 0x003f003fu) * (uint32_t)sc + bias;  // bytes 1, 3
+                        lo[4 * cx + t] = __byte_perm(e, o, 0x6240);
+                        hi[4 * cx + t] = __byte_perm(e, o, 0x7351) ^ 0x80808080u;
+                    }
+                }
+                tmem_st8(ta + 16 * s + 8 * c2, lo);
+                tmem_st8(ta + 32 + 16 * s + 8 * c2, hi);
             }
-            tmem_st8(ta + 8 * cw, o1);
-            tmem_st8(ta + 32 + 8 * cw, o2);
         }
     }
-    __device__ static __forceinline__ void emit_min(const Pre&, const Ctx&, uint8_t*, int, int) {}
-    __device__ static __forceinline__ float scale_of(uint32_t hdr) { return half_bits_to_float((uint16_t)hdr); }
 };
 
 // Matrices without copies, repacked on their way (candle_moe_api.cu).  The forms that take such a layer otherwise gate with expf and
@@ -563,43 +555,14 @@ struct GemmQ6KOnTheWay : GemmQ6K {
 // Half h of a 256-block is its half-tile block h; word cw of chunk t of region s holds elements 16 cw + 4 t .. + 3.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ80 {
-    static constexpr bool EXACT_GATE = false;
-    static constexpr bool HAS_MIN = false;
-    static constexpr int A_COLS = 32, A_PARTS = 1, A_PAIRS = 4;
-    static constexpr int B_PARTS = 1;
-    static constexpr bool STAGE_W = true;
-    static constexpr bool HALF_TILES = true;  // staged as half-tile blocks, one bulk copy per 8 rows
-    static constexpr int W_ROW_BYTES = 2 * Q80_HTB_BYTES / 8;
-    static constexpr int W_STAGES_WIDE = 2;  // staged blocks beside 128-wide activation stages
-    struct Row {};
-    __device__ static __forceinline__ Row row(const uint8_t*, int, int) { return Row{}; }
-    struct Pre {
-        uint2 sc;       // 4 f16 scales
-        uint4 q[2][4];  // per slab: chunks t = 0..3
-    };
-    __device__ static __forceinline__ void load(Pre&, const Row&, int, int) {}
-    // ht_addr: the row's half-tile (both blocks) in the stage, g: its row inside
-    __device__ static __forceinline__ void load_half_tile(Pre& pr, uint32_t ht_addr, int g, int h) {
-        const uint32_t b = ht_addr + h * Q80_HTB_BYTES;
-        pr.sc = lds64_o<1024>(b + 8 * g);
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const uint32_t c = b + 16 * chunk_pos(g, t);
-            pr.q[0][t] = lds128_o<0>(c);
-            pr.q[1][t] = lds128_o<512>(c);
-        }
-    }
-    __device__ static __forceinline__ void load_staged(Pre&, uint32_t, int) {}
-    __device__ static __forceinline__ uint32_t staged_words(const Pre& pr) {
-        uint32_t v = pr.sc.x;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) v |= pr.q[0][t].x | pr.q[1][t].x;
-        return v;
-    }
-    __device__ static __forceinline__ uint32_t hdr_of(const Pre&) { return 0u; }
+    static constexpr bool EXACT_GATE = false, I8 = false, HAS_MIN = false;
+    static constexpr int A_PARTS = 1, B_PARTS = 1;
+    static constexpr bool HALF_TILES = true;
+    static constexpr int W_UNITS = 2;  // a stage is the half-tile blocks of one half
+    static constexpr int W_UNIT_BYTES = G_TILE_M / 8 * Q80_HTB_BYTES;
     struct Ctx {};
-    __device__ static __forceinline__ void begin(const Pre&, Ctx&, int) {}
-    __device__ static __forceinline__ float scale_of(uint32_t) { return 1.0f; }  // the scales are inside the operands
+    __device__ static __forceinline__ void begin(Ctx&, uint32_t, int) {}
+    __device__ static __forceinline__ float scale_of(const Ctx&) { return 1.0f; }  // the scales are inside the operands
     // 4 int8 -> 2 columns of fp16 pairs (k0, k2), (k1, k3): the byte plus 128 is dropped into the mantissa of 1024
     // (0x6400 | b + 128 = 1152 + b), 1152 comes off exactly, one multiply rounds
     __device__ static __forceinline__ void split4(uint32_t v, __half2& e, __half2& f) {
@@ -611,25 +574,27 @@ struct GemmQ80 {
         e = __hsub2(h2_bits(a), k1152);
         f = __hsub2(h2_bits(b), k1152);
     }
-    // scales of the two 32-element blocks of slab s
-    __device__ static __forceinline__ __half2 scales(const Pre& pr, int s) { return h2_bits(s ? pr.sc.y : pr.sc.x); }
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx&, uint32_t ta) {
-        const __half2 d2 = scales(pr, s);
-        uint32_t o[32];
+    __device__ static __forceinline__ void emit(const Ctx&, uint32_t row, int g, int, uint32_t, uint32_t ta) {
+        const uint2 sc = lds64_o<1024>(row + 8 * g);  // 4 f16 scales, two per slab
 #pragma unroll
-        for (int cw = 0; cw < 4; ++cw) {
-            const __half2 d = cw < 2 ? __low2half2(d2) : __high2half2(d2);
+        for (int s = 0; s < 2; ++s) {
+            const __half2 d2 = h2_bits(s ? sc.y : sc.x);
+            uint32_t o[32];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-                __half2 e, f;
-                split4(w4(pr.q[s][t], cw), e, f);
-                o[8 * cw + 2 * t] = bits_h2(__hmul2(e, d));
-                o[8 * cw + 2 * t + 1] = bits_h2(__hmul2(f, d));
+                const uint4 q = lds128_o<0>(row + 512 * s + 16 * chunk_pos(g, t));
+#pragma unroll
+                for (int cw = 0; cw < 4; ++cw) {
+                    __half2 e, f;
+                    split4(w4(q, cw), e, f);
+                    const __half2 d = cw < 2 ? __low2half2(d2) : __high2half2(d2);
+                    o[8 * cw + 2 * t] = bits_h2(__hmul2(e, d));
+                    o[8 * cw + 2 * t + 1] = bits_h2(__hmul2(f, d));
+                }
             }
+            tmem_st32(ta + 32 * s, o);
         }
-        tmem_st32(ta, o);
     }
-    __device__ static __forceinline__ void emit_min(const Pre&, const Ctx&, uint8_t*, int, int) {}
 };
 
 // ------------------------------------------------------------------------------------------------
@@ -639,48 +604,80 @@ struct GemmQ80 {
 //   weights      4096 d_w q  = A0 + A1      (the power of two keeps the residuals out of the fp16 subnormals;
 //   activations    64 d_a q  = B0 + B1       both come off again in the epilogue's scale)
 // and the tensor core accumulates A0 B0 + A1 B0 + A0 B1 in f32 (A1 B1 is below 2^-22 of a term).  Three MMAs per
-// K step; the activation operand is twice as large, so its two shared-memory stages hold half a block each (see the
-// kernel).
+// K step; the activation operand is twice as large.
 // ------------------------------------------------------------------------------------------------
 struct GemmQ80X : GemmQ80 {
-    static constexpr int A_COLS = 64, A_PARTS = 2, A_PAIRS = 2;
-    static constexpr int B_PARTS = 2;
-    static constexpr int W_STAGES_WIDE = 2;
-    __device__ static __forceinline__ float scale_of(uint32_t) { return 1.0f / 4096.0f; }
-    __device__ static __forceinline__ void emit(int s, const Pre& pr, const Ctx&, uint32_t ta) {
-        const __half2 d2 = __hmul2(scales(pr, s), __float2half2_rn(4096.f));  // exact (a power of two)
+    static constexpr int A_PARTS = 2, B_PARTS = 2;
+    __device__ static __forceinline__ float scale_of(const Ctx&) { return 1.0f / 4096.0f; }
+    __device__ static __forceinline__ void emit(const Ctx&, uint32_t row, int g, int, uint32_t, uint32_t ta) {
+        const uint2 sc = lds64_o<1024>(row + 8 * g);
+#pragma unroll 1
+        for (int s = 0; s < 2; ++s) {
+            const __half2 d2 = __hmul2(h2_bits(s ? sc.y : sc.x), __float2half2_rn(4096.f));  // exact (a power of two)
+            uint4 q[4];
 #pragma unroll
-        for (int c2 = 0; c2 < 2; ++c2) {  // one 32-element block of the slab
-            const __half2 d = c2 ? __high2half2(d2) : __low2half2(d2);
-            uint32_t p0[16], p1[16];
+            for (int t = 0; t < 4; ++t) q[t] = lds128_o<0>(row + 512 * s + 16 * chunk_pos(g, t));
 #pragma unroll
-            for (int cw = 0; cw < 2; ++cw)
+            for (int c2 = 0; c2 < 2; ++c2) {  // one 32-element block of the slab
+                const __half2 d = c2 ? __high2half2(d2) : __low2half2(d2);
+                uint32_t p0[16], p1[16];
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    __half2 e, f;
-                    split4(w4(pr.q[s][t], 2 * c2 + cw), e, f);
-                    const __half2 re = __hmul2(e, d), rf = __hmul2(f, d);
-                    p0[8 * cw + 2 * t] = bits_h2(re);
-                    p0[8 * cw + 2 * t + 1] = bits_h2(rf);
-                    p1[8 * cw + 2 * t] = bits_h2(__hfma2(e, d, __hneg2(re)));  // exact: the residual of a 19-bit product has at most 8 bits
-                    p1[8 * cw + 2 * t + 1] = bits_h2(__hfma2(f, d, __hneg2(rf)));
-                }
-            tmem_st16(ta + 16 * c2, p0);
-            tmem_st16(ta + 32 + 16 * c2, p1);
+                for (int cw = 0; cw < 2; ++cw)
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        __half2 e, f;
+                        split4(w4(q[t], 2 * c2 + cw), e, f);
+                        const __half2 re = __hmul2(e, d), rf = __hmul2(f, d);
+                        p0[8 * cw + 2 * t] = bits_h2(re);
+                        p0[8 * cw + 2 * t + 1] = bits_h2(rf);
+                        p1[8 * cw + 2 * t] = bits_h2(__hfma2(e, d, __hneg2(re)));  // exact: the residual of a 19-bit product has at most 8 bits
+                        p1[8 * cw + 2 * t + 1] = bits_h2(__hfma2(f, d, __hneg2(rf)));
+                    }
+                tmem_st16(ta + 64 * s + 16 * c2, p0);
+                tmem_st16(ta + 64 * s + 32 + 16 * c2, p1);
+            }
         }
     }
 };
 
-// one activation stage: a 256-wide block (four slabs) or the half of one with two operand parts, + the min-term box
+// How a kernel is laid out for a format and a position tile.  The rings of the kernel are short and their lengths divide the two
+// blocks that the issuing loops are unrolled over, so that every address in them is a constant: with ring positions kept in
+// registers a pair cost the MMA thread 680 clocks beside busy unpack warps, with constants 240.
 template <class F, int TN>
-__host__ __device__ constexpr int b_stage_bytes() {
-    return 4 * (TN * G_SLAB_K * 2) + (F::HAS_MIN ? TN * G_MIN_K * 4 : 0);
-}
-// raw weight blocks staged per CTA (see the kernel): what fits beside the activation stages
-template <class F, int TN>
-__host__ __device__ constexpr int w_stages() {
-    return !F::STAGE_W ? 1 : (TN <= 64 ? (F::HALF_TILES ? 4 : 6) : F::W_STAGES_WIDE);
-}
+struct GemmCfg {
+    static constexpr int EPI_WARPS = TN == 32 ? 4 : 8;  // a warp drains 32 rows x CH columns
+    static constexpr int CH = TN / (EPI_WARPS / 4);
+    static constexpr int GROUPS = 2;                    // of four unpack warps: every other block (Q8_0: every other pair)
+    static constexpr int WARPS = EPI_WARPS + 4 * GROUPS + 4, THREADS = 32 * WARPS;
+    // registers per thread after the trade (setmaxnreg): their sum over the warpgroups is at most the launch allocation
+    static constexpr int REGS_LAUNCH = WARPS == 20 ? 96 : 128;
+    static constexpr bool WIDE_I8 = F::I8 && TN == 128;
+    static constexpr int REGS_EPI = TN == 32 ? 160 : (WIDE_I8 ? 152 : 136);
+    static constexpr int REGS_DQ = TN == 32 ? 128 : (WIDE_I8 ? 72 : 72), REGS_MISC = TN == 32 ? 96 : (WIDE_I8 ? 32 : 64);
+    static_assert(EPI_WARPS / 4 * REGS_EPI + GROUPS * REGS_DQ + REGS_MISC <= WARPS / 4 * REGS_LAUNCH, "more registers than the launch has");
+    static_assert(THREADS * REGS_LAUNCH <= 65536, "");
+    // pairs of weight slabs (half blocks) in flight, each with its activation stage: two blocks, one with two-part operands
+    static constexpr int RING = F::A_PARTS == 2 ? 2 : 4;
+    // int8 products have two accumulators per position; 128-wide tiles then go through a block's positions in two passes,
+    // one of which is drained during the other
+    static constexpr int PASSES = F::I8 && TN == 128 ? 2 : 1;
+    static constexpr int ACC_COLS = F::I8 ? 2 * TN / PASSES : TN;  // of one of the two accumulators
+    // tensor memory: [two accumulators | pairs of weight slabs | min operands of two blocks (in shared memory beside 128-wide tiles)]
+    static constexpr bool MIN_TM = F::HAS_MIN && TN < 128, MIN_SM = F::HAS_MIN && TN == 128;
+    static constexpr int SLAB_COLS = 32 * F::A_PARTS, PAIR_COLS = 2 * SLAB_COLS;
+    static constexpr int TM_A = 2 * ACC_COLS, TM_MIN = TM_A + RING * PAIR_COLS;
+    static_assert(TM_MIN + (MIN_TM ? 2 * G_MIN_K : 0) <= G_TMEM_COLS, "");
+    // shared memory: activation stages (half blocks: two slabs, B_PARTS times), min operands per block, weight stages
+    static constexpr int B_TILE = TN * G_SLAB_K * 2;                        // [TN x 64] fp16 or [TN x 128] int8
+    static constexpr int B_BYTES = F::I8 ? B_TILE : 2 * F::B_PARTS * B_TILE;
+    static constexpr int M_BYTES = F::HAS_MIN ? TN * G_MIN_K * 4 : 0, MA_BYTES = MIN_SM ? G_TILE_M * G_MIN_K * 4 : 0;
+    static constexpr int W_BYTES = F::W_UNIT_BYTES;
+    static constexpr int FIXED = RING * B_BYTES + 2 * (M_BYTES + MA_BYTES);
+    static constexpr int W_ROOM = 232448 - 1024 - 3072 /* barriers, offsets, weight scales */ - 4 * TN * 4 - FIXED;
+    static constexpr int W_STAGES = W_ROOM / W_BYTES < G_W_BARS ? W_ROOM / W_BYTES : G_W_BARS;
+    static_assert(W_STAGES >= 2, "");
+    static constexpr int SMEM = FIXED + W_STAGES * W_BYTES + 1024 /* alignment slack */;
+};
 
 // weight row of tile row r: gate_up tiles hold 8 rows of W1, then the same 8 rows of W3, and so on (64 rows of each)
 template <bool GATE_UP>
@@ -709,8 +706,17 @@ struct TileWalk {
         : offs(offs_), E(E_), m_tiles(m_tiles_), ksplit(ksplit_), blocks(kb / ksplit_), tile(blockIdx.x), first(0), e(0) {
         n_tiles = (offs[1] - offs[0] + TN - 1) / TN;
     }
+    // how many tiles this CTA has (before the first next())
+    __device__ __forceinline__ uint32_t tiles() const {
+        uint32_t all = 0;
+#pragma unroll 1
+        for (uint32_t i = 0; i < E; ++i) all += (offs[i + 1] - offs[i] + TN - 1) / TN;
+        all *= ksplit * m_tiles;
+        return all > blockIdx.x ? (all - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    }
     __device__ __forceinline__ bool next(TileCoord& tc) {
         uint32_t per_mt = n_tiles * ksplit;
+#pragma unroll 1
         while (tile - first >= per_mt * m_tiles) {
             first += per_mt * m_tiles;
             if (++e >= E) {
@@ -737,90 +743,70 @@ struct TileWalk {
 };
 
 template <class F, bool GATE_UP, int TN>
-__global__ void __launch_bounds__(G_THREADS, 1)
+__global__ void __launch_bounds__(GemmCfg<F, TN>::THREADS, 1)
 expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_bs) {
+    using C = GemmCfg<F, TN>;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_a[4], empty_a[4], full_b[G_B_STAGES], empty_b[G_B_STAGES];  // A: per pair of slabs
-    __shared__ uint64_t tmem_full[2], epi_done[2], full_w[G_W_STAGES_MAX], empty_w[G_W_STAGES_MAX];
+    // per pair: both operands there (four unpack warps and the copy), and its MMAs done
+    __shared__ uint64_t full_p[C::RING], done_p[C::RING];
+    __shared__ uint64_t acc_full[2], acc_free[2], full_w[G_W_BARS], empty_w[G_W_BARS];
     __shared__ uint32_t s_offs[CANDLE_MOE_MAX_EXPERTS + 1];
-    constexpr int CH = TN / 2;            // columns (positions) per epilogue warp: two warps share a TMEM lane quarter
-    constexpr int B_TILE = TN * G_SLAB_K * 2;  // one [TN x 64] fp16 activation slab
-    __shared__ __align__(16) float s_d8[G_EPI_WARPS][2][CH];  // per epilogue warp: activation scales of its columns
-    __shared__ float s_dw[8][G_TILE_M];  // per block (ring of 8) and tile row: the weight scale the drain multiplies by
+    constexpr int CH = C::CH;
+    __shared__ __align__(16) float s_d8[4][TN];  // activation scales of the positions, per block (ring of 4)
+    __shared__ float s_dw[4][G_TILE_M];  // per block (ring of 4) and tile row: the weight scale the drain multiplies by
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
+    constexpr int WARP_DQ0 = C::EPI_WARPS, WARP_MISC0 = WARP_DQ0 + 4 * C::GROUPS;
+    constexpr int WARP_LOAD = WARP_MISC0, WARP_D8 = WARP_MISC0 + 1, WARP_TMA = WARP_MISC0 + 2, WARP_MMA = WARP_MISC0 + 3;
     // the warp index through a shuffle: the compiler then knows that it is warp-uniform and keeps role
     // dispatch, loop counters and MMA / TMA operands in uniform registers
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     pdl_trigger();
-    pdl_wait();
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    // One activation stage holds a whole 256-wide block (four slabs, + the min-term box for Q4_K).  With two operand
-    // parts (exact Q8_0) a whole block would be twice that, so there the two stages are the two HALVES of a block
-    // -- stage pr = the slabs of pair pr: [part 0: slab 2 pr, 2 pr + 1 | part 1: slab 2 pr, 2 pr + 1] -- each
-    // refilled for the next block as soon as its own pair's MMAs are done; the same shared memory then takes
-    // 128-wide position tiles.
-    constexpr bool B_HALF = F::B_PARTS == 2;
-    constexpr int G_STAGE_BYTES = b_stage_bytes<F, TN>();
-    uint8_t* smem_min_a = smem + G_B_STAGES * G_STAGE_BYTES;  // Q4_K: 2 slots of the min operand (weights side)
-    // staged raw blocks of the tile rows: a ring of WS blocks, so that the copy of block b + WS - 1 is in flight while
-    // block b is unpacked.  (Q4_K, 128-wide position tiles: one block and requests into L2 ahead of it, with a min-term box
-    // of 32 floats per row, against three blocks beside 16 floats: 2048 rows 2470 -> 2422 us, 8 small experts at 257
-    // rows 78.0 -> 75.0, [4096, 4096] at 777 rows 53.9 -> 52.9.)
-    constexpr int WS = w_stages<F, TN>();
-    constexpr int W_STAGE_BYTES = G_TILE_M * F::W_ROW_BYTES;
-    uint8_t* smem_w = smem_min_a + (F::HAS_MIN ? 2 : 0) * G_MIN_A_BYTES;
-    for (int i = threadIdx.x; i <= P.E; i += G_THREADS) s_offs[i] = P.offsets[i];
+    uint8_t* smem_min_b = smem + C::RING * C::B_BYTES;
+    uint8_t* smem_min_a = smem_min_b + 2 * C::M_BYTES;
+    uint8_t* smem_w = smem_min_a + 2 * C::MA_BYTES;
     if (threadIdx.x == 0) {
         s_abort = 0;
-        for (int s = 0; s < 4; ++s) {
-            mbar_init(&full_a[s], G_DQ_WARPS / 2);
-            mbar_init(&empty_a[s], 1);
-        }
-        for (int s = 0; s < G_B_STAGES; ++s) {
-            mbar_init(&full_b[s], 1);
-            mbar_init(&empty_b[s], 1);
+        for (int s = 0; s < C::RING; ++s) {
+            mbar_init(&full_p[s], 4 + 1);
+            mbar_init(&done_p[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
-            mbar_init(&tmem_full[b], 1);
-            mbar_init(&epi_done[b], G_EPI_WARPS);
+            mbar_init(&acc_full[b], 2);  // the accumulator and the scales of its positions
+            mbar_init(&acc_free[b], C::EPI_WARPS / C::PASSES);
         }
-        for (int s = 0; s < G_W_STAGES_MAX; ++s) {
+        for (int s = 0; s < G_W_BARS; ++s) {
             mbar_init(&full_w[s], 1);
-            mbar_init(&empty_w[s], G_DQ_WARPS);
+            mbar_init(&empty_w[s], 4);
         }
         fence_barrier_init();
     }
-    if (warp == G_WARP_TMA) tmem_alloc(&s_tmem_base, G_TMEM_COLS);
+    if (warp == WARP_TMA) tmem_alloc(&s_tmem_base, G_TMEM_COLS);
+    pdl_wait();  // nothing above touches what the kernels before leave
+    for (int i = threadIdx.x; i <= P.E; i += C::THREADS) s_offs[i] = P.offsets[i];
     tc5_fence_before_sync();
     __syncthreads();
     tc5_fence_after_sync();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, s_tmem_base, 0);
     volatile int* abort_flag = &s_abort;
     TileWalk<TN> walk(s_offs, P.E, P.m_tiles, P.ksplit, P.kb);
-    constexpr uint32_t IDESC = umma_idesc_f16(G_TILE_M, TN), IDESC_TF32 = umma_idesc_tf32(G_TILE_M, TN);
 
-    // Register budget: launched with 96 per thread; the TMA/MMA warpgroup hands 64 per thread back to the CTA's
-    // pool and the two epilogue warpgroups take 32 more each, so the total stays what the launch allocated (a
-    // request beyond the pool would wait forever).
-    if (warp >= G_WARP_DQ0 + G_DQ_WARPS) reg_dealloc<G_REGS_MISC>();  // the whole last warpgroup (two idle warps, TMA, MMA)
-    if (warp < G_WARP_DQ0) {
-        reg_alloc<G_REGS_EPI>();
+    // Register budget: the warpgroup with the issuing warps (and the unpack warps, where they need fewer) hands registers back to
+    // the CTA's pool and the epilogue takes them, so the total stays what the launch allocated (a request beyond the pool
+    // would wait forever).
+    if (warp >= WARP_MISC0) reg_dealloc<C::REGS_MISC>();
+    else if (warp >= WARP_DQ0 && C::REGS_DQ < C::REGS_LAUNCH) reg_dealloc<C::REGS_DQ>();
+    if (warp < WARP_DQ0) {
+        if (C::REGS_EPI > C::REGS_LAUNCH) reg_alloc<C::REGS_EPI>();
         // ===================== epilogue =====================
-        const int quarter = warp & 3, colhalf = (warp - G_WARP_EPI0) >> 2, ew = warp - G_WARP_EPI0;
+        const int quarter = warp & 3, colhalf = warp >> 2;
         const int r = 32 * quarter + lane;  // tile row = TMEM lane
-        const uint32_t ta_lane = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(colhalf * CH);
+        const uint32_t ta_lane = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(C::PASSES == 2 ? colhalf * C::ACC_COLS : colhalf * CH);
         uint32_t ab = 0;
-        TileCoord tc, tcn;
-        bool have = walk.next(tc);
-        if (have) {
-            const float* dp = P.d8t + (size_t)tc.kb0 * P.P_pad + tc.p0 + colhalf * CH;
-            for (int i = lane; i < CH; i += 32) s_d8[ew][0][i] = dp[i];
-            __syncwarp();
-        }
-        while (have) {
-            const bool have_n = walk.next(tcn);
+        TileCoord tc;
+        while (walk.next(tc)) {
             // the accumulators are kept as pairs of columns: one packed fused multiply-add per pair and block
             uint64_t acc2[CH / 2];
 #pragma unroll
@@ -835,58 +821,50 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
             }
             for (int blk = tc.kb0; blk < tc.kb1;) {
               const int stop = RUNS ? min(blk + G_RUN, tc.kb1) : tc.kb1;
+#pragma unroll 1
               for (; blk < stop; ++blk, ++ab) {
-                const int buf = ab & 1;
-                // scales of the next block (maybe of the next tile): in flight while this block is drained
-                float d8_n0 = 0.f, d8_n1 = 0.f;
-                const float* dp = nullptr;
-                if (blk + 1 < tc.kb1)
-                    dp = P.d8t + (size_t)(blk + 1) * P.P_pad + tc.p0 + colhalf * CH + lane;
-                else if (have_n)
-                    dp = P.d8t + (size_t)tcn.kb0 * P.P_pad + tcn.p0 + colhalf * CH + lane;
-                const bool pre = dp != nullptr;
-                if (pre) {
-                    if (lane < CH) d8_n0 = dp[0];
-                    if (CH > 32) d8_n1 = dp[32];
-                }
-                mbar_wait(&tmem_full[buf], (ab >> 1) & 1, abort_flag);
+                const int buf = C::PASSES == 2 ? colhalf : (int)(ab & 1);
+                mbar_wait_tight(&acc_full[buf], C::PASSES == 2 ? ab & 1 : (ab >> 1) & 1, abort_flag);
                 tc5_fence_after_sync();
-                const float dw = s_dw[ab & 7][r];  // left by the unpack warps when they produced this block
+                const float dw = s_dw[ab & 3][r];  // left by the unpack warps when they produced this block
                 const uint64_t dw2 = f32x2_pack(dw, dw);
-                const uint32_t t_main = ta_lane + (uint32_t)(G_TM_MAIN + buf * TN);
-                const uint32_t d8_addr = smem_u32(&s_d8[ew][buf][0]);
-                // Four steps of 16 columns; the load of step i+1 is in flight while step i is scaled into
+                const uint32_t t_main = ta_lane + (uint32_t)(C::PASSES == 2 ? 0 : buf * C::ACC_COLS);
+                const uint32_t d8_addr = smem_u32(&s_d8[ab & 3][colhalf * CH]);
+                // Steps of 16 columns; the load of step i+1 is in flight while step i is scaled into
                 // the register accumulators: acc += (d8[col] * dw[row]) * v.
-                constexpr int NS = CH / 16;  // steps of 16 columns
-                uint32_t stg[2][16];
+                constexpr int NS = CH / 16, PL = C::ACC_COLS / 2;
+                uint32_t stg[2][16], sth[2][F::I8 ? 16 : 1];  // int8: low and high plane
                 tmem_ld16(t_main, stg[0]);
+                if constexpr (F::I8) tmem_ld16(t_main + PL, sth[0]);
                 tmem_ld_wait();
                 static_for<NS>([&](auto Cc) {
-                    constexpr int c = decltype(Cc)::value;
-                    if (c + 1 < NS) tmem_ld16(t_main + 16 * (c + 1), stg[(c + 1) & 1]);
+                    constexpr int c = decltype(Cc)::value, s = c & 1;
+                    if constexpr (c + 1 < NS) {
+                        tmem_ld16(t_main + 16 * (c + 1), stg[s ^ 1]);
+                        if constexpr (F::I8) tmem_ld16(t_main + PL + 16 * (c + 1), sth[s ^ 1]);
+                    }
+                    if constexpr (F::I8) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) stg[s][i] = __float_as_uint((float)((int)stg[s][i] + 256 * (int)sth[s][i]));
+                    }
                     static_for<4>([&](auto Qc) {
                         constexpr int q = decltype(Qc)::value;
                         const uint4 dv = lds128_o<64 * c + 16 * q>(d8_addr);  // base + constant: no address arithmetic
                         // per column pair: the two scale products in one packed multiply, the two accumulations in one
                         // packed fused multiply-add (each half is the IEEE fma of the scalar form)
                         acc2[8 * c + 2 * q] = f32x2_fma(f32x2_mul(dw2, f32x2_pack_bits(dv.x, dv.y)),
-                                                        f32x2_pack_bits(stg[c & 1][4 * q], stg[c & 1][4 * q + 1]), acc2[8 * c + 2 * q]);
+                                                        f32x2_pack_bits(stg[s][4 * q], stg[s][4 * q + 1]), acc2[8 * c + 2 * q]);
                         acc2[8 * c + 2 * q + 1] = f32x2_fma(f32x2_mul(dw2, f32x2_pack_bits(dv.z, dv.w)),
-                                                            f32x2_pack_bits(stg[c & 1][4 * q + 2], stg[c & 1][4 * q + 3]),
+                                                            f32x2_pack_bits(stg[s][4 * q + 2], stg[s][4 * q + 3]),
                                                             acc2[8 * c + 2 * q + 1]);
                     });
                     if (c + 1 < NS) tmem_ld_wait();
-                    if (c == (NS >= 2 ? NS - 2 : 0)) {  // every column of this thread has been read: the buffer may be overwritten
+                    if (c == NS - 2) {  // every column of this thread has been read: the accumulator may be overwritten
                         tc5_fence_before_sync();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&epi_done[buf]);
+                        if (lane == 0) mbar_arrive(&acc_free[buf]);
                     }
                 });
-                if (pre) {
-                    if (lane < CH) s_d8[ew][buf ^ 1][lane] = d8_n0;
-                    if (CH > 32) s_d8[ew][buf ^ 1][lane + 32] = d8_n1;
-                }
-                __syncwarp();
               }
               if (RUNS && blk < tc.kb1) {
 #pragma unroll
@@ -919,133 +897,106 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                 for (int c = 0; c < CH; ++c)
                     if (pc0 + c < tc.p_end) out_k[(size_t)(pc0 + c) * P.N + n] = acc[c];
             }
-            tc = tcn;
-            have = have_n;
         }
-    } else if (warp < G_WARP_DQ0 + G_DQ_WARPS) {
-        // ===================== weight unpack -> fp16 operand in tensor memory =====================
-        const int quarter = warp & 3, h = (warp - G_WARP_DQ0) >> 2;
+    } else if (warp < WARP_MISC0) {
+        // ===================== weight unpack -> operand in tensor memory =====================
+        // A group takes every other block, a thread a whole row of it (Q8_0, whose halves stand on their own: every other
+        // half), so that a header is decoded once, and the waits, the shared-memory reads and the hand-over of one block lie
+        // behind the arithmetic of the other.  The loops stay rolled: the warps of a scheduler share its instruction cache
+        // with the issuing warps, whose few instructions everything waits for.
+        const int quarter = warp & 3, group = (warp - WARP_DQ0) >> 2;
         const int r = 32 * quarter + lane;
-        const uint32_t ta_lane = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)G_TM_A;
-        const uint32_t min_row_off = (uint32_t)(r * G_MIN_K * 4);
-        uint32_t ab = 0;
-        TileCoord tc, tcn;
-        bool have = walk.next(tc);
-        typename F::Row rowc{}, rown{};
-        typename F::Pre cur, nxt;
+        const uint32_t ta_lane = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)C::TM_A;
         // where tile row r lies in a stage: rows (gate_up: the W1 rows first, then the W3 rows) or half-tiles in tile order
         const uint32_t w_row = smem_u32(smem_w) +
-                               (F::HALF_TILES ? (uint32_t)((r >> 3) * 8 * F::W_ROW_BYTES)
-                                : GATE_UP ? (uint32_t)((((r >> 3) & 1) * (G_TILE_M / 2) + (r >> 4) * 8 + (r & 7)) * F::W_ROW_BYTES)
-                                          : (uint32_t)(r * F::W_ROW_BYTES));
-        const bool is_w3 = GATE_UP && ((r >> 3) & 1);
-        if (have && !F::STAGE_W) {
-            rowc = F::row(is_w3 ? P.wb.p[tc.e] : P.wa.p[tc.e], weight_row<GATE_UP>(tc.mt, r), P.kb);
-            F::load(cur, rowc, tc.kb0, h);
-            nxt = cur;
-        }
-        while (have) {
-            const bool have_n = walk.next(tcn);
-            if (have_n && !F::STAGE_W)
-                rown = F::row(is_w3 ? P.wb.p[tcn.e] : P.wa.p[tcn.e], weight_row<GATE_UP>(tcn.mt, r), P.kb);
-            for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
-                if (F::STAGE_W) {
-                    // this block's raw bytes were copied to shared memory by the loader warp
-                    mbar_wait(&full_w[ab % WS], (ab / WS) & 1, abort_flag);
-                    if constexpr (F::HALF_TILES)
-                        F::load_half_tile(cur, w_row + (ab % WS) * W_STAGE_BYTES, r & 7, h);
-                    else
-                        F::load_staged(cur, w_row + (ab % WS) * W_STAGE_BYTES, h);
-                } else if (blk + 1 < tc.kb1) {
-                    F::load(nxt, rowc, blk + 1, h);
-                } else if (have_n) {
-                    F::load(nxt, rown, tcn.kb0, h);
-                }
-                typename F::Ctx ctx;
-                F::begin(cur, ctx, h);
-                if (h == 0) s_dw[ab & 7][r] = F::scale_of(F::hdr_of(cur));  // read by the epilogue when it drains this block
-                // Handing the stage back to the loader as soon as the staged words have ARRIVED in registers.  The loads are
-                // plain shared-memory loads, their results are not needed until the emits below, and an arrive that
-                // merely follows them in program order was observed to overtake them -- the refill then landed under
-                // loads still waiting behind the (long) wait for a free operand slot, and the first rows of a tile came
-                // out with the next block's weights, rarely and only when the MMAs are the bottleneck.  So the barrier's
-                // ADDRESS is made to depend on one word of every load of every lane (OR-reduced over the warp, masked
-                // with a kernel parameter that is zero at run time): the arrive cannot be issued before those words
-                // exist.  (Released after the emits instead, a ring of two stages gave a copy less than the time of one
-                // block's emits: all-Q8_0 layer of 60 experts, 4096 rows, gate_up 562 -> 531 us, shared down 136 -> 125 us.)
-                // A ring of three or four stages (narrow position tiles) has that time, and there the reduction costs more than it
-                // gives: released after the emits (nothing reads the stage later than that, whatever the order of the
-                // instructions), gate_up of the Mixtral-shaped layer at 100 rows takes 201 us, released here 212.
-                if (F::STAGE_W && WS <= 2) {
-                    const uint32_t dep = __reduce_or_sync(0xffffffffu, F::staged_words(cur)) & P.zero;
-                    if (lane == 0) mbar_arrive(&empty_w[ab % WS + dep]);
-                }
-                // The pair goes to tensor memory; the ring holds A_PAIRS pairs (Q4_K: two blocks).  The barriers
-                // go by (block parity, pair) -- each has ONE waiting MMA warp that sees every phase, so a parity
-                // wait is never ambiguous -- while the TMEM slot is the pair index modulo the ring size: before
-                // writing it, wait for the MMAs of the block that used it last.
-                const uint32_t bidx = 2 * (ab & 1) + h, slot = bidx % F::A_PAIRS;
-                if (ab >= F::A_PAIRS / 2) {
-                    const uint32_t abp = ab - F::A_PAIRS / 2;
-                    mbar_wait_relaxed(&empty_a[2 * (abp & 1) + h], (abp >> 1) & 1, abort_flag);
-                }
+                               (F::HALF_TILES ? (uint32_t)((r >> 3) * (F::W_UNIT_BYTES * 8 / G_TILE_M))
+                                : GATE_UP ? (uint32_t)((((r >> 3) & 1) * (G_TILE_M / 2) + (r >> 4) * 8 + (r & 7)) * (F::W_UNIT_BYTES / G_TILE_M))
+                                          : (uint32_t)(r * (F::W_UNIT_BYTES / G_TILE_M)));
+        const int g = r & 7;
+        const uint32_t n_units = walk.tiles() * walk.blocks * F::W_UNITS;  // weight stages of this CTA: blocks or halves
+        uint32_t ws = group;
+#pragma unroll 1
+        for (uint32_t u = group, n = 0; u < n_units; u += 2, ++n) {
+            uint64_t* const bar_w = &empty_w[u % G_W_BARS];
+            const uint32_t row = w_row + ws * C::W_BYTES;
+            // the raw bytes were copied to shared memory by the loader warp
+            mbar_wait_tight(&full_w[u % G_W_BARS], (u / G_W_BARS) & 1, abort_flag);
+            typename F::Ctx ctx;
+            F::begin(ctx, row, g);
+            constexpr int H = 3 - F::W_UNITS;  // pairs of a unit
+            // a ring slot is taken again by the same group: pass counts its uses so far
+            const uint32_t first = H == 2 ? 2 * group : (C::RING == 4 ? u & 3 : u & 1);
+            const uint32_t pass = H == 1 && C::RING == 4 ? n >> 1 : n;
+#pragma unroll 1
+            for (int h = 0; h < H; ++h) {
+                const uint32_t slot = first + h;
+                if (pass > 0) mbar_wait_tight(&done_p[slot], (pass - 1) & 1, abort_flag);  // the MMAs that read it last
                 tc5_fence_after_sync();
-                F::emit(0, cur, ctx, ta_lane + (uint32_t)(2 * slot * F::A_COLS));
-                F::emit(1, cur, ctx, ta_lane + (uint32_t)((2 * slot + 1) * F::A_COLS));
-                if (F::HAS_MIN) {
-                    // weight side of the min term.  Its slot was last read by the min MMAs of block ab - 2, issued
-                    // before the commit of that block's second pair.
-                    if (h == 0 && ab >= 2) mbar_wait_relaxed(&empty_a[2 * (ab & 1) + 1], ((ab - 2) >> 1) & 1, abort_flag);
-                    F::emit_min(cur, ctx, smem_min_a + (size_t)(ab & 1) * G_MIN_A_BYTES + min_row_off, h, (r >> 1) & 3);
-                    fence_proxy_async_smem();
+                if (H == 2 ? h == 0 : group == 0) s_dw[(H == 2 ? u : u >> 1) & 3][r] = F::scale_of(ctx);  // for the drain of this block
+                F::emit(ctx, row, g, h, P.magic, ta_lane + slot * C::PAIR_COLS);
+                if constexpr (F::HAS_MIN) {
+                    if (h == 1) {
+                        // (the last min MMAs on these operands came before the commit just waited for)
+                        uint32_t rho[16];
+                        F::min_operand(ctx, rho);
+                        if constexpr (C::MIN_TM) {
+                            tmem_st16(tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(C::TM_MIN + group * G_MIN_K), rho);
+                        } else {
+                            uint8_t* const a = smem_min_a + group * C::MA_BYTES + r * (G_MIN_K * 4);
+                            const int sw = (r >> 1) & 3;  // 64-byte swizzle
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                *reinterpret_cast<uint4*>(a + ((j ^ sw) << 4)) = make_uint4(rho[4 * j], rho[4 * j + 1], rho[4 * j + 2], rho[4 * j + 3]);
+                            fence_proxy_async_smem();
+                        }
+                    }
                 }
                 tmem_st_wait();
                 tc5_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(&full_a[bidx]);
-                    if (F::STAGE_W && WS > 2) mbar_arrive(&empty_w[ab % WS]);
+                    mbar_arrive(&full_p[slot]);
+                    if (h == H - 1) mbar_arrive(bar_w);  // every byte of the stage has been used
                 }
-                if (!F::STAGE_W) cur = nxt;
             }
-            tc = tcn;
-            rowc = rown;
-            have = have_n;
+            ws += 2;
+            if (ws >= C::W_STAGES) ws -= C::W_STAGES;
         }
-    } else if (warp == G_WARP_LOAD) {
+    } else if (warp == WARP_LOAD) {
         // ===================== weight loader: raw blocks of the tile rows -> shared memory =====================
-        // One TMA box per matrix and block: [64 or 128 rows x 144 bytes] of the byte matrix [n_rows, row_bytes]
-        // (gate_up: the W1 rows, then the W3 rows; a TMA destination must be 128-byte aligned, so the halves cannot
-        // be skewed against each other and neighbouring lanes, which alternate between them, share banks two by
-        // two).
+        uint32_t unit = 0, ws = 0;
+        bool ok = true;
+        TileCoord tc;
         if constexpr (F::HALF_TILES) {
             // half-tile blocks of the repacked layout: one bulk copy per 8 tile rows, lane i < 16 copies half-tile i
             // (gate_up: W1 and W3 half-tiles alternate).  No requests into L2 ahead: the CTAs of a weight tile's position tiles
             // run together and share the lines, and sixteen more instructions per block held the copies up (all-Q8_0 layer of
             // 60 experts, 4096 rows, down 236 -> 218 us, shared down 127 -> 106 us without them).
-            uint32_t ab = 0;
-            TileCoord tc;
-            constexpr int HT_BYTES = 8 * F::W_ROW_BYTES;  // a half-tile over one 256-block
+            constexpr int HT_BYTES = F::W_UNIT_BYTES * 8 / G_TILE_M;
             const bool active = lane < G_TILE_M / 8, is_w3 = GATE_UP && (lane & 1);
-            while (walk.next(tc)) {
+            while (ok && walk.next(tc)) {
                 const int ht = GATE_UP ? tc.mt * 8 + (lane >> 1) : tc.mt * 16 + lane;
-                const uint8_t* src = active ? (is_w3 ? P.wb.p[tc.e] : P.wa.p[tc.e]) + (size_t)ht * P.kb * HT_BYTES : nullptr;
-                for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
-                    const uint32_t ws = ab % WS;
-                    if (ab >= (uint32_t)WS) mbar_wait(&empty_w[ws], ((ab / WS) - 1) & 1, abort_flag);
-                    if (lane == 0) mbar_expect_tx(&full_w[ws], G_TILE_M * F::W_ROW_BYTES);
+                const uint8_t* src = active ? (is_w3 ? P.wb.p[tc.e] : P.wa.p[tc.e]) + (size_t)ht * P.kb * F::W_UNITS * HT_BYTES : nullptr;
+#pragma unroll 1
+                for (int u = tc.kb0 * F::W_UNITS; u < tc.kb1 * F::W_UNITS; ++u, ++unit) {
+                    const uint32_t last = unit - C::W_STAGES;
+                    uint64_t* const bar = &full_w[unit % G_W_BARS];
+                    if (unit >= (uint32_t)C::W_STAGES) ok = mbar_wait_tight(&empty_w[last % G_W_BARS], (last / G_W_BARS) & 1, abort_flag);
+                    if (!(ok = __all_sync(0xffffffffu, ok))) break;  // nothing is issued after a wait that gave up
+                    if (lane == 0) mbar_expect_tx(bar, F::W_UNIT_BYTES);
                     __syncwarp();
-                    if (active && !*abort_flag)
-                        bulk_g2s(smem_w + ws * W_STAGE_BYTES + lane * HT_BYTES, src + (size_t)blk * HT_BYTES, HT_BYTES, &full_w[ws]);
-                    __syncwarp();
+                    if (active) bulk_g2s(smem_w + ws * C::W_BYTES + lane * HT_BYTES, src + (size_t)u * HT_BYTES, HT_BYTES, bar);
+                    if (++ws == C::W_STAGES) ws = 0;
                 }
             }
-        } else if constexpr (F::STAGE_W) {
-            uint32_t ab = 0;
+        } else {
+            // One TMA box per matrix and block: [64 rows x 144 bytes] of the byte matrix [n_rows, row_bytes]
+            // (gate_up: the W1 rows, then the W3 rows; a TMA destination must be 128-byte aligned, so the halves cannot
+            // be skewed against each other and neighbouring lanes, which alternate between them, share banks two by
+            // two).
             int fenced = -1;
-            TileCoord tc;
-            constexpr int HALF = G_TILE_M / 2 * F::W_ROW_BYTES;  // 9216
-            while (walk.next(tc)) {
+            constexpr int ROW_BYTES = F::W_UNIT_BYTES / G_TILE_M, HALF = F::W_UNIT_BYTES / 2;
+            while (ok && walk.next(tc)) {
                 const CUtensorMap* m0 = P.wmaps + 2 * tc.e;
                 // the maps were written by a kernel earlier on the stream: fence an expert's once, before their first use by this
                 // warp (every lane fences: any may be elected)
@@ -1055,135 +1006,226 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                     if (GATE_UP) tensormap_fence_acquire(m0 + 1);
                 }
                 const int y0 = GATE_UP ? tc.mt * 64 : tc.mt * 128;
-                for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
-                    const uint32_t ws = ab % WS;
-                    if (ab >= (uint32_t)WS) mbar_wait(&empty_w[ws], ((ab / WS) - 1) & 1, abort_flag);
+#pragma unroll 1
+                for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++unit) {
+                    const uint32_t last = unit - C::W_STAGES;
+                    uint64_t* const bar = &full_w[unit % G_W_BARS];
+                    if (unit >= (uint32_t)C::W_STAGES) ok = mbar_wait_tight(&empty_w[last % G_W_BARS], (last / G_W_BARS) & 1, abort_flag);
+                    if (!(ok = __all_sync(0xffffffffu, ok))) break;
                     if (elect_one()) {
-                        uint8_t* dst = smem_w + ws * W_STAGE_BYTES;
-                        mbar_expect_tx(&full_w[ws], G_TILE_M * F::W_ROW_BYTES);
-                        if (GATE_UP) {
-                            tma_load_2d(dst, m0, blk * F::W_ROW_BYTES, y0, &full_w[ws]);
-                            tma_load_2d(dst + HALF, m0 + 1, blk * F::W_ROW_BYTES, y0, &full_w[ws]);
+                        uint8_t* dst = smem_w + ws * C::W_BYTES;
+                        mbar_expect_tx(bar, F::W_UNIT_BYTES);
+                        tma_load_2d(dst, m0, blk * ROW_BYTES, y0, bar);
+                        if (GATE_UP)
+                            tma_load_2d(dst + HALF, m0 + 1, blk * ROW_BYTES, y0, bar);
+                        else
+                            tma_load_2d(dst + HALF, m0, blk * ROW_BYTES, y0 + 64, bar);
+                    }
+                    __syncwarp();
+                    if (++ws == C::W_STAGES) ws = 0;
+                }
+            }
+        }
+    } else if (warp == WARP_D8) {
+        // ===================== activation scales of the drain =====================
+        // From global memory two blocks ahead, to shared memory when the accumulator they go with has been drained of what it
+        // held before: the epilogue then waits for one barrier per block.  (Loaded by the epilogue itself, a block's scales held
+        // it for the latency of L2; requested there by asynchronous copies, for the instructions that this took, 300 clocks of
+        // 1700 beside busy unpack warps.)
+        constexpr int NR = TN / C::PASSES >= 64 ? (TN / C::PASSES) / 32 : 1;  // values per lane and pass
+        TileCoord tc;
+        int blk = 0, end = 0;
+        bool more = true;
+        const auto fetch = [&](float (&v)[NR * C::PASSES]) {  // the next block's scales
+            if (blk == end) {
+                more = more && walk.next(tc);
+                blk = tc.kb0;
+                end = tc.kb1;
+            }
+            if (more) {
+                const float* dp = P.d8t + (size_t)blk * P.P_pad + tc.p0 + lane;
+#pragma unroll
+                for (int i = 0; i < NR * C::PASSES; ++i) v[i] = dp[32 * i];
+                ++blk;
+            }
+            return more;
+        };
+        float v0[NR * C::PASSES], v1[NR * C::PASSES];
+        bool have = fetch(v0), have_n = have && fetch(v1), ok = true;
+        for (uint32_t ab = 0; have && ok; ++ab) {
+#pragma unroll
+            for (int ps = 0; ps < C::PASSES; ++ps) {
+                const int buf = C::PASSES == 2 ? ps : (int)(ab & 1);
+                if (ab >= 2 / C::PASSES) ok = mbar_wait_tight(&acc_free[buf], C::PASSES == 2 ? (ab & 1) ^ 1 : ((ab >> 1) & 1) ^ 1, abort_flag);
+#pragma unroll
+                for (int i = 0; i < NR; ++i) s_d8[ab & 3][32 * (NR * ps + i) + lane] = v0[NR * ps + i];
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_full[buf]);
+            }
+            have = have_n;
+#pragma unroll
+            for (int i = 0; i < NR * C::PASSES; ++i) v0[i] = v1[i];
+            have_n = have && fetch(v1);
+        }
+    } else if (warp == WARP_TMA) {
+        // ===================== TMA: activation operand =====================
+        // One stage = the slabs of one pair: [part 0: two slabs | part 1: two slabs], int8: the 128 bytes of the half in one box;
+        // a row of two-part operands holds [256 of part 0 | 256 of part 1] per block.  The min operand of a block comes with its
+        // second pair.  Unrolled over two blocks, like the MMA loop.
+        if (elect_one()) {
+            TileCoord tc;
+            uint32_t it = 0;
+            bool second = false;
+            const auto load_block = [&](auto Bc, int blk) {
+                constexpr int B = decltype(Bc)::value, R = C::RING;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int st = (2 * B + h) % R;
+                    // use it (ring of two blocks) or 2 it + B (of one) of this stage
+                    if (R == 4 ? it > 0 : it > 0 || B > 0)
+                        if (!mbar_wait_tight(&done_p[st], R == 4 ? (it & 1) ^ 1 : (B & 1) ^ 1, abort_flag)) return false;
+                    uint8_t* dst = smem + st * C::B_BYTES;
+                    mbar_expect_tx(&full_p[st], C::B_BYTES + (h == 1 ? C::M_BYTES : 0));
+                    if constexpr (F::I8) {
+                        tma_load_2d(dst, &map_b, blk * 256 + h * 128, (int)tc.p0, &full_p[st]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 2 * F::B_PARTS; ++j)
+                            tma_load_2d(dst + j * C::B_TILE, &map_b, blk * 256 * F::B_PARTS + (j >> 1) * 256 + (2 * h + (j & 1)) * 64,
+                                        (int)tc.p0, &full_p[st]);
+                    }
+                    if (F::HAS_MIN && h == 1) tma_load_2d(smem_min_b + B * C::M_BYTES, &map_bs, blk * G_MIN_K, (int)tc.p0, &full_p[st]);
+                }
+                return true;
+            };
+            while (walk.next(tc)) {
+                int blk = tc.kb0;
+                if (second) goto tma_second;
+#pragma unroll 1
+                for (;;) {
+                    second = true;
+                    if (!load_block(std::integral_constant<int, 0>{}, blk)) goto tma_done;
+                    if (++blk == tc.kb1) break;
+                tma_second:
+                    second = false;
+                    if (!load_block(std::integral_constant<int, 1>{}, blk)) goto tma_done;
+                    ++it;
+                    if (++blk == tc.kb1) break;
+                }
+            }
+        tma_done:;
+        }
+        __syncwarp();
+    } else if (warp == WARP_MMA) {
+        // ===================== MMA issue =====================
+        // Everything else of the kernel waits for this loop, and beside busy warps each instruction in it counts at its full
+        // latency and its place in the instruction cache: one barrier to wait for per pair, constant addresses (see GemmCfg); the
+        // whole warp walks it, so that operands stay in uniform registers, and one elected lane issues.
+        TileCoord tc;
+        uint32_t it = 0, n_eff = 0, idesc[2] = {0, 0}, idesc_min = 0;
+        bool second = false;
+        const uint64_t b_desc = umma_desc_sw128(smem_u32(smem));
+        const uint64_t mb_desc = umma_desc_sw64(smem_u32(smem_min_b)), ma_desc = umma_desc_sw64(smem_u32(smem_min_a));
+        const auto block = [&](auto Bc) {  // block 2 it + B of this CTA
+            constexpr int B = decltype(Bc)::value, R = C::RING;
+#pragma unroll
+            for (int ps = 0; ps < C::PASSES; ++ps) {
+                const int buf = C::PASSES == 2 ? ps : B;
+                // the drain of what this accumulator held last: block ab - 2, with two passes ab - 1
+                if (C::PASSES == 2 ? it > 0 || B > 0 : it > 0)
+                    mbar_wait_tight(&acc_free[buf], C::PASSES == 2 ? (B & 1) ^ 1 : (it & 1) ^ 1, abort_flag);
+                const uint32_t d_main = tmem_base + buf * C::ACC_COLS;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int st = (2 * B + h) % R;
+                    if (ps == 0) mbar_wait_tight(&full_p[st], R == 4 ? it & 1 : B & 1, abort_flag);
+                    tc5_fence_after_sync();
+                    if (elect_one()) {
+                        const uint32_t a_t = tmem_base + C::TM_A + st * C::PAIR_COLS;
+                        const uint64_t db = umma_desc_add(b_desc, st * (C::B_BYTES >> 4));
+                        if constexpr (F::I8) {
+                            uint32_t id0 = idesc[0], id1 = idesc[1];
+                            if (ps == 1) {  // positions 64 .. 127
+                                const uint32_t n = n_eff > 64 ? n_eff - 64 : 0;
+                                id0 = umma_idesc_i8(G_TILE_M, 0, false) | ((n >> 3) << 17);
+                                id1 = umma_idesc_i8(G_TILE_M, 0, true) | ((n >> 3) << 17);
+                            }
+                            if (ps == 0 || n_eff > 64) {
+                                const uint64_t dp = umma_desc_add(db, ps * (64 * 128 >> 4));
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {  // K steps of 32: 8 columns of A, 32 bytes of B
+                                    umma_i8_ts(d_main, a_t + 8 * k, umma_desc_add(dp, 2 * k), id0, (h | k) != 0);
+                                    umma_i8_ts(d_main + C::ACC_COLS / 2, a_t + 32 + 8 * k, umma_desc_add(dp, 2 * k), id1, (h | k) != 0);
+                                }
+                            }
                         } else {
-                            tma_load_2d(dst, m0, blk * F::W_ROW_BYTES, y0, &full_w[ws]);
-                            tma_load_2d(dst + HALF, m0, blk * F::W_ROW_BYTES, y0 + 64, &full_w[ws]);
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {  // two slabs of four K steps
+                                const uint32_t a_k = a_t + (k >> 2) * C::SLAB_COLS + 8 * (k & 3);
+                                const uint64_t b_k = umma_desc_add(db, (k >> 2) * (C::B_TILE >> 4) + 2 * (k & 3));
+                                umma_f16_ts(d_main, a_k, b_k, idesc[0], (h | k) != 0);
+                                if (F::A_PARTS == 2) umma_f16_ts(d_main, a_k + 32, b_k, idesc[0], true);
+                                if (F::B_PARTS == 2) umma_f16_ts(d_main, a_k, umma_desc_add(b_k, 2 * (C::B_TILE >> 4)), idesc[0], true);
+                            }
                         }
+                        if (F::HAS_MIN && h == 1) {
+                            // the min term joins the same accumulator: three tf32 steps r1 b1 + r2 b1 + r1 b2, last in the block
+                            const uint64_t dm = umma_desc_add(mb_desc, B * (C::M_BYTES >> 4));
+                            if constexpr (C::MIN_TM) {
+                                const uint32_t da = tmem_base + C::TM_MIN + B * G_MIN_K;
+                                umma_tf32_ts(d_main, da, dm, idesc_min, true);
+                                umma_tf32_ts(d_main, da + 8, dm, idesc_min, true);
+                                umma_tf32_ts(d_main, da, umma_desc_add(dm, 2), idesc_min, true);
+                            } else {
+                                const uint64_t da = umma_desc_add(ma_desc, B * (C::MA_BYTES >> 4));
+                                umma_tf32(d_main, da, dm, idesc_min, true);
+                                umma_tf32(d_main, umma_desc_add(da, 2), dm, idesc_min, true);
+                                umma_tf32(d_main, da, umma_desc_add(dm, 2), idesc_min, true);
+                            }
+                        }
+                        // the pair's operands may be overwritten once these MMAs have read them
+                        if (ps == C::PASSES - 1) umma_commit(&done_p[st]);
+                        if (h == 1) umma_commit(&acc_full[buf]);
                     }
                     __syncwarp();
                 }
             }
-        }
-    } else if (warp == G_WARP_TMA) {
-        // ===================== TMA: activation operand =====================
-        // the whole warp walks the loop (uniform control flow and addresses), one elected lane issues
-        uint32_t ab = 0;
-        TileCoord tc;
-        while (walk.next(tc)) {
-            for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
-                if constexpr (B_HALF) {
-                    // stage pr of every block: free once the MMAs of pair pr of the block before are done
-#pragma unroll
-                    for (int pr = 0; pr < 2; ++pr) {
-                        if (ab >= 1) mbar_wait_relaxed(&empty_b[pr], (ab - 1) & 1, abort_flag);
-                        uint8_t* dst = smem + (size_t)pr * G_STAGE_BYTES;
-                        if (elect_one()) {
-                            mbar_expect_tx(&full_b[pr], G_STAGE_BYTES);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)  // a row holds [256 of part 0 | 256 of part 1] per block
-                                tma_load_2d(dst + j * B_TILE, &map_b, blk * 512 + (j >> 1) * 256 + (2 * pr + (j & 1)) * 64, (int)tc.p0,
-                                            &full_b[pr]);
-                        }
-                        __syncwarp();
-                    }
-                    continue;
-                }
-                // one stage = the whole 256-wide block: four slabs (+ the activation side of the min term), one barrier
-                const int st = ab & 1;
-                if (ab >= 2) mbar_wait_relaxed(&empty_b[st], ((ab >> 1) & 1) ^ 1, abort_flag);
-                uint8_t* dst = smem + (size_t)st * G_STAGE_BYTES;
-                if (elect_one()) {
-                    mbar_expect_tx(&full_b[st], G_STAGE_BYTES);
-#pragma unroll
-                    for (int s4 = 0; s4 < 4; ++s4)
-                        tma_load_2d(dst + s4 * B_TILE, &map_b, blk * 256 + s4 * 64, (int)tc.p0, &full_b[st]);
-                    if (F::HAS_MIN) tma_load_2d(dst + 4 * B_TILE, &map_bs, blk * G_MIN_K, (int)tc.p0, &full_b[st]);
-                }
-                __syncwarp();
-            }
-        }
-    } else if (warp == G_WARP_MMA) {
-        // ===================== MMA issue =====================
-        // (Splitting the blocks by parity over two issuing warps was measured: no gain.)
-        uint32_t ita = 0, ab = 0;
-        TileCoord tc;
-        const uint32_t a_base = tmem_base + (uint32_t)G_TM_A;
-        const uint64_t b_desc0 = umma_desc_sw128(smem_u32(smem));
-        const uint64_t ma_desc0 = umma_desc_sw64(smem_u32(smem_min_a)), mb_desc0 = umma_desc_sw64(smem_u32(smem) + 4 * B_TILE);
-        bool rdy_a = false, rdy_b = false;
-        while (walk.next(tc)) {
+        };
+        // (after a wait that gave up, the rest of the tile is issued all the same: the lanes stay together)
+        while (!__any_sync(0xffffffffu, *abort_flag) && walk.next(tc)) {
+            uint32_t left = walk.blocks;
             // The last position tile of an expert is rarely full: its MMAs run N = the rows it holds, rounded up to 16
             // (an MMA's time goes with N; the columns beyond are neither computed nor stored).
-            const uint32_t n_eff = min((uint32_t)TN, (tc.p_end - tc.p0 + 15u) & ~15u);
-            const uint32_t idesc = (IDESC & ~(0x3Fu << 17)) | ((n_eff >> 3) << 17);
-            const uint32_t idesc_tf32 = (IDESC_TF32 & ~(0x3Fu << 17)) | ((n_eff >> 3) << 17);
-            for (int blk = tc.kb0; blk < tc.kb1; ++blk, ++ab) {
-                const int buf = ab & 1;  // main accumulator and B stage of this block
-                // the drain of block ab - 2 has released this main accumulator
-                if (ab >= 2) mbar_wait(&epi_done[buf], ((ab >> 1) & 1) ^ 1, abort_flag);
-                const uint32_t d_main = tmem_base + (uint32_t)(G_TM_MAIN + buf * TN);
-                const uint64_t db = b_desc0 + (uint64_t)((B_HALF ? 0 : buf) * (G_STAGE_BYTES >> 4));
-#pragma unroll
-                for (int pr = 0; pr < 2; ++pr, ita += 2) {
-                    const uint32_t bidx = 2 * (ab & 1) + pr, slot = bidx % F::A_PAIRS;  // barrier, TMEM slot (see the unpack warps)
-                    if (!rdy_a) mbar_wait(&full_a[bidx], (ab >> 1) & 1, abort_flag);
-                    if constexpr (B_HALF) {
-                        mbar_wait(&full_b[pr], ab & 1, abort_flag);
-                    } else {
-                        if (pr == 0 && !rdy_b) mbar_wait(&full_b[buf], (ab >> 1) & 1, abort_flag);
-                    }
-                    tc5_fence_after_sync();
-                    // look at this warp's next barriers now: the answers arrive while the MMAs are issued
-                    rdy_a = pr == 0 ? mbar_test(&full_a[bidx + 1], (ab >> 1) & 1)                    // second pair of this block
-                                    : mbar_test(&full_a[2 * ((ab + 1) & 1)], ((ab + 1) >> 1) & 1);  // first pair of the next
-                    if (!B_HALF && pr == 1) rdy_b = mbar_test(&full_b[buf ^ 1], ((ab + 1) >> 1) & 1);
-                    const uint32_t a_t = a_base + (uint32_t)(2 * slot * F::A_COLS);
-                    if (elect_one()) {
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {  // two slabs of four K steps
-                            const uint32_t a_k = a_t + (uint32_t)((k >> 2) * F::A_COLS + 8 * (k & 3));
-                            // slab of this K step inside its stage: whole-block stages hold slabs 0..3, half-block
-                            // stages [part 0: two slabs | part 1: two slabs] of pair pr
-                            const uint64_t b_k = db + (uint64_t)((B_HALF ? pr * 4 + (k >> 2) : 2 * pr + (k >> 2)) * (B_TILE >> 4) + 2 * (k & 3));
-                            umma_f16_ts(d_main, a_k, b_k, idesc, (pr | k) != 0);
-                            if (F::A_PARTS == 2) umma_f16_ts(d_main, a_k + 32, b_k, idesc, true);
-                            if (F::B_PARTS == 2) umma_f16_ts(d_main, a_k, b_k + (uint64_t)(2 * (B_TILE >> 4)), idesc, true);
-                        }
-                        if (pr == 1 && F::HAS_MIN) {
-                            // the min term joins the same accumulator: three tf32 steps, last in the block
-                            const uint64_t da = ma_desc0 + (uint64_t)(buf * (G_MIN_A_BYTES >> 4)), dm = mb_desc0 + (uint64_t)(buf * (G_STAGE_BYTES >> 4));
-                            umma_tf32(d_main, da, dm, idesc_tf32, true);      // r1 b1
-                            umma_tf32(d_main, da + 2, dm, idesc_tf32, true);  // r2 b1
-                            umma_tf32(d_main, da, dm + 2, idesc_tf32, true);  // r1 b2
-                        }
-                        umma_commit(&empty_a[bidx]);  // the stages may be refilled once these MMAs have read them
-                        if (B_HALF) umma_commit(&empty_b[pr]);
-                        if (pr == 1) {
-                            if (!B_HALF) umma_commit(&empty_b[buf]);
-                            umma_commit(&tmem_full[buf]);
-                        }
-                    }
-                    __syncwarp();
-                }
+            n_eff = min((uint32_t)TN, (tc.p_end - tc.p0 + 15u) & ~15u);
+            if constexpr (F::I8) {
+                const uint32_t n = min(n_eff, (uint32_t)(TN / C::PASSES));
+                idesc[0] = umma_idesc_i8(G_TILE_M, 0, false) | ((n >> 3) << 17);  // low plane: unsigned bytes
+                idesc[1] = umma_idesc_i8(G_TILE_M, 0, true) | ((n >> 3) << 17);
+            } else {
+                idesc[0] = umma_idesc_f16(G_TILE_M, 0) | ((n_eff >> 3) << 17);
+                idesc_min = umma_idesc_tf32(G_TILE_M, 0) | ((n_eff >> 3) << 17);
+            }
+            if (second) goto mma_second;
+#pragma unroll 1
+            for (;;) {
+                second = true;
+                block(std::integral_constant<int, 0>{});
+                if (--left == 0) break;
+            mma_second:
+                second = false;
+                block(std::integral_constant<int, 1>{});
+                ++it;
+                if (--left == 0) break;
             }
         }
     }
     tc5_fence_before_sync();
     __syncthreads();
-    // After a wait that gave up, copies and MMAs of this CTA may still be under way (the issuing warps have run through their
-    // remaining blocks): give them time, some microseconds each at most, before the shared and tensor memory go
+    // After a wait that gave up, copies and MMAs of this CTA may still be under way (the issuing warps have stopped): give them
+    // time, some microseconds each at most, before the shared and tensor memory go
     if (s_abort)
         for (int i = 0; i < 5000; ++i) __nanosleep(1000);
-    if (warp == G_WARP_TMA) {
+    if (warp == WARP_TMA) {
         tc5_fence_after_sync();
         tmem_dealloc(tmem_base, G_TMEM_COLS);
     }
@@ -1236,12 +1278,11 @@ int g_gemm_sms = -1;
 
 template <class F, bool GATE_UP, int TN>
 cudaError_t launch_gemm_kernel(cudaStream_t st, const GemmParams& G, const CUtensorMap& map_b, const CUtensorMap& map_bs) {
-    const int smem_bytes = G_B_STAGES * b_stage_bytes<F, TN>() + (F::HAS_MIN ? 2 : 0) * G_MIN_A_BYTES +
-                           (F::STAGE_W ? w_stages<F, TN>() * G_TILE_M * F::W_ROW_BYTES : 0) + 1024 /* alignment slack */;
+    using C = GemmCfg<F, TN>;
     auto kfn = expert_gemm_kernel<F, GATE_UP, TN>;
-    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e != cudaSuccess) return e;
-    return launch_k(kfn, dim3(g_gemm_sms), dim3(G_THREADS), (size_t)smem_bytes, st, G, map_b, map_bs);
+    return launch_k(kfn, dim3(g_gemm_sms), dim3(C::THREADS), (size_t)C::SMEM, st, G, map_b, map_bs);
 }
 
 }  // namespace
@@ -1301,6 +1342,8 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     const int64_t p_pad = P + G_PAD_ROWS;
     uint8_t* base = static_cast<uint8_t*>(scratch);
     __half* bf16 = reinterpret_cast<__half*>(base);
+    int8_t* b8 = reinterpret_cast<int8_t*>(base);  // Q6_K: int8 operand in the same place
+    const bool i8 = dtype == CANDLE_GGML_Q6K;
     float* bmin = reinterpret_cast<float*>(base + align_up((size_t)p_pad * K * 2 * parts, 256));
     float* d8t = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bmin) + align_up((size_t)p_pad * kb * G_MIN_K * 4, 256));
     const bool has_min = dtype == CANDLE_GGML_Q4K;
@@ -1339,17 +1382,19 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     else if (x_f32)
         e = q80 ? launch_k(prep_gemm_f32_q80_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K_in, K, q80x ? 1 : 0, bf16,
                            d8t, single_group)
-                : launch_k(prep_gemm_f32_q8k_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K, bf16,
-                           has_min ? bmin : (float*)nullptr, d8t, single_group, first);
+                : launch_k(prep_gemm_f32_q8k_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K, i8 ? b8 : (int8_t*)nullptr,
+                           bf16, has_min ? bmin : (float*)nullptr, d8t, single_group, first);
     else
         e = q80 ? launch_k(prep_gemm_b_q80_kernel, prep_grid, dim3(256), 0, st, aq, ascale, row_of, (int)P, (int)p_pad, K_in, K,
                            q80x ? 1 : 0, bf16, d8t)
-                : launch_k(prep_gemm_b_kernel, prep_grid, dim3(256), 0, st, aq, ascale, absum, row_of, (int)P, (int)p_pad, K, bf16,
-                           has_min ? bmin : (float*)nullptr, d8t, first);
+            : i8 ? launch_k(prep_gemm_i8_kernel, prep_grid, dim3(256), 0, st, aq, ascale, row_of, (int)P, (int)p_pad, K, b8, d8t)
+                 : launch_k(prep_gemm_b_kernel, prep_grid, dim3(256), 0, st, aq, ascale, absum, row_of, (int)P, (int)p_pad, K, bf16, bmin, d8t,
+                            first);
     if (e != cudaSuccess) return e;
 
     CUtensorMap map_b, map_bs;
-    if (!make_map_2d(&map_b, bf16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)p_pad, (uint64_t)K * parts, G_SLAB_K, tn))
+    if (i8 ? !make_map_2d(&map_b, b8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)p_pad, (uint64_t)K, 2 * G_SLAB_K, tn)
+           : !make_map_2d(&map_b, bf16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)p_pad, (uint64_t)K * parts, G_SLAB_K, tn))
         return cudaErrorNotSupported;
     if (!make_map_2d(&map_bs, bmin, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)p_pad, (uint64_t)kb * G_MIN_K, G_MIN_K, tn, CU_TENSOR_MAP_SWIZZLE_64B))
         return cudaErrorNotSupported;
@@ -1399,8 +1444,8 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     }
     G.ksplit = ksplit;
     G.out = ksplit == 1 && out_whole ? out_whole : out;
-    G.zero = 0;
     G.split_stride = split_stride;
+    G.magic = 0x64006400u;
     e = stream_status_ptr(&G.status);
     if (e != cudaSuccess) return e;
     if (dtype == CANDLE_GGML_Q4K) {

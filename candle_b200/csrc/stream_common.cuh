@@ -60,6 +60,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     *abort_flag = 1;
     return false;
 }
+// The same in as few instructions as possible, for kernels whose warps share their instruction caches with warps that do
+// something else: the form above, written out at every wait, made the large-batch GEMM 90 KB of code.
+__device__ __forceinline__ bool mbar_wait_tight(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    int n = SPIN_LIMIT;
+#pragma unroll 1
+    while (!mbar_try_wait(bar, parity)) {
+        if (*abort_flag || --n == 0) {
+            *abort_flag = 1;
+            return false;
+        }
+    }
+    return true;
+}
 // After a wait that gave up: a copy that was issued completes this phase, whatever the abort flag says, so its CTA must not
 // leave before (bounded, as every wait: a phase whose copies were never issued runs into the limit).
 __device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity, int limit = SPIN_LIMIT) {
@@ -179,6 +192,9 @@ __device__ __forceinline__ uint64_t lds64u(uint32_t addr) {
 // 16-byte asynchronous global -> shared copy (per thread, bypassing L1) and its group fences
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
