@@ -885,17 +885,21 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                 // the lane with bit 3 clear holds w1 x, its partner w3 x of the same output row: the first finishes the
                 // first half of this warp's columns, the other the second half, one exchange per pair of columns
                 const bool up = lane & 8;
+                const uint32_t p0 = pc0 + (up ? CH / 2 : 0);
+                const int rows = (int)(tc.p_end - p0);
+                float* const out_p = out_k + (size_t)p0 * P.N + n;
 #pragma unroll
                 for (int c = 0; c < CH / 2; ++c) {
                     const float recv = __shfl_xor_sync(0xffffffffu, up ? acc[c] : acc[c + CH / 2], 8);
                     const float gv = up ? recv : acc[c], uv = up ? acc[c + CH / 2] : recv;
-                    const uint32_t p = pc0 + c + (up ? CH / 2 : 0);
-                    if (p < tc.p_end) out_k[(size_t)p * P.N + n] = (F::EXACT_GATE ? silu_f(gv) : __fdividef(gv, 1.0f + __expf(-gv))) * uv;
+                    if (c < rows) out_p[(size_t)c * P.N] = (F::EXACT_GATE ? silu_f(gv) : __fdividef(gv, 1.0f + __expf(-gv))) * uv;
                 }
             } else {
+                const int rows = (int)(tc.p_end - pc0);
+                float* const out_p = out_k + (size_t)pc0 * P.N + n;
 #pragma unroll
                 for (int c = 0; c < CH; ++c)
-                    if (pc0 + c < tc.p_end) out_k[(size_t)(pc0 + c) * P.N + n] = acc[c];
+                    if (c < rows) out_p[(size_t)c * P.N] = acc[c];
             }
         }
     } else if (warp < WARP_MISC0) {
@@ -1032,58 +1036,57 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         // held before: the epilogue then waits for one barrier per block.  (Loaded by the epilogue itself, a block's scales held
         // it for the latency of L2; requested there by asynchronous copies, for the instructions that this took, 300 clocks of
         // 1700 beside busy unpack warps.)
-        constexpr int NR = TN / C::PASSES >= 64 ? (TN / C::PASSES) / 32 : 1;  // values per lane and pass
+        constexpr int NR = TN / C::PASSES / 32;  // values per lane and pass
         TileCoord tc;
-        int blk = 0, end = 0;
-        bool more = true;
-        const auto fetch = [&](float (&v)[NR * C::PASSES]) {  // the next block's scales
-            if (blk == end) {
-                more = more && walk.next(tc);
-                blk = tc.kb0;
-                end = tc.kb1;
+        float v[NR * C::PASSES], old[NR * C::PASSES];
+        const float* dp = nullptr;
+        uint32_t left = 0;
+#pragma unroll 1
+        for (uint32_t ab = 0;; ++ab) {  // asks for the scales of block ab, hands over those of block ab - 1
+            bool more = true;
+            if (left == 0) {
+                more = walk.next(tc);
+                left = more ? walk.blocks : 0;
+                dp = P.d8t + (size_t)tc.kb0 * P.P_pad + tc.p0 + lane;
             }
             if (more) {
-                const float* dp = P.d8t + (size_t)blk * P.P_pad + tc.p0 + lane;
 #pragma unroll
                 for (int i = 0; i < NR * C::PASSES; ++i) v[i] = dp[32 * i];
-                ++blk;
+                dp += P.P_pad;
+                --left;
             }
-            return more;
-        };
-        float v0[NR * C::PASSES], v1[NR * C::PASSES];
-        bool have = fetch(v0), have_n = have && fetch(v1), ok = true;
-        for (uint32_t ab = 0; have && ok; ++ab) {
+            if (ab > 0) {
+                const uint32_t bl = ab - 1;
 #pragma unroll
-            for (int ps = 0; ps < C::PASSES; ++ps) {
-                const int buf = C::PASSES == 2 ? ps : (int)(ab & 1);
-                if (ab >= 2 / C::PASSES) ok = mbar_wait_tight(&acc_free[buf], C::PASSES == 2 ? (ab & 1) ^ 1 : ((ab >> 1) & 1) ^ 1, abort_flag);
+                for (int ps = 0; ps < C::PASSES; ++ps) {
+                    const uint32_t buf = C::PASSES == 2 ? ps : bl & 1, turn = C::PASSES == 2 ? bl : bl >> 1;  // uses of this accumulator so far
+                    if (turn > 0) mbar_wait_tight(&acc_free[buf], (turn - 1) & 1, abort_flag);
 #pragma unroll
-                for (int i = 0; i < NR; ++i) s_d8[ab & 3][32 * (NR * ps + i) + lane] = v0[NR * ps + i];
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_full[buf]);
+                    for (int i = 0; i < NR; ++i) s_d8[bl & 3][32 * (NR * ps + i) + lane] = old[NR * ps + i];
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_full[buf]);
+                }
             }
-            have = have_n;
+            if (!more) break;
 #pragma unroll
-            for (int i = 0; i < NR * C::PASSES; ++i) v0[i] = v1[i];
-            have_n = have && fetch(v1);
+            for (int i = 0; i < NR * C::PASSES; ++i) old[i] = v[i];
         }
     } else if (warp == WARP_TMA) {
         // ===================== TMA: activation operand =====================
         // One stage = the slabs of one pair: [part 0: two slabs | part 1: two slabs], int8: the 128 bytes of the half in one box;
         // a row of two-part operands holds [256 of part 0 | 256 of part 1] per block.  The min operand of a block comes with its
         // second pair.  Unrolled over two blocks, like the MMA loop.
-        if (elect_one()) {
-            TileCoord tc;
-            uint32_t it = 0;
-            bool second = false;
-            const auto load_block = [&](auto Bc, int blk) {
-                constexpr int B = decltype(Bc)::value, R = C::RING;
+        TileCoord tc;
+        uint32_t it = 0;
+        bool second = false, ok = true;
+        const auto load_block = [&](auto Bc, int blk) {
+            constexpr int B = decltype(Bc)::value, R = C::RING;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int st = (2 * B + h) % R;
-                    // use it (ring of two blocks) or 2 it + B (of one) of this stage
-                    if (R == 4 ? it > 0 : it > 0 || B > 0)
-                        if (!mbar_wait_tight(&done_p[st], R == 4 ? (it & 1) ^ 1 : (B & 1) ^ 1, abort_flag)) return false;
+            for (int h = 0; h < 2; ++h) {
+                const int st = (2 * B + h) % R;
+                // use it (ring of two blocks) or 2 it + B (of one) of this stage
+                if (R == 4 ? it > 0 : it > 0 || B > 0) ok = ok && mbar_wait_tight(&done_p[st], R == 4 ? (it & 1) ^ 1 : (B & 1) ^ 1, abort_flag);
+                if (elect_one() && ok) {  // nothing is issued after a wait that gave up
                     uint8_t* dst = smem + st * C::B_BYTES;
                     mbar_expect_tx(&full_p[st], C::B_BYTES + (h == 1 ? C::M_BYTES : 0));
                     if constexpr (F::I8) {
@@ -1096,26 +1099,24 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                     }
                     if (F::HAS_MIN && h == 1) tma_load_2d(smem_min_b + B * C::M_BYTES, &map_bs, blk * G_MIN_K, (int)tc.p0, &full_p[st]);
                 }
-                return true;
-            };
-            while (walk.next(tc)) {
-                int blk = tc.kb0;
-                if (second) goto tma_second;
-#pragma unroll 1
-                for (;;) {
-                    second = true;
-                    if (!load_block(std::integral_constant<int, 0>{}, blk)) goto tma_done;
-                    if (++blk == tc.kb1) break;
-                tma_second:
-                    second = false;
-                    if (!load_block(std::integral_constant<int, 1>{}, blk)) goto tma_done;
-                    ++it;
-                    if (++blk == tc.kb1) break;
-                }
+                __syncwarp();
             }
-        tma_done:;
+        };
+        while (walk.next(tc)) {
+            int blk = tc.kb0;
+            if (second) goto tma_second;
+#pragma unroll 1
+            for (;;) {
+                second = true;
+                load_block(std::integral_constant<int, 0>{}, blk);
+                if (++blk == tc.kb1) break;
+            tma_second:
+                second = false;
+                load_block(std::integral_constant<int, 1>{}, blk);
+                ++it;
+                if (++blk == tc.kb1) break;
+            }
         }
-        __syncwarp();
     } else if (warp == WARP_MMA) {
         // ===================== MMA issue =====================
         // Everything else of the kernel waits for this loop, and beside busy warps each instruction in it counts at its full
