@@ -53,7 +53,7 @@ constexpr int G_PAD_ROWS = 128;                // zero rows after the last posit
 constexpr int G_W_BARS = 8;
 constexpr int G_MIN_K = 16;     // min term of Q4_K: floats per row and block, two K steps of tf32 (64-byte rows, 64-byte swizzle)
 constexpr int G_TMEM_COLS = 512;
-constexpr int G_RUN = 8;  // blocks that narrow tiles add in a row
+constexpr int G_RUN = 4;  // blocks that narrow tiles add in a row
 
 // Tensor maps of the weight matrices reach device memory as kernel PARAMETERS -- of the operand preparation that runs before the
 // GEMM anyway, and of a small copy kernel for what does not fit there -- never
@@ -91,10 +91,23 @@ __global__ void __launch_bounds__(128) write_maps_kernel(const __grid_constant__
 // 16 floats [b1 (8) | b2 (8)], matched by [r1 | r2] on the weight side.  The main
 // sum stays an exact integer until these last three steps; what they add in error is of the order of the
 // reference's own f32 rounding (2^-23 of the min term).
+//
+// Position tiles of up to 64 have the tensor memory for an accumulator of its own: sum_j m_j bsum32_j is ONE fp16 step of exact
+// integers per block, [m (8) | m (8)] against [c1 (8) | c2 (8)] with bsum32 = c1 + c2, c1 a multiple of 4, and the drain adds
+// d8 * (d M - dmin Mm) like the reference.  Relative error against 64-bit arithmetic (K = 4096, 12800 rows): 1.55e-7 with the
+// joined min term, 0.87e-7 (the streaming form 1.16e-7); a layer at 100 rows is as fast.
 // ---------------------------------------------------------------------------------------------
 // nearest value with a 10-bit mantissa (the 13 low bits of the fp32 container zero)
 __device__ __forceinline__ float tf32_head(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u); }
 
+// first part of a sum of 32 activations: its ten leading bits, or (fp16 steps) its multiple of 4
+__device__ __forceinline__ float min_head(float bv, int fp16) { return fp16 ? 4.0f * rintf(0.25f * bv) : tf32_head(bv); }
+__device__ __forceinline__ void store_min(float* bmin, int64_t i, float v, int fp16) {
+    if (fp16)
+        reinterpret_cast<__half*>(bmin)[i] = __float2half_rn(v);
+    else
+        bmin[i] = v;
+}
 // four integers of at most 128 as bytes: 2^23 + 2^22 + v has v in its low bits
 __device__ __forceinline__ uint32_t pack_s8(float a, float b, float c, float d) {
     const uint32_t ab = __byte_perm(__float_as_uint(a + 12582912.f), __float_as_uint(b + 12582912.f), 0x0040);
@@ -126,7 +139,7 @@ prep_gemm_i8_kernel(const int8_t* __restrict__ aq, const float* __restrict__ asc
 __global__ void __launch_bounds__(256)
 prep_gemm_b_kernel(const int8_t* __restrict__ aq, const float* __restrict__ ascale, const int16_t* __restrict__ absum,
                    const uint32_t* __restrict__ row_of, int P, int P_pad, int K, __half* __restrict__ bf16,
-                   float* __restrict__ bmin, float* __restrict__ d8t, const __grid_constant__ MapChunk maps) {
+                   float* __restrict__ bmin, int min_fp16, float* __restrict__ d8t, const __grid_constant__ MapChunk maps) {
     pdl_trigger();
     pdl_wait();
     if (blockIdx.x == 0) write_maps(maps);
@@ -151,11 +164,11 @@ prep_gemm_b_kernel(const int8_t* __restrict__ aq, const float* __restrict__ asca
         const int j = lane & 7;  // word j: b1_j, word 8 + j: b2_j
         const int16_t* bs = absum + row * (K / 16) + blk * 16 + 2 * j;
         const float bv = (float)((int)bs[0] + (int)bs[1]);
-        const float b1 = tf32_head(bv), b2 = bv - b1;  // exact: |bv| < 4096, so b2 is -1, 0 or 1
+        const float b1 = min_head(bv, min_fp16), b2 = bv - b1;  // exact: |bv| <= 4096
         bm = lane < 8 ? b1 : b2;
     }
     *reinterpret_cast<uint4*>(bf16 + (int64_t)p * K + blk * 256 + lane * 8) = o;
-    if (lane < G_MIN_K) bmin[((int64_t)p * kb + blk) * G_MIN_K + lane] = bm;
+    if (lane < G_MIN_K) store_min(bmin, ((int64_t)p * kb + blk) * G_MIN_K + lane, bm, min_fp16);
     if (lane == 0) d8t[(int64_t)blk * P_pad + p] = d8;
 }
 
@@ -212,7 +225,7 @@ prep_gemm_b_q80_kernel(const int8_t* __restrict__ aq, const float* __restrict__ 
 constexpr int PREP_UNITS = 2;
 __global__ void __launch_bounds__(256)
 prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, int8_t* __restrict__ b8, __half* __restrict__ bf16, float* __restrict__ bmin,
-                         float* __restrict__ d8t, uint32_t* __restrict__ single_group, const __grid_constant__ MapChunk maps) {
+                         int min_fp16, float* __restrict__ d8t, uint32_t* __restrict__ single_group, const __grid_constant__ MapChunk maps) {
     pdl_trigger();
     pdl_wait();
     if (blockIdx.x == 0) write_maps(maps);
@@ -257,8 +270,8 @@ prep_gemm_f32_q8k_kernel(const float* __restrict__ x, int P, int P_pad, int K, i
             s += __shfl_xor_sync(0xffffffffu, s, 1);
             s += __shfl_xor_sync(0xffffffffu, s, 2);  // 32 elements = four lanes
             const int j = lane & 7;  // the words of prep_gemm_b_kernel
-            const float bv = __shfl_sync(0xffffffffu, s, 4 * j), b1 = tf32_head(bv), b2 = bv - b1;
-            if (lane < G_MIN_K) bmin[((int64_t)p[u] * kb + blk[u]) * G_MIN_K + lane] = lane < 8 ? b1 : b2;
+            const float bv = __shfl_sync(0xffffffffu, s, 4 * j), b1 = min_head(bv, min_fp16), b2 = bv - b1;
+            if (lane < G_MIN_K) store_min(bmin, ((int64_t)p[u] * kb + blk[u]) * G_MIN_K + lane, lane < 8 ? b1 : b2, min_fp16);
         }
         if (lane == 0) d8t[(int64_t)blk[u] * P_pad + p[u]] = d8;
     }
@@ -460,6 +473,17 @@ struct GemmQ4K {
     }
     // weight side of the min term (see prep_gemm_b_kernel): -rho_j = -dmin m_j / d split into tf32 terms [r1 (8) | r2 (8)].
     // 2^23 + m as float bits is 0x4B000000 | m.
+    // one fp16 step: the eight mins, for the tiles that accumulate them on their own
+    __device__ static __forceinline__ void min_operand16(const Ctx& c, uint32_t (&r)[4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t v;  // 1024 + m in both halves
+            asm("prmt.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(c.mn[i >> 1]), "r"(0x64646464u), "r"(0x4140u + 0x0202u * (i & 1)));
+            r[i] = bits_h2(__hsub2(h2_bits(v), __float2half2_rn(1024.f)));
+        }
+    }
+    __device__ static __forceinline__ float d_of(const Ctx& c) { return half_bits_to_float((uint16_t)c.dd); }
+    __device__ static __forceinline__ float neg_dmin_of(const Ctx& c) { return -half_bits_to_float((uint16_t)(c.dd >> 16)); }
     __device__ static __forceinline__ void min_operand(const Ctx& c, uint32_t (&r)[16]) {
         const float ratio = -__fdividef(half_bits_to_float((uint16_t)(c.dd >> 16)), scale_of(c));
 #pragma unroll
@@ -534,12 +558,16 @@ struct GemmQ6K {
     }
 };
 
-// Matrices without copies, repacked on their way (candle_moe_api.cu).  The forms that take such a layer otherwise gate with expf and
+// Matrices without copies, repacked on their way (candle_moe_api.cu), and batches that the decode kernels or the streaming form
+// would take as well.  The forms that take such a layer otherwise gate with expf and
 // an exact division (silu_f); the hidden rows are quantized to int8 again, where a difference in the last bit can become a
 // step, so this one does the same: largest relative error of a gate 2.4e-7 (8.1e-7 with __expf and an approximate division), of
 // the hidden rows against 64-bit arithmetic 0.98-1.01e-7 (streaming form 0.98-1.01e-7, row-per-warp form 1.2-1.5e-7, without
 // the exact gate 1.01-1.05e-7).  It costs 3-6 % of a layer of small matrices (8 experts of 1536 x 2560, 400 rows: 457 -> 470 us).
-struct GemmQ6KOnTheWay : GemmQ6K {
+struct GemmQ6KExact : GemmQ6K {
+    static constexpr bool EXACT_GATE = true;
+};
+struct GemmQ4KExact : GemmQ4K {
     static constexpr bool EXACT_GATE = true;
 };
 
@@ -661,19 +689,22 @@ struct GemmCfg {
     // int8 products have two accumulators per position; 128-wide tiles then go through a block's positions in two passes,
     // one of which is drained during the other
     static constexpr int PASSES = F::I8 && TN == 128 ? 2 : 1;
-    static constexpr int ACC_COLS = F::I8 ? 2 * TN / PASSES : TN;  // of one of the two accumulators
-    // tensor memory: [two accumulators | pairs of weight slabs | min operands of two blocks (in shared memory beside 128-wide tiles)]
-    static constexpr bool MIN_TM = F::HAS_MIN && TN < 128, MIN_SM = F::HAS_MIN && TN == 128;
+    // Q4_K beside narrow tiles: the min term has an accumulator of its own (see prep_gemm_b_kernel)
+    static constexpr bool MIN_ACC = F::HAS_MIN && TN <= 64;
+    static constexpr int ACC_COLS = F::I8 || MIN_ACC ? 2 * TN / PASSES : TN;  // of one of the two accumulators
+    // tensor memory: [two accumulators | pairs of weight slabs | min operands of two blocks (32-wide tiles; else in shared memory)]
+    static constexpr bool MIN_TM = F::HAS_MIN && TN == 32, MIN_SM = F::HAS_MIN && !MIN_TM;
     static constexpr int SLAB_COLS = 32 * F::A_PARTS, PAIR_COLS = 2 * SLAB_COLS;
     static constexpr int TM_A = 2 * ACC_COLS, TM_MIN = TM_A + RING * PAIR_COLS;
-    static_assert(TM_MIN + (MIN_TM ? 2 * G_MIN_K : 0) <= G_TMEM_COLS, "");
+    static_assert(TM_MIN + (MIN_TM ? 2 * G_MIN_K / 2 : 0) <= G_TMEM_COLS, "");
     // shared memory: activation stages (half blocks: two slabs, B_PARTS times), min operands per block, weight stages
     static constexpr int B_TILE = TN * G_SLAB_K * 2;                        // [TN x 64] fp16 or [TN x 128] int8
     static constexpr int B_BYTES = F::I8 ? B_TILE : 2 * F::B_PARTS * B_TILE;
-    static constexpr int M_BYTES = F::HAS_MIN ? TN * G_MIN_K * 4 : 0, MA_BYTES = MIN_SM ? G_TILE_M * G_MIN_K * 4 : 0;
+    static constexpr int M_ROW = G_MIN_K * (MIN_ACC ? 2 : 4);  // bytes: fp16 or tf32
+    static constexpr int M_BYTES = F::HAS_MIN ? TN * M_ROW : 0, MA_BYTES = MIN_SM ? G_TILE_M * M_ROW : 0;
     static constexpr int W_BYTES = F::W_UNIT_BYTES;
     static constexpr int FIXED = RING * B_BYTES + 2 * (M_BYTES + MA_BYTES);
-    static constexpr int W_ROOM = 232448 - 1024 - 3072 /* barriers, offsets, weight scales */ - 4 * TN * 4 - FIXED;
+    static constexpr int W_ROOM = 232448 - 1024 - 3072 /* barriers, offsets, weight scales */ - (MIN_ACC ? 2048 : 0) - 4 * TN * 4 - FIXED;
     static constexpr int W_STAGES = W_ROOM / W_BYTES < G_W_BARS ? W_ROOM / W_BYTES : G_W_BARS;
     static_assert(W_STAGES >= 2, "");
     static constexpr int SMEM = FIXED + W_STAGES * W_BYTES + 1024 /* alignment slack */;
@@ -755,6 +786,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
     constexpr int CH = C::CH;
     __shared__ __align__(16) float s_d8[4][TN];  // activation scales of the positions, per block (ring of 4)
     __shared__ float s_dw[4][G_TILE_M];  // per block (ring of 4) and tile row: the weight scale the drain multiplies by
+    __shared__ float s_dm[C::MIN_ACC ? 4 : 1][C::MIN_ACC ? G_TILE_M : 1];  // ... and -dmin
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     constexpr int WARP_DQ0 = C::EPI_WARPS, WARP_MISC0 = WARP_DQ0 + 4 * C::GROUPS;
@@ -811,8 +843,8 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
             uint64_t acc2[CH / 2];
 #pragma unroll
             for (int i = 0; i < CH / 2; ++i) acc2[i] = 0ull;
-            // Narrow tiles have registers to add the blocks in runs of RUN, the runs on their own ([32000, 4096] Q6_K at 32
-            // rows, relative error against 64-bit arithmetic: 7.8e-8 in one run of 16, 6.5e-8 in two; 48.8 -> 49.6 us)
+            // Narrow tiles have registers to add the blocks in runs of G_RUN, the runs on their own ([32000, 4096] Q6_K at 32
+            // rows, relative error against 64-bit arithmetic: 7.8e-8 in one run of 16, 6.5e-8 in two, 6.2e-8 in four)
             constexpr bool RUNS = TN <= 64;
             uint64_t run2[RUNS ? CH / 2 : 1];
             if (RUNS) {
@@ -828,20 +860,26 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                 tc5_fence_after_sync();
                 const float dw = s_dw[ab & 3][r];  // left by the unpack warps when they produced this block
                 const uint64_t dw2 = f32x2_pack(dw, dw);
+                uint64_t dm2 = 0;
+                if constexpr (C::MIN_ACC) {
+                    const float dm = s_dm[ab & 3][r];
+                    dm2 = f32x2_pack(dm, dm);
+                }
                 const uint32_t t_main = ta_lane + (uint32_t)(C::PASSES == 2 ? 0 : buf * C::ACC_COLS);
                 const uint32_t d8_addr = smem_u32(&s_d8[ab & 3][colhalf * CH]);
                 // Steps of 16 columns; the load of step i+1 is in flight while step i is scaled into
                 // the register accumulators: acc += (d8[col] * dw[row]) * v.
                 constexpr int NS = CH / 16, PL = C::ACC_COLS / 2;
-                uint32_t stg[2][16], sth[2][F::I8 ? 16 : 1];  // int8: low and high plane
+                constexpr bool TWO = F::I8 || C::MIN_ACC;
+                uint32_t stg[2][16], sth[2][TWO ? 16 : 1];  // int8: low and high plane; Q4_K: main sum and min term
                 tmem_ld16(t_main, stg[0]);
-                if constexpr (F::I8) tmem_ld16(t_main + PL, sth[0]);
+                if constexpr (TWO) tmem_ld16(t_main + PL, sth[0]);
                 tmem_ld_wait();
                 static_for<NS>([&](auto Cc) {
                     constexpr int c = decltype(Cc)::value, s = c & 1;
                     if constexpr (c + 1 < NS) {
                         tmem_ld16(t_main + 16 * (c + 1), stg[s ^ 1]);
-                        if constexpr (F::I8) tmem_ld16(t_main + PL + 16 * (c + 1), sth[s ^ 1]);
+                        if constexpr (TWO) tmem_ld16(t_main + PL + 16 * (c + 1), sth[s ^ 1]);
                     }
                     if constexpr (F::I8) {
 #pragma unroll
@@ -850,13 +888,17 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                     static_for<4>([&](auto Qc) {
                         constexpr int q = decltype(Qc)::value;
                         const uint4 dv = lds128_o<64 * c + 16 * q>(d8_addr);  // base + constant: no address arithmetic
-                        // per column pair: the two scale products in one packed multiply, the two accumulations in one
-                        // packed fused multiply-add (each half is the IEEE fma of the scalar form)
-                        acc2[8 * c + 2 * q] = f32x2_fma(f32x2_mul(dw2, f32x2_pack_bits(dv.x, dv.y)),
-                                                        f32x2_pack_bits(stg[s][4 * q], stg[s][4 * q + 1]), acc2[8 * c + 2 * q]);
-                        acc2[8 * c + 2 * q + 1] = f32x2_fma(f32x2_mul(dw2, f32x2_pack_bits(dv.z, dv.w)),
-                                                            f32x2_pack_bits(stg[s][4 * q + 2], stg[s][4 * q + 3]),
-                                                            acc2[8 * c + 2 * q + 1]);
+                        // per column pair packed operations (each half is the IEEE operation of the scalar form)
+                        static_for<2>([&](auto Ic) {
+                            constexpr int i = decltype(Ic)::value, j = 4 * q + 2 * i;
+                            const uint64_t d8 = i ? f32x2_pack_bits(dv.z, dv.w) : f32x2_pack_bits(dv.x, dv.y);
+                            const uint64_t main = f32x2_pack_bits(stg[s][j], stg[s][j + 1]);
+                            uint64_t& a = acc2[8 * c + 2 * q + i];
+                            if constexpr (C::MIN_ACC)  // d8 * (d M - dmin Mm): the two cancel before anything is rounded to the sum
+                                a = f32x2_fma(f32x2_fma(dm2, f32x2_pack_bits(sth[s][j], sth[s][j + 1]), f32x2_mul(dw2, main)), d8, a);
+                            else
+                                a = f32x2_fma(f32x2_mul(dw2, d8), main, a);
+                        });
                     });
                     if (c + 1 < NS) tmem_ld_wait();
                     if (c == NS - 2) {  // every column of this thread has been read: the accumulator may be overwritten
@@ -936,17 +978,35 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                 const uint32_t slot = first + h;
                 if (pass > 0) mbar_wait_tight(&done_p[slot], (pass - 1) & 1, abort_flag);  // the MMAs that read it last
                 tc5_fence_after_sync();
-                if (H == 2 ? h == 0 : group == 0) s_dw[(H == 2 ? u : u >> 1) & 3][r] = F::scale_of(ctx);  // for the drain of this block
+                if (H == 2 ? h == 0 : group == 0) {  // for the drain of this block
+                    if constexpr (C::MIN_ACC) {
+                        s_dw[u & 3][r] = F::d_of(ctx);
+                        s_dm[u & 3][r] = F::neg_dmin_of(ctx);
+                    } else {
+                        s_dw[(H == 2 ? u : u >> 1) & 3][r] = F::scale_of(ctx);
+                    }
+                }
                 F::emit(ctx, row, g, h, P.magic, ta_lane + slot * C::PAIR_COLS);
                 if constexpr (F::HAS_MIN) {
                     if (h == 1) {
                         // (the last min MMAs on these operands came before the commit just waited for)
-                        uint32_t rho[16];
-                        F::min_operand(ctx, rho);
-                        if constexpr (C::MIN_TM) {
-                            tmem_st16(tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(C::TM_MIN + group * G_MIN_K), rho);
+                        if constexpr (C::MIN_ACC) {
+                            uint32_t m[4];
+                            F::min_operand16(ctx, m);
+                            if constexpr (C::MIN_TM) {
+                                const uint32_t t = tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(C::TM_MIN + group * (G_MIN_K / 2));
+                                tmem_st4(t, m);
+                                tmem_st4(t + 4, m);
+                            } else {
+                                uint8_t* const a = smem_min_a + group * C::MA_BYTES + r * C::M_ROW;  // both halves alike: no swizzle to mind
+                                *reinterpret_cast<uint4*>(a) = make_uint4(m[0], m[1], m[2], m[3]);
+                                *reinterpret_cast<uint4*>(a + 16) = make_uint4(m[0], m[1], m[2], m[3]);
+                                fence_proxy_async_smem();
+                            }
                         } else {
-                            uint8_t* const a = smem_min_a + group * C::MA_BYTES + r * (G_MIN_K * 4);
+                            uint32_t rho[16];
+                            F::min_operand(ctx, rho);
+                            uint8_t* const a = smem_min_a + group * C::MA_BYTES + r * C::M_ROW;
                             const int sw = (r >> 1) & 3;  // 64-byte swizzle
 #pragma unroll
                             for (int j = 0; j < 4; ++j)
@@ -1126,7 +1186,8 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         uint32_t it = 0, n_eff = 0, idesc[2] = {0, 0}, idesc_min = 0;
         bool second = false;
         const uint64_t b_desc = umma_desc_sw128(smem_u32(smem));
-        const uint64_t mb_desc = umma_desc_sw64(smem_u32(smem_min_b)), ma_desc = umma_desc_sw64(smem_u32(smem_min_a));
+        const uint64_t mb_desc = C::MIN_ACC ? umma_desc_sw32(smem_u32(smem_min_b)) : umma_desc_sw64(smem_u32(smem_min_b));
+        const uint64_t ma_desc = C::MIN_ACC ? umma_desc_sw32(smem_u32(smem_min_a)) : umma_desc_sw64(smem_u32(smem_min_a));
         const auto block = [&](auto Bc) {  // block 2 it + B of this CTA
             constexpr int B = decltype(Bc)::value, R = C::RING;
 #pragma unroll
@@ -1170,15 +1231,14 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                             }
                         }
                         if (F::HAS_MIN && h == 1) {
-                            // the min term joins the same accumulator: three tf32 steps r1 b1 + r2 b1 + r1 b2, last in the block
                             const uint64_t dm = umma_desc_add(mb_desc, B * (C::M_BYTES >> 4));
+                            const uint64_t da = umma_desc_add(ma_desc, B * (C::MA_BYTES >> 4));
                             if constexpr (C::MIN_TM) {
-                                const uint32_t da = tmem_base + C::TM_MIN + B * G_MIN_K;
-                                umma_tf32_ts(d_main, da, dm, idesc_min, true);
-                                umma_tf32_ts(d_main, da + 8, dm, idesc_min, true);
-                                umma_tf32_ts(d_main, da, umma_desc_add(dm, 2), idesc_min, true);
+                                umma_f16_ts(d_main + TN, tmem_base + C::TM_MIN + B * (G_MIN_K / 2), dm, idesc[0], false);
+                            } else if constexpr (C::MIN_ACC) {
+                                umma_f16(d_main + TN, da, dm, idesc[0], false);
                             } else {
-                                const uint64_t da = umma_desc_add(ma_desc, B * (C::MA_BYTES >> 4));
+                                // the min term joins the same accumulator: three tf32 steps r1 b1 + r2 b1 + r1 b2, last in the block
                                 umma_tf32(d_main, da, dm, idesc_min, true);
                                 umma_tf32(d_main, umma_desc_add(da, 2), dm, idesc_min, true);
                                 umma_tf32(d_main, da, umma_desc_add(dm, 2), idesc_min, true);
@@ -1384,12 +1444,12 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         e = q80 ? launch_k(prep_gemm_f32_q80_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K_in, K, q80x ? 1 : 0, bf16,
                            d8t, single_group)
                 : launch_k(prep_gemm_f32_q8k_kernel, prep_grid, dim3(256), 0, st, x_f32, (int)P, (int)p_pad, K, i8 ? b8 : (int8_t*)nullptr,
-                           bf16, has_min ? bmin : (float*)nullptr, d8t, single_group, first);
+                           bf16, has_min ? bmin : (float*)nullptr, tn <= 64 ? 1 : 0, d8t, single_group, first);
     else
         e = q80 ? launch_k(prep_gemm_b_q80_kernel, prep_grid, dim3(256), 0, st, aq, ascale, row_of, (int)P, (int)p_pad, K_in, K,
                            q80x ? 1 : 0, bf16, d8t)
             : i8 ? launch_k(prep_gemm_i8_kernel, prep_grid, dim3(256), 0, st, aq, ascale, row_of, (int)P, (int)p_pad, K, b8, d8t)
-                 : launch_k(prep_gemm_b_kernel, prep_grid, dim3(256), 0, st, aq, ascale, absum, row_of, (int)P, (int)p_pad, K, bf16, bmin, d8t,
+                 : launch_k(prep_gemm_b_kernel, prep_grid, dim3(256), 0, st, aq, ascale, absum, row_of, (int)P, (int)p_pad, K, bf16, bmin, tn <= 64 ? 1 : 0, d8t,
                             first);
     if (e != cudaSuccess) return e;
 
@@ -1397,7 +1457,8 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     if (i8 ? !make_map_2d(&map_b, b8, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)p_pad, (uint64_t)K, 2 * G_SLAB_K, tn)
            : !make_map_2d(&map_b, bf16, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)p_pad, (uint64_t)K * parts, G_SLAB_K, tn))
         return cudaErrorNotSupported;
-    if (!make_map_2d(&map_bs, bmin, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)p_pad, (uint64_t)kb * G_MIN_K, G_MIN_K, tn, CU_TENSOR_MAP_SWIZZLE_64B))
+    if (tn <= 64 ? !make_map_2d(&map_bs, bmin, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (uint64_t)p_pad, (uint64_t)kb * G_MIN_K, G_MIN_K, tn, CU_TENSOR_MAP_SWIZZLE_32B)
+                 : !make_map_2d(&map_bs, bmin, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)p_pad, (uint64_t)kb * G_MIN_K, G_MIN_K, tn, CU_TENSOR_MAP_SWIZZLE_64B))
         return cudaErrorNotSupported;
 
     GemmParams G{};
@@ -1450,6 +1511,11 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     e = stream_status_ptr(&G.status);
     if (e != cudaSuccess) return e;
     if (dtype == CANDLE_GGML_Q4K) {
+        if (gate_up && exact_gate) {
+            if (tn == 32) return launch_gemm_kernel<GemmQ4KExact, true, 32>(st, G, map_b, map_bs);
+            if (tn == 64) return launch_gemm_kernel<GemmQ4KExact, true, 64>(st, G, map_b, map_bs);
+            return launch_gemm_kernel<GemmQ4KExact, true, 128>(st, G, map_b, map_bs);
+        }
         if (tn == 32)
             return gate_up ? launch_gemm_kernel<GemmQ4K, true, 32>(st, G, map_b, map_bs) : launch_gemm_kernel<GemmQ4K, false, 32>(st, G, map_b, map_bs);
         if (tn == 64)
@@ -1467,9 +1533,9 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
         return launch_gemm_kernel<GemmQ80, false, 128>(st, G, map_b, map_bs);
     }
     if (gate_up && exact_gate) {
-        if (tn == 32) return launch_gemm_kernel<GemmQ6KOnTheWay, true, 32>(st, G, map_b, map_bs);
-        if (tn == 64) return launch_gemm_kernel<GemmQ6KOnTheWay, true, 64>(st, G, map_b, map_bs);
-        return launch_gemm_kernel<GemmQ6KOnTheWay, true, 128>(st, G, map_b, map_bs);
+        if (tn == 32) return launch_gemm_kernel<GemmQ6KExact, true, 32>(st, G, map_b, map_bs);
+        if (tn == 64) return launch_gemm_kernel<GemmQ6KExact, true, 64>(st, G, map_b, map_bs);
+        return launch_gemm_kernel<GemmQ6KExact, true, 128>(st, G, map_b, map_bs);
     }
     if (tn == 32)
         return gate_up ? launch_gemm_kernel<GemmQ6K, true, 32>(st, G, map_b, map_bs) : launch_gemm_kernel<GemmQ6K, false, 32>(st, G, map_b, map_bs);

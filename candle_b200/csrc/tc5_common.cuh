@@ -132,6 +132,16 @@ __device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t smem_addr) {
     d |= (uint64_t)4 << 61;  // layout: SWIZZLE_64B
     return d;
 }
+// Rows of 32 bytes with 32-byte swizzle: 8-row atoms of 256 B.
+__device__ __forceinline__ uint64_t umma_desc_sw32(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(256 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)6 << 61;  // layout: SWIZZLE_32B
+    return d;
+}
 // Instruction descriptor for kind::f16: A and B fp16, both K-major, D fp32, tile M x N.
 __host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N) {
     return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
