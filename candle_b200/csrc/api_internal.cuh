@@ -35,6 +35,7 @@ struct ExpertBufs {
     void* gemm;     // scratch of the large-batch GEMM (may be null)
     uint8_t* repack = nullptr;  // room for one expert's Q6_K matrices repacked on the way (null: that form is not used)
     void* repack_gemm = nullptr;  // ... and that form's operand scratch
+    int64_t gemm_above = -1;      // rows above which the GEMM takes the products (-1: the tuning key's)
 };
 
 // The shared expert's products beside the routed ones (run_experts takes them where the decode kernels do): what each needs,

@@ -12,11 +12,9 @@ using namespace cmoe;
 
 namespace {
 
-// Above this bound on the rows of one expert (default 96) the tensor-core GEMM takes the k-quant products (below,
-// the decode kernels); the tuning key GEMM_MIN_ROWS changes it.
-// A single-device forward only knows the bound T on the rows of an expert, and its experts usually hold about
-// k T / E rows, i.e. a few of the decode kernels' 16-row groups.  Measured on the Mixtral-shaped layer (decode
-// kernels / GEMM, microseconds per step): T = 64 308 / 419, 80 376 / 421, 96 425 / 423, 112 504 / 449, 128 507 / 450.
+// Rows per step above which the tensor-core GEMM takes the products (below, the decode kernels).  The tuning key GEMM_MIN_ROWS
+// sets them; at its default (96) a single-device forward over repacked copies goes by the rows that an expert holds on average,
+// k T / E, because the decode kernels pay for every eight of them and the GEMM hardly at all (gemm_rows below).
 inline int64_t gemm_min_rows() { return tuning_get(TUNE_GEMM_MIN_ROWS); }
 // When the caller knows the ACTUAL largest row count of an expert (or, in the slot form of expert parallelism, a
 // bound five quarters of the expected one, so that the tile width leaves a margin), the GEMM takes over above 32 rows.
@@ -32,6 +30,24 @@ constexpr int64_t GEMM_MIN_ROWS_EXACT = 32;
 // faster in all of 300 sizes from 1024 to 32000 by 512 to 4096).  Every sixteen rows are one more pass over the copy.
 constexpr int64_t QMM_DIRECT_MAX_ROWS = 64;
 constexpr int64_t QMM_GEMM_MIN_ROWS = 48;  // the dense product: one matrix, rows known exactly
+// Measured, decode kernels / GEMM, us per block.  Mixtral-shaped (8 experts, top-2): T = 32 217 / 277, 48 261 / 282, 56 283 / 276, 64 300 /
+// 281, 96 385 / 294; all Q4_K: 48 232 / 241, 56 249 / 241; d = 2048, ff = 8192: 48 105 / 115, 64 119 / 114; d = ff = 4096, Q6_K: 16 138 / 136,
+// 48 171 / 138.  Q8_0 with a shared expert: 60 experts, top-4: 100 205 / 296, 256 299 / 323, 384 401 / 358; 16 experts, top-2: 192 166 / 169,
+// 256 202 / 178; 32 experts, top-4: 128 175 / 209, 192 228 / 228, 256 269 / 233.
+// Without copies, streaming form / GEMM for Q4_K (Q6_K products stay where they are): d = ff = 4096: 8 91 / 100, 12 111 / 100, 16 112 / 101,
+// 96 228 / 107; d = 2048, ff = 8192: 8 110 / 98, 32 153 / 99; d = 1024, ff = 3584: 8 56 / 44, 64 102 / 50; Mixtral-shaped with a Q6_K down
+// product: 8 283 / 277, 32 412 / 342, 96 793 / 503.
+// Only where an expert's rows are expected in a narrow tile, whose gate is as exact as that of the forms before.
+inline int64_t gemm_rows(const candle_moe_weights_t* w) {
+    const int64_t rows = gemm_min_rows(), E = w->n_experts, k = w->top_k;
+    if (rows != TUNE_GEMM_MIN_ROWS_DEFAULT) return rows;
+    const bool q80_13 = w->dtype_w13 == CANDLE_GGML_Q8_0, q80_2 = w->dtype_w2 == CANDLE_GGML_Q8_0;
+    const bool copies = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked;
+    if (copies && q80_13 && q80_2) return std::max(rows, std::min<int64_t>(22 * E / k, 512));  // (not measured beyond)
+    if (q80_13 || q80_2 || 5 * k * rows > 4 * 64 * E) return rows;
+    if (copies) return std::min(rows, 12 * E / k);
+    return w->dtype_w13 == CANDLE_GGML_Q4K ? std::min(rows, 5 * E / (2 * k)) : rows;
+}
 // Decode-sized batches may split K finely (more parallel items, smaller resident activations);
 // larger batches get four slots, enough for the streaming form's activation rows to fit.
 inline int k_split_slots(int64_t T) { return T <= gemm_min_rows() ? MAX_K_SPLITS : 4; }
@@ -137,8 +153,9 @@ Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_, size_t a
         ws.so = carve<float>(base, off, (size_t)T * d * k_split_slots(T));
         free_at = off;
     }
-    if (T > gemm_min_rows()) {
-        // large batches: fp16 activation operand of the tcgen05 GEMM (Q4_K matrices), reused by gate_up and down
+    size_t gemm_ext = 0;  // end of the GEMM's operand scratch where a workspace need not have it
+    if (T > std::min(gemm_min_rows(), gemm_rows(w))) {
+        // large batches: activation operand of the tcgen05 GEMM, reused by gate_up and down
         size_t g = 0;
         const auto takes = [](int dt, const void* packed) {
             return dt == CANDLE_GGML_Q4K || ((dt == CANDLE_GGML_Q6K || dt == CANDLE_GGML_Q8_0) && packed != nullptr);
@@ -150,14 +167,16 @@ Workspace layout(const candle_moe_weights_t* w, int64_t T, void* base_, size_t a
             w->shared_w2_prepacked)
             g = std::max(g, std::max(expert_gemm_scratch_bytes(T, (int)d, 2), expert_gemm_scratch_bytes(T, w->d_ff_shared)));
         if (g) {
-            off = align_up(off, 1024);
-            ws.gemm = base ? base + off : nullptr;
+            const size_t at = align_up(off, 1024);
+            const bool optional = T <= gemm_min_rows();  // the decode kernels take the batch without it
+            if (!optional) off = at + g;
+            else gemm_ext = align_up(at + g, 256);
+            if (!optional || avail >= gemm_ext) ws.gemm = base ? base + at : nullptr;
             if (!base) ws.gemm = reinterpret_cast<void*>(1);  // size query: only the extent matters
-            off += g;
         }
     }
     ws.total = align_up(off, 256);
-    ws.total_ext = ws.total;
+    ws.total_ext = std::max(ws.total, gemm_ext);
     if (T > gemm_min_rows()) {
         const bool r13 = repacks_on_the_way(w->dtype_w13, w->w1_prepacked && w->w3_prepacked, w->d_ff, w->d_model, true, (int64_t)Tk, w->n_experts);
         const bool r2 = repacks_on_the_way(w->dtype_w2, w->w2_prepacked != nullptr, w->d_model, w->d_ff, false, (int64_t)Tk, w->n_experts);
@@ -362,9 +381,10 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
                 bool marks, bool rows_exact, const uint32_t* row_limit, int64_t total_rows_hint, SharedRun* shared) {
     if (total_rows_hint <= 0) total_rows_hint = P;
     const int E = w->n_experts, d = w->d_model, ff = w->d_ff;
-    const bool large = b.gemm && max_rows > (rows_exact ? GEMM_MIN_ROWS_EXACT : gemm_min_rows()) && gemm_enabled();
+    const int64_t gemm_above = b.gemm_above >= 0 ? b.gemm_above : gemm_min_rows();
+    const bool large = b.gemm && max_rows > (rows_exact ? GEMM_MIN_ROWS_EXACT : gemm_above) && gemm_enabled();
     bool use_prepacked = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked &&
-                         max_rows <= std::max<int64_t>(gemm_min_rows(), 64) && !large;
+                         max_rows <= std::max<int64_t>({gemm_min_rows(), gemm_above, 64}) && !large;
     bool gate_done = false, down_done = false;
     *eo_splits = 1;
     ExpertPtrs q1, q3, q2;
@@ -404,8 +424,9 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
         const cudaError_t ce = !rp && b.repack && repacks_on_the_way(w->dtype_w13, false, ff, d, true, P, E)
                                    ? gemm_repacking(st, true, p1, p3, E, d, ff, offsets, row_of, P, tile_rows, xq, xs, xb, b.hidden, b,
                                                     nullptr, 0, nullptr)
-                                   : launch_expert_gemm(st, true, g1, g3, w->dtype_w13, rp, E, d, ff, offsets, row_of, P, tile_rows, xq,
-                                                  xs, xb, b.hidden, b.gemm);
+                                   : launch_expert_gemm(st, true, g1, g3, w->dtype_w13, rp, E, d, ff, offsets, row_of, P, tile_rows, xq, xs, xb,
+                                                        b.hidden, b.gemm, 1, nullptr, 0, nullptr, nullptr, nullptr, false,
+                                                        !rows_exact && max_rows <= gemm_min_rows());
         if (ce == cudaSuccess)
             gate_done = true;
         else if (ce != cudaErrorNotSupported)
@@ -533,15 +554,17 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
     mark(st, 2);
     // a token selects an expert at most once: no expert sees more than T rows
     int eo_splits = 1, so_splits = 1;
-    const ExpertBufs eb{ws.hidden, ws.hq, ws.hs, ws.hb, ws.eo, ws.gemm, ws.repack, ws.repack_gemm};
+    const int64_t gemm_above = gemm_rows(w);
+    const ExpertBufs eb{ws.hidden, ws.hq, ws.hs, ws.hb, ws.eo, ws.gemm, ws.repack, ws.repack_gemm, gemm_above};
     // over repacked Q8_0 copies the shared expert takes the decode kernels -- in the launches of the routed experts where those
     // are Q8_0 too -- and for large batches the tensor-core GEMM
     const bool sh_packed = w->d_ff_shared > 0 && w->dtype_shared13 == CANDLE_GGML_Q8_0 && w->dtype_shared2 == CANDLE_GGML_Q8_0 &&
                            w->shared_w1_prepacked && w->shared_w3_prepacked && w->shared_w2_prepacked &&
                            !((reinterpret_cast<uintptr_t>(w->shared_w1_prepacked) | reinterpret_cast<uintptr_t>(w->shared_w3_prepacked) |
                               reinterpret_cast<uintptr_t>(w->shared_w2_prepacked)) & 15);
-    const bool sh_gemm = sh_packed && ws.gemm && T > gemm_min_rows() && gemm_enabled();
-    const bool sh_direct = sh_packed && !sh_gemm && T <= std::max<int64_t>(gemm_min_rows(), 64);
+    const int64_t sh_above = std::max(gemm_min_rows(), gemm_above);
+    const bool sh_gemm = sh_packed && ws.gemm && T > sh_above && gemm_enabled();
+    const bool sh_direct = sh_packed && !sh_gemm && T <= std::max<int64_t>(sh_above, 64);
     SharedRun sr;
     const bool sh_joins = sh_direct && w->dtype_w13 == CANDLE_GGML_Q8_0 && w->dtype_w2 == CANDLE_GGML_Q8_0 && ws.sxq == ws.xq;
     if (sh_joins) {

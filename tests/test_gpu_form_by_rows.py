@@ -1,7 +1,72 @@
-"""The narrow GEMM tiles whose Q4_K min term has its own accumulator."""
+"""Which kernels take a batch of a single-device forward: the rows on either side of the rule's lines (candle_moe_api.cu, gemm_rows),
+with repacked copies and without, against the oracle; and the narrow GEMM tiles whose Q4_K min term has its own accumulator."""
+import ctypes as C
+
+import numpy as np
 import pytest
 
+from tests import helpers as H
+
 pytestmark = pytest.mark.gpu
+
+
+def _check(orc, torch, cfg, T, prepack):
+    from candle_b200 import _lib
+    blk, mw = H.random_device_block(orc, torch, cfg, 5)
+    if prepack:
+        blk.prepack()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn((T, cfg["d"]), generator=g, device="cuda", dtype=torch.float32)
+    y = blk.forward(x).clone()
+    assert torch.equal(y, blk.forward(x))
+    v = C.c_int32(-1)
+    assert _lib.load().candle_moe_device_status(C.byref(v)) == 0 and v.value == 0
+    xs = x.cpu().numpy()
+    ref = orc.moe_forward(mw, xs)
+    ids = blk.last_routing(T)[0].numpy().astype(np.uint32)
+    probs = orc.router_topk(xs, mw.router, cfg["k"], cfg["renorm"], mw.router_bias)[0]
+    H.check_routing(probs, ref.topk_ids, ids)
+    same = (ref.topk_ids == ids).all(axis=1)
+    assert H.max_rel(y.cpu().numpy()[same], ref.y[same]) <= H.MAX_REL_TOL
+    assert H.rel_l2(y.cpu().numpy()[same], ref.y[same]) <= H.REL_L2_TOL
+    return blk, x, y
+
+
+def _cfg(dt13, dt2, E, k, d=512, ff=1024, fs=0):
+    return dict(d=d, ff=ff, E=E, k=k, dt13=dt13, dt2=dt2, renorm=True, ff_shared=fs, zipf=False)
+
+
+@pytest.mark.parametrize("dt13,dt2,prepack,E,k,rows", [
+    (12, 14, True, 8, 2, (48, 49, 96, 97)),   # 12 rows of an expert
+    (14, 14, True, 8, 2, (48, 49)),
+    (12, 12, True, 3, 2, (18, 19, 96)),       # few experts: wide tiles, the old line
+    (12, 12, False, 8, 2, (10, 11, 64)),      # 2.5 rows of an expert, GGUF blocks
+    (12, 14, False, 8, 2, (11, 96)),          # the down product stays where it was
+    (14, 12, False, 8, 2, (11, 96)),
+    (8, 8, True, 32, 4, (97, 176, 177)),      # 22 rows of an expert
+    (8, 8, False, 32, 4, (97,)),
+])
+def test_rows_on_either_side_of_the_lines(orc, torch_cuda, dt13, dt2, prepack, E, k, rows):
+    for T in rows:
+        _check(orc, torch_cuda, _cfg(dt13, dt2, E, k, fs=512 if dt13 == 8 and prepack else 0), T, prepack)
+
+
+@pytest.mark.parametrize("dt13,dt2,prepack", [(12, 14, True), (12, 12, False)])
+def test_smallest_workspace_of_a_batch_stays_enough(orc, torch_cuda, dt13, dt2, prepack):
+    """Up to 96 rows the GEMM's operand scratch is optional: a workspace without it is taken, by the other kernels."""
+    torch = torch_cuda
+    from candle_b200 import _lib
+    lib, T = _lib.load(), 64
+    blk, x, y = _check(orc, torch, _cfg(dt13, dt2, 8, 2), T, prepack)
+    w = blk._cw
+    small, full = H.smallest_workspace(_lib, w, T), C.c_size_t(0)
+    assert lib.candle_moe_workspace_bytes(C.byref(w), T, C.byref(full)) == 0
+    assert small < full.value
+    ws = torch.empty(small, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(y)
+    assert lib.candle_moe_forward(torch.cuda.current_stream().cuda_stream, C.byref(w), x.data_ptr(), T, out.data_ptr(), ws.data_ptr(), small) == 0
+    # the hidden rows are quantized to int8 in between: the bound of two orders of the f32 sums
+    assert H.rel_l2(out.cpu().numpy(), y.cpu().numpy()) <= H.REL_L2_TOL
 
 
 @pytest.mark.parametrize("rows,n,k", [(17, 12800, 256), (32, 12800, 2304), (33, 12800, 768), (49, 256, 4096), (64, 1024, 1024), (65, 1024, 1024)])
