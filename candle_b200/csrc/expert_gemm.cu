@@ -1032,24 +1032,32 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         bool ok = true;
         TileCoord tc;
         if constexpr (F::HALF_TILES) {
-            // half-tile blocks of the repacked layout: one bulk copy per 8 tile rows, lane i < 16 copies half-tile i
-            // (gate_up: W1 and W3 half-tiles alternate).  No requests into L2 ahead: the CTAs of a weight tile's position tiles
-            // run together and share the lines, and sixteen more instructions per block held the copies up (all-Q8_0 layer of
-            // 60 experts, 4096 rows, down 236 -> 218 us, shared down 127 -> 106 us without them).
-            constexpr int HT_BYTES = F::W_UNIT_BYTES * 8 / G_TILE_M;
-            const bool active = lane < G_TILE_M / 8, is_w3 = GATE_UP && (lane & 1);
+            // half-tile blocks of the repacked layout: one bulk copy per 8 tile rows (gate_up: W1 and W3 half-tiles alternate), all
+            // issued by one lane from uniform registers: issued by sixteen lanes, they went out one after the other all the same,
+            // about 80 clocks each, and the loader held up the all-Q8_0 products (60 experts, 4096 rows: down
+            // 202 -> 164 us, shared down 144 -> 106, gate_up 467 -> 452).
+            // No requests into L2 ahead: the CTAs of a weight tile's position tiles run together and share the lines.
+            constexpr int HT_BYTES = F::W_UNIT_BYTES * 8 / G_TILE_M, N_HT = G_TILE_M / 8;
+            const size_t pitch = (size_t)P.kb * F::W_UNITS * HT_BYTES;  // from a half-tile of rows to the next
             while (ok && walk.next(tc)) {
-                const int ht = GATE_UP ? tc.mt * 8 + (lane >> 1) : tc.mt * 16 + lane;
-                const uint8_t* src = active ? (is_w3 ? P.wb.p[tc.e] : P.wa.p[tc.e]) + (size_t)ht * P.kb * F::W_UNITS * HT_BYTES : nullptr;
+                const size_t off = (size_t)tc.mt * (GATE_UP ? N_HT / 2 : N_HT) * pitch + (size_t)tc.kb0 * F::W_UNITS * HT_BYTES;
+                const uint8_t *src = P.wa.p[tc.e] + off, *src3 = GATE_UP ? P.wb.p[tc.e] + off : nullptr;
 #pragma unroll 1
-                for (int u = tc.kb0 * F::W_UNITS; u < tc.kb1 * F::W_UNITS; ++u, ++unit) {
+                for (uint32_t left = walk.blocks * F::W_UNITS; left > 0; --left, ++unit) {
                     const uint32_t last = unit - C::W_STAGES;
                     uint64_t* const bar = &full_w[unit % G_W_BARS];
                     if (unit >= (uint32_t)C::W_STAGES) ok = mbar_wait_tight(&empty_w[last % G_W_BARS], (last / G_W_BARS) & 1, abort_flag);
                     if (!(ok = __all_sync(0xffffffffu, ok))) break;  // nothing is issued after a wait that gave up
-                    if (lane == 0) mbar_expect_tx(bar, F::W_UNIT_BYTES);
+                    if (elect_one()) {
+                        uint8_t* const dst = smem_w + ws * C::W_BYTES;
+                        mbar_expect_tx(bar, F::W_UNIT_BYTES);
+#pragma unroll
+                        for (int i = 0; i < N_HT; ++i)
+                            bulk_g2s(dst + i * HT_BYTES, GATE_UP ? (i & 1 ? src3 : src) + (i >> 1) * pitch : src + i * pitch, HT_BYTES, bar);
+                    }
                     __syncwarp();
-                    if (active) bulk_g2s(smem_w + ws * C::W_BYTES + lane * HT_BYTES, src + (size_t)u * HT_BYTES, HT_BYTES, bar);
+                    src += HT_BYTES;
+                    if (GATE_UP) src3 += HT_BYTES;
                     if (++ws == C::W_STAGES) ws = 0;
                 }
             }
