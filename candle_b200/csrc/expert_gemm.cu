@@ -1213,7 +1213,7 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         // whole warp walks it, so that operands stay in uniform registers, and one elected lane issues.
         TileCoord tc;
         uint32_t it = 0, n_eff = 0, idesc[2] = {0, 0}, idesc_min = 0;
-        bool second = false;
+        bool second = false, full_n = false, free_n = false;
         const uint64_t b_desc = umma_desc_sw128(smem_u32(smem));
         const uint64_t mb_desc = C::MIN_ACC ? umma_desc_sw32(smem_u32(smem_min_b)) : umma_desc_sw64(smem_u32(smem_min_b));
         const uint64_t ma_desc = C::MIN_ACC ? umma_desc_sw32(smem_u32(smem_min_a)) : umma_desc_sw64(smem_u32(smem_min_a));
@@ -1223,14 +1223,23 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
             for (int ps = 0; ps < C::PASSES; ++ps) {
                 const int buf = C::PASSES == 2 ? ps : B;
                 // the drain of what this accumulator held last: block ab - 2, with two passes ab - 1
-                if (C::PASSES == 2 ? it > 0 || B > 0 : it > 0)
+                if (C::PASSES == 2 ? it > 0 || B > 0 : it > 0 && !free_n)
                     mbar_wait_tight(&acc_free[buf], C::PASSES == 2 ? (B & 1) ^ 1 : (it & 1) ^ 1, abort_flag);
                 const uint32_t d_main = tmem_base + buf * C::ACC_COLS;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int st = (2 * B + h) % R;
-                    if (ps == 0) mbar_wait_tight(&full_p[st], R == 4 ? it & 1 : B & 1, abort_flag);
+                    if (ps == 0 && !full_n) mbar_wait_tight(&full_p[st], R == 4 ? it & 1 : B & 1, abort_flag);
                     tc5_fence_after_sync();
+                    if constexpr (C::PASSES == 1 && TN == 128) {
+                        // ask the next barriers now: the answers, 200 to 300 clocks away, arrive while the MMAs are issued (gate_up of
+                        // the Mixtral-shaped layer, 2048 rows 960 -> 930 us, [4096, 4096] at 777 rows 41.5 -> 39.5; narrow tiles, whose MMAs are
+                        // over by then, gain nothing)
+                        const uint32_t next_it = B == 1 && h == 1 ? it + 1 : it;
+                        const int nb = h == 0 ? B : B ^ 1, nst = (2 * nb + (h ^ 1)) % R;
+                        full_n = mbar_test(&full_p[nst], R == 4 ? next_it & 1 : nb & 1);
+                        if (h == 1) free_n = mbar_test(&acc_free[nb], (next_it & 1) ^ 1);
+                    }
                     if (elect_one()) {
                         const uint32_t a_t = tmem_base + C::TM_A + st * C::PAIR_COLS;
                         const uint64_t db = umma_desc_add(b_desc, st * (C::B_BYTES >> 4));
