@@ -473,6 +473,37 @@ cudaError_t launch_router_topk(cudaStream_t st, const float* x, const float* rou
 // ------------------------------------------------------------------------------------------------
 constexpr int PERMUTE_THREADS = 1024;
 
+// s_off[e]: counts -> exclusive prefix sums, and both to memory (offsets[E] = the total); by one warp
+__device__ __forceinline__ void scan_counts(uint32_t* s_off, int lane, int E, uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets) {
+    constexpr int PER = CANDLE_MOE_MAX_EXPERTS / 32;
+    uint32_t v[PER], sum = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = lane * PER + j;
+        v[j] = e < E ? s_off[e] : 0u;
+        sum += v[j];
+    }
+    uint32_t run = sum;  // inclusive over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += up;
+    }
+    run -= sum;
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = lane * PER + j;
+        if (e < E) {
+            counts[e] = v[j];
+            offsets[e] = run;
+            s_off[e] = run;
+            run += v[j];
+            if (e == E - 1) offsets[E] = run;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(PERMUTE_THREADS)
 permute_kernel(const uint32_t* __restrict__ ids, int64_t n_pairs, int k, int E, uint32_t* __restrict__ counts,
                uint32_t* __restrict__ offsets, uint32_t* __restrict__ perm_token, uint32_t* __restrict__ pair_pos) {
@@ -496,35 +527,7 @@ permute_kernel(const uint32_t* __restrict__ ids, int64_t n_pairs, int k, int E, 
         if (lane == 0) s_off[e] = c;
     }
     __syncthreads();
-    if (warp == 0) {
-        constexpr int PER = CANDLE_MOE_MAX_EXPERTS / 32;
-        uint32_t v[PER], sum = 0;
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int e = lane * PER + j;
-            v[j] = e < E ? s_off[e] : 0u;
-            sum += v[j];
-        }
-        uint32_t run = sum;  // inclusive over the lanes
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t up = __shfl_up_sync(0xffffffffu, run, o);
-            if (lane >= o) run += up;
-        }
-        run -= sum;
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int e = lane * PER + j;
-            if (e < E) {
-                counts[e] = v[j];
-                offsets[e] = run;
-                s_off[e] = run;
-                run += v[j];
-                if (e == E - 1) offsets[E] = run;
-            }
-        }
-    }
+    if (warp == 0) scan_counts(s_off, lane, E, counts, offsets);
     __syncthreads();
     for (int e = warp; e < E; e += n_warps) {
         uint32_t base = s_off[e];
@@ -579,32 +582,35 @@ permute_scan_kernel(uint32_t* __restrict__ table, int n_chunks, int E, uint32_t*
                     uint32_t* __restrict__ offsets) {
     pdl_trigger();
     pdl_wait();
-    __shared__ uint32_t s_count[CANDLE_MOE_MAX_EXPERTS], s_off[CANDLE_MOE_MAX_EXPERTS + 1];
+    __shared__ uint32_t s_off[CANDLE_MOE_MAX_EXPERTS + 1];
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         uint32_t c = 0;
+#pragma unroll 8
         for (int b = 0; b < n_chunks; ++b) c += table[(size_t)b * E + e];
-        s_count[e] = c;
+        s_off[e] = c;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int e = 0; e < E; ++e) {
-            s_off[e] = run;
-            run += s_count[e];
-        }
-        s_off[E] = run;
-    }
+    if (threadIdx.x < 32) scan_counts(s_off, threadIdx.x, E, counts, offsets);
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        counts[e] = s_count[e];
         uint32_t run = s_off[e];
-        for (int b = 0; b < n_chunks; ++b) {
+        int b = 0;
+        for (; b + 8 <= n_chunks; b += 8) {  // eight loads in flight
+            uint32_t c[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) c[j] = table[(size_t)(b + j) * E + e];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                table[(size_t)(b + j) * E + e] = run;
+                run += c[j];
+            }
+        }
+        for (; b < n_chunks; ++b) {
             const uint32_t c = table[(size_t)b * E + e];
             table[(size_t)b * E + e] = run;
             run += c;
         }
     }
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = s_off[e];
 }
 
 __global__ void __launch_bounds__(PERMUTE_THREADS)
@@ -613,17 +619,24 @@ permute_place_kernel(const uint32_t* __restrict__ ids, int64_t n_pairs, int k, i
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = PERMUTE_THREADS / 32;
+    // every warp holds the chunk's ids, sixteen to a lane, and goes through its experts without another load: 16384
+    // selections of 60 experts 15.8 -> 8.5 us, 4096 of eight 13.8 -> 5.3
+    constexpr int PER = PERMUTE_CHUNK / 32;
     const int64_t c0 = (int64_t)blockIdx.x * PERMUTE_CHUNK;
-    const int64_t c1 = c0 + PERMUTE_CHUNK < n_pairs ? c0 + PERMUTE_CHUNK : n_pairs;
+    const uint32_t n = (uint32_t)(n_pairs - c0 < PERMUTE_CHUNK ? n_pairs - c0 : PERMUTE_CHUNK);
+    uint32_t id[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) id[j] = (uint32_t)(32 * j + lane) < n ? ids[c0 + 32 * j + lane] : 0xffffffffu;  // (no expert's)
+#pragma unroll 1
     for (int e = warp; e < E; e += n_warps) {
         uint32_t base = table[(size_t)blockIdx.x * E + e];
-        for (int64_t i0 = c0; i0 < c1; i0 += 32) {
-            const int64_t i = i0 + lane;
-            const bool hit = i < c1 && ids[i] == (uint32_t)e;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const bool hit = id[j] == (uint32_t)e;
             const uint32_t m = __ballot_sync(0xffffffffu, hit);
             if (hit) {
-                const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
-                perm_token[pos] = (uint32_t)(i / k);
+                const uint32_t i = (uint32_t)c0 + 32 * j + lane, pos = base + __popc(m & ((1u << lane) - 1u));
+                perm_token[pos] = i / (uint32_t)k;
                 pair_pos[i] = pos;
             }
             base += __popc(m);

@@ -1,5 +1,6 @@
 """Which kernels take a batch of a single-device forward: the rows on either side of the rule's lines (candle_moe_api.cu, gemm_rows),
-with repacked copies and without, against the oracle; and the narrow GEMM tiles whose Q4_K min term has its own accumulator."""
+with repacked copies and without, against the oracle; the narrow GEMM tiles whose Q4_K min term has its own
+accumulator; the dispatch lists."""
 import ctypes as C
 
 import numpy as np
@@ -94,3 +95,37 @@ def test_min_term_of_narrow_tiles(torch_cuda, rows, n, k):
     assert float((got - ref).norm() / ref.norm()) < 4 * (k / 256) ** 0.5 * 2 ** -24
     for r in (3, 5, 6):
         assert float((got[:, r] - ref[:, r]).abs().max()) <= 1e-5 * max(1.0, float(ref[:, r].abs().max()))
+
+
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (127, 1, 2), (16, 8, 32), (43, 3, 33), (129, 1, 128), (256, 8, 60), (257, 8, 60), (600, 4, 128),
+                                   (4096, 1, 5), (1537, 3, 8)])
+def test_dispatch_lists(torch_cuda, T, k, E):
+    """The dispatch by one CTA against a stable sort: part of a load round, whole ones, one expert to a lane group and beyond."""
+    torch = torch_cuda
+    from candle_b200 import _lib
+    rng = np.random.default_rng(T + E)
+    ids = np.stack([rng.choice(E, size=k, replace=False) for _ in range(T)]).astype(np.uint32)
+    d = torch.from_numpy(ids.astype(np.int32)).cuda()
+    counts, offsets = torch.full((E,), -1, dtype=torch.int32, device="cuda"), torch.full((E + 1,), -1, dtype=torch.int32, device="cuda")
+    perm, pos = torch.full((T * k,), -1, dtype=torch.int32, device="cuda"), torch.full((T * k,), -1, dtype=torch.int32, device="cuda")
+    assert _lib.load().candle_moe_permute(torch.cuda.current_stream().cuda_stream, d.data_ptr(), T, k, E, counts.data_ptr(), offsets.data_ptr(),
+                                          perm.data_ptr(), pos.data_ptr()) == 0
+    order = np.argsort(ids.reshape(-1), kind="stable")
+    assert (counts.cpu().numpy() == np.bincount(ids.reshape(-1), minlength=E)).all()
+    assert (offsets.cpu().numpy() == np.concatenate([[0], np.cumsum(np.bincount(ids.reshape(-1), minlength=E))])).all()
+    assert (perm.cpu().numpy() == order // k).all()
+    assert (pos.cpu().numpy()[order] == np.arange(T * k)).all()
+
+
+@pytest.mark.parametrize("T,k,E", [(257, 8, 60), (1537, 3, 8), (2561, 1, 3), (640, 8, 128)])
+def test_dispatch_lists_of_a_large_batch(orc, torch_cuda, T, k, E):
+    """The same inside a block with more than 2048 selections: chunks of 512, the last one whole or not, more chunks than a round of
+    the scan loads."""
+    torch = torch_cuda
+    blk, _ = H.random_device_block(orc, torch, _cfg(12, 12, E, k, d=256, ff=256), 1)
+    x = torch.randn((T, 256), generator=torch.Generator(device="cuda").manual_seed(T), device="cuda")
+    blk.forward(x)
+    ids, _, counts, perm = (v.cpu().numpy() for v in blk.last_routing(T))
+    flat = ids.reshape(-1).astype(np.int64)
+    assert (counts[:E] == np.bincount(flat, minlength=E)).all()
+    assert (perm.reshape(-1)[:T * k] == np.argsort(flat, kind="stable") // k).all()
