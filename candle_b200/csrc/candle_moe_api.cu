@@ -373,8 +373,8 @@ static cudaError_t gemm_repacking(cudaStream_t st, bool gate_up, const ExpertPtr
 }
 
 // The routed experts over P rows grouped by expert (device offsets [E + 1]); no expert has more than max_rows
-// rows.  Picks, per product, the decode kernels over the repacked copies (max_rows <= 128), the tensor-core GEMM
-// (more than that, scratch present), or the streaming / row forms.  Leaves *eo_splits partial outputs in b.eo.
+// rows.  Picks, per product, the decode kernels over the repacked copies, the tensor-core GEMM
+// (from b.gemm_above rows on, scratch present), or the streaming / row forms.  Leaves *eo_splits partial outputs in b.eo.
 int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs& p1, const ExpertPtrs& p3,
                 const ExpertPtrs& p2, int64_t max_rows, int64_t P, const uint32_t* offsets, const uint32_t* row_of,
                 const int8_t* xq, const float* xs, const int16_t* xb, const ExpertBufs& b, int slots, int* eo_splits,

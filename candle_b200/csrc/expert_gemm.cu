@@ -875,6 +875,8 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                 tmem_ld16(t_main, stg[0]);
                 if constexpr (TWO) tmem_ld16(t_main + PL, sth[0]);
                 tmem_ld_wait();
+                tmem_ld_pin(stg[0]);
+                if constexpr (TWO) tmem_ld_pin(sth[0]);
                 static_for<NS>([&](auto Cc) {
                     constexpr int c = decltype(Cc)::value, s = c & 1;
                     if constexpr (c + 1 < NS) {
@@ -900,7 +902,11 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                                 a = f32x2_fma(f32x2_mul(dw2, d8), main, a);
                         });
                     });
-                    if (c + 1 < NS) tmem_ld_wait();
+                    if constexpr (c + 1 < NS) {
+                        tmem_ld_wait();
+                        tmem_ld_pin(stg[s ^ 1]);
+                        if constexpr (TWO) tmem_ld_pin(sth[s ^ 1]);
+                    }
                     if (c == NS - 2) {  // every column of this thread has been read: the accumulator may be overwritten
                         tc5_fence_before_sync();
                         __syncwarp();

@@ -82,19 +82,6 @@ __device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity, int l
     }
     return false;
 }
-// The same wait for warps that run ahead of their consumer (producers waiting for a free stage): they sleep
-// between polls so that their polling does not take issue slots from the warps that work.  (try_wait with a
-// suspend-time hint is no alternative: it is expanded into exactly such a loop.)
-__device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    for (int i = 0; i < SPIN_LIMIT; ++i) {
-        __nanosleep(100);
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
 // global -> shared bulk copy (16-byte aligned addresses, size a multiple of 16), completion counted
 // in bytes on `bar`.  No multicast.
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -192,9 +179,6 @@ __device__ __forceinline__ uint64_t lds64u(uint32_t addr) {
 // 16-byte asynchronous global -> shared copy (per thread, bypassing L1) and its group fences
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>

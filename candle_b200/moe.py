@@ -105,7 +105,7 @@ class MlpOrMoe:
 
     def prepack(self) -> "MlpOrMoe":
         """Make the optional repacked copies of every expert matrix (one-time, doubles the weight memory of this
-        block): for the decode kernels (batches of up to 96 rows), and Q6_K and Q8_0 in the large-batch GEMM."""
+        block): for the decode kernels (small batches), and Q6_K and Q8_0 in the large-batch GEMM."""
         def copies(mats):
             # every matrix of the family or none: a shape the repack does not take (CANDLE_MOE_E_SHAPE, e.g. Q6_K rows
             # with an odd number of 256-blocks) leaves the family on its GGUF blocks
