@@ -1223,19 +1223,25 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
         const uint64_t b_desc = umma_desc_sw128(smem_u32(smem));
         const uint64_t mb_desc = C::MIN_ACC ? umma_desc_sw32(smem_u32(smem_min_b)) : umma_desc_sw64(smem_u32(smem_min_b));
         const uint64_t ma_desc = C::MIN_ACC ? umma_desc_sw32(smem_u32(smem_min_a)) : umma_desc_sw64(smem_u32(smem_min_a));
-        const auto block = [&](auto Bc) {  // block 2 it + B of this CTA
+        // The whole warp's answer: after a wait that gave up, on whichever lane, it leaves its loop, and no MMA or commit is issued.
+        // (known: the answer to a barrier asked ahead, looked at here, after it has had its time)
+        const auto wait = [&](bool known, uint64_t* bar, uint32_t parity) {
+            return (bool)__all_sync(0xffffffffu, known || mbar_wait_tight(bar, parity, abort_flag));
+        };
+        const auto block = [&](auto Bc) {  // block 2 it + B of this CTA; false: a wait gave up
             constexpr int B = decltype(Bc)::value, R = C::RING;
 #pragma unroll
             for (int ps = 0; ps < C::PASSES; ++ps) {
                 const int buf = C::PASSES == 2 ? ps : B;
                 // the drain of what this accumulator held last: block ab - 2, with two passes ab - 1
-                if (C::PASSES == 2 ? it > 0 || B > 0 : it > 0 && !free_n)
-                    mbar_wait_tight(&acc_free[buf], C::PASSES == 2 ? (B & 1) ^ 1 : (it & 1) ^ 1, abort_flag);
+                if (C::PASSES == 2 ? it > 0 || B > 0 : it > 0) {
+                    if (!wait(free_n, &acc_free[buf], C::PASSES == 2 ? (B & 1) ^ 1 : (it & 1) ^ 1)) return false;
+                }
                 const uint32_t d_main = tmem_base + buf * C::ACC_COLS;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int st = (2 * B + h) % R;
-                    if (ps == 0 && !full_n) mbar_wait_tight(&full_p[st], R == 4 ? it & 1 : B & 1, abort_flag);
+                    if (ps == 0 && !wait(full_n, &full_p[st], R == 4 ? it & 1 : B & 1)) return false;
                     tc5_fence_after_sync();
                     if constexpr (C::PASSES == 1 && TN == 128) {
                         // ask the next barriers now: the answers, 200 to 300 clocks away, arrive while the MMAs are issued (gate_up of
@@ -1295,8 +1301,8 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
                     __syncwarp();
                 }
             }
+            return true;
         };
-        // (after a wait that gave up, the rest of the tile is issued all the same: the lanes stay together)
         while (!__any_sync(0xffffffffu, *abort_flag) && walk.next(tc)) {
             uint32_t left = walk.blocks;
             // The last position tile of an expert is rarely full: its MMAs run N = the rows it holds, rounded up to 16
@@ -1314,15 +1320,16 @@ expert_gemm_kernel(const __grid_constant__ GemmParams P, const __grid_constant__
 #pragma unroll 1
             for (;;) {
                 second = true;
-                block(std::integral_constant<int, 0>{});
+                if (!block(std::integral_constant<int, 0>{})) goto mma_end;
                 if (--left == 0) break;
             mma_second:
                 second = false;
-                block(std::integral_constant<int, 1>{});
+                if (!block(std::integral_constant<int, 1>{})) goto mma_end;
                 ++it;
                 if (--left == 0) break;
             }
         }
+    mma_end:;
     }
     tc5_fence_before_sync();
     __syncthreads();
