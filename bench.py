@@ -499,6 +499,7 @@ def run_ours(args, cfg):
     from candle_b200 import _lib as _cm
     gmin = C.c_int64(96)
     _cm.load().candle_moe_get_tuning(_cm.TUNE_GEMM_MIN_ROWS, C.byref(gmin))
+    gmin.value = 96 if gmin.value == _cm.GEMM_ROWS_AUTO else gmin.value
     if T > gmin.value:
         # large batches run tensor-core grouped products: the bound is the tensor pipe.  Algorithmic flops of the
         # dominant product (the second multiply of every Q6_K slab is not counted).

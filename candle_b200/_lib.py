@@ -28,6 +28,7 @@ ERROR_NAMES = {
 
 # candle_moe_set_tuning keys
 TUNE_GEMM_ENABLED, TUNE_GEMM_MIN_ROWS, TUNE_STREAM_MAX_ROWS, TUNE_FORCE_ROWS, TUNE_MID_ENABLED = range(5)
+GEMM_ROWS_AUTO = -2 ** 63  # value of TUNE_GEMM_MIN_ROWS unless it is set
 
 
 class CandleMoeError(RuntimeError):

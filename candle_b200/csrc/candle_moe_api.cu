@@ -13,9 +13,10 @@ using namespace cmoe;
 namespace {
 
 // Rows per step above which the tensor-core GEMM takes the products (below, the decode kernels).  The tuning key GEMM_MIN_ROWS
-// sets them; at its default (96) a single-device forward over repacked copies goes by the rows that an expert holds on average,
+// sets them; left to itself it stands for 96, and a single-device forward goes by the rows that an expert holds on average,
 // k T / E, because the decode kernels pay for every eight of them and the GEMM hardly at all (gemm_rows below).
-inline int64_t gemm_min_rows() { return tuning_get(TUNE_GEMM_MIN_ROWS); }
+inline bool gemm_rows_auto() { return tuning_get(TUNE_GEMM_MIN_ROWS) == CANDLE_MOE_GEMM_ROWS_AUTO; }
+inline int64_t gemm_min_rows() { return gemm_rows_auto() ? 96 : tuning_get(TUNE_GEMM_MIN_ROWS); }
 // When the caller knows the ACTUAL largest row count of an expert (or, in the slot form of expert parallelism, a
 // bound five quarters of the expected one, so that the tile width leaves a margin), the GEMM takes over above 32 rows.
 // Measured on one GPU with the experts of one rank of the Mixtral-shaped layer (decode kernels / GEMM, microseconds
@@ -40,7 +41,7 @@ constexpr int64_t QMM_GEMM_MIN_ROWS = 48;  // the dense product: one matrix, row
 // Only where an expert's rows are expected in a narrow tile, whose gate is as exact as that of the forms before.
 inline int64_t gemm_rows(const candle_moe_weights_t* w) {
     const int64_t rows = gemm_min_rows(), E = w->n_experts, k = w->top_k;
-    if (rows != TUNE_GEMM_MIN_ROWS_DEFAULT) return rows;
+    if (!gemm_rows_auto()) return rows;
     const bool q80_13 = w->dtype_w13 == CANDLE_GGML_Q8_0, q80_2 = w->dtype_w2 == CANDLE_GGML_Q8_0;
     const bool copies = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked;
     if (copies && q80_13 && q80_2) return std::max(rows, std::min<int64_t>(22 * E / k, 512));  // (not measured beyond)

@@ -144,7 +144,6 @@ enum TuningKey {
     TUNE_MID_ENABLED = CANDLE_MOE_TUNE_MID_ENABLED,
     TUNE_N_KEYS
 };
-constexpr int64_t TUNE_GEMM_MIN_ROWS_DEFAULT = 96;
 int64_t tuning_get(int key);
 bool tuning_set(int key, int64_t value);  // false: unknown key
 

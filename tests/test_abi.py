@@ -152,6 +152,31 @@ def test_tuning_switches_round_trip(lib):
     assert L.candle_moe_set_tuning(99, 1) == -2 and L.candle_moe_get_tuning(99, C.byref(v)) == -2
 
 
+def test_every_line_of_the_gemm_can_be_chosen(lib):
+    """96 rows, the line of everything that does not go by the rows of an expert, is a fixed line like any other when it is
+    set: a layer over copies then has no GEMM scratch at 90 rows, and has it again when the value found before is put back."""
+    L, out, v = lib.load(), C.c_size_t(0), C.c_int64(-1)
+    some = (C.c_void_p * 8)(*[4096] * 8)
+    w = _weights(lib, w1_prepacked=some, w3_prepacked=some, w2_prepacked=some)
+
+    def size(T):
+        assert L.candle_moe_workspace_bytes(C.byref(w), T, C.byref(out)) == 0
+        return out.value
+
+    auto = size(90)
+    assert L.candle_moe_get_tuning(lib.TUNE_GEMM_MIN_ROWS, C.byref(v)) == 0
+    old = v.value
+    try:
+        sizes = {}
+        for line in (95, 96, 97):
+            assert L.candle_moe_set_tuning(lib.TUNE_GEMM_MIN_ROWS, line) == 0
+            sizes[line] = size(90)
+        assert sizes[95] == sizes[96] == sizes[97] < auto
+    finally:
+        assert L.candle_moe_set_tuning(lib.TUNE_GEMM_MIN_ROWS, old) == 0
+    assert size(90) == auto
+
+
 def _ep_cfg(lib, **kw):
     cfg = lib.EpConfigC()
     cfg.rank, cfg.world, cfg.n_experts_global, cfg.top_k, cfg.renorm, cfg.max_tokens = 0, 2, 8, 2, 1, 32
