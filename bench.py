@@ -364,13 +364,21 @@ def parity_vs_oracle(orc, mw, x_rows, y_rows, ids_rows):
             "bounds": {"rel_l2": 1e-3, "max_rel": 2e-3}}
 
 
-def block_launches(cfg, T, prepacked, gemm_min_rows):
+def gemm_rows(weights):
+    """Rows above which a forward over these weights (candle_moe_weights_t) takes the tensor-core GEMM."""
+    from candle_b200 import _lib
+    rows = C.c_int64(0)
+    _lib.check("candle_moe_forward_gemm_rows", _lib.load().candle_moe_forward_gemm_rows(C.byref(weights), C.byref(rows)))
+    return rows.value
+
+
+def block_launches(cfg, T, prepacked, weights):
     """Kernels one forward of the block launches (the library's own, counted from its launch sequence)."""
     q8 = cfg["dt13"] == 8
     pairs = T * cfg["k"]
     n = 1 + (0 if T == 1 else (3 if pairs > 2048 else 1)) + (1 if q8 else 0)  # router (+ x quantization fused unless Q8_0), dispatch
     maps = lambda E: (2 * E + 15) // 16 - 1                                    # tensor-map copies beyond the 16 of the preparation
-    gemm = T > gemm_min_rows
+    gemm = T > gemm_rows(weights)
     def product(dt, E, takes_gemm):
         if gemm and takes_gemm:
             return 1 + (maps(E) if dt == 12 else 0) + 1                         # operand preparation, maps, GEMM
@@ -496,11 +504,7 @@ def run_ours(args, cfg):
             "frac": ach / peak, "traffic": NCU_TRAFFIC_BYTES.get((args.workload, T, top)),
             "peak_source": f"{peak_kind} copy bandwidth",
             "algorithmic_bytes_per_launch": top_bytes, "kernel_ms": stage_ms[top]}
-    from candle_b200 import _lib as _cm
-    gmin = C.c_int64(96)
-    _cm.load().candle_moe_get_tuning(_cm.TUNE_GEMM_MIN_ROWS, C.byref(gmin))
-    gmin.value = 96 if gmin.value == _cm.GEMM_ROWS_AUTO else gmin.value
-    if T > gmin.value:
+    if T > gemm_rows(blk._cw):
         # large batches run tensor-core grouped products: the bound is the tensor pipe.  Algorithmic flops of the
         # dominant product (the second multiply of every Q6_K slab is not counted).
         flops = 2.0 * T * cfg["k"] * d * cfg["ff"] * (2 if top == "gate_up" else 1)
@@ -525,7 +529,7 @@ def run_ours(args, cfg):
         "e2e": {"value": T * world / (ms_e2e / args.steps * 1e-3), "unit": "tokens/s",
                 "h2d_bytes_per_step": T * d * 4, "d2h_bytes_per_step": T * d * 4,
                 "ms_per_step": ms_e2e / args.steps},
-        "gpu_launches": block_launches(cfg, T, not args.no_prepack, gmin.value) * args.steps,
+        "gpu_launches": block_launches(cfg, T, not args.no_prepack, blk._cw) * args.steps,
         "clocks": clocks,
     }
     print(json.dumps(line))

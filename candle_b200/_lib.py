@@ -74,6 +74,7 @@ SYMBOLS = {
     "candle_moe_set_tuning": (C.c_int, [C.c_int32, C.c_int64]),
     "candle_moe_get_tuning": (C.c_int, [C.c_int32, C.POINTER(C.c_int64)]),
     "candle_moe_workspace_bytes": (C.c_int, [C.POINTER(MoeWeightsC), _I64, C.POINTER(_SZ)]),
+    "candle_moe_forward_gemm_rows": (C.c_int, [C.POINTER(MoeWeightsC), C.POINTER(_I64)]),
     "candle_moe_router_topk": (C.c_int, [_P, _P, _P, _P, _I64, _I32, _I32, _I32, _I32, _P, _P]),
     "candle_moe_permute": (C.c_int, [_P, _P, _I64, _I32, _I32, _P, _P, _P, _P]),
     "candle_moe_quantize_act": (C.c_int, [_P, _P, _I64, _I32, _I32, _P, _P, _P]),

@@ -277,6 +277,13 @@ int candle_moe_workspace_bytes(const candle_moe_weights_t* w, int64_t max_tokens
     return CANDLE_MOE_OK;
 }
 
+int candle_moe_forward_gemm_rows(const candle_moe_weights_t* w, int64_t* out_rows) {
+    if (!out_rows) return CANDLE_MOE_E_NULL;
+    CM_TRY(check_weights(w));
+    *out_rows = gemm_enabled() ? gemm_rows(w) : INT64_MAX;
+    return CANDLE_MOE_OK;
+}
+
 int candle_moe_router_topk(void* stream, const float* x, const float* router, const float* bias, int64_t T,
                            int32_t d, int32_t E, int32_t k, int32_t renorm, uint32_t* topk_ids, float* topk_w) {
     if (!x || !router || !topk_ids || !topk_w) return CANDLE_MOE_E_NULL;

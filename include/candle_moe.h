@@ -122,6 +122,11 @@ CANDLE_MOE_API const char* candle_moe_version(void);
  * 321 and the zeros_like/index_add copies of quantized_llama.rs:184,202). */
 CANDLE_MOE_API int candle_moe_workspace_bytes(const candle_moe_weights_t* w, int64_t max_tokens, size_t* out_bytes);
 
+/* The number of rows above which candle_moe_forward takes the tensor-core GEMM for these weights, where their formats and
+ * layouts allow it and the workspace is one of candle_moe_workspace_bytes; up to it the decode kernels over repacked copies or the
+ * streaming form run.  INT64_MAX where CANDLE_MOE_TUNE_GEMM_ENABLED is 0.  Host only; the tables' entries are not read. */
+CANDLE_MOE_API int candle_moe_forward_gemm_rows(const candle_moe_weights_t* w, int64_t* out_rows);
+
 /* Router: logits = x . Wg^T (+ bias), softmax over all experts, stable descending top-k (ties keep
  * the lower expert id), optional renormalisation.  Replaces quantized_llama.rs:153-179
  * (QMatMul::forward on the f32 gate, candle_nn::ops::softmax_last_dim, the host-side sort).

@@ -152,6 +152,29 @@ def test_tuning_switches_round_trip(lib):
     assert L.candle_moe_set_tuning(99, 1) == -2 and L.candle_moe_get_tuning(99, C.byref(v)) == -2
 
 
+def test_the_benchmark_counts_the_kernels_of_the_form_that_runs(lib):
+    """Launches of a layer on either side of the rows from which the GEMM takes it, which the library names."""
+    import bench
+    L, some = lib.load(), (C.c_void_p * 8)(*[4096] * 8)
+    rows = C.c_int64(0)
+    cfg = {"dt13": 12, "dt2": 14, "E": 8, "k": 2, "ff_shared": 0}
+    w = _weights(lib, w1_prepacked=some, w3_prepacked=some, w2_prepacked=some)
+    assert L.candle_moe_forward_gemm_rows(C.byref(w), C.byref(rows)) == 0 and 32 < rows.value < 96
+    # router, dispatch, gate_up, quantizer, down, combine; with the GEMM two preparations in place of the quantizer
+    assert bench.block_launches(cfg, rows.value, True, w) == 6
+    assert bench.block_launches(cfg, rows.value + 1, True, w) == 7
+    assert bench.block_launches(cfg, 1, True, w) == 5
+    old = C.c_int64(0)
+    assert L.candle_moe_get_tuning(lib.TUNE_GEMM_ENABLED, C.byref(old)) == 0
+    try:
+        assert L.candle_moe_set_tuning(lib.TUNE_GEMM_ENABLED, 0) == 0
+        assert bench.block_launches(cfg, rows.value + 1, True, w) == 6
+    finally:
+        assert L.candle_moe_set_tuning(lib.TUNE_GEMM_ENABLED, old.value) == 0
+    assert L.candle_moe_forward_gemm_rows(C.byref(_weights(lib, top_k=9)), C.byref(rows)) == -2
+    assert L.candle_moe_forward_gemm_rows(C.byref(w), None) == -1
+
+
 def test_every_line_of_the_gemm_can_be_chosen(lib):
     """96 rows, the line of everything that does not go by the rows of an expert, is a fixed line like any other when it is
     set: a layer over copies then has no GEMM scratch at 90 rows, and has it again when the value found before is put back."""
