@@ -390,7 +390,8 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     if (total_rows_hint <= 0) total_rows_hint = P;
     const int E = w->n_experts, d = w->d_model, ff = w->d_ff;
     const int64_t gemm_above = b.gemm_above >= 0 ? b.gemm_above : gemm_min_rows();
-    const bool large = b.gemm && max_rows > (rows_exact ? GEMM_MIN_ROWS_EXACT : gemm_above) && gemm_enabled();
+    const bool gemm_here = b.gemm && gemm_enabled();
+    bool large = gemm_here && max_rows > (rows_exact ? GEMM_MIN_ROWS_EXACT : gemm_above);
     bool use_prepacked = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked &&
                          max_rows <= std::max<int64_t>({gemm_min_rows(), gemm_above, 64}) && !large;
     bool gate_done = false, down_done = false;
@@ -404,6 +405,11 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
         if (st_copies != CANDLE_MOE_OK && w->dtype_w13 != CANDLE_GGML_Q8_0 && w->dtype_w2 != CANDLE_GGML_Q8_0) return st_copies;
         use_prepacked = st_copies == CANDLE_MOE_OK;
     }
+    // More than gemm_min_rows() rows that the line leaves to the decode kernels: the GEMM takes what they refuse -- rows too long for
+    // their shared memory (Q8_0 gate_up from d = 5120 on, down from K = 20480), tables that are no use to them.  (16 experts of 5120 x
+    // 1536, top-1, 128 rows: 126 us that way, 320 on the tile kernel over the GGUF blocks.)
+    const bool gemm_second = gemm_here && !large && use_prepacked && max_rows > gemm_min_rows();
+    if (gemm_here && !use_prepacked && max_rows > gemm_min_rows()) large = true;
     if (use_prepacked) {
         cudaError_t ce = cudaErrorNotSupported;
         const SharedGroup* const tries[2] = {shared ? &shared->gate : nullptr, nullptr};  // with the shared expert, or without
@@ -421,7 +427,7 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     // Position-tile width of the GEMM: from the actual largest row count when it is known, else from five quarters
     // of the average (an expert beyond the tile width simply takes a second tile)
     const int64_t tile_rows = rows_exact ? max_rows : std::min<int64_t>(max_rows, (5 * total_rows_hint + 4 * E - 1) / (4 * E));
-    if (!gate_done && large) {
+    if (!gate_done && (large || gemm_second)) {
         // Q6_K and Q8_0 are read from the repacked copies (their GGUF blocks are only 2-byte aligned)
         const bool rp = (w->dtype_w13 == CANDLE_GGML_Q6K || w->dtype_w13 == CANDLE_GGML_Q8_0) && w->w1_prepacked && w->w3_prepacked;
         ExpertPtrs g1 = p1, g3 = p3;
@@ -471,7 +477,7 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
         else
             *eo_splits = 1;
     }
-    if (!down_done && large) {
+    if (!down_done && (large || gemm_second)) {
         ExpertPtrs g2 = p2;
         if (rp2) CM_TRY(fill_ptrs(w->w2_prepacked, E, g2));
         const cudaError_t ce = repack2 ? gemm_repacking(st, false, p2, p2, E, ff, d, offsets, nullptr, P, tile_rows, b.hq, b.hs, b.hb, b.eo, b,
@@ -598,15 +604,18 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
         if (ws.sxq != ws.xq)
             CM_TRY(rc(launch_quantize_act(st, x, T, d, w->dtype_shared13, ws.sxq, ws.sxs, ws.sxb)));
         bool sh_done = sr.gate_done;
+        const bool sh_second = sh_direct && ws.gemm && T > gemm_min_rows() && gemm_enabled();  // as gemm_second in run_experts
         if (!sh_done && (sh_gemm || sh_direct)) {
             ExpertPtrs r1{}, r3{};
             r1.p[0] = static_cast<const uint8_t*>(w->shared_w1_prepacked);
             r3.p[0] = static_cast<const uint8_t*>(w->shared_w3_prepacked);
-            const cudaError_t ce =
-                sh_gemm ? launch_expert_gemm(st, true, r1, r3, CANDLE_GGML_Q8_0, true, 1, d, fs, ws.sh_offsets, nullptr, T, T, ws.sxq,
-                                             ws.sxs, ws.sxb, ws.shidden, ws.gemm)
-                        : launch_expert_direct(st, true, r1, r3, CANDLE_GGML_Q8_0, 1, d, fs, ws.sh_offsets, nullptr, T, ws.sxq, ws.sxs,
-                                               ws.sxb, ws.shidden, nullptr, 0, 1, 0, T);
+            cudaError_t ce = cudaErrorNotSupported;
+            if (sh_direct)
+                ce = launch_expert_direct(st, true, r1, r3, CANDLE_GGML_Q8_0, 1, d, fs, ws.sh_offsets, nullptr, T, ws.sxq, ws.sxs, ws.sxb,
+                                          ws.shidden, nullptr, 0, 1, 0, T);
+            if (ce == cudaErrorNotSupported && (sh_gemm || sh_second))
+                ce = launch_expert_gemm(st, true, r1, r3, CANDLE_GGML_Q8_0, true, 1, d, fs, ws.sh_offsets, nullptr, T, T, ws.sxq, ws.sxs,
+                                        ws.sxb, ws.shidden, ws.gemm);
             if (ce == cudaSuccess)
                 sh_done = true;
             else if (ce != cudaErrorNotSupported)
@@ -621,12 +630,14 @@ static int forward_impl(void* stream, const candle_moe_weights_t* w, const float
         if (!sh_done && (sh_gemm || sh_direct)) {
             ExpertPtrs r2{};
             r2.p[0] = static_cast<const uint8_t*>(w->shared_w2_prepacked);
-            const cudaError_t ce =
-                sh_gemm ? launch_expert_gemm(st, false, r2, r2, CANDLE_GGML_Q8_0, true, 1, fs, d, ws.sh_offsets, nullptr, T, T, ws.shq,
-                                             ws.shs, ws.shb, ws.so, ws.gemm, k_split_slots(T), &so_splits, T * (int64_t)d, nullptr,
-                                             fuse_sh ? ws.shidden : nullptr)
-                        : launch_expert_direct(st, false, r2, r2, CANDLE_GGML_Q8_0, 1, fs, d, ws.sh_offsets, nullptr, T, ws.shq,
-                                               ws.shs, ws.shb, ws.so, &so_splits, T * (int64_t)d, k_split_slots(T), 1, T);
+            cudaError_t ce = cudaErrorNotSupported;
+            if (sh_direct)
+                ce = launch_expert_direct(st, false, r2, r2, CANDLE_GGML_Q8_0, 1, fs, d, ws.sh_offsets, nullptr, T, ws.shq, ws.shs,
+                                          ws.shb, ws.so, &so_splits, T * (int64_t)d, k_split_slots(T), 1, T);
+            if (ce == cudaErrorNotSupported && (sh_gemm || sh_second))
+                ce = launch_expert_gemm(st, false, r2, r2, CANDLE_GGML_Q8_0, true, 1, fs, d, ws.sh_offsets, nullptr, T, T, ws.shq, ws.shs,
+                                        ws.shb, ws.so, ws.gemm, k_split_slots(T), &so_splits, T * (int64_t)d, nullptr,
+                                        fuse_sh ? ws.shidden : nullptr);
             if (ce == cudaSuccess)
                 sh_done = true;
             else if (ce != cudaErrorNotSupported || fuse_sh)

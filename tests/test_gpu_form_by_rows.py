@@ -129,3 +129,30 @@ def test_dispatch_lists_of_a_large_batch(orc, torch_cuda, T, k, E):
     flat = ids.reshape(-1).astype(np.int64)
     assert (counts[:E] == np.bincount(flat, minlength=E)).all()
     assert (perm.reshape(-1)[:T * k] == np.argsort(flat, kind="stable") // k).all()
+
+
+def _tuned(key, value, fn):
+    """fn() with a kernel-selection switch set"""
+    from candle_b200 import _lib
+    L, old = _lib.load(), C.c_int64(0)
+    assert L.candle_moe_get_tuning(key, C.byref(old)) == 0 and L.candle_moe_set_tuning(key, value) == 0
+    try:
+        return fn()
+    finally:
+        assert L.candle_moe_set_tuning(key, old.value) == 0
+
+
+@pytest.mark.parametrize("cfg,T", [
+    (_cfg(8, 8, 8, 1, d=5120, ff=1024), 100),         # gate_up: sixteen rows of 5120 and the rings are more than shared memory
+    (_cfg(8, 8, 8, 1, d=512, ff=1024, fs=20480), 100),  # the shared expert's down product, four splits of 5120
+])
+def test_products_that_the_decode_kernels_refuse_go_to_the_gemm(orc, torch_cuda, cfg, T):
+    """Q8_0 batches above 96 rows which the line leaves to the decode kernels: without the GEMM the refused product is the tile kernel's
+    over the GGUF blocks, whose sums run in another order."""
+    from candle_b200 import _lib
+    blk, x, y = _check(orc, torch_cuda, cfg, T, True)
+    rows = C.c_int64(0)
+    assert _lib.load().candle_moe_forward_gemm_rows(C.byref(blk._cw), C.byref(rows)) == 0 and rows.value >= T
+    tiles = _tuned(_lib.TUNE_GEMM_ENABLED, 0, lambda: blk.forward(x).clone())
+    assert not torch_cuda.equal(y, tiles)
+    assert H.rel_l2(y.cpu().numpy(), tiles.cpu().numpy()) <= H.REL_L2_TOL
