@@ -31,10 +31,29 @@ constexpr int64_t GEMM_MIN_ROWS_EXACT = 32;
 // faster in all of 300 sizes from 1024 to 32000 by 512 to 4096).  Every sixteen rows are one more pass over the copy.
 constexpr int64_t QMM_DIRECT_MAX_ROWS = 64;
 constexpr int64_t QMM_GEMM_MIN_ROWS = 48;  // the dense product: one matrix, rows known exactly
+// The line for Q8_0 over repacked copies, from estimated times of both forms in microseconds: the GEMM costs .33 more per expert and .065
+// less per million routed weights saved (W), the decode kernels .009 W more for every row of an expert beyond eight; a shared expert, whose
+// group holds every row, joins the decode kernels' launches (14 us of launches and .6 per million of its weights, S, saved) and costs them
+// .006 S more per row.  Fitted to 330 sizes (8 to 128 experts, top-1 to top-8, d = 1024 to 4096, ff = 512 to 4096, with and without a
+// shared expert of 2816 to 5632, 97 to 512 rows): 0.3 % slower than the better form on average, at worst 11 %.  Decode kernels / GEMM --
+// 60 experts of 2048 x 1408, top-2: 160 rows 172 / 189, 352 192 / 196, 512 260 / 229; with a shared expert of 5632: 160 rows 220 / 254, 272
+// 263 / 259, 512 406 / 302; 32 experts, top-2, and that shared expert: 97 rows 147 / 161, 192 183 / 180, 352 273 / 193; 128 experts of
+// 2048 x 768, top-8: 97 rows 258 / 267, 160 279 / 275, 352 376 / 279; 16 experts of 1024 x 1024, top-2: 97 rows 54 / 46.  (By 22 rows of an expert
+// alone, with a shared expert or not: 7 % slower than the better form on average, at worst 46 %.)
+inline int64_t gemm_rows_q80(const candle_moe_weights_t* w, int64_t rows) {
+    const double E = w->n_experts, k = w->top_k, W = 3e-6 * E * w->d_model * w->d_ff;
+    const double S = w->d_ff_shared > 0 && w->dtype_shared13 == CANDLE_GGML_Q8_0 && w->dtype_shared2 == CANDLE_GGML_Q8_0 && w->shared_w1_prepacked &&
+                             w->shared_w3_prepacked && w->shared_w2_prepacked
+                         ? 3e-6 * w->d_model * w->d_ff_shared
+                         : 0.0;
+    const double gain = 0.065 * W - 0.33 * E + (S > 0 ? 14.0 + 0.6 * S : 0.0);
+    const double eight = 8.0 * E / k, per_row = 0.009 * W * k / E, per_shared_row = 0.006 * S;
+    const double line = gain <= per_shared_row * eight ? (S > 0 ? gain / per_shared_row : 0.0) : (gain + per_row * eight) / (per_row + per_shared_row);
+    return std::max(rows, (int64_t)std::min(line, 512.0));  // (not measured beyond)
+}
 // Measured, decode kernels / GEMM, us per block.  Mixtral-shaped (8 experts, top-2): T = 32 217 / 277, 48 261 / 282, 56 283 / 276, 64 300 /
 // 281, 96 385 / 294; all Q4_K: 48 232 / 241, 56 249 / 241; d = 2048, ff = 8192: 48 105 / 115, 64 119 / 114; d = ff = 4096, Q6_K: 16 138 / 136,
-// 48 171 / 138.  Q8_0 with a shared expert: 60 experts, top-4: 100 205 / 296, 256 299 / 323, 384 401 / 358; 16 experts, top-2: 192 166 / 169,
-// 256 202 / 178; 32 experts, top-4: 128 175 / 209, 192 228 / 228, 256 269 / 233.
+// 48 171 / 138.
 // Without copies, streaming form / GEMM for Q4_K (Q6_K products stay where they are): d = ff = 4096: 8 91 / 100, 12 111 / 100, 16 112 / 101,
 // 96 228 / 107; d = 2048, ff = 8192: 8 110 / 98, 32 153 / 99; d = 1024, ff = 3584: 8 56 / 44, 64 102 / 50; Mixtral-shaped with a Q6_K down
 // product: 8 283 / 277, 32 412 / 342, 96 793 / 503.
@@ -44,7 +63,7 @@ inline int64_t gemm_rows(const candle_moe_weights_t* w) {
     if (!gemm_rows_auto()) return rows;
     const bool q80_13 = w->dtype_w13 == CANDLE_GGML_Q8_0, q80_2 = w->dtype_w2 == CANDLE_GGML_Q8_0;
     const bool copies = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked;
-    if (copies && q80_13 && q80_2) return std::max(rows, std::min<int64_t>(22 * E / k, 512));  // (not measured beyond)
+    if (copies && q80_13 && q80_2) return gemm_rows_q80(w, rows);
     if (q80_13 || q80_2 || 5 * k * rows > 4 * 64 * E) return rows;
     if (copies) return std::min(rows, 12 * E / k);
     return w->dtype_w13 == CANDLE_GGML_Q4K ? std::min(rows, 5 * E / (2 * k)) : rows;

@@ -175,6 +175,30 @@ def test_the_benchmark_counts_the_kernels_of_the_form_that_runs(lib):
     assert L.candle_moe_forward_gemm_rows(C.byref(w), None) == -1
 
 
+def _line(lib, E, k, d, ff, dt13, dt2, copies=True, fs=0):
+    """rows above which the GEMM takes a layer"""
+    some = (C.c_void_p * E)(*[4096] * E)
+    w = _weights(lib, n_experts=E, top_k=k, d_model=d, d_ff=ff, dtype_w13=dt13, dtype_w2=dt2)
+    if copies:
+        w.w1_prepacked = w.w3_prepacked = w.w2_prepacked = some
+    if fs:
+        w.d_ff_shared, w.dtype_shared13, w.dtype_shared2 = fs, 8, 8
+        w.shared_w1_prepacked = w.shared_w3_prepacked = w.shared_w2_prepacked = 4096
+    rows = C.c_int64(0)
+    assert lib.load().candle_moe_forward_gemm_rows(C.byref(w), C.byref(rows)) == 0
+    return rows.value
+
+
+# rows that were measured faster on the decode kernels, and on the GEMM
+@pytest.mark.parametrize("E,k,d,ff,fs,decode,gemm", [
+    (60, 4, 2048, 1408, 5632, 160, 224), (60, 2, 2048, 1408, 5632, 224, 352), (60, 2, 2048, 1408, 0, 272, 448), (32, 2, 2048, 1408, 5632, 144, 224),
+    (32, 2, 2048, 1408, 0, 160, 224), (16, 1, 2048, 1408, 5632, 144, 192), (16, 2, 4096, 4096, 0, 96, 128), (16, 1, 4096, 4096, 0, 192, 272),
+    (64, 8, 3584, 2560, 0, 97, 128), (128, 8, 2048, 768, 2816, 128, 192), (128, 1, 1024, 1024, 4096, 96, 272), (32, 4, 1024, 1024, 0, 96, 112),
+])
+def test_line_of_q80_layers(lib, E, k, d, ff, fs, decode, gemm):
+    assert decode <= _line(lib, E, k, d, ff, 8, 8, fs=fs) < gemm
+
+
 def test_every_line_of_the_gemm_can_be_chosen(lib):
     """96 rows, the line of everything that does not go by the rows of an expert, is a fixed line like any other when it is
     set: a layer over copies then has no GEMM scratch at 90 rows, and has it again when the value found before is put back."""
