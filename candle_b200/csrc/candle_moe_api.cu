@@ -51,9 +51,21 @@ inline int64_t gemm_rows_q80(const candle_moe_weights_t* w, int64_t rows) {
     const double line = gain <= per_shared_row * eight ? (S > 0 ? gain / per_shared_row : 0.0) : (gain + per_row * eight) / (per_row + per_shared_row);
     return std::max(rows, (int64_t)std::min(line, 512.0));  // (not measured beyond)
 }
-// Measured, decode kernels / GEMM, us per block.  Mixtral-shaped (8 experts, top-2): T = 32 217 / 277, 48 261 / 282, 56 283 / 276, 64 300 /
-// 281, 96 385 / 294; all Q4_K: 48 232 / 241, 56 249 / 241; d = 2048, ff = 8192: 48 105 / 115, 64 119 / 114; d = ff = 4096, Q6_K: 16 138 / 136,
-// 48 171 / 138.
+// Rows of an expert above which k-quant products over repacked copies take the GEMM: where both forms cross, which is later for layers
+// of many weights (the GEMM's time per block is the same, the decode kernels gain on longer items) and for Q6_K down products (1.2 us a
+// block of the GEMM instead of 0.7).  Decode kernels / GEMM, us per layer, w13 / w2.  8 experts, top-2 -- 4096 x 14336, Q4_K / Q6_K: 48 rows
+// 242 / 287, 58 266 / 296, 64 310 / 302, 72 330 / 302; Q4_K / Q4_K: 52 230 / 252, 60 260 / 253; 2560 x 6144, Q4_K / Q6_K: 50 103 / 117, 60 109 /
+// 113, 64 114 / 111; Q6_K / Q6_K: 50 120 / 129, 60 134 / 129; 1024 x 3584, Q4_K / Q6_K: 52 52 / 56, 60 57 / 56; Q4_K / Q4_K: 48 51 / 50, 60 54 / 52.
+// 4 experts of 4096 x 14336, top-2, Q4_K / Q6_K: 25 rows 138 / 176, 32 182 / 170.  60 of 2048 x 1536, top-8: 96 rows 191 / 210.  16 of 2048 x
+// 1024, top-4: 48 rows 62 / 59; 32 of them, top-8: 48 90 / 92, 57 97 / 93.  Twelve for all of them, as before, cost 3 to 25 % between the lines.
+// Q6_K rows of 4096 and more are too long for the decode kernels' gate_up with two position tiles: 4096 x 14336: 48 rows 477 / 352.
+inline int64_t gemm_expert_rows(const candle_moe_weights_t* w) {
+    const bool q6_13 = w->dtype_w13 == CANDLE_GGML_Q6K, q6_2 = w->dtype_w2 == CANDLE_GGML_Q6K;
+    if (!expert_direct_takes_gate_up(w->dtype_w13, w->d_model)) return 12;
+    const double millions = 3e-6 * w->n_experts * w->d_model * w->d_ff;
+    if (millions >= 350.0) return q6_13 && q6_2 ? 14 : 15;
+    return w->n_experts > 8 ? 12 : (q6_2 ? 14 : 13);
+}
 // Without copies, streaming form / GEMM for Q4_K (Q6_K products stay where they are): d = ff = 4096: 8 91 / 100, 12 111 / 100, 16 112 / 101,
 // 96 228 / 107; d = 2048, ff = 8192: 8 110 / 98, 32 153 / 99; d = 1024, ff = 3584: 8 56 / 44, 64 102 / 50; Mixtral-shaped with a Q6_K down
 // product: 8 283 / 277, 32 412 / 342, 96 793 / 503.
@@ -65,7 +77,7 @@ inline int64_t gemm_rows(const candle_moe_weights_t* w) {
     const bool copies = w->w1_prepacked && w->w3_prepacked && w->w2_prepacked;
     if (copies && q80_13 && q80_2) return gemm_rows_q80(w, rows);
     if (q80_13 || q80_2 || 5 * k * rows > 4 * 64 * E) return rows;
-    if (copies) return std::min(rows, 12 * E / k);
+    if (copies) return std::min(rows, gemm_expert_rows(w) * E / k);
     return w->dtype_w13 == CANDLE_GGML_Q4K ? std::min(rows, 5 * E / (2 * k)) : rows;
 }
 // Decode-sized batches may split K finely (more parallel items, smaller resident activations);

@@ -224,6 +224,8 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
                                  const int16_t* absum, float* out, int* n_splits_out, int64_t split_stride,
                                  int max_splits, int max_active_experts = 0, int64_t total_rows = 0, float* out_whole = nullptr,
                                  const SharedGroup* shared = nullptr);
+// whether that kernel has the shared memory for a gate_up over rows of K with two position tiles
+bool expert_direct_takes_gate_up(int dtype, int K);
 // large-batch grouped GEMM on tcgen05 / TMEM: Q4_K in GGUF layout (repacked = false), Q6_K in the repacked
 // layout (repacked = true); `scratch` of expert_gemm_scratch_bytes(P, K) bytes
 size_t expert_gemm_scratch_bytes(int64_t P, int K, int parts = 1);  // parts = 2: the exact Q8_0 gate_up operand

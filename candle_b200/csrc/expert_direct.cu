@@ -713,6 +713,37 @@ cudaError_t launch_prepack(cudaStream_t st, int dtype, const void* raw, int64_t 
     return cudaGetLastError();
 }
 
+// Shared memory of a CTA for `ks_blocks` K-blocks of a group's rows: the rows' int8 values, scales and block sums, the warps' rings
+// of K-blocks (4 slots for Q4_K, 2368 B each, and Q8_0, 2176 B, 3 for Q6_K, 3360 B) and, with one position tile, their partial sums.
+struct DirectSmem {
+    int act_stride;
+    uint32_t off_act, off_scale, off_bs, off_ring, off_part, total;
+};
+static DirectSmem direct_smem(int dtype, int NT, int ks_blocks) {
+    const bool q80 = dtype == CANDLE_GGML_Q8_0;
+    const int blk = q80 ? DirQ80::BLK : 256, MT = 8 * NT, bs_per_block = q80 ? 0 : (dtype == CANDLE_GGML_Q4K ? 8 : 16);
+    DirectSmem m{};
+    auto take = [&](uint32_t bytes) {
+        m.total = (m.total + 127u) & ~127u;
+        const uint32_t o = m.total;
+        m.total += bytes;
+        return o;
+    };
+    m.act_stride = ks_blocks * blk + 16;
+    m.off_act = take((uint32_t)MT * m.act_stride);
+    m.off_scale = take((uint32_t)MT * ks_blocks * 4 * (q80 ? DirQ80::SC_PER_BLOCK : 1));
+    m.off_bs = take((uint32_t)2 * MT * ks_blocks * bs_per_block);
+    const int depth = dtype == CANDLE_GGML_Q6K ? 3 : 4;
+    m.off_ring = take((uint32_t)DIRECT_WARPS * depth * 2u * (q80 ? Q80_HTB_BYTES : (dtype == CANDLE_GGML_Q4K ? Q4K_HTB_BYTES : Q6K_HTB_BYTES)));
+    m.off_part = NT == 1 ? take((uint32_t)DIRECT_WARPS * 512u) : 0u;
+    return m;
+}
+constexpr uint32_t DIRECT_MAX_SMEM = 232448;  // what a CTA of sm_100a can have
+bool expert_direct_takes_gate_up(int dtype, int K) {
+    const int blk = dtype == CANDLE_GGML_Q8_0 ? DirQ80::BLK : 256;
+    return direct_smem(dtype, 2, (K + blk - 1) / blk).total <= DIRECT_MAX_SMEM - 1024;
+}
+
 // Plans and launches the prepacked-weight kernel; cudaErrorNotSupported when the shape is not taken.
 cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int dtype,
                                  int E, int K, int N, const uint32_t* offsets, const uint32_t* row_of,
@@ -747,7 +778,6 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
     if (shared && few_rows && max_rows_per_expert > 8 && shared->rows > 16) return cudaErrorNotSupported;
     const int NT = max_rows_per_expert <= 8 || few_rows ? 1 : 2;
     const int MT = 8 * NT;
-    const int bs_per_block = q80 ? 0 : (dtype == CANDLE_GGML_Q4K ? 8 : 16);
     DirectParams P{};
     P.wa = wa;
     P.wb = wb;
@@ -773,22 +803,14 @@ cudaError_t launch_expert_direct(cudaStream_t st, bool gate_up, const ExpertPtrs
             if (sh_splits > (gate_up ? 1 : std::min(8, shared->max_splits))) return cudaErrorNotSupported;
             ks_blocks = std::max(ks_blocks, (sh_kb + sh_splits - 1) / sh_splits);
         }
-        uint32_t off = 0;
-        auto take = [&](uint32_t bytes) {
-            off = (off + 127u) & ~127u;
-            const uint32_t o = off;
-            off += bytes;
-            return o;
-        };
-        P.act_stride = ks_blocks * blk + 16;
-        P.off_act = take((uint32_t)MT * P.act_stride);
-        P.off_scale = take((uint32_t)MT * ks_blocks * 4 * (q80 ? DirQ80::SC_PER_BLOCK : 1));
-        P.off_bs = take((uint32_t)2 * MT * ks_blocks * bs_per_block);
-        // per-warp rings of DEPTH K-blocks: 4 slots for Q4_K (2368 B each) and Q8_0 (2176 B), 3 for Q6_K (3360 B)
-        const int depth = dtype == CANDLE_GGML_Q6K ? 3 : 4;
-        const uint32_t slot_bytes = 2u * (q80 ? Q80_HTB_BYTES : (dtype == CANDLE_GGML_Q4K ? Q4K_HTB_BYTES : Q6K_HTB_BYTES));
-        P.off_ring = take((uint32_t)DIRECT_WARPS * depth * slot_bytes);
-        P.off_part = NT == 1 ? take((uint32_t)DIRECT_WARPS * 512u) : 0u;
+        const DirectSmem m = direct_smem(dtype, NT, ks_blocks);
+        P.act_stride = m.act_stride;
+        P.off_act = m.off_act;
+        P.off_scale = m.off_scale;
+        P.off_bs = m.off_bs;
+        P.off_ring = m.off_ring;
+        P.off_part = m.off_part;
+        const uint32_t off = m.total;
         if ((int)off > g_dir_max_smem - 1024) continue;
         P.splits = splits;
         int bs = 0;

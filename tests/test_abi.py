@@ -199,6 +199,15 @@ def test_line_of_q80_layers(lib, E, k, d, ff, fs, decode, gemm):
     assert decode <= _line(lib, E, k, d, ff, 8, 8, fs=fs) < gemm
 
 
+@pytest.mark.parametrize("E,k,d,ff,dt13,dt2,decode,gemm", [
+    (8, 2, 4096, 14336, 12, 14, 60, 64), (8, 2, 4096, 14336, 12, 12, 56, 64), (8, 2, 4096, 14336, 14, 14, 0, 49), (8, 2, 2048, 8192, 12, 14, 58, 64),
+    (8, 2, 2560, 6144, 12, 14, 60, 64), (8, 2, 2560, 6144, 14, 14, 56, 62), (8, 2, 1024, 3584, 12, 14, 54, 64), (8, 2, 1024, 3584, 12, 12, 0, 54),
+    (4, 2, 4096, 14336, 12, 14, 28, 34), (60, 8, 2048, 1536, 12, 14, 96, 97), (16, 4, 2048, 1024, 12, 14, 0, 50), (16, 8, 2048, 2048, 12, 14, 0, 28),
+])
+def test_line_of_k_quant_layers_over_copies(lib, E, k, d, ff, dt13, dt2, decode, gemm):
+    assert decode <= _line(lib, E, k, d, ff, dt13, dt2) < gemm
+
+
 def test_every_line_of_the_gemm_can_be_chosen(lib):
     """96 rows, the line of everything that does not go by the rows of an expert, is a fixed line like any other when it is
     set: a layer over copies then has no GEMM scratch at 90 rows, and has it again when the value found before is put back."""

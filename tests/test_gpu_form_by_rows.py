@@ -38,8 +38,10 @@ def _cfg(dt13, dt2, E, k, d=512, ff=1024, fs=0):
 
 
 @pytest.mark.parametrize("dt13,dt2,prepack,E,k,rows", [
-    (12, 14, True, 8, 2, (48, 49, 96, 97)),   # 12 rows of an expert
-    (14, 14, True, 8, 2, (48, 49)),
+    (12, 14, True, 8, 2, (48, 56, 57, 96, 97)),  # 14 rows of an expert
+    (12, 12, True, 8, 2, (52, 53)),           # 13
+    (14, 14, True, 8, 2, (48, 56, 57)),
+    (12, 14, True, 16, 4, (48, 49)),          # 12
     (12, 12, True, 3, 2, (18, 19, 96)),       # few experts: wide tiles, the old line
     (12, 12, False, 8, 2, (10, 11, 64)),      # 2.5 rows of an expert, GGUF blocks
     (12, 14, False, 8, 2, (11, 96)),          # the down product stays where it was
