@@ -66,9 +66,23 @@ inline int64_t gemm_expert_rows(const candle_moe_weights_t* w) {
     if (millions >= 350.0) return q6_13 && q6_2 ? 14 : 15;
     return w->n_experts > 8 ? 12 : (q6_2 ? 14 : 13);
 }
-// Without copies, streaming form / GEMM for Q4_K (Q6_K products stay where they are): d = ff = 4096: 8 91 / 100, 12 111 / 100, 16 112 / 101,
-// 96 228 / 107; d = 2048, ff = 8192: 8 110 / 98, 32 153 / 99; d = 1024, ff = 3584: 8 56 / 44, 64 102 / 50; Mixtral-shaped with a Q6_K down
-// product: 8 283 / 277, 32 412 / 342, 96 793 / 503.
+// Rows of a step above which a layer without copies takes the GEMM, for Q4_K products beside a Q4_K gate_up (Q6_K ones stay where they are).
+// Up to eight rows the streaming form has one position tile and is the faster for most layers; beyond, it pays for two, and the GEMM wins from 2.5 rows of an expert on, its
+// launches for the tensor maps of many experts included -- where its tiles fill the SMs and the weights outweigh its launches.
+// Streaming form / GEMM, us per layer.  8 experts, top-2 -- 1024 x 3584: 10 rows 64 / 53, 60 98 / 51; 4096 x 4096: 8 77 / 94, 10 104 / 101,
+// 60 163 / 103; 4096 x 14336: 10 293 / 239, 60 500 / 240, Q6_K down 320 / 302, 579 / 415; 512 x 1024: 16 33 / 34, 32 36 / 34; top-4, 4096 x
+// 4096: 6 83 / 100, 8 89 / 101, 10 110 / 100.  64 of 2048 x 1024, top-8: 21 rows 184 / 133; 128 of 2048 x 768, top-8: 42 rows 303 / 222; 32 of 512
+// x 512, top-4: 24 rows 54 / 57, 64 60 / 56.  Few experts -- 4 of 4096 x 4096, top-2: 8 rows 56 / 67, 12 72 / 66; 4 of 4096 x 14336: 8 136 /
+// 155, 10 174 / 153; 3 of 4096 x 4096, top-1: 9 59 / 63, 22 65 / 63; 2 of 2048 x 4096, top-1: 8 33 / 39, 12 39 / 39; 3 of 1024 x 1024: 42 rows 31 / 33.
+inline int64_t gemm_rows_gguf(const candle_moe_weights_t* w, int64_t rows) {
+    const int64_t E = w->n_experts;
+    const double millions = 3e-6 * E * w->d_model * w->d_ff;
+    int64_t halves = 5;  // of a row of an expert
+    if (millions < (E < 6 ? 18.0 : 8.0)) return rows;
+    if (E < 6 && millions < 500.0) halves = 12;
+    else if (millions < std::max(20.0, 0.8 * E)) halves = 16;
+    return std::min(rows, std::max<int64_t>(8, halves * E / (2 * w->top_k)));
+}
 // Only where an expert's rows are expected in a narrow tile, whose gate is as exact as that of the forms before.
 inline int64_t gemm_rows(const candle_moe_weights_t* w) {
     const int64_t rows = gemm_min_rows(), E = w->n_experts, k = w->top_k;
@@ -78,7 +92,7 @@ inline int64_t gemm_rows(const candle_moe_weights_t* w) {
     if (copies && q80_13 && q80_2) return gemm_rows_q80(w, rows);
     if (q80_13 || q80_2 || 5 * k * rows > 4 * 64 * E) return rows;
     if (copies) return std::min(rows, gemm_expert_rows(w) * E / k);
-    return w->dtype_w13 == CANDLE_GGML_Q4K ? std::min(rows, 5 * E / (2 * k)) : rows;
+    return w->dtype_w13 == CANDLE_GGML_Q4K ? gemm_rows_gguf(w, rows) : rows;
 }
 // Decode-sized batches may split K finely (more parallel items, smaller resident activations);
 // larger batches get four slots, enough for the streaming form's activation rows to fit.

@@ -208,6 +208,15 @@ def test_line_of_k_quant_layers_over_copies(lib, E, k, d, ff, dt13, dt2, decode,
     assert decode <= _line(lib, E, k, d, ff, dt13, dt2) < gemm
 
 
+@pytest.mark.parametrize("E,k,d,ff,decode,gemm", [
+    (8, 2, 1024, 3584, 8, 12), (8, 2, 4096, 4096, 8, 12), (8, 4, 4096, 4096, 8, 10), (16, 8, 4096, 4096, 8, 10), (128, 8, 2048, 768, 8, 60), (64, 8, 2048, 1024, 8, 40),
+    (4, 2, 4096, 4096, 8, 16), (4, 2, 4096, 14336, 8, 10), (3, 1, 4096, 4096, 14, 28), (2, 1, 2048, 4096, 8, 20), (3, 1, 1024, 1024, 42, 97), (8, 2, 512, 512, 48, 97),
+    (8, 2, 512, 1024, 20, 48), (32, 4, 512, 512, 32, 96),
+])
+def test_line_of_q4k_layers_without_copies(lib, E, k, d, ff, decode, gemm):
+    assert decode <= _line(lib, E, k, d, ff, 12, 12, copies=False) < gemm
+
+
 def test_every_line_of_the_gemm_can_be_chosen(lib):
     """96 rows, the line of everything that does not go by the rows of an expert, is a fixed line like any other when it is
     set: a layer over copies then has no GEMM scratch at 90 rows, and has it again when the value found before is put back."""

@@ -43,8 +43,10 @@ def _cfg(dt13, dt2, E, k, d=512, ff=1024, fs=0):
     (14, 14, True, 8, 2, (48, 56, 57)),
     (12, 14, True, 16, 4, (48, 49)),          # 12
     (12, 12, True, 3, 2, (18, 19, 96)),       # few experts: wide tiles, the old line
-    (12, 12, False, 8, 2, (10, 11, 64)),      # 2.5 rows of an expert, GGUF blocks
-    (12, 14, False, 8, 2, (11, 96)),          # the down product stays where it was
+    (12, 12, False, 8, 2, (10, 11, 32, 33, 64)),  # GGUF blocks, a small layer: 8 rows of an expert
+    (12, 12, False, 32, 8, (8, 10, 11, 40)),  # 2.5; four chunks of tensor maps
+    (12, 12, False, 4, 1, (9, 64)),           # few experts of a small layer: the old line
+    (12, 14, False, 8, 2, (11, 33, 96)),      # the down product stays where it was
     (14, 12, False, 8, 2, (11, 96)),
     (8, 8, True, 32, 4, (97, 176, 177)),      # 22 rows of an expert
     (8, 8, False, 32, 4, (97,)),
