@@ -442,11 +442,19 @@ int run_experts(cudaStream_t st, const candle_moe_weights_t* w, const ExpertPtrs
     bool gate_done = false, down_done = false;
     *eo_splits = 1;
     ExpertPtrs q1, q3, q2;
+    // Tables with a missing or misaligned entry: an error with k-quants at every batch that the decode kernels may take, whether this
+    // one takes them or not (Q4_K products on the GEMM read none)
+    const bool check_copies = large && !rows_exact && max_rows <= gemm_min_rows() && w->w1_prepacked && w->w3_prepacked && w->w2_prepacked;
+    if (check_copies && w->dtype_w13 != CANDLE_GGML_Q8_0 && w->dtype_w2 != CANDLE_GGML_Q8_0) {
+        CM_TRY(fill_ptrs(w->w1_prepacked, E, q1));
+        CM_TRY(fill_ptrs(w->w3_prepacked, E, q3));
+        CM_TRY(fill_ptrs(w->w2_prepacked, E, q2));
+    }
     if (use_prepacked) {
         int st_copies = fill_ptrs(w->w1_prepacked, E, q1);
         if (st_copies == CANDLE_MOE_OK) st_copies = fill_ptrs(w->w3_prepacked, E, q3);
         if (st_copies == CANDLE_MOE_OK) st_copies = fill_ptrs(w->w2_prepacked, E, q2);
-        // tables with a missing or misaligned entry: an error for k-quants, left alone with Q8_0 matrices (which need no copies here)
+        // (left alone with Q8_0 matrices, which need no copies here)
         if (st_copies != CANDLE_MOE_OK && w->dtype_w13 != CANDLE_GGML_Q8_0 && w->dtype_w2 != CANDLE_GGML_Q8_0) return st_copies;
         use_prepacked = st_copies == CANDLE_MOE_OK;
     }

@@ -160,3 +160,26 @@ def test_products_that_the_decode_kernels_refuse_go_to_the_gemm(orc, torch_cuda,
     tiles = _tuned(_lib.TUNE_GEMM_ENABLED, 0, lambda: blk.forward(x).clone())
     assert not torch_cuda.equal(y, tiles)
     assert H.rel_l2(y.cpu().numpy(), tiles.cpu().numpy()) <= H.REL_L2_TOL
+
+
+@pytest.mark.parametrize("bad,status", [(None, -1), (8, -5)])
+def test_bad_tables_of_copies_are_refused_on_either_side_of_the_line(orc, torch_cuda, bad, status):
+    """A missing or misaligned entry among the copies of a Q4_K layer: an error up to 96 rows, also where the GEMM, which reads the
+    GGUF blocks, takes the batch; beyond, the tables are not looked at."""
+    torch = torch_cuda
+    from candle_b200 import _lib
+    blk, _ = H.random_device_block(orc, torch, _cfg(12, 12, 8, 2), 5)
+    blk.prepack()
+    lib, table = _lib.load(), blk._cw.w3_prepacked
+    keep = table[7]
+    for T, expected in ((16, status), (64, status), (96, status), (97, 0)):
+        x = torch.randn((T, 512), device="cuda")
+        y, ws = torch.empty_like(x), torch.empty(blk.workspace_bytes(T) + 256, dtype=torch.uint8, device="cuda")
+        at = (ws.data_ptr() + 255) // 256 * 256
+        run = lambda: lib.candle_moe_forward(torch.cuda.current_stream().cuda_stream, C.byref(blk._cw), x.data_ptr(), T, y.data_ptr(), at,
+                                             ws.numel() - 256)
+        table[7] = None if bad is None else keep + bad
+        assert run() == expected, T
+        table[7] = keep
+        assert run() == 0, T
+    torch.cuda.synchronize()
