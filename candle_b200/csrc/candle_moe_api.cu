@@ -342,6 +342,7 @@ int candle_moe_permute(void* stream, const uint32_t* topk_ids, int64_t T, int32_
                        uint32_t* expert_counts, uint32_t* expert_offsets, uint32_t* perm_token, uint32_t* pair_pos) {
     if (!topk_ids || !expert_counts || !expert_offsets || !perm_token || !pair_pos) return CANDLE_MOE_E_NULL;
     if (T < 0 || k <= 0 || k > CANDLE_MOE_MAX_TOPK || E <= 0 || E > CANDLE_MOE_MAX_EXPERTS) return CANDLE_MOE_E_SHAPE;
+    if (T > (int64_t)UINT32_MAX / k) return CANDLE_MOE_E_SHAPE;  // the lists hold 32-bit positions, the kernel 32-bit indices
     return rc(launch_permute((cudaStream_t)stream, topk_ids, T, k, E, expert_counts, expert_offsets, perm_token,
                              pair_pos));
 }

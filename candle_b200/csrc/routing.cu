@@ -514,10 +514,13 @@ permute_kernel(const uint32_t* __restrict__ ids, int64_t n_pairs, int k, int E, 
     __shared__ uint32_t s_off[CANDLE_MOE_MAX_EXPERTS + 1];  // counts, then offsets
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = PERMUTE_THREADS / 32;
     const uint32_t n = (uint32_t)n_pairs, none = 0xffffffffu;  // (no expert has that id)
+    // rounds are counted: an index that ran to n would wrap behind the last round of nearly 2^32 pairs and never end (within that round
+    // the largest index is a multiple of 128 less one, 2^32 - 1 at most)
+    const uint32_t rounds = (uint32_t)((n_pairs + 127) / 128);
     for (int e = warp; e < E; e += n_warps) {
-        uint32_t c = 0;
+        uint32_t c = 0, i0 = lane;
 #pragma unroll 1
-        for (uint32_t i0 = lane; i0 - lane < n; i0 += 128) {
+        for (uint32_t round = 0; round < rounds; ++round, i0 += 128) {
             uint32_t id[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) id[j] = i0 + 32 * j < n ? ids[i0 + 32 * j] : none;
@@ -530,9 +533,9 @@ permute_kernel(const uint32_t* __restrict__ ids, int64_t n_pairs, int k, int E, 
     if (warp == 0) scan_counts(s_off, lane, E, counts, offsets);
     __syncthreads();
     for (int e = warp; e < E; e += n_warps) {
-        uint32_t base = s_off[e];
+        uint32_t base = s_off[e], i0 = lane;
 #pragma unroll 1
-        for (uint32_t i0 = lane; i0 - lane < n; i0 += 128) {
+        for (uint32_t round = 0; round < rounds; ++round, i0 += 128) {
             uint32_t id[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) id[j] = i0 + 32 * j < n ? ids[i0 + 32 * j] : none;

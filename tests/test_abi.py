@@ -217,6 +217,28 @@ def test_line_of_q4k_layers_without_copies(lib, E, k, d, ff, decode, gemm):
     assert decode <= _line(lib, E, k, d, ff, 12, 12, copies=False) < gemm
 
 
+@pytest.mark.parametrize("T,k", [(2 ** 32, 1), (2 ** 29, 8), (2 ** 61, 8)])
+def test_dispatch_of_more_selections_than_its_lists_can_number_is_refused(lib, T, k):
+    assert lib.load().candle_moe_permute(None, 4096, T, k, 8, 4096, 4096, 4096, 4096) == -2
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 2 ** 31, 2 ** 32 - 129, 2 ** 32 - 128, 2 ** 32 - 127, 2 ** 32 - 1])
+def test_rounds_of_the_small_dispatch_end_at_every_length(n):
+    """permute_kernel's loop in its own 32-bit arithmetic: the condition as the source has it, at the first and the last rounds."""
+    src = open(os.path.join(ROOT, "candle_b200", "csrc", "routing.cu")).read()
+    kernel = src[src.index("permute_kernel(const"):src.index("permute_count_kernel(")]
+    loops = re.findall(r"for \(([^;]*; [^;]*; [^)]*i0 \+= 128)\)", kernel)
+    assert len(loops) == 2 and len(set(loops)) == 1
+    m = 2 ** 32
+    rounds = (n + 127) // 128
+    last = (rounds - 1) * 128 + 31  # i0 of the last lane there
+    if "round < rounds" in loops[0]:
+        assert "rounds = (uint32_t)((n_pairs + 127) / 128)" in kernel
+    else:  # an index against n: behind the last round it must not have wrapped
+        assert "i0 - lane < n" in loops[0] and (last + 128 - 31) % m >= n
+    assert last + 96 < m  # no index of the last round wraps
+
+
 def test_every_line_of_the_gemm_can_be_chosen(lib):
     """96 rows, the line of everything that does not go by the rows of an expert, is a fixed line like any other when it is
     set: a layer over copies then has no GEMM scratch at 90 rows, and has it again when the value found before is put back."""
