@@ -19,8 +19,8 @@ inline bool gemm_rows_auto() { return tuning_get(TUNE_GEMM_MIN_ROWS) == CANDLE_M
 inline int64_t gemm_min_rows() { return gemm_rows_auto() ? 96 : tuning_get(TUNE_GEMM_MIN_ROWS); }
 // When the caller knows the ACTUAL largest row count of an expert (or, in the slot form of expert parallelism, a
 // bound five quarters of the expected one, so that the tile width leaves a margin), the GEMM takes over above 32 rows.
-// Measured on one GPU with the experts of one rank of the Mixtral-shaped layer (decode kernels / GEMM, microseconds
-// per step): one expert, 32 rows 92 / 98, 48 rows 122 / 98, 64 rows 134 / 103, 96 rows 190 / 129, 128 rows 229 / 129;
+// Measured on one GPU with the experts of one rank of the Mixtral-shaped layer and a former GEMM, with which the line was not measured
+// again (decode kernels / GEMM, microseconds per step): one expert, 32 rows 92 / 98, 48 rows 122 / 98, 64 rows 134 / 103, 96 rows 190 / 129, 128 rows 229 / 129;
 // two experts, 32 rows each 163 / 159, 40 rows 193 / 165, 64 rows 246 / 200; four experts, 32 rows 272 / 262, 40 rows
 // 323 / 263.  (An earlier measurement of 248 us for two experts of ~33 rows had position tiles of 32, so that every
 // expert with a row more than expected took a second, almost empty tile.)  A single-device forward only knows the
@@ -1032,8 +1032,10 @@ struct QmmWorkspace {
     size_t total;
 };
 // One group holds every row, so the row count is exact.  The tensor-core GEMM takes the product above 48 rows, and
-// from 17 rows on when the matrix has enough 128-row tiles to fill the SMs by itself (measured at 32 rows:
-// [32000, 4096] Q6_K 76 us through the GEMM against 108 us through the streaming form, [4096, 4096] Q4_K 25 against 23).
+// from 17 rows on when the matrix has enough 128-row tiles to fill the SMs by itself.  Both lines are those of a former GEMM ([4096, 4096]
+// Q4_K at 32 rows 25 us against 23 through the streaming form); the present one is ahead below them too.  Streaming form / GEMM on the
+// device, us, 17 and 48 rows: [1024, 4096] Q4_K 13 / 11, 15 / 13; [4096, 4096] 20 / 15, 26 / 15; [6144, 4096] 24 / 16, 33 / 17; [12800, 4096] 36 /
+// 20, 51 / 23; [32000, 4096] Q6_K 103 / 45, 160 / 50.
 inline bool qmm_takes_gemm(int dtype, int64_t rows, int n) {
     return dtype != CANDLE_GGML_Q8_0 && (rows > QMM_GEMM_MIN_ROWS || (rows > 16 && n >= 12800));
 }

@@ -240,7 +240,7 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
                                bool operand_ready = false, bool exact_gate = false, int max_run = 0);
 // whether launch_expert_gemm takes the product (given scratch).  Its x_f32: the f32 rows in grouped order instead of their
 // quantization (aq, ascale, absum are then not read); single_group: as in launch_quantize_act, with x_f32 only; exact_gate: the
-// gate of a Q4_K or Q6_K gate_up by silu_f; max_run: K is split (within max_splits) until no sum goes over more blocks
+// gate of a Q6_K gate_up by silu_f, of a Q4_K one in tiles of up to 64 positions (such batches alone ask for it); max_run: K is split (within max_splits) until no sum goes over more blocks
 bool expert_gemm_takes(bool gate_up, int dtype, bool repacked, int K, int N, int64_t P);
 // Q8_0 grouped products for many rows per expert (expert_q80.cu); cudaErrorNotSupported for other shapes
 cudaError_t launch_expert_q80(cudaStream_t st, bool gate_up, const ExpertPtrs& wa, const ExpertPtrs& wb, int E, int K, int N,

@@ -7,8 +7,9 @@
 // Q8K rows, and the weight operand holds (sub-block scale) x (quant).  After every 256-element block
 // the accumulator is drained and scaled by d_w(row, block) * d8(position, block) on the CUDA cores.
 //   Q4_K: fp16 operand sc_j * q (at most 63 * 15, exact), `tcgen05.mma kind::f16`, fp32 accumulation in tensor memory
-//         -- exact while a block's sum stays below 2^24, which it does by a wide margin for real data; the min
-//         term joins the same accumulator as three tf32 steps per block against dmin / d (see prep_gemm_b_kernel).
+//         -- exact while a block's sum stays below 2^24, which it does by a wide margin for real data.  The min term: beside
+//         up to 64 positions exact integers in an accumulator of its own, beside 128 three tf32 steps per block against
+//         dmin / d into the main one (see prep_gemm_b_kernel).
 //   Q6_K: sc_j * (q - 32) reaches 4096 and is not always an fp16 integer: two int8 planes, `kind::i8`, int32
 //         accumulation (exact).  Reads the repacked layout of the decode kernels (16-byte aligned pieces; the
 //         210-byte GGUF blocks are only 2-byte aligned).
@@ -30,7 +31,8 @@
 // the operand copies taken out: the MMA warp walked its few dozen instructions per pair of slabs at several clocks each beside
 // busy warps, behind an instruction cache that 60-90 KB of code -- every wait written out with its give-up path at every place
 // -- did not fit.  Hence constant ring addresses, waits of a few instructions (mbar_wait_tight), no tile search in the unpack
-// warps, one barrier per pair for both operands, masks fused with the fp16 magic number (field).  Layers, before -> after: Mixtral-shaped,
+// warps, one barrier per pair for both operands, masks fused with the fp16 magic number (field).  Counters of the result, gate_up / down:
+// issue slots busy 64 / 66 % of the active cycles at 100 rows, 66 / 72 % at 2048; tensor pipe 23 / 13 and 67 / 40 %.  Layers, before -> after: Mixtral-shaped,
 // 100 rows 388 -> 315 us, 2048 rows 2471 -> 2079; 8 small experts from GGUF blocks, 257 rows 79.4 -> 72.3; 60 Q8_0 experts,
 // 4096 rows 1776 -> 1710; [32000, 4096] Q6_K at 32 rows 49.4 -> 44.4, [4096, 4096] Q4_K at 777 rows 53.8 -> 48.7.
 // Every mbarrier wait is bounded (see stream_common.cuh); nothing here uses cluster multicast.
@@ -471,9 +473,7 @@ struct GemmQ4K {
             tmem_st32(ta + 32 * s, o);
         }
     }
-    // weight side of the min term (see prep_gemm_b_kernel): -rho_j = -dmin m_j / d split into tf32 terms [r1 (8) | r2 (8)].
-    // 2^23 + m as float bits is 0x4B000000 | m.
-    // one fp16 step: the eight mins, for the tiles that accumulate them on their own
+    // weight side of the min term (see prep_gemm_b_kernel): the eight mins, one fp16 step, for the tiles that accumulate them on their own
     __device__ static __forceinline__ void min_operand16(const Ctx& c, uint32_t (&r)[4]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -484,6 +484,7 @@ struct GemmQ4K {
     }
     __device__ static __forceinline__ float d_of(const Ctx& c) { return half_bits_to_float((uint16_t)c.dd); }
     __device__ static __forceinline__ float neg_dmin_of(const Ctx& c) { return -half_bits_to_float((uint16_t)(c.dd >> 16)); }
+    // ... and for the others -rho_j = -dmin m_j / d split into tf32 terms [r1 (8) | r2 (8)].  2^23 + m as float bits is 0x4B000000 | m.
     __device__ static __forceinline__ void min_operand(const Ctx& c, uint32_t (&r)[16]) {
         const float ratio = -__fdividef(half_bits_to_float((uint16_t)(c.dd >> 16)), scale_of(c));
 #pragma unroll
@@ -681,7 +682,7 @@ struct GemmCfg {
     static constexpr int REGS_LAUNCH = WARPS == 20 ? 96 : 128;
     static constexpr bool WIDE_I8 = F::I8 && TN == 128;
     static constexpr int REGS_EPI = TN == 32 ? 160 : (WIDE_I8 ? 152 : 136);
-    static constexpr int REGS_DQ = TN == 32 ? 128 : (WIDE_I8 ? 72 : 72), REGS_MISC = TN == 32 ? 96 : (WIDE_I8 ? 32 : 64);
+    static constexpr int REGS_DQ = TN == 32 ? 128 : 72, REGS_MISC = TN == 32 ? 96 : (WIDE_I8 ? 32 : 64);
     static_assert(EPI_WARPS / 4 * REGS_EPI + GROUPS * REGS_DQ + REGS_MISC <= WARPS / 4 * REGS_LAUNCH, "more registers than the launch has");
     static_assert(THREADS * REGS_LAUNCH <= 65536, "");
     // pairs of weight slabs (half blocks) in flight, each with its activation stage: two blocks, one with two-part operands
@@ -1562,10 +1563,9 @@ cudaError_t launch_expert_gemm(cudaStream_t st, bool gate_up, const ExpertPtrs& 
     e = stream_status_ptr(&G.status);
     if (e != cudaSuccess) return e;
     if (dtype == CANDLE_GGML_Q4K) {
-        if (gate_up && exact_gate) {
+        if (gate_up && exact_gate && tn <= 64) {
             if (tn == 32) return launch_gemm_kernel<GemmQ4KExact, true, 32>(st, G, map_b, map_bs);
-            if (tn == 64) return launch_gemm_kernel<GemmQ4KExact, true, 64>(st, G, map_b, map_bs);
-            return launch_gemm_kernel<GemmQ4KExact, true, 128>(st, G, map_b, map_bs);
+            return launch_gemm_kernel<GemmQ4KExact, true, 64>(st, G, map_b, map_bs);
         }
         if (tn == 32)
             return gate_up ? launch_gemm_kernel<GemmQ4K, true, 32>(st, G, map_b, map_bs) : launch_gemm_kernel<GemmQ4K, false, 32>(st, G, map_b, map_bs);

@@ -55,7 +55,7 @@ bool tuning_set(int key, int64_t value) {
 // expert, from k on -1); writes the token's ids and weights.  A round is two warp-wide integer reductions and the loop is
 // rolled: eight rounds of five exchanges of three values each, written out, were 16 KB of code at the end of every router kernel,
 // fetched by every launch of it (Mixtral-shaped layer at one row: 10.0 -> 8.3 us, layer 75.3 -> 73.0; 60 experts, 16 rows: 12.7 -> 11.5,
-// 4096 rows: layer 1364 -> 1326).
+// 4096 rows: layer 1364 -> 1326 in short runs).
 __device__ __forceinline__ int softmax_topk_warp(const float* s_logits, int lane, int E, int k, int renorm,
                                                  uint32_t* __restrict__ ids_row, float* __restrict__ w_row) {
     // softmax over E (candle-nn/src/ops.rs:326-339): exp(v - max) / sum, true division
