@@ -682,7 +682,10 @@ struct GemmCfg {
     static constexpr int REGS_LAUNCH = WARPS == 20 ? 96 : 128;
     static constexpr bool WIDE_I8 = F::I8 && TN == 128;
     static constexpr int REGS_EPI = TN == 32 ? 160 : (WIDE_I8 ? 152 : 136);
-    static constexpr int REGS_DQ = TN == 32 ? 128 : 72, REGS_MISC = TN == 32 ? 96 : (WIDE_I8 ? 32 : 64);
+    // (64-wide tiles of Q4_K: with 72 for the unpack warps they spilled 32 bytes; Mixtral-shaped layer, 200 rows 366 -> 359 us.  128-wide
+    // ones spill 8, and gain nothing that way)
+    static constexpr bool WIDE_UNPACK = F::HAS_MIN && TN == 64;
+    static constexpr int REGS_DQ = TN == 32 ? 128 : (WIDE_UNPACK ? 80 : 72), REGS_MISC = TN == 32 ? 96 : (WIDE_I8 ? 32 : (WIDE_UNPACK ? 48 : 64));
     static_assert(EPI_WARPS / 4 * REGS_EPI + GROUPS * REGS_DQ + REGS_MISC <= WARPS / 4 * REGS_LAUNCH, "more registers than the launch has");
     static_assert(THREADS * REGS_LAUNCH <= 65536, "");
     // pairs of weight slabs (half blocks) in flight, each with its activation stage: two blocks, one with two-part operands
